@@ -100,8 +100,8 @@ int sma_ctx_create(int device, sma_ctx **out) {
     DeviceGuard g(device);
     auto *ctx = new sma_ctx();
     ctx->device = device;
-    const char *at = std::getenv("SMA_AUTOTUNE");
-    ctx->autotune = !(at && std::string(at) == "0");
+    const char *at = std::getenv("SMA_AUTOTUNE"), *av = std::getenv("SMA_AUTOTUNE_VERBOSE");
+    ctx->tune = av && std::string(av) == "1" && !(at && std::string(at) == "0");
     const char *fg = std::getenv("SMA_FILTER_GRAPHS");
     ctx->filter_graphs = !(fg && std::string(fg) == "0");
     const char *pe = std::getenv("SMA_PERSISTENT");
@@ -453,10 +453,6 @@ int sma_apply_poly_block_percol_dev(sma_op *op, const double *coeffs, int64_t K,
       require(std::isfinite(coeffs[i]), SMA_ERR_ARG, "non-finite coefficient");
     DeviceGuard g(op->ctx->device);
     cudaStream_t st = op->ctx->stream;
-    std::vector<int> idn(b);
-    for (int64_t j = 0; j < b; ++j) idn[j] = (int)j;
-    DevBuf<int> colseg(b, st);
-    SMA_CUDA(cudaMemcpyAsync(colseg.p, idn.data(), b * sizeof(int), cudaMemcpyHostToDevice, st));
     auto run = [&](auto zero) {
       using T = decltype(zero);
       std::vector<T> ch((K + 1) * b);
@@ -464,8 +460,8 @@ int sma_apply_poly_block_percol_dev(sma_op *op, const double *coeffs, int64_t K,
       DevBuf<T> coef(ch.size(), st), B1(n * b, st), B2(n * b, st), TMP(n * b, st), AX;
       if (op->kind != OP_CSR) AX.alloc(n * b, st);
       SMA_CUDA(cudaMemcpyAsync(coef.p, ch.data(), ch.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-      percol_filter<T>(op, st, coef.p, K, smin, smax, (const T *)Q_dev, (T *)Y_dev, b, colseg.p,
-                       B1.p, B2.p, TMP.p, AX.p);
+      percol_filter<T>(op, st, coef.p, K, smin, smax, (const T *)Q_dev, (T *)Y_dev, b, B1.p, B2.p,
+                       TMP.p, AX.p);
       SMA_CUDA(cudaStreamSynchronize(st));
     };
     if (precision == SMA_PREC_FP64) {

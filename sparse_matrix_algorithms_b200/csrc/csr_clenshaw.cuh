@@ -1,33 +1,39 @@
-// The fused CSR Clenshaw step and its online autotuner (included by csr_clenshaw_f64.cu and
-// csr_clenshaw_f32.cu, one translation unit per element type).
+// The fused CSR Clenshaw step (included by csr_clenshaw_f64.cu and csr_clenshaw_f32.cu, one
+// translation unit per element type).
 //
 //   out[i, :] = ck*Q[i, :] + alpha * sum_j A[i,j] B1[j, :] + beta*B1[i, :] - B2[i, :]
 //
-// One CTA of 256 threads owns 256/G consecutive rows; a group of G threads owns one row and
-// each thread covers V consecutive columns of every G*V-wide column pass (V*sizeof(T) is
-// 8..32 bytes: one or two 16-byte loads per neighbour row).  Gathers are issued U at a
-// time so that U neighbour rows are in flight per thread, and the epilogue operands (the
-// row of Q, B1, B2) are requested before the gathers.  Two families differ in how a
-// thread obtains its row's (column, value) pairs:
-//   DIRECT  every thread reads them itself; the G lanes of a group read the same
-//           addresses, which the L1 cache serves as one broadcast;
-//   STAGED  the CTA first copies the pairs of all its rows (one contiguous CSR range)
-//           into shared memory with coalesced loads, then reads them from there.
-// Both families are launched as programmatic dependents of the previous step (when the
-// context allows it): a CTA first lets the next step's grid be scheduled, reads what no
-// step writes (its CSR rows and the row of Q), and only then waits for the previous grid
-// to complete (griddepcontrol.wait) before it reads B1 or B2 or writes anything -- so the
-// next step's CTAs fill the SMs that this step's last wave leaves idle.  Launched without
-// the attribute, both instructions are no-ops.
+// A thread owns V consecutive columns of one row (V*sizeof(T) = 32 bytes where the widths,
+// strides and addresses allow it: one 256-bit access per neighbour row); a CTA of 128 threads
+// owns the whole rows that fit.  Blocks wider than 64 vectors are cut into panels, the panel
+// being the slow grid dimension, so that the neighbour rows of a panel are still in L2 when
+// their last reader comes.
+//
+// What bounds it.  The n x b streams (Q, B1, B2, out) come from HBM when they exceed the L2,
+// the neighbour rows from L2 (15 TB/s measured), and between a row's pointer, its column
+// indices and its gathers lie two dependent latencies that only resident warps can hide.  So
+// registers go to occupancy, not to operands in flight: at most U = 4 neighbour rows are held
+// at a time, the epilogue's rows are prefetched into L2 at the start and loaded only after the
+// gathers, and 40 registers keep 12 CTAs on an SM.  Measured on the 3D Anderson lattice
+// (n = 262144, 7 entries a row), step after step on one B200:
+//   FP32 b = 64   66 -> 43 us (6.6 TB/s of algorithmic bytes),  b = 768   640 -> 522 us,
+//   FP64 b = 64  121 -> 85 us (6.6 TB/s).
+// Against the kernel before it: 16-byte halves at a 32-byte stride doubled the L1 wavefronts
+// (73 % of the LSU data pipe), and 63 registers left 45 % of the warps (DRAM 4.0 TB/s).
+//
+// Steps alternate the direction in which they walk the rows (rev): what the last CTAs of a
+// step touched is what the first CTAs of the next read from L2 (FP64 b = 64: 97 -> 93 us).
+//
+// Steps are launched as programmatic dependents of the previous step (when the context allows
+// it): a CTA reads what no step writes -- its row pointers -- and starts the prefetch of its
+// row of Q, then waits for the previous grid before it touches B1 or B2 or writes anything.
+//
 // Every configuration accumulates with FMA in ascending column order -- the order of the
-// reference's CSC product on a symmetric matrix -- so all configurations write
-// bit-identical results, and the autotuner may run real recurrence steps with different
-// configurations while it measures them.
+// reference's CSC product on a symmetric matrix -- so all write bit-identical results.
 #pragma once
 
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
 
 #include "sma_internal.h"
 #include "vec.cuh"
@@ -35,770 +41,329 @@
 namespace sma {
 namespace csr {
 
-constexpr int kThreads = 256;
-constexpr int kStage = 1024;  // CSR entries a STAGED CTA keeps in shared memory
+constexpr int kThreads = 128;
+constexpr int kPanel = 64;  // vectors of a row in one panel
 
-template <typename T, int V, bool HQ, bool HS, bool HB>
-__device__ __forceinline__ void epilogue(T *__restrict__ out, const T (&acc)[V], const T (&q)[V],
-                                         const T (&s)[V], const T (&t)[V], const T (&ck)[V],
-                                         T alpha, T beta) {
-  T r[V];
-#pragma unroll
-  for (int v = 0; v < V; ++v)
-    r[v] = clenshaw_combine<HQ, HS, HB>(acc[v], q[v], s[v], t[v], ck[v], alpha, beta);
-  stv<T, V>(out, r);
+// What one launch needs; leading dimensions in bytes.
+template <typename T>
+struct Step {
+  const int *rowptr, *colind;
+  const T *val;
+  const T *Q, *B1, *B2;
+  T *out;
+  const T *cseg;      // per-column coefficients (PC), else null
+  const int *colseg;  // PC: the coefficient of column c is cseg[colseg[c]], or cseg[c] when null
+  uint64_t ldq, ldb, ldo;
+  T ck, alpha, beta;
+  uint32_t n, b;      // rows, columns
+  uint32_t lanes;     // vectors of a row in one panel
+  uint32_t rows;      // rows of a CTA (rows * lanes <= kThreads)
+  uint32_t divlanes;  // ceil(2^16 / lanes): tid / lanes = tid * divlanes >> 16 for tid < 128
+  int rev;
+};
+
+template <typename T>
+__device__ __forceinline__ const T *at(const T *p, uint64_t bytes) {
+  return reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + bytes);
 }
 
-// The Q coefficient of each of a thread's V columns c0 .. c0+V-1: the step's scalar ck, or
-// (PC) the coefficient of the column's segment, cseg[colseg[c]].
-template <typename T, int V, bool PC>
-__device__ __forceinline__ void coeffs_of(T (&ckv)[V], T ck, const T *__restrict__ cseg,
-                                          const int *__restrict__ colseg, int c0) {
-#pragma unroll
-  for (int v = 0; v < V; ++v) {
-    if constexpr (PC) ckv[v] = __ldg(cseg + __ldg(colseg + c0 + v));
-    else ckv[v] = ck;
-  }
+// Byte offset of a gathered row: 32 x 32 -> 64 bit product unless the leading dimension itself
+// needs 64 bits (W).
+template <bool W>
+__device__ __forceinline__ uint64_t row_bytes(uint32_t row, uint64_t ld) {
+  if constexpr (W) return (uint64_t)row * ld;
+  return (uint64_t)row * (uint32_t)ld;
 }
 
-// R consecutive entries from j: all R gathers are issued before the first FMA, so R
-// neighbour rows are in flight at once; FMAs in ascending entry order.
-template <typename T, int V, int R>
-__device__ __forceinline__ void chunk(const int *__restrict__ cols, const T *__restrict__ vals,
-                                      int off, int j, const T *__restrict__ B1c, int64_t ldb,
-                                      T (&acc)[V]) {
+// R consecutive entries from j: all R gathers are issued before the first FMA; FMAs in
+// ascending entry order.
+template <typename T, int V, int R, bool W>
+__device__ __forceinline__ void chunk(const Step<T> &a, int j, const T *B1c, T (&acc)[V]) {
   int c[R];
-  T x[R][V], a[R];
+  T x[R][V], v[R];
 #pragma unroll
-  for (int u = 0; u < R; ++u) c[u] = cols[j + u - off];
+  for (int u = 0; u < R; ++u) c[u] = __ldg(a.colind + j + u);
 #pragma unroll
-  for (int u = 0; u < R; ++u) ldv<T, V>(B1c + (int64_t)c[u] * ldb, x[u]);
+  for (int u = 0; u < R; ++u) ldv<T, V>(at(B1c, row_bytes<W>((uint32_t)c[u], a.ldb)), x[u]);
 #pragma unroll
-  for (int u = 0; u < R; ++u) a[u] = vals[j + u - off];
+  for (int u = 0; u < R; ++u) v[u] = __ldg(a.val + j + u);
 #pragma unroll
   for (int u = 0; u < R; ++u)
 #pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = fma(a[u], x[u][v], acc[v]);
+    for (int i = 0; i < V; ++i) acc[i] = fma(v[u], x[u][i], acc[i]);
 }
 
-// acc += sum over the row's entries j in [start, end) of vals[j-off] * B1c[cols[j-off] * ldb]:
-// chunks of U, then the r < U remaining entries as ONE chunk of exactly r (a switch over
-// r), so that a row shorter than U -- the 7-entry rows of the Anderson lattice under
-// U = 8 -- still has all its gathers in flight together.
-template <typename T, int V, int U>
-__device__ __forceinline__ void row_product(const int *__restrict__ cols, const T *__restrict__ vals,
-                                            int off, int start, int end, const T *__restrict__ B1c,
-                                            int64_t ldb, T (&acc)[V]) {
-  int j = start;
-  for (; j + U <= end; j += U) chunk<T, V, U>(cols, vals, off, j, B1c, ldb, acc);
+// acc += the row's entries [j, end): chunks of U, then the r < U remaining entries as ONE chunk
+// of exactly r (a switch over r).
+template <typename T, int V, int U, bool W>
+__device__ __forceinline__ void row_product(const Step<T> &a, int j, int end, const T *B1c,
+                                            T (&acc)[V]) {
+  for (; j + U <= end; j += U) chunk<T, V, U, W>(a, j, B1c, acc);
   switch (end - j) {
-    case 7: if constexpr (U > 7) chunk<T, V, 7>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 6: if constexpr (U > 6) chunk<T, V, 6>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 5: if constexpr (U > 5) chunk<T, V, 5>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 4: if constexpr (U > 4) chunk<T, V, 4>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 3: chunk<T, V, 3>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 2: chunk<T, V, 2>(cols, vals, off, j, B1c, ldb, acc); break;
-    case 1: chunk<T, V, 1>(cols, vals, off, j, B1c, ldb, acc); break;
+    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(a, j, B1c, acc); break;
+    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(a, j, B1c, acc); break;
+    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(a, j, B1c, acc); break;
+    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(a, j, B1c, acc); break;
+    case 3: chunk<T, V, 3, W>(a, j, B1c, acc); break;
+    case 2: chunk<T, V, 2, W>(a, j, B1c, acc); break;
+    case 1: chunk<T, V, 1, W>(a, j, B1c, acc); break;
     default: break;
   }
 }
 
-// Programmatic dependent launch: let the next grid in the stream be scheduled; wait until
-// the grids this one depends on have completed and their writes are visible.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The Q coefficients of the thread's V columns.
+template <typename T, int V, bool PC>
+__device__ __forceinline__ void coefficients(const Step<T> &a, uint32_t c0, T (&ck)[V]) {
+  if constexpr (!PC) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) ck[i] = a.ck;
+  } else if (a.colseg == nullptr) {  // one polynomial per column: its coefficients side by side
+    ldv<T, V>(a.cseg + c0, ck);
+  } else {  // segments are runs of columns: equal ends, one coefficient
+    const int s0 = __ldg(a.colseg + c0), s1 = __ldg(a.colseg + c0 + V - 1);
+    ck[0] = __ldg(a.cseg + s0);
+#pragma unroll
+    for (int i = 1; i < V; ++i)
+      ck[i] = s0 == s1 ? ck[0] : __ldg(a.cseg + __ldg(a.colseg + c0 + i));
+  }
+}
 
-template <typename T, int V, int G, int U, bool HQ, bool HS, bool HB, bool PC>
-__global__ void __launch_bounds__(kThreads)
-direct_kernel(const int *__restrict__ rowptr, const int *__restrict__ colind,
-              const T *__restrict__ val, int64_t n, int b, const T *__restrict__ Q, int64_t ldq,
-              const T *__restrict__ B1, const T *__restrict__ B2, int64_t ldb,
-              T *__restrict__ out, int64_t ldo, T ck, T alpha, T beta,
-              const T *__restrict__ cseg, const int *__restrict__ colseg) {
-  constexpr int kRows = kThreads / G;
-  pdl_trigger();
-  const int64_t row = (int64_t)blockIdx.x * kRows + threadIdx.x / G;
-  const bool live = row < n;
-  const int lane = threadIdx.x % G;
+// HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W>
+__global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
+  const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+  const uint32_t r = threadIdx.x * a.divlanes >> 16;
+  const uint32_t row = bx * a.rows + r;
+  const uint32_t c0 = (by * a.lanes + threadIdx.x - r * a.lanes) * V;
+  const bool in = r < a.rows && row < a.n && c0 < a.b;
   int start = 0, end = 0;
-  T q[V], s[V], t[V];
-  if (live) {  // what no step writes: the CSR row and the first pass's row of Q
-    start = __ldg(rowptr + row);
-    end = __ldg(rowptr + row + 1);
-    if constexpr (HQ) if (lane * V < b) ldv<T, V>(Q + row * ldq + lane * V, q);
+  if (in) {
+    start = __ldg(a.rowptr + row);
+    end = __ldg(a.rowptr + row + 1);
+    if constexpr (HQ) prefetch_l2(at(a.Q + c0, row * a.ldq));
   }
-  pdl_wait();
-  if (!live) return;
-  for (int c0 = lane * V; c0 < b; c0 += G * V) {
-    T acc[V];
+  pdl_wait_then_trigger();
+  if (!in) return;
+  const uint64_t own = row * a.ldb;
+  if constexpr (HB) prefetch_l2(at(a.B2 + c0, own));
+  T acc[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = T(0);
-    if constexpr (HQ) if (c0 != lane * V) ldv<T, V>(Q + row * ldq + c0, q);
-    if constexpr (HS) ldv<T, V>(B1 + row * ldb + c0, s);
-    if constexpr (HB) ldv<T, V>(B2 + row * ldb + c0, t);
-    row_product<T, V, U>(colind, val, 0, start, end, B1 + c0, ldb, acc);
-    T ckv[V];
-    coeffs_of<T, V, PC>(ckv, ck, cseg, colseg, c0);
-    epilogue<T, V, HQ, HS, HB>(out + row * ldo + c0, acc, q, s, t, ckv, alpha, beta);
-  }
+  for (int i = 0; i < V; ++i) acc[i] = T(0);
+  row_product<T, V, U, W>(a, start, end, a.B1 + c0, acc);
+  T q[V], s[V], t[V], ck[V], o[V];
+  if constexpr (HQ) ldv<T, V, false>(at(a.Q + c0, row * a.ldq), q);
+  if constexpr (HB) ldv<T, V, false>(at(a.B2 + c0, own), t);
+  if constexpr (HS) ldv<T, V>(at(a.B1 + c0, own), s);
+  if constexpr (HQ) coefficients<T, V, PC>(a, c0, ck);
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    o[i] = clenshaw_combine<HQ, HS, HB>(acc[i], q[i], s[i], t[i], ck[i], a.alpha, a.beta);
+  stv<T, V>(const_cast<T *>(at(a.out + c0, row * a.ldo)), o);
 }
 
-template <typename T, int V, int G, int U, bool HQ, bool HS, bool HB, bool PC>
-__global__ void __launch_bounds__(kThreads)
-staged_kernel(const int *__restrict__ rowptr, const int *__restrict__ colind,
-              const T *__restrict__ val, int64_t n, int b, const T *__restrict__ Q, int64_t ldq,
-              const T *__restrict__ B1, const T *__restrict__ B2, int64_t ldb,
-              T *__restrict__ out, int64_t ldo, T ck, T alpha, T beta,
-              const T *__restrict__ cseg, const int *__restrict__ colseg) {
-  constexpr int kRows = kThreads / G;
-  __shared__ int s_col[kStage];
-  __shared__ T s_val[kStage];
-  pdl_trigger();
-  const int64_t row0 = (int64_t)blockIdx.x * kRows;
-  const int64_t row = row0 + threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  const bool live = row < n;
-  T q[V], s[V], t[V];
-  if constexpr (HQ) if (live && lane * V < b) ldv<T, V>(Q + row * ldq + lane * V, q);
-  const int64_t rlast = min(n, row0 + kRows);
-  const int base = __ldg(rowptr + row0);
-  const int top = __ldg(rowptr + rlast);
-  const bool staged = top - base <= kStage;
-  if (staged) {
-    for (int i = threadIdx.x; i < top - base; i += kThreads) {
-      s_col[i] = __ldg(colind + base + i);
-      s_val[i] = __ldg(val + base + i);
-    }
-  }
-  __syncthreads();
-  pdl_wait();  // B1 and B2 come from the previous steps
-  if (!live) return;  // no barrier follows
-  const int start = __ldg(rowptr + row);
-  const int end = __ldg(rowptr + row + 1);
-  for (int c0 = lane * V; c0 < b; c0 += G * V) {
-    T acc[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = T(0);
-    if constexpr (HQ) if (c0 != lane * V) ldv<T, V>(Q + row * ldq + c0, q);
-    if constexpr (HS) ldv<T, V>(B1 + row * ldb + c0, s);
-    if constexpr (HB) ldv<T, V>(B2 + row * ldb + c0, t);
-    if (staged) row_product<T, V, U>(s_col, s_val, base, start, end, B1 + c0, ldb, acc);
-    else row_product<T, V, U>(colind, val, 0, start, end, B1 + c0, ldb, acc);
-    T ckv[V];
-    coeffs_of<T, V, PC>(ckv, ck, cseg, colseg, c0);
-    epilogue<T, V, HQ, HS, HB>(out + row * ldo + c0, acc, q, s, t, ckv, alpha, beta);
-  }
-}
+}  // namespace csr
+}  // namespace sma
 
-// ASYNC family: every thread moves exactly 16 bytes (V = 16/sizeof(T) elements) of each
-// neighbour row it needs with cp.async (global -> shared, asynchronous), for up to NB
-// neighbours at a time plus the epilogue rows of Q, B1 and B2, then waits for its own
-// copies only and computes from shared memory.  All of a row's gathers are in flight at
-// once without holding registers, so a row costs one memory latency.  Each thread reads
-// back only the chunks it copied itself, so no barrier is needed.  CTAs are 128 threads;
-// shared memory per CTA is (NB + 3) * 128 * 16 bytes (22.5 KB for NB = 8, 38.9 KB for 16).
-constexpr int kAsyncThreads = 128;
+#include "csr_bulk.cuh"
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
+namespace sma {
+namespace csr {
 
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-template <typename T, int G, int NB, bool HQ, bool HS, bool HB>
-__global__ void __launch_bounds__(kAsyncThreads)
-async_kernel(const int *__restrict__ rowptr, const int *__restrict__ colind,
-             const T *__restrict__ val, int64_t n, int b, const T *__restrict__ Q, int64_t ldq,
-             const T *__restrict__ B1, const T *__restrict__ B2, int64_t ldb,
-             T *__restrict__ out, int64_t ldo, T ck, T alpha, T beta) {
-  constexpr int V = 16 / (int)sizeof(T);
-  constexpr int kRows = kAsyncThreads / G;
-  __shared__ uint4 buf[NB + 3][kAsyncThreads];  // slot-major: a warp's copies are contiguous
-  const int64_t row = (int64_t)blockIdx.x * kRows + threadIdx.x / G;
-  if (row >= n) return;
-  const int tid = threadIdx.x;
-  const int lane = tid % G;
-  const int start = __ldg(rowptr + row);
-  const int end = __ldg(rowptr + row + 1);
-  for (int c0 = lane * V; c0 < b; c0 += G * V) {
-    if constexpr (HQ) cp_async16(&buf[NB][tid], Q + row * ldq + c0);
-    if constexpr (HS) cp_async16(&buf[NB + 1][tid], B1 + row * ldb + c0);
-    if constexpr (HB) cp_async16(&buf[NB + 2][tid], B2 + row * ldb + c0);
-    T acc[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = T(0);
-    for (int j0 = start; j0 < end; j0 += NB) {
-      const int cnt = min(NB, end - j0);
-      for (int u = 0; u < cnt; ++u)
-        cp_async16(&buf[u][tid], B1 + (int64_t)__ldg(colind + j0 + u) * ldb + c0);
-      cp_async_wait_all();
-      for (int u = 0; u < cnt; ++u) {
-        const T a = __ldg(val + j0 + u);
-        const T *x = reinterpret_cast<const T *>(&buf[u][tid]);
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] = fma(a, x[v], acc[v]);
-      }
-    }
-    cp_async_wait_all();  // epilogue rows of an empty row
-    T q[V], s[V], t[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      if constexpr (HQ) q[v] = reinterpret_cast<const T *>(&buf[NB][tid])[v];
-      if constexpr (HS) s[v] = reinterpret_cast<const T *>(&buf[NB + 1][tid])[v];
-      if constexpr (HB) t[v] = reinterpret_cast<const T *>(&buf[NB + 2][tid])[v];
-    }
-    T ckv[V];
-    coeffs_of<T, V, false>(ckv, ck, nullptr, nullptr, c0);
-    epilogue<T, V, HQ, HS, HB>(out + row * ldo + c0, acc, q, s, t, ckv, alpha, beta);
-  }
-}
-
-// BULK family: a CTA of kBulkThreads threads owns RC = kBulkThreads / G rows (G threads of V
-// elements each cover a row in ONE pass, b = G V) and first stages everything its step
-// reads into shared memory: its CSR pairs (plain coalesced loads), then with 1D bulk copies
-// (cp.async.bulk global -> this CTA's shared memory; no multicast, local memory only) the
-// rows of Q, B1 and B2 it updates and every neighbour row of B1 its pairs name, all
-// completing on one mbarrier.  Every row a CTA needs is in flight at once without holding
-// registers, and the arithmetic reads shared memory only, in the same order as the other
-// families (bit-identical results).  Whole rows move, so rows must be 16..512 bytes and all
-// leading dimensions multiples of 16 bytes.  The host sizes the shared memory for the
-// largest CTA of the operator.  The wait on the mbarrier is bounded by elapsed time
-// (%globaltimer, one second): a CTA that gives up sets *err, waits (bounded again) for its
-// copies, and returns without writing; the host then reports SMA_ERR_TIMEOUT.
-constexpr int kBulkThreads = 256;
-constexpr unsigned long long kBulkWaitNs = 1000000000ull;
-
-__device__ __forceinline__ unsigned long long bulk_clock_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void bulk_copy(void *smem_dst, const void *gsrc, unsigned bytes,
-                                          unsigned mbar) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-      ::"r"(d), "l"(gsrc), "r"(bytes), "r"(mbar) : "memory");
-}
-
-// Waits for phase 0 of the mbarrier; false when `limit_ns` of elapsed time passed first.
-__device__ __forceinline__ bool bulk_wait(unsigned mbar, unsigned long long limit_ns) {
-  const unsigned long long t0 = bulk_clock_ns();
-  for (unsigned long long spin = 0;; ++spin) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(mbar) : "memory");
-    if (done) return true;
-    if (bulk_clock_ns() - t0 > limit_ns || spin > (1ull << 34)) return false;
-  }
-}
-
-template <typename T, int V, int G, bool HQ, bool HS, bool HB>
-__global__ void __launch_bounds__(kBulkThreads)
-bulk_kernel(const int *__restrict__ rowptr, const int *__restrict__ colind,
-            const T *__restrict__ val, int64_t n, int b, const T *__restrict__ Q, int64_t ldq,
-            const T *__restrict__ B1, const T *__restrict__ B2, int64_t ldb,
-            T *__restrict__ out, int64_t ldo, T ck, T alpha, T beta, int cap, int *err) {
-  constexpr int RC = kBulkThreads / G;
-  constexpr int NR = (HQ ? 1 : 0) + (HS ? 1 : 0) + (HB ? 1 : 0);
-  extern __shared__ __align__(16) unsigned char bulk_smem[];
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(bulk_smem);
-  T *rows = reinterpret_cast<T *>(bulk_smem + 16);  // NR x RC rows: Q, B1, B2 (those present)
-  T *nbr = rows + (size_t)NR * RC * b;               // cap neighbour rows
-  T *sval = nbr + (size_t)cap * b;
-  int *scol = reinterpret_cast<int *>(sval + cap);
-  const unsigned mbar = static_cast<unsigned>(__cvta_generic_to_shared(bar));
-  const unsigned rb = (unsigned)b * sizeof(T);
-  const int64_t row0 = (int64_t)blockIdx.x * RC;
-  const int nrows = (int)min((int64_t)RC, n - row0);
-  const int base = __ldg(rowptr + row0);
-  const int cnt = __ldg(rowptr + row0 + nrows) - base;
-  if (cnt > cap) {  // the host sized shared memory for the largest CTA: never taken
-    if (threadIdx.x == 0) atomicExch(err, 2);
-    return;
-  }
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  for (int i = threadIdx.x; i < cnt; i += kBulkThreads) {
-    scol[i] = __ldg(colind + base + i);
-    sval[i] = __ldg(val + base + i);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned bytes = ((unsigned)cnt + (unsigned)(NR * nrows)) * rb;
-    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n"
-                 ::"r"(mbar), "r"(bytes) : "memory");
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < cnt; i += kBulkThreads)
-    bulk_copy(nbr + (size_t)i * b, B1 + (int64_t)scol[i] * ldb, rb, mbar);
-  {
-    int slot = 0;
-    const T *src[3];
-    int64_t ld[3];
-    if constexpr (HQ) { src[slot] = Q; ld[slot] = ldq; ++slot; }
-    if constexpr (HS) { src[slot] = B1; ld[slot] = ldb; ++slot; }
-    if constexpr (HB) { src[slot] = B2; ld[slot] = ldb; ++slot; }
-    for (int e = threadIdx.x; e < NR * nrows; e += kBulkThreads) {
-      const int k = e / nrows, r = e % nrows;
-      bulk_copy(rows + ((size_t)k * RC + r) * b, src[k] + (row0 + r) * ld[k], rb, mbar);
-    }
-  }
-  if (!bulk_wait(mbar, kBulkWaitNs)) {
-    if (threadIdx.x == 0) atomicExch(err, 1);
-    bulk_wait(mbar, kBulkWaitNs);  // let the copies in flight land before the CTA exits
-    return;
-  }
-  const int r = threadIdx.x / G;
-  if (r >= nrows) return;
-  const int c0 = (threadIdx.x % G) * V;
-  const int64_t row = row0 + r;
-  const int start = __ldg(rowptr + row) - base, end = __ldg(rowptr + row + 1) - base;
-  T acc[V], q[V], sv[V], t[V], ckv[V];
-#pragma unroll
-  for (int v = 0; v < V; ++v) {
-    acc[v] = T(0);
-    ckv[v] = ck;
-  }
-  for (int e = start; e < end; ++e) {
-    const T a = sval[e];
-    const T *x = nbr + (size_t)e * b + c0;
-#pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = fma(a, x[v], acc[v]);
-  }
-  int slot = 0;
-  if constexpr (HQ) {
-#pragma unroll
-    for (int v = 0; v < V; ++v) q[v] = rows[((size_t)slot * RC + r) * b + c0 + v];
-    ++slot;
-  }
-  if constexpr (HS) {
-#pragma unroll
-    for (int v = 0; v < V; ++v) sv[v] = rows[((size_t)slot * RC + r) * b + c0 + v];
-    ++slot;
-  }
-  if constexpr (HB) {
-#pragma unroll
-    for (int v = 0; v < V; ++v) t[v] = rows[((size_t)slot * RC + r) * b + c0 + v];
-  }
-  epilogue<T, V, HQ, HS, HB>(out + row * ldo + c0, acc, q, sv, t, ckv, alpha, beta);
-}
-
-// ------------------------------------------------------------------ configurations
-// Encoded as fam | V << 4 | G << 8 | U << 16 (for the ASYNC family U is NB).
-inline int enc(int fam, int V, int G, int U) { return fam | (V << 4) | (G << 8) | (U << 16); }
-inline int fam_of(int c) { return c & 15; }
-inline int v_of(int c) { return (c >> 4) & 15; }
-inline int g_of(int c) { return (c >> 8) & 255; }
-inline int u_of(int c) { return c >> 16; }
-
-template <typename T>
-struct Args {
-  const sma_op *op;
-  cudaStream_t st;
-  int64_t b;
-  const T *Q;
-  int64_t ldq;
-  const T *B1, *B2;
-  int64_t ldb;
-  T *out;
-  int64_t ldo;
-  double ck, alpha, beta;
-  // per-segment coefficients of this step (cseg[segment]) and the segment of every column
-  // (colseg[column]); null for one coefficient.  Batched spectrum slicing maps a window's
-  // columns to its segment; the POLFED polish gives every column its own polynomial.
-  const T *cseg = nullptr;
-  const int *colseg = nullptr;
-};
-
-// Launch of a DIRECT or STAGED step: as a programmatic dependent of the previous launch in
-// the stream when the context allows it (the kernels wait for their predecessor before
-// they touch B1, B2 or the output), else an ordinary launch.
-template <typename... KArgs, typename... Args>
-void launch_step(const sma_op *op, void (*kernel)(KArgs...), unsigned grid, cudaStream_t st,
-                 Args... args) {
+// ------------------------------------------------------------------ launch
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W>
+void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = op->ctx->pdl ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W>, a));
   SMA_CHECK_LAUNCH();
 }
 
-template <typename T, int V, int G, int U, bool HQ, bool HS, bool HB>
-void launch_one(int fam, const Args<T> &a) {
-  const T *val;
-  if constexpr (sizeof(T) == 8) val = (const T *)a.op->val64;
-  else val = (const T *)a.op->val32;
-  constexpr int kRows = kThreads / G;
-  const unsigned grid = (unsigned)((a.op->n + kRows - 1) / kRows);
-  const sma_op *op = a.op;
-  if constexpr (HQ && HS && HB) {
-    if (a.cseg) {
-      auto k = fam == 0 ? direct_kernel<T, V, G, U, true, true, true, true>
-                        : staged_kernel<T, V, G, U, true, true, true, true>;
-      return launch_step(op, k, grid, a.st, op->rowptr, op->colind, val, op->n, (int)a.b, a.Q,
-                         a.ldq, a.B1, a.B2, a.ldb, a.out, a.ldo, T(0), (T)a.alpha, (T)a.beta,
-                         a.cseg, a.colseg);
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W>
+void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
+  const uint32_t vecs = a.b / V;
+  // as few panels as keep a row within kPanel vectors, each a multiple of 4 vectors (128 bytes)
+  const uint32_t panels = (vecs + kPanel - 1) / kPanel;
+  a.lanes = panels == 1 ? vecs : ((vecs + panels - 1) / panels + 3) / 4 * 4;
+  a.rows = kThreads / a.lanes;
+  a.divlanes = (65536 + a.lanes - 1) / a.lanes;
+  const uint32_t gx = (a.n + a.rows - 1) / a.rows;
+  // Fewer than six waves of 8-CTA residency: a step is then a latency, not a stream, and twice
+  // the gathers in flight at half the occupancy is the faster kernel (Anderson L = 20, b = 64
+  // FP64: 3.7 us against 5.0; XXZ L = 18, b = 32: 13.5 against 14.2; with 2 M threads 43.8
+  // against 42.5).
+  const bool small = gathers ? gathers == 8
+                             : (int64_t)a.n * vecs < 6LL * 8 * kThreads * op->ctx->num_sms;
+  constexpr uint32_t kGridY = 65535;
+  const uint32_t ny = (vecs + a.lanes - 1) / a.lanes;
+  const uint32_t span = kGridY * a.lanes * V, width = a.b;
+  for (uint32_t p = 0; p < ny; p += kGridY) {  // more than one pass only beyond 65535 panels
+    if (p) {
+      a.B1 += span;
+      a.out += span;
+      if (HQ) a.Q += span;
+      if (HB) a.B2 += span;
+      if (PC) { if (a.colseg) a.colseg += span; else a.cseg += span; }
     }
+    a.b = width - p * a.lanes * V;
+    const dim3 grid(gx, std::min(kGridY, ny - p));
+    if (small) launch<T, V, 8, 8, HQ, HS, HB, PC, W>(op, st, a, grid);
+    else launch<T, V, 4, 12, HQ, HS, HB, PC, W>(op, st, a, grid);
   }
-  if (a.cseg) throw Error(SMA_ERR_INTERNAL, "segmented Clenshaw step needs the full variant");
-  auto k = fam == 0 ? direct_kernel<T, V, G, U, HQ, HS, HB, false>
-                    : staged_kernel<T, V, G, U, HQ, HS, HB, false>;
-  launch_step(op, k, grid, a.st, op->rowptr, op->colind, val, op->n, (int)a.b, a.Q, a.ldq, a.B1,
-              a.B2, a.ldb, a.out, a.ldo, (T)a.ck, (T)a.alpha, (T)a.beta, (const T *)nullptr,
-              (const int *)nullptr);
 }
 
-template <typename T, int G, int NB, bool HQ, bool HS, bool HB>
-void launch_async(const Args<T> &a) {
-  if (a.cseg) throw Error(SMA_ERR_INTERNAL, "the asynchronous family has no segmented variant");
-  const T *val;
-  if constexpr (sizeof(T) == 8) val = (const T *)a.op->val64;
-  else val = (const T *)a.op->val32;
-  constexpr int kRows = kAsyncThreads / G;
-  const unsigned grid = (unsigned)((a.op->n + kRows - 1) / kRows);
-  async_kernel<T, G, NB, HQ, HS, HB><<<grid, kAsyncThreads, 0, a.st>>>(
-      a.op->rowptr, a.op->colind, val, a.op->n, (int)a.b, a.Q, a.ldq, a.B1, a.B2, a.ldb, a.out,
-      a.ldo, (T)a.ck, (T)a.alpha, (T)a.beta);
-  SMA_CHECK_LAUNCH();
+// ------------------------------------------------------------------ the tuning table
+// With SMA_AUTOTUNE_VERBOSE=1 in the environment (and SMA_AUTOTUNE not 0) the first launches of
+// each shape of an operator with n >= 20000 run every configuration in turn, four times, on the
+// real steps, bracketed by events; then the table is printed and the fastest kept.  A check of
+// the rules above: without the variable they alone choose.
+struct Config {
+  bool bulk;
+  int V, gathers;
+};
+
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
+void launch_config(const sma_op *op, cudaStream_t st, const Step<T> &a, const Config &c) {
+  if constexpr (!PC)
+    if (c.bulk) return launch_bulk<T, V, HQ, HS, HB>(op, st, a);
+  launch_width<T, V, HQ, HS, HB, PC, false>(op, st, a, c.gathers);
 }
 
-// The most CSR entries held by any CTA of RC consecutive rows (cached per RC).
-inline int bulk_max_pairs(const sma_op *op, int RC) {
-  sma_op *o = const_cast<sma_op *>(op);
-  const auto it = o->bulk_pairs.find(RC);
-  if (it != o->bulk_pairs.end()) return it->second;
-  if (o->host_rowptr.empty()) {
-    o->host_rowptr.resize(op->n + 1);
-    SMA_CUDA(cudaMemcpy(o->host_rowptr.data(), op->rowptr, (op->n + 1) * sizeof(int),
-                        cudaMemcpyDeviceToHost));
-  }
-  int mx = 0;
-  for (int64_t r = 0; r < op->n; r += RC) {
-    const int64_t e = std::min<int64_t>(op->n, r + RC);
-    mx = std::max(mx, o->host_rowptr[e] - o->host_rowptr[r]);
-  }
-  o->bulk_pairs[RC] = mx;
-  return mx;
-}
-
-inline size_t bulk_smem_bytes(int RC, int nr, int b, int cap, size_t elem) {
-  return 16 + (size_t)nr * RC * b * elem + (size_t)cap * (b * elem + elem + sizeof(int));
-}
-
-template <typename T, int V, int G, bool HQ, bool HS, bool HB>
-void launch_bulk(const Args<T> &a) {
-  if (a.cseg) throw Error(SMA_ERR_INTERNAL, "the bulk family has no segmented variant");
-  const sma_op *op = a.op;
-  if (a.b != (int64_t)G * V) throw Error(SMA_ERR_INTERNAL, "bulk family: b != G V");
-  const T *val;
-  if constexpr (sizeof(T) == 8) val = (const T *)op->val64;
-  else val = (const T *)op->val32;
-  constexpr int RC = kBulkThreads / G;
-  constexpr int NR = (HQ ? 1 : 0) + (HS ? 1 : 0) + (HB ? 1 : 0);
-  const int cap = std::max(1, bulk_max_pairs(op, RC));
-  const size_t smem = bulk_smem_bytes(RC, NR, (int)a.b, cap, sizeof(T));
-  require(op->bulk_err != nullptr, SMA_ERR_INTERNAL, "bulk family without its error flag");
-  SMA_CUDA(cudaFuncSetAttribute(bulk_kernel<T, V, G, HQ, HS, HB>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const unsigned grid = (unsigned)((op->n + RC - 1) / RC);
-  bulk_kernel<T, V, G, HQ, HS, HB><<<grid, kBulkThreads, smem, a.st>>>(
-      op->rowptr, op->colind, val, op->n, (int)a.b, a.Q, a.ldq, a.B1, a.B2, a.ldb, a.out, a.ldo,
-      (T)a.ck, (T)a.alpha, (T)a.beta, cap, op->bulk_err);
-  SMA_CHECK_LAUNCH();
-}
-
-// Whether the BULK family can take this step: whole rows of 16..512 bytes, every leading
-// dimension and base address on 16 bytes, and the largest CTA's rows within shared memory.
-template <typename T, bool HQ, bool HS, bool HB>
-bool bulk_fits(const Args<T> &a, int V) {
-  const int64_t rb = a.b * (int64_t)sizeof(T);
-  if (a.cseg || rb < 16 || rb > 512 || rb % 16 || a.b % V) return false;
-  const int64_t G = a.b / V;
-  if (G != 4 && G != 8 && G != 16 && G != 32) return false;
-  auto al = [](const void *p) { return p == nullptr || ((uintptr_t)p & 15) == 0; };
-  if ((a.ldb * sizeof(T)) % 16 || (HQ && (a.ldq * sizeof(T)) % 16) || !al(a.Q) || !al(a.B1) ||
-      !al(a.B2))
-    return false;
-  const int RC = kBulkThreads / (int)G;
-  const int nr = (HQ ? 1 : 0) + (HS ? 1 : 0) + (HB ? 1 : 0);
-  const int cap = std::max(1, bulk_max_pairs(a.op, RC));
-  return bulk_smem_bytes(RC, nr, (int)a.b, cap, sizeof(T)) <= 200 * 1024;
-}
-
-template <typename T, int V, bool HQ, bool HS, bool HB>
-void launch_v(int c, const Args<T> &a) {
-  const int fam = fam_of(c);
-  if (fam == 3) {
-    switch (g_of(c)) {
-      case 4: return launch_bulk<T, V, 4, HQ, HS, HB>(a);
-      case 8: return launch_bulk<T, V, 8, HQ, HS, HB>(a);
-      case 16: return launch_bulk<T, V, 16, HQ, HS, HB>(a);
-      case 32: return launch_bulk<T, V, 32, HQ, HS, HB>(a);
-      default: throw Error(SMA_ERR_INTERNAL, "bad bulk CSR kernel configuration");
-    }
-  }
-  if (fam == 2) {
-    if constexpr (V * sizeof(T) == 16) {
-      switch (g_of(c) * 100 + u_of(c)) {
-        case 408: return launch_async<T, 4, 8, HQ, HS, HB>(a);
-        case 416: return launch_async<T, 4, 16, HQ, HS, HB>(a);
-        case 808: return launch_async<T, 8, 8, HQ, HS, HB>(a);
-        case 816: return launch_async<T, 8, 16, HQ, HS, HB>(a);
-        case 1608: return launch_async<T, 16, 8, HQ, HS, HB>(a);
-        case 1616: return launch_async<T, 16, 16, HQ, HS, HB>(a);
-        case 3208: return launch_async<T, 32, 8, HQ, HS, HB>(a);
-        case 3216: return launch_async<T, 32, 16, HQ, HS, HB>(a);
-        default: break;
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
+bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
+  if (!op->ctx->tune || op->n < 20000) return false;
+  cudaStreamCaptureStatus cap;
+  SMA_CUDA(cudaStreamIsCapturing(st, &cap));
+  CsrTune &t = const_cast<sma_op *>(op)->tuned[{(int64_t)sizeof(T) * 8 + V, HQ * 8 + HS * 4 + HB * 2 + PC, a.b}];
+  std::vector<Config> cfg = {{false, V, 8}, {false, V, 4}};
+  if constexpr (!PC) {
+    if (bulk_fits<T, V, HQ, HS, HB>(op, a)) {
+      if (!op->bulk_err && cap == cudaStreamCaptureStatusNone) {
+        SMA_CUDA(cudaMalloc((void **)&const_cast<sma_op *>(op)->bulk_err, sizeof(int)));
+        SMA_CUDA(cudaMemset(op->bulk_err, 0, sizeof(int)));
       }
-    }
-    throw Error(SMA_ERR_INTERNAL, "bad asynchronous CSR kernel configuration");
-  }
-  switch (g_of(c) * 100 + u_of(c)) {
-    case 404: return launch_one<T, V, 4, 4, HQ, HS, HB>(fam, a);
-    case 408: return launch_one<T, V, 4, 8, HQ, HS, HB>(fam, a);
-    case 804: return launch_one<T, V, 8, 4, HQ, HS, HB>(fam, a);
-    case 808: return launch_one<T, V, 8, 8, HQ, HS, HB>(fam, a);
-    case 1604: return launch_one<T, V, 16, 4, HQ, HS, HB>(fam, a);
-    case 1608: return launch_one<T, V, 16, 8, HQ, HS, HB>(fam, a);
-    case 3204: return launch_one<T, V, 32, 4, HQ, HS, HB>(fam, a);
-    case 3208: return launch_one<T, V, 32, 8, HQ, HS, HB>(fam, a);
-    default: throw Error(SMA_ERR_INTERNAL, "bad CSR kernel configuration");
-  }
-}
-
-template <typename T, bool HQ, bool HS, bool HB>
-void launch_cfg(int c, const Args<T> &a) {
-  switch (v_of(c)) {
-    case 1: return launch_v<T, 1, HQ, HS, HB>(c, a);
-    case 2: return launch_v<T, 2, HQ, HS, HB>(c, a);
-    case 4: return launch_v<T, 4, HQ, HS, HB>(c, a);
-    default:
-      if constexpr (sizeof(T) == 4) {
-        if (v_of(c) == 8) return launch_v<T, 8, HQ, HS, HB>(c, a);
-      }
-      throw Error(SMA_ERR_INTERNAL, "bad CSR vector width");
-  }
-}
-
-inline bool aligned(const void *p, int bytes) { return p == nullptr || ((uintptr_t)p % bytes) == 0; }
-
-// Online autotuner.  The first 2 x (number of candidates) launches for a given operator,
-// element type, variant, width and leading dimension run the candidates in turn on the
-// real recurrence steps, bracketed by CUDA events; after the last of them one event
-// synchronization reads the times, and the four fastest candidates (best of two runs) run
-// four times more each, in turn; the fastest of those (best of its four runs) is kept for
-// the operator's lifetime.  Single runs of a 50-100 us step vary by 10 % or more with
-// clocks and neighbouring launches, so the second round guards the choice against a
-// lucky or unlucky trial.  Candidates: both families; the widest vector the
-// alignment allows, and half of it when that is 32 bytes; the narrowest power-of-two
-// group covering the block in one column pass, and the half-width group; U = 4 and 8.
-// Small operators (n < 20000) and contexts with autotuning off use the first candidate.
-template <typename T, bool HQ, bool HS, bool HB>
-void step(const Args<T> &a) {
-  const sma_op *op = a.op;
-  auto ok = [&](int v) {
-    const int bytes = std::min(16, v * (int)sizeof(T));
-    return a.b % v == 0 && a.ldb % v == 0 && a.ldo % v == 0 && (!HQ || a.ldq % v == 0) &&
-           aligned(a.Q, bytes) && aligned(a.B1, bytes) && aligned(a.B2, bytes) &&
-           aligned(a.out, bytes);
-  };
-  int vmax = 1;
-  for (int v : {2, 4, 8})
-    if (v * (int)sizeof(T) <= 32 && ok(v)) vmax = v;
-  const uint64_t key = ((uint64_t)sizeof(T) << 56) | ((uint64_t)vmax << 52) |
-                       ((uint64_t)((HQ ? 4 : 0) | (HS ? 2 : 0) | (HB ? 1 : 0)) << 48) |
-                       (a.cseg ? (1ull << 51) : 0ull) | ((uint64_t)a.b << 24) |
-                       (uint64_t)std::min<int64_t>(a.ldb, 0xFFFFFF);
-  CsrTune &tu = const_cast<sma_op *>(op)->tuned[key];
-  if (tu.chosen >= 0) return launch_cfg<T, HQ, HS, HB>(tu.chosen, a);
-  if (tu.cands.empty()) {
-    for (int fam : {1, 0})
-      for (int V : {vmax, vmax / 2}) {
-        if (V < 1 || (V != vmax && vmax * (int)sizeof(T) < 32)) continue;
-        const int64_t lanes = (a.b + V - 1) / V;
-        const int g0 = lanes <= 4 ? 4 : lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
-        for (int G : {g0, g0 / 2}) {
-          if (G < 4) continue;
-          tu.cands.push_back(enc(fam, V, G, 8));
-          tu.cands.push_back(enc(fam, V, G, 4));
-        }
-      }
-    for (int V : {vmax, vmax / 2}) {  // the BULK family: whole rows staged by bulk copies
-      // (a key with 16-byte vectors guarantees 16-byte pointers and leading dimensions)
-      if (V >= 1 && vmax * (int)sizeof(T) >= 16 && bulk_fits<T, HQ, HS, HB>(a, V)) {
-        if (!op->bulk_err) {
-          SMA_CUDA(cudaMalloc((void **)&const_cast<sma_op *>(op)->bulk_err, sizeof(int)));
-          SMA_CUDA(cudaMemset(op->bulk_err, 0, sizeof(int)));
-        }
-        tu.cands.push_back(enc(3, V, (int)(a.b / V), 0));
-      }
-    }
-    if (vmax * (int)sizeof(T) >= 16 && !a.cseg) {  // the ASYNC family moves 16-byte chunks
-      const int V = 16 / (int)sizeof(T);
-      const int64_t lanes = (a.b + V - 1) / V;
-      const int g0 = lanes <= 4 ? 4 : lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
-      tu.cands.push_back(enc(2, V, g0, 8));
-      tu.cands.push_back(enc(2, V, g0, 16));
-      if (g0 >= 8) tu.cands.push_back(enc(2, V, g0 / 2, 8));
-    }
-    if (!op->ctx->autotune || op->n < 20000) {
-      tu.chosen = tu.cands[0];
-      return launch_cfg<T, HQ, HS, HB>(tu.chosen, a);
+      if (op->bulk_err) cfg.push_back({true, V, 0});
     }
   }
-  const int kReps = tu.round == 0 ? 2 : 4;
-  const size_t ncand = tu.cands.size();
-  const size_t idx = tu.trial.size();
-  const int c = tu.cands[idx % ncand];
-  cudaEvent_t e0, e1;
-  SMA_CUDA(cudaEventCreate(&e0));
-  SMA_CUDA(cudaEventCreate(&e1));
-  tu.events.push_back(e0);
-  tu.events.push_back(e1);
-  tu.trial.push_back(c);
-  SMA_CUDA(cudaEventRecord(e0, a.st));
-  launch_cfg<T, HQ, HS, HB>(c, a);
-  SMA_CUDA(cudaEventRecord(e1, a.st));
-  if (idx + 1 < kReps * ncand) return;
-  SMA_CUDA(cudaEventSynchronize(e1));
-  std::vector<float> best(ncand, INFINITY);
-  for (size_t i = 0; i < tu.trial.size(); ++i) {
+  if (t.chosen >= 0) {
+    launch_config<T, V, HQ, HS, HB, PC>(op, st, a, cfg[std::min(t.chosen, (int)cfg.size() - 1)]);
+    return true;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return false;
+  cudaEvent_t e[2];
+  const size_t i = t.events.size() / 2;
+  for (cudaEvent_t &x : e) {
+    SMA_CUDA(cudaEventCreate(&x));
+    t.events.push_back(x);
+  }
+  SMA_CUDA(cudaEventRecord(e[0], st));
+  launch_config<T, V, HQ, HS, HB, PC>(op, st, a, cfg[i % cfg.size()]);
+  SMA_CUDA(cudaEventRecord(e[1], st));
+  if (i + 1 < 4 * cfg.size()) return true;
+  SMA_CUDA(cudaEventSynchronize(e[1]));
+  std::vector<float> best(cfg.size(), INFINITY);
+  for (size_t k = 0; k <= i; ++k) {
     float ms = 0.f;
-    SMA_CUDA(cudaEventElapsedTime(&ms, tu.events[2 * i], tu.events[2 * i + 1]));
-    best[i % ncand] = std::min(best[i % ncand], ms);
+    SMA_CUDA(cudaEventElapsedTime(&ms, t.events[2 * k], t.events[2 * k + 1]));
+    best[k % cfg.size()] = std::min(best[k % cfg.size()], ms);
   }
-  if (tu.round == 0 && ncand > 4) {  // the four best run again
-    std::vector<size_t> order(ncand);
-    for (size_t i = 0; i < ncand; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return best[x] < best[y]; });
-    std::vector<int> top;
-    for (size_t i = 0; i < 4; ++i) top.push_back(tu.cands[order[i]]);
-    if (const char *vb = std::getenv("SMA_AUTOTUNE_VERBOSE"); vb && vb[0] == '1') {
-      fprintf(stderr, "sma autotune round 1: %s n=%lld b=%lld ld=%lld ->", sizeof(T) == 8 ? "fp64" : "fp32",
-              (long long)op->n, (long long)a.b, (long long)a.ldb);
-      for (size_t i = 0; i < ncand; ++i)
-        fprintf(stderr, " %s/V%d/G%d/U%d=%.1fus",
-                fam_of(tu.cands[i]) == 3   ? "bulk"
-                : fam_of(tu.cands[i]) == 2 ? "async"
-                : fam_of(tu.cands[i])      ? "staged"
-                                           : "direct",
-                v_of(tu.cands[i]), g_of(tu.cands[i]), u_of(tu.cands[i]), 1e3 * best[i]);
-      fprintf(stderr, "\n");
-    }
-    tu.release();
-    tu.cands = top;
-    tu.round = 1;
-    return;
-  }
-  const size_t w = std::min_element(best.begin(), best.end()) - best.begin();
-  tu.chosen = tu.cands[w];
-  tu.release();
-  if (const char *vb = std::getenv("SMA_AUTOTUNE_VERBOSE"); vb && vb[0] == '1') {
-    fprintf(stderr, "sma autotune: %s n=%lld b=%lld ld=%lld variant=%d%d%d ->", sizeof(T) == 8 ? "fp64" : "fp32",
-            (long long)op->n, (long long)a.b, (long long)a.ldb, (int)HQ, (int)HS, (int)HB);
-    for (size_t i = 0; i < ncand; ++i)
-      fprintf(stderr, " %s%s/V%d/G%d/U%d=%.1fus", i == w ? "*" : "",
-              fam_of(tu.cands[i]) == 3   ? "bulk"
-              : fam_of(tu.cands[i]) == 2 ? "async"
-              : fam_of(tu.cands[i])      ? "staged"
-                                         : "direct",
-              v_of(tu.cands[i]), g_of(tu.cands[i]), u_of(tu.cands[i]), 1e3 * best[i]);
-    fprintf(stderr, "\n");
-  }
+  t.release();
+  t.chosen = (int)(std::min_element(best.begin(), best.end()) - best.begin());
+  fprintf(stderr, "sma autotune: %s n=%lld b=%lld variant=%d%d%d ->", sizeof(T) == 8 ? "fp64" : "fp32",
+          (long long)op->n, (long long)a.b, (int)HQ, (int)HS, (int)HB);
+  for (size_t k = 0; k < cfg.size(); ++k)
+    fprintf(stderr, " %s%s/V%d/U%d=%.1fus", (int)k == t.chosen ? "*" : "",
+            cfg[k].bulk ? "bulk" : "rows", V, cfg[k].gathers, 1e3 * best[k]);
+  fprintf(stderr, "\n");
+  return true;
 }
 
-template <typename T>
-void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
-                   const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                   double alpha, double beta, bool has_self) {
-  const Args<T> a{op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta};
-  if (Q && has_self && B2) return step<T, true, true, true>(a);
-  if (Q && has_self && !B2) return step<T, true, true, false>(a);
-  if (!Q && !has_self && !B2) return step<T, false, false, false>(a);
-  throw Error(SMA_ERR_INTERNAL, "unsupported Clenshaw step variant");
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
+void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
+  if (!tuned_step<T, V, HQ, HS, HB, PC>(op, st, a)) launch_width<T, V, HQ, HS, HB, PC, false>(op, st, a);
+}
+
+inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
+
+// Picks the vector width: the widest that widths, strides and addresses allow, but narrower
+// while the step would not give every SM a CTA (XXZ L = 14, b = 8 FP64: 4.4, 3.3 and 3.1 us a
+// step with 4, 2 and 1 columns a thread).
+template <typename T, bool HQ, bool HS, bool HB, bool PC>
+void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
+  if (op->n == 0 || b == 0) return;
+  require(b < (int64_t)1 << 31, SMA_ERR_ARG, "block too wide");
+  if constexpr (sizeof(T) == 8) a.val = op->val64;
+  else a.val = op->val32;
+  a.rowptr = op->rowptr;
+  a.colind = op->colind;
+  a.n = (uint32_t)op->n;
+  a.b = (uint32_t)b;
+  auto fits = [&](int v) {
+    const int bytes = v * (int)sizeof(T);
+    return b % v == 0 && a.ldb % bytes == 0 && a.ldo % bytes == 0 && aligned(a.B1, bytes) &&
+           aligned(a.out, bytes) && (!HQ || (a.ldq % bytes == 0 && aligned(a.Q, bytes))) &&
+           (!HB || aligned(a.B2, bytes)) && (!PC || a.colseg || aligned(a.cseg, bytes));
+  };
+  const int64_t want = (int64_t)op->ctx->num_sms * kThreads;
+  auto take = [&](int v) { return fits(v) && op->n * (b / v) >= want; };
+  if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true>(op, st, a);
+  if constexpr (sizeof(T) == 4)
+    if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC>(op, st, a);
+  if (take(4)) return launch_rule<T, 4, HQ, HS, HB, PC>(op, st, a);
+  if (take(2)) return launch_rule<T, 2, HQ, HS, HB, PC>(op, st, a);
+  launch_width<T, 1, HQ, HS, HB, PC, false>(op, st, a);
 }
 
 }  // namespace csr
-}  // namespace sma
 
-namespace sma {
 template <typename T>
 void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                        const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                       double alpha, double beta, bool has_self) {
-  csr::clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self);
-}
-}  // namespace sma
-
-namespace sma {
-namespace csr {
-
-// The CSR step without the autotuner: the operator's tuned configuration for this key when
-// one has been chosen, else the autotuner's first candidate.  Creates no events and never
-// inserts into the tuning cache (used by the allocation-free entry point).
-template <typename T, bool HQ, bool HS, bool HB>
-void step_untuned(const Args<T> &a) {
-  auto ok = [&](int v) {
-    const int bytes = std::min(16, v * (int)sizeof(T));
-    return a.b % v == 0 && a.ldb % v == 0 && a.ldo % v == 0 && (!HQ || a.ldq % v == 0) &&
-           aligned(a.Q, bytes) && aligned(a.B1, bytes) && aligned(a.B2, bytes) &&
-           aligned(a.out, bytes);
-  };
-  int vmax = 1;
-  for (int v : {2, 4, 8})
-    if (v * (int)sizeof(T) <= 32 && ok(v)) vmax = v;
-  const uint64_t key = ((uint64_t)sizeof(T) << 56) | ((uint64_t)vmax << 52) |
-                       ((uint64_t)((HQ ? 4 : 0) | (HS ? 2 : 0) | (HB ? 1 : 0)) << 48) |
-                       (a.cseg ? (1ull << 51) : 0ull) | ((uint64_t)a.b << 24) |
-                       (uint64_t)std::min<int64_t>(a.ldb, 0xFFFFFF);
-  const auto it = a.op->tuned.find(key);
-  if (it != a.op->tuned.end() && it->second.chosen >= 0)
-    return launch_cfg<T, HQ, HS, HB>(it->second.chosen, a);
-  const int64_t lanes = (a.b + vmax - 1) / vmax;
-  const int g0 = lanes <= 4 ? 4 : lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
-  launch_cfg<T, HQ, HS, HB>(enc(1, vmax, g0, 8), a);
-}
-
-}  // namespace csr
-
-template <typename T>
-void csr_clenshaw_step_untuned(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
-                               int64_t ldq, const T *B1, const T *B2, int64_t ldb, T *out,
-                               int64_t ldo, double ck, double alpha, double beta, bool has_self) {
-  const csr::Args<T> a{op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta};
-  if (Q && has_self && B2) return csr::step_untuned<T, true, true, true>(a);
-  if (Q && has_self && !B2) return csr::step_untuned<T, true, true, false>(a);
+                       double alpha, double beta, bool has_self, bool rev) {
+  csr::Step<T> a{};
+  a.Q = Q;
+  a.B1 = B1;
+  a.B2 = B2;
+  a.out = out;
+  a.ldq = (uint64_t)ldq * sizeof(T);
+  a.ldb = (uint64_t)ldb * sizeof(T);
+  a.ldo = (uint64_t)ldo * sizeof(T);
+  a.ck = (T)ck;
+  a.alpha = (T)alpha;
+  a.beta = (T)beta;
+  a.rev = rev;
+  if (Q && has_self && B2) return csr::step<T, true, true, true, false>(op, st, b, a);
+  if (Q && has_self && !B2) return csr::step<T, true, true, false, false>(op, st, b, a);
+  if (!Q && !has_self && !B2) return csr::step<T, false, false, false, false>(op, st, b, a);
   throw Error(SMA_ERR_INTERNAL, "unsupported Clenshaw step variant");
 }
 
-// The segmented step: column c takes the coefficient cseg[colseg[c]]; Q, B1 and B2 are all
-// read.  tuned = false uses the operator's cached configuration (or the default one) and
-// creates no events, so that it may be recorded into a CUDA graph.
+// The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
+// cseg[c] when colseg is null; Q, B1 and B2 are all read.
 template <typename T>
 void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
-                           const T *cseg, const int *colseg, double alpha, double beta,
-                           bool tuned) {
-  csr::Args<T> a{op, st, b, Q, ldq, B1, B2, ldb, out, ldo, 0.0, alpha, beta};
+                           const T *cseg, const int *colseg, double alpha, double beta, bool rev) {
+  csr::Step<T> a{};
+  a.Q = Q;
+  a.B1 = B1;
+  a.B2 = B2;
+  a.out = out;
   a.cseg = cseg;
   a.colseg = colseg;
-  if (tuned) return csr::step<T, true, true, true>(a);
-  csr::step_untuned<T, true, true, true>(a);
+  a.ldq = (uint64_t)ldq * sizeof(T);
+  a.ldb = (uint64_t)ldb * sizeof(T);
+  a.ldo = (uint64_t)ldo * sizeof(T);
+  a.alpha = (T)alpha;
+  a.beta = (T)beta;
+  a.rev = rev;
+  csr::step<T, true, true, true, true>(op, st, b, a);
 }
 }  // namespace sma

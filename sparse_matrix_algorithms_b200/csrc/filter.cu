@@ -91,24 +91,12 @@ static void matblock_apply(const sma_op *op, cudaStream_t st, const T *X, T *AX,
   }
 }
 
-// One fused step for device operators: the autotuned CSR launch, or (tuned = false, for
-// graph recording) the operator's cached configuration with no events.
-template <typename T>
-static void fused_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
-                       const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                       double alpha, double beta, bool tuned) {
-  if (!tuned && op->kind == OP_CSR)
-    csr_clenshaw_step_untuned<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, true);
-  else
-    launch_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, true);
-}
-
 // The launches of one filter (K >= 1); returns the step count and algorithmic bytes.
 template <typename T>
 static FilterCount record_filter(const sma_op *op, cudaStream_t st,
                                  const std::vector<double> &coeffs, double smin, double smax,
                                  const T *Q, int64_t ldq, T *Y, int64_t ldy, int64_t b,
-                                 ClenshawWork<T> &work, bool tuned) {
+                                 ClenshawWork<T> &work) {
   FilterCount fc;
   const int64_t n = op->n;
   const int64_t K = (int64_t)coeffs.size() - 1;
@@ -127,8 +115,8 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   for (int64_t ci = K - 1; ci >= 1; --ci) {
     if (fused) {
-      fused_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, TMP, ld, coeffs[ci], alpha,
-                    beta, tuned);
+      launch_clenshaw_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, TMP, ld,
+                              coeffs[ci], alpha, beta, true, ci & 1);
     } else {
       matblock_apply<T>(op, st, B1, work.ax.p, ld, b);
       launch_clenshaw_axpy<T>(st, n, b, Q, ldq, work.ax.p, ld, B1, b2_zero ? nullptr : B2, ld,
@@ -144,8 +132,8 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   }
   // final step: Y = c_0 Q + invd*A B1 - c*invd*B1 - B2
   if (fused) {
-    fused_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, Y, ldy, coeffs[0], invd,
-                  -(c * invd), tuned);
+    launch_clenshaw_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, Y, ldy, coeffs[0],
+                            invd, -(c * invd), true, false);
   } else {
     matblock_apply<T>(op, st, B1, work.ax.p, ld, b);
     launch_clenshaw_axpy<T>(st, n, b, Q, ldq, work.ax.p, ld, B1, b2_zero ? nullptr : B2, ld, Y,
@@ -183,7 +171,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
   }
   if (op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF || K < kGraphMinDegree ||
       !op->ctx->filter_graphs)
-    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work, true);
+    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work);
   // repeated filter -> CUDA graph on the staging blocks
   const bool same = work.g_op == op && work.g_b == b && work.g_smin == smin &&
                     work.g_smax == smax && work.g_coeffs == coeffs;
@@ -196,8 +184,8 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     work.g_coeffs = coeffs;
   }
   work.g_calls += 1;
-  if (work.g_calls == 1)  // first call: eager, so the kernel autotuner sees real steps
-    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work, true);
+  if (work.g_calls == 1)  // first call: eager, a graph pays from its second use
+    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work);
   if (!work.q.p) {
     work.q.alloc(n * work.bcap, st);
     work.y.alloc(n * work.bcap, st);
@@ -207,7 +195,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     const int64_t l0 = g_kernel_launches.load();
     SMA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
-      fc = record_filter<T>(op, st, coeffs, smin, smax, work.q.p, b, work.y.p, b, b, work, false);
+      fc = record_filter<T>(op, st, coeffs, smin, smax, work.q.p, b, work.y.p, b, b, work);
     } catch (...) {
       cudaGraph_t g = nullptr;
       cudaStreamEndCapture(st, &g);

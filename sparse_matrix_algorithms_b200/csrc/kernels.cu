@@ -532,10 +532,11 @@ __global__ void check_csr_kernel(int64_t n, const int *__restrict__ rowptr,
 template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                          double alpha, double beta, bool has_self) {
+                          double alpha, double beta, bool has_self, bool rev) {
   if (op->n == 0 || b == 0) return;
   if (op->kind == OP_CSR) {
-    csr_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self);
+    csr_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self,
+                         rev);
   } else if (op->kind == OP_LAP1D) {
     Lap1dRows<T> rows{op->n};
     dispatch_flags<T>(rows, st, op->n, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self);
@@ -582,10 +583,10 @@ void launch_copy_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int
 
 template void launch_clenshaw_step<double>(const sma_op *, cudaStream_t, int64_t, const double *,
                                            int64_t, const double *, const double *, int64_t,
-                                           double *, int64_t, double, double, double, bool);
+                                           double *, int64_t, double, double, double, bool, bool);
 template void launch_clenshaw_step<float>(const sma_op *, cudaStream_t, int64_t, const float *,
                                           int64_t, const float *, const float *, int64_t, float *,
-                                          int64_t, double, double, double, bool);
+                                          int64_t, double, double, double, bool, bool);
 template void launch_scale_block<double>(cudaStream_t, int64_t, int64_t, const double *, int64_t,
                                          double *, int64_t, double);
 template void launch_scale_block<float>(cudaStream_t, int64_t, int64_t, const float *, int64_t,

@@ -29,11 +29,6 @@
 
 namespace sma {
 
-template <typename T>
-void csr_clenshaw_step_untuned(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
-                               int64_t ldq, const T *B1, const T *B2, int64_t ldb, T *out,
-                               int64_t ldo, double ck, double alpha, double beta, bool has_self);
-
 namespace {
 
 constexpr int64_t kNoAllocMaxElems = int64_t(1) << 21;
@@ -71,17 +66,6 @@ struct CurrentDevice {
   }
 };
 
-// One fused step on the operator: the CSR form without the autotuner (which creates
-// events), or the stencil form.
-void step(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
-          const double *B1, const double *B2, double *out, int64_t ldo, double ck, double alpha,
-          double beta) {
-  if (op->kind == OP_CSR)
-    csr_clenshaw_step_untuned<double>(op, st, b, Q, ldq, B1, B2, b, out, ldo, ck, alpha, beta, true);
-  else
-    launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, B2, b, out, ldo, ck, alpha, beta, true);
-}
-
 void filter_noalloc(sma_op *op, const double *coeffs, int64_t K, double smin, double smax,
                     const double *Q, int64_t ldq, double *Y, int64_t ldy, int64_t b) {
   require(op != nullptr && op->ctx != nullptr, SMA_ERR_ARG, "null operator");
@@ -114,17 +98,19 @@ void filter_noalloc(sma_op *op, const double *coeffs, int64_t K, double smin, do
     launch_scale_block<double>(st, n, b, Q, ldq, B1, b, coeffs[K]);
     bool b2_zero = true;
     for (int64_t ci = K - 1; ci >= 1; --ci) {
-      step(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, TMP, b, coeffs[ci], alpha, beta);
+      launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, b, TMP, b,
+                                   coeffs[ci], alpha, beta, true, ci & 1);
       double *t = B2;
       B2 = B1;
       B1 = TMP;
       TMP = t;
       b2_zero = false;
     }
-    step(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, Y, ldy, coeffs[0], invd, -(c * invd));
+    launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, b, Y, ldy,
+                                 coeffs[0], invd, -(c * invd), true, false);
   }
   SMA_CUDA(cudaStreamSynchronize(st));
-  check_bulk_error(op, st);  // a tuned bulk-copy step reports a wait that gave up
+  check_bulk_error(op, st);  // a bulk-copy step reports a wait that gave up
 }
 
 }  // namespace

@@ -33,6 +33,14 @@ constexpr int kThreads = 256;
 
 // ---- L2-only vector loads for the blocks written during the launch
 template <typename T, int V>
+struct Vec;
+template <> struct Vec<double, 1> { using type = double; };
+template <> struct Vec<double, 2> { using type = double2; };
+template <> struct Vec<float, 1> { using type = float; };
+template <> struct Vec<float, 2> { using type = float2; };
+template <> struct Vec<float, 4> { using type = float4; };
+
+template <typename T, int V>
 __device__ __forceinline__ void ldcg1(const T *p, T *f) {
   using VT = typename Vec<T, V>::type;
   const VT x = __ldcg(reinterpret_cast<const VT *>(p));

@@ -97,13 +97,13 @@ int grid_of(int64_t total) {
 
 // Y = q(A_hat) Q where column j of the n x b blocks (ld = b) runs its own polynomial with
 // coefficients coef[m * b + j], m = 0..K (row-major (K+1) x b table, FP32 or FP64 like
-// the blocks).  colseg is the identity map 0..b-1 on the device; B1, B2, TMP (and AX for
-// operators without a fused step) are n x b work blocks.  The recurrence starts from zero
+// the blocks).  B1, B2, TMP (and AX for operators without a fused step) are n x b work
+// blocks.  The recurrence starts from zero
 // blocks, so its first product multiplies zeros (one extra step out of K+1).
 template <typename T>
 FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int64_t K,
-                          double smin, double smax, const T *Q, T *Y, int64_t b,
-                          const int *colseg, T *B1, T *B2, T *TMP, T *AX) {
+                          double smin, double smax, const T *Q, T *Y, int64_t b, T *B1, T *B2,
+                          T *TMP, T *AX) {
   FilterCount fc;
   const int64_t n = op->n;
   require(op->kind != OP_MATBLOCK, SMA_ERR_ARG, "the per-column filter needs a device operator");
@@ -113,9 +113,9 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
   SMA_CUDA(cudaMemsetAsync(B1, 0, bytes, st));
   SMA_CUDA(cudaMemsetAsync(B2, 0, bytes, st));
   const bool fused = op->kind == OP_CSR;
-  auto step = [&](const T *crow, T *out, double al, double be) {
+  auto step = [&](const T *crow, T *out, double al, double be, bool rev) {
     if (fused) {
-      csr_clenshaw_step_seg<T>(op, st, b, Q, b, B1, B2, b, out, b, crow, colseg, al, be, true);
+      csr_clenshaw_step_seg<T>(op, st, b, Q, b, B1, B2, b, out, b, crow, nullptr, al, be, rev);
     } else {
       if (op->kind == OP_CSR_HALF)
         half_product<T>(op, st, B1, b, AX, b, b);
@@ -129,13 +129,13 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
   const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   const double blk = (double)n * (double)b * sizeof(T);
   for (int64_t k = K; k >= 1; --k) {
-    step(coef + k * b, TMP, alpha, beta);
+    step(coef + k * b, TMP, alpha, beta, k & 1);
     T *t = B2;  // B1, B2, TMP = TMP, B1, B2
     B2 = B1;
     B1 = TMP;
     TMP = t;
   }
-  step(coef, Y, invd, -(c * invd));
+  step(coef, Y, invd, -(c * invd), false);
   check_bulk_error(op, st);
   fc.steps = K + 1;
   fc.bytes = (double)(K + 1) * (mat_bytes + 4 * blk);
@@ -144,10 +144,10 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
 
 template FilterCount percol_filter<float>(const sma_op *, cudaStream_t, const float *, int64_t,
                                           double, double, const float *, float *, int64_t,
-                                          const int *, float *, float *, float *, float *);
+                                          float *, float *, float *, float *);
 template FilterCount percol_filter<double>(const sma_op *, cudaStream_t, const double *, int64_t,
                                            double, double, const double *, double *, int64_t,
-                                           const int *, double *, double *, double *, double *);
+                                           double *, double *, double *, double *);
 
 // Coefficients e_0..e_{K-1} of q_t (p's divided difference at t) and p(t), from the
 // Clenshaw intermediates of p at t.
@@ -214,13 +214,7 @@ PolishOut polish_mixed(const sma_op *op, const PolishCoeffs &coeffs_of, int64_t 
     coef32.alloc(Kmax * kap, st);
     if (op->kind != OP_CSR) AX32.alloc(n * kap, st);
   };
-  DevBuf<int> colseg(kpad, st), act_d(kpad, st), slot_d(k, st);
-  {
-    std::vector<int> idn(kpad);
-    for (int64_t j = 0; j < kpad; ++j) idn[j] = (int)j;
-    SMA_CUDA(cudaMemcpyAsync(colseg.p, idn.data(), kpad * sizeof(int), cudaMemcpyHostToDevice, st));
-    SMA_CUDA(cudaStreamSynchronize(st));
-  }
+  DevBuf<int> act_d(kpad, st), slot_d(k, st);
   // Rayleigh-Ritz with A on span(V) (V n x k, orthonormalized in place): X = V E,
   // out.lam/out.res its Ritz values (ascending) and residual norms.
   auto rayleigh_ritz = [&](double *V) {
@@ -353,7 +347,7 @@ PolishOut polish_mixed(const sma_op *op, const PolishCoeffs &coeffs_of, int64_t 
                                                            theta_d.p, inv_s_d.p, R32.p);
     SMA_CHECK_LAUNCH();
     const FilterCount f = percol_filter<float>(op, st, coef32.p, K - 1, smin, smax, R32.p, Z32.p,
-                                               kapad, colseg.p, B1.p, B2.p, TMP.p, AX32.p);
+                                               kapad, B1.p, B2.p, TMP.p, AX32.p);
     fc.steps += f.steps;
     fc.bytes += f.bytes;
     combine_kernel<<<grid_of(n * k), 256, 0, st>>>(n, k, X, k, Z32.p, kapad, slot_d.p, pt_d.p,

@@ -9,9 +9,9 @@
 // The three recurrence blocks start zeroed, which makes a joining window's first step
 // exactly its B1 = c_K Q and its second step exactly the one without B2: every window's
 // filtered block is bit-identical to the single-window filter of filter.cu, while the
-// sparse matrix is read once per index for all windows.  After one eager call (during
-// which the kernel autotuner measures the widths it meets) the whole recurrence is
-// recorded into a CUDA graph and replayed for as long as the set of windows is unchanged.
+// sparse matrix is read once per index for all windows.  After one eager call the whole
+// recurrence is recorded into a CUDA graph and replayed for as long as the set of windows is
+// unchanged.
 #pragma once
 
 #include "solver_common.h"
@@ -93,22 +93,17 @@ struct SliceBatch {
   // One step at index k over the first b columns.  One segment: the unsegmented step with
   // the scalar c_k (the same arithmetic on the same values -- (T) c_k either way -- without
   // the per-column coefficient lookups); several: the segmented step.
-  void step(int64_t k, int64_t b, const T *B1, const T *B2, T *out, double al, double be,
-            bool tuned) {
+  void step(int64_t k, int64_t b, const T *B1, const T *B2, T *out, double al, double be) {
     const int64_t nseg = (int64_t)wins.size();
-    if (nseg == 1) {
-      if (tuned)
-        csr_clenshaw_step<T>(op, st, b, q.p, W, B1, B2, W, out, W, coef1[k], al, be, true);
-      else
-        csr_clenshaw_step_untuned<T>(op, st, b, q.p, W, B1, B2, W, out, W, coef1[k], al, be, true);
-      return;
-    }
+    if (nseg == 1)
+      return csr_clenshaw_step<T>(op, st, b, q.p, W, B1, B2, W, out, W, coef1[k], al, be, true,
+                                  k & 1);
     csr_clenshaw_step_seg<T>(op, st, b, q.p, W, B1, B2, W, out, W, coef.p + k * nseg, colseg.p,
-                             al, be, tuned);
+                             al, be, k & 1);
   }
 
-  // The whole recurrence on q -> y.  tuned = false for graph recording.
-  void record(bool tuned) {
+  // The whole recurrence on q -> y.
+  void record() {
     const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
     const double alpha = 2.0 * invd, beta = -2.0 * c * invd;
     const size_t bytes = (size_t)(n * W) * sizeof(T);
@@ -117,13 +112,13 @@ struct SliceBatch {
     SMA_CUDA(cudaMemsetAsync(tmp.p, 0, bytes, st));
     T *B1 = b1.p, *B2 = b2.p, *TMP = tmp.p;
     for (int64_t k = Kmax; k >= 1; --k) {
-      step(k, active[k], B1, B2, TMP, alpha, beta, tuned);
+      step(k, active[k], B1, B2, TMP, alpha, beta);
       T *t = B2;
       B2 = B1;
       B1 = TMP;
       TMP = t;
     }
-    step(0, W, B1, B2, y.p, invd, -(c * invd), tuned);
+    step(0, W, B1, B2, y.p, invd, -(c * invd));
   }
 
   // Algorithmic bytes of one batched filter: every step reads the matrix once and Q, B1,
@@ -145,7 +140,7 @@ struct SliceBatch {
       const int64_t l0 = g_kernel_launches.load();
       SMA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
-        record(false);
+        record();
       } catch (...) {
         cudaGraph_t g = nullptr;
         cudaStreamEndCapture(st, &g);
@@ -162,7 +157,7 @@ struct SliceBatch {
       g_kernel_launches.fetch_add(recorded_launches);
       return 1;
     }
-    record(true);
+    record();
     return 0;
   }
 };

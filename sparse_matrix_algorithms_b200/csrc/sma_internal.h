@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
+#include <array>
 #include <atomic>
 #include <functional>
 #include <cstdint>
@@ -66,21 +67,17 @@ inline void require(bool ok, int code, const std::string &msg) {
   if (!ok) throw Error(code, msg);
 }
 
-// Online autotuner state of the CSR Clenshaw step for one (element type, vector width,
-// variant, block width, leading dimension) key of an operator (csr_clenshaw.cuh).
+// Timed launches of the CSR step for one (type and vector width, variant, width) of an operator
+// (the tuning table of csr_clenshaw.cuh).
 struct CsrTune {
-  std::vector<int> cands;           // encoded candidate configurations
-  std::vector<int> trial;           // configuration of each timed launch so far
-  std::vector<cudaEvent_t> events;  // start/stop event pair per timed launch
-  int round = 0;                    // 0: every candidate twice; 1: the four best again
-  int chosen = -1;                  // encoded winner once decided
+  std::vector<cudaEvent_t> events;  // start and stop of each timed launch so far
+  int chosen = -1;                  // the configuration kept once all have been timed
   CsrTune() = default;
   CsrTune(const CsrTune &) = delete;
   CsrTune &operator=(const CsrTune &) = delete;
   void release() {
     for (cudaEvent_t e : events) cudaEventDestroy(e);
     events.clear();
-    trial.clear();
   }
   ~CsrTune() { release(); }
 };
@@ -94,7 +91,7 @@ struct sma_ctx {
   cublasHandle_t cublas = nullptr;
   cusolverDnHandle_t cusolver = nullptr;
   int num_sms = 148;
-  bool autotune = true;  // SMA_AUTOTUNE=0 in the environment turns the kernel autotuner off
+  bool tune = false;  // SMA_AUTOTUNE_VERBOSE=1 and SMA_AUTOTUNE not 0: time the CSR step's kernels
   // SMA_FILTER_GRAPHS=0 turns off the CUDA-graph replay of repeated filters (filter.cu)
   bool filter_graphs = true;
   // SMA_PERSISTENT=1: CSR filters run as one persistent cooperative launch (persistent.cu)
@@ -136,11 +133,10 @@ struct sma_op {
   // caller callback
   sma_matblock_fn fn = nullptr;
   void *user = nullptr;
-  // autotuned CSR kernel configurations
-  std::map<uint64_t, sma::CsrTune> tuned;
-  // BULK family of the CSR step (csr_clenshaw.cuh): the most CSR entries any CTA of RC rows
-  // holds, per RC (from a host copy of the row pointers), and the device flag its bounded
-  // wait sets when it gives up
+  // the tuning table of the CSR step; for its BULK family the most CSR entries any CTA of RC rows
+  // holds, per RC (from a host copy of the row pointers), and the device flag its bounded wait
+  // sets when it gives up
+  std::map<std::array<int64_t, 3>, sma::CsrTune> tuned;
   std::map<int, int> bulk_pairs;
   std::vector<int> host_rowptr;
   int *bulk_err = nullptr;
@@ -190,31 +186,26 @@ struct Block {
 
 // ------------------------------------------------------------------ kernels (kernels.cu)
 // out = ck*Q + alpha*(A*B1) + beta*B1 - B2 over b columns (one Clenshaw step).
-// Q may be null (ck ignored), B2 may be null, has_self=false drops the beta*B1 term.
+// Q may be null (ck ignored), B2 may be null, has_self=false drops the beta*B1 term.  rev: the
+// rows are walked from the last to the first; a recurrence alternates it from step to step.
 template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                          double alpha, double beta, bool has_self);
+                          double alpha, double beta, bool has_self, bool rev = false);
 // The CSR form of launch_clenshaw_step (csr_clenshaw_f64.cu / csr_clenshaw_f32.cu).
 template <typename T>
 void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                        const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                       double alpha, double beta, bool has_self);
+                       double alpha, double beta, bool has_self, bool rev);
 // Throws SMA_ERR_TIMEOUT (and clears the flag) when a BULK-family launch of the CSR step on
 // this operator gave up its bounded wait; synchronizes the stream when the family was used.
 void check_bulk_error(const sma_op *op, cudaStream_t st);
-// The CSR step without the autotuner (cached or default configuration, no events).
-template <typename T>
-void csr_clenshaw_step_untuned(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
-                               int64_t ldq, const T *B1, const T *B2, int64_t ldb, T *out,
-                               int64_t ldo, double ck, double alpha, double beta, bool has_self);
-// The segmented CSR step (batched slicing, the POLFED polish): column c uses the
-// coefficient cseg[colseg[c]] (csr_clenshaw.cuh).
+// The segmented CSR step (batched slicing, the POLFED polish): column c uses the coefficient
+// cseg[colseg[c]] (colseg nondecreasing), or cseg[c] when colseg is null (csr_clenshaw.cuh).
 template <typename T>
 void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
-                           const T *cseg, const int *colseg, double alpha, double beta,
-                           bool tuned);
+                           const T *cseg, const int *colseg, double alpha, double beta, bool rev);
 // out = ck * Q
 template <typename T>
 void launch_scale_block(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq, T *out,
@@ -387,11 +378,11 @@ int64_t orthonormalize(sma_ctx *ctx, int64_t n, int64_t k, double *X, int64_t ld
 
 // ------------------------------------------------------------------ polish (polish.cu)
 // Y = q(A_hat) Q with a polynomial per column: coef[m * b + j] is coefficient m of column
-// j (m = 0..K), blocks n x b row-major with ld = b, colseg the identity map on the device.
+// j (m = 0..K), blocks n x b row-major with ld = b.
 template <typename T>
 FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int64_t K,
-                          double smin, double smax, const T *Q, T *Y, int64_t b,
-                          const int *colseg, T *B1, T *B2, T *TMP, T *AX);
+                          double smin, double smax, const T *Q, T *Y, int64_t b, T *B1, T *B2,
+                          T *TMP, T *AX);
 // e[0..K-1]: Chebyshev coefficients of (p(s) - p(t)) / (s - t) for p = sum c_m T_m; *pt = p(t).
 void divided_difference(const std::vector<double> &c, double t, double *e, double *pt);
 struct PolishOut {

@@ -1,64 +1,85 @@
-// Vector loads/stores of V consecutive elements (V*sizeof(T) <= 32 bytes, issued as one
-// or two accesses of at most 16 bytes).  Read-only data goes through the non-coherent
-// path (__ldg); it is written only by earlier kernel launches.
+// Vector loads/stores of V consecutive elements, V*sizeof(T) = 4..32 bytes, each ONE access:
+// a 32-byte vector is a 256-bit load or store (sm_100), so that a warp's request covers whole
+// 128-byte lines -- two 16-byte halves at a 32-byte stride touch every line twice.  Read-only
+// data goes through the non-coherent path; it is written only by earlier kernel launches.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 namespace sma {
 
-template <typename T, int V>
-struct Vec;
-template <> struct Vec<double, 1> { using type = double; };
-template <> struct Vec<double, 2> { using type = double2; };
-template <> struct Vec<float, 1> { using type = float; };
-template <> struct Vec<float, 2> { using type = float2; };
-template <> struct Vec<float, 4> { using type = float4; };
-
-template <typename T, int V>
-__device__ __forceinline__ void ldv1(const T *__restrict__ p, T *f) {
-  using VT = typename Vec<T, V>::type;
-  const VT x = __ldg(reinterpret_cast<const VT *>(p));
-  if constexpr (V == 1) {
-    f[0] = x;
-  } else if constexpr (V == 2) {
-    f[0] = x.x; f[1] = x.y;
+// KEEP = false: the line is not kept in L1 (rows that one thread reads once)
+template <bool KEEP, int BYTES>
+__device__ __forceinline__ void ld_words(const void *p, unsigned (&w)[BYTES / 4]) {
+  static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16 || BYTES == 32, "vector width");
+  if constexpr (BYTES == 32) {
+    if constexpr (KEEP)
+      asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+            "=r"(w[7])
+          : "l"(p));
+    else
+      asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+            "=r"(w[7])
+          : "l"(p));
+  } else if constexpr (BYTES == 16) {
+    if constexpr (KEEP)
+      asm("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];"
+          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p));
+    else
+      asm("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
+          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p));
+  } else if constexpr (BYTES == 8) {
+    if constexpr (KEEP) asm("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
+    else
+      asm("ld.global.nc.L1::no_allocate.v2.b32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
   } else {
-    f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
+    if constexpr (KEEP) asm("ld.global.nc.b32 %0, [%1];" : "=r"(w[0]) : "l"(p));
+    else asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(w[0]) : "l"(p));
   }
 }
 
-template <typename T, int V>
-__device__ __forceinline__ void stv1(T *__restrict__ p, const T *f) {
-  using VT = typename Vec<T, V>::type;
-  VT x;
-  if constexpr (V == 1) {
-    x = f[0];
-  } else if constexpr (V == 2) {
-    x.x = f[0]; x.y = f[1];
-  } else {
-    x.x = f[0]; x.y = f[1]; x.z = f[2]; x.w = f[3];
-  }
-  *reinterpret_cast<VT *>(p) = x;
-}
-
-template <typename T, int V>
+template <typename T, int V, bool KEEP = true>
 __device__ __forceinline__ void ldv(const T *__restrict__ p, T (&f)[V]) {
-  constexpr int kPer = (V * (int)sizeof(T) <= 16) ? V : 16 / (int)sizeof(T);
-#pragma unroll
-  for (int k = 0; k < V / kPer; ++k) ldv1<T, kPer>(p + k * kPer, f + k * kPer);
+  unsigned w[V * sizeof(T) / 4];
+  ld_words<KEEP, V * (int)sizeof(T)>(p, w);
+  memcpy(f, w, sizeof(w));
 }
 
 template <typename T, int V>
 __device__ __forceinline__ void stv(T *__restrict__ p, const T (&f)[V]) {
-  constexpr int kPer = (V * (int)sizeof(T) <= 16) ? V : 16 / (int)sizeof(T);
-#pragma unroll
-  for (int k = 0; k < V / kPer; ++k) stv1<T, kPer>(p + k * kPer, f + k * kPer);
+  constexpr int kBytes = V * (int)sizeof(T);
+  unsigned w[kBytes / 4];
+  memcpy(w, f, sizeof(w));
+  if constexpr (kBytes == 32)
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  else if constexpr (kBytes == 16)
+    asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(w[0]), "r"(w[1]),
+                 "r"(w[2]), "r"(w[3]) : "memory");
+  else if constexpr (kBytes == 8)
+    asm volatile("st.global.v2.b32 [%0], {%1, %2};" ::"l"(p), "r"(w[0]), "r"(w[1]) : "memory");
+  else
+    asm volatile("st.global.b32 [%0], %1;" ::"l"(p), "r"(w[0]) : "memory");
 }
 
-}  // namespace sma
+// Brings the line into L2 without holding a register for it.
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 
-namespace sma {
+// Programmatic dependent launch: wait until the grids this one depends on have completed and
+// their writes are visible; let the next grid in the stream be scheduled.  The second always
+// comes AFTER the first: a grid then starts while its predecessor runs, but never while its
+// predecessor's predecessor still does, so no cache line that an older step read into L1 can
+// outlive the write that replaced it.  Launched without the attribute both are no-ops.
+__device__ __forceinline__ void pdl_wait_then_trigger() {
+  asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // Round-to-nearest products and sums that the compiler never contracts into FMAs.
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
