@@ -331,46 +331,72 @@ __global__ void randn_kernel(int64_t n, int64_t m, uint64_t seed, double *__rest
 }
 
 // ------------------------------------------------------------------ column reductions
-__global__ void colred_stage1(int mode, int64_t n, int64_t k, const double *__restrict__ X,
-                              int64_t ldx, const double *__restrict__ Y, int64_t ldy,
-                              const double *__restrict__ lam, double *__restrict__ partial,
-                              int64_t rows_per_chunk) {
-  __shared__ double sh[8][33];
-  const int cl = threadIdx.x % 32, rl = threadIdx.x / 32;
-  const int64_t col = (int64_t)blockIdx.y * 32 + cl;
+// Stage 1: a CTA sums one chunk of rows of up to 32 columns.  The 2^lc threads of a row group
+// sit on consecutive columns, so that narrow blocks (k = 16 of the KPM vectors) still use every
+// lane; 256 >> lc rows are in flight per pass.  mode 2 forms sum X Y and, `plane` further on, sum
+// Y Y from one read of both blocks.
+__global__ void __launch_bounds__(256)
+colred_stage1(int mode, int lc, int64_t n, int64_t k, const double *__restrict__ X, int64_t ldx,
+              const double *__restrict__ Y, int64_t ldy, const double *__restrict__ lam,
+              double *__restrict__ partial, int64_t rows_per_chunk, int64_t plane) {
+  __shared__ double sh[2][256];
+  const int tid = threadIdx.x, cl = tid & ((1 << lc) - 1), rl = tid >> lc, R = 256 >> lc;
+  const int64_t col = ((int64_t)blockIdx.y << lc) + cl;
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_chunk;
   const int64_t r1 = min(n, r0 + rows_per_chunk);
-  double s = 0.0;
+  double s = 0.0, s2 = 0.0;
   if (col < k) {
     const double l = mode == 1 ? lam[col] : 0.0;
-    for (int64_t i = r0 + rl; i < r1; i += 8) {
+#pragma unroll 4
+    for (int64_t i = r0 + rl; i < r1; i += R) {
       const double x = X[i * ldx + col];
       const double y = Y[i * ldy + col];
-      if (mode == 0) {
-        s = fma(x, y, s);
-      } else {
+      if (mode == 1) {
         const double d = y - l * x;
         s = fma(d, d, s);
+      } else {
+        s = fma(x, y, s);
+        s2 = fma(y, y, s2);
       }
     }
   }
-  sh[rl][cl] = s;
-  __syncthreads();
+  sh[0][tid] = s;
+  sh[1][tid] = s2;
+  for (int h = 128; h >= 1 << lc; h >>= 1) {
+    __syncthreads();
+    if (tid < h) {
+      sh[0][tid] += sh[0][tid + h];
+      sh[1][tid] += sh[1][tid + h];
+    }
+  }
   if (rl == 0 && col < k) {
-    double t = 0.0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) t += sh[r][cl];
-    partial[(int64_t)blockIdx.x * k + col] = t;
+    partial[(int64_t)blockIdx.x * k + col] = sh[0][tid];
+    if (mode == 2) partial[plane + (int64_t)blockIdx.x * k + col] = sh[1][tid];
   }
 }
 
-__global__ void colred_stage2(int mode, int64_t chunks, int64_t k, const double *__restrict__ partial,
-                              double *__restrict__ out) {
-  for (int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; col < k;
-       col += (int64_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (int64_t c = 0; c < chunks; ++c) t += partial[c * k + col];
-    out[col] = mode == 1 ? sqrt(t) : t;
+// Stage 2: out[g k + col] = the sum over the chunks of group g (groups of chunks x k partials one
+// after the other), eight row groups of a CTA sharing the chunks: a serial sum of the 1184
+// partials of a KPM reduction took 80 of its 90 us.
+__global__ void __launch_bounds__(256)
+colred_stage2(int mode, int64_t chunks, int64_t k, int64_t total, const double *__restrict__ partial,
+              double *__restrict__ out) {
+  __shared__ double sh[8][33];
+  const int cl = threadIdx.x % 32, rl = threadIdx.x / 32;
+  const int64_t e = (int64_t)blockIdx.x * 32 + cl;
+  double t = 0.0;
+  if (e < total) {
+    const double *p = partial + (e / k) * chunks * k + e % k;
+#pragma unroll 4
+    for (int64_t c = rl; c < chunks; c += 8) t += p[c * k];
+  }
+  sh[rl][cl] = t;
+  __syncthreads();
+  if (rl == 0 && e < total) {
+    t = 0.0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) t += sh[r][cl];
+    out[e] = mode == 1 ? sqrt(t) : t;
   }
 }
 
@@ -612,21 +638,40 @@ void launch_randn(cudaStream_t st, int64_t n, int64_t m, uint64_t seed, double *
   SMA_CHECK_LAUNCH();
 }
 
+void column_partials(cudaStream_t st, int mode, int64_t n, int64_t k, const double *X, int64_t ldx,
+                     const double *Y, int64_t ldy, const double *lam, double *partial) {
+  int lc = 0;
+  while (lc < 5 && (1 << lc) < k) ++lc;
+  const int64_t ctiles = (k + (1 << lc) - 1) >> lc;
+  const int64_t chunks = column_chunks(n, k);
+  const dim3 grid((unsigned)chunks, (unsigned)ctiles);
+  colred_stage1<<<grid, 256, 0, st>>>(mode, lc, n, k, X, ldx, Y, ldy, lam, partial,
+                                      (n + chunks - 1) / chunks, chunks * k);
+  SMA_CHECK_LAUNCH();
+}
+
+// Chunks of rows: four CTAs an SM over the whole grid, each thread summing at least eight rows.
+int64_t column_chunks(int64_t n, int64_t k) {
+  const int64_t ctiles = (k + 31) / 32;
+  const int64_t rows = k >= 32 ? 64 : 8 * (256 / std::max<int64_t>(k, 1));
+  return std::max<int64_t>(1, std::min<int64_t>((n + rows - 1) / rows, (148 * 4 + ctiles - 1) / ctiles));
+}
+
+void column_totals(cudaStream_t st, int mode, int64_t chunks, int64_t k, int64_t groups,
+                   const double *partial, double *out) {
+  const int64_t total = groups * k;
+  colred_stage2<<<(unsigned)((total + 31) / 32), 256, 0, st>>>(mode, chunks, k, total, partial, out);
+  SMA_CHECK_LAUNCH();
+}
+
 void column_reduce(cudaStream_t st, int mode, int64_t n, int64_t k, const double *X, int64_t ldx,
                    const double *Y, int64_t ldy, const double *lam, double *out,
                    DevBuf<double> &scratch) {
   if (k == 0) return;
-  const int64_t ctiles = (k + 31) / 32;
-  int64_t chunks = std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, (148 * 8 + ctiles - 1) / ctiles));
-  const int64_t rows_per_chunk = (n + chunks - 1) / chunks;
-  chunks = std::max<int64_t>(1, (n + rows_per_chunk - 1) / rows_per_chunk);
+  const int64_t chunks = column_chunks(n, k);
   if (scratch.count < (size_t)(chunks * k)) scratch.alloc(chunks * k, st);
-  dim3 grid((unsigned)chunks, (unsigned)ctiles);
-  colred_stage1<<<grid, 256, 0, st>>>(mode, n, k, X, ldx, Y, ldy, lam, scratch.p, rows_per_chunk);
-  SMA_CHECK_LAUNCH();
-  colred_stage2<<<(unsigned)std::max<int64_t>(1, (k + 255) / 256), 256, 0, st>>>(mode, chunks, k,
-                                                                                scratch.p, out);
-  SMA_CHECK_LAUNCH();
+  column_partials(st, mode, n, k, X, ldx, Y, ldy, lam, scratch.p);
+  column_totals(st, mode, chunks, k, 1, scratch.p, out);
 }
 
 static void transpose(cudaStream_t st, int64_t R, int64_t C, const double *in, int64_t ldi,

@@ -51,8 +51,13 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   require(M >= 1 && R >= 1, SMA_ERR_ARG, "need at least one moment and one vector");
   require(smax > smin, SMA_ERR_ARG, "need smin < smax");
   const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
-  DevBuf<double> t0(n * R, st), t1(n * R, st), t2(n * R, st), dots(2 * (M / 2 + 1) * R, st),
-      scratch;
+  // dots of one step: <T_{k+1}, T_k> and <T_k, T_k>, chunks x R partials each; the partials of
+  // `batch` steps are summed by one launch
+  const int64_t chunks = column_chunks(n, R), set = 2 * chunks * R;
+  const int64_t steps = (M + 1) / 2;
+  const int64_t batch = std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
+  DevBuf<double> t0(n * R, st), t1(n * R, st), t2(n * R, st), dots(2 * steps * R, st),
+      partial(batch * set, st);
   {
     const int64_t total = n * R;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
@@ -65,46 +70,47 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   const bool product_then_axpy = op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF;
   if (product_then_axpy) ax.alloc(n * R, st);
   auto step = [&](const double *Q, const double *B1, double *out, double ck, double alpha,
-                  double beta) {
+                  double beta, bool rev) {
     if (product_then_axpy) {
       op_apply(op, st, B1, R, ax.p, R, R);
       launch_clenshaw_axpy<double>(st, n, R, Q, R, ax.p, R, B1, nullptr, R, out, R, ck, alpha, beta);
     } else {
-      launch_clenshaw_step<double>(op, st, R, Q, R, B1, nullptr, R, out, R, ck, alpha, beta, true);
+      launch_clenshaw_step<double>(op, st, R, Q, R, B1, nullptr, R, out, R, ck, alpha, beta, true, rev);
     }
   };
-  // dots[2k] = <T_k, T_k>, dots[2k+1] = <T_{k+1}, T_k> (R values each)
-  double *Tprev = t0.p, *Tcur = t1.p, *Tnext = t2.p;
-  column_reduce(st, 0, n, R, t0.p, R, t0.p, R, nullptr, dots.p, scratch);  // <T0, T0>
-  if (M > 1) {
-    // T1 = A_hat T0 = invd A T0 - c invd T0 (Q term with coefficient 0)
-    step(t0.p, t0.p, Tcur, 0.0, invd, -c * invd);
-    column_reduce(st, 0, n, R, Tcur, R, t0.p, R, nullptr, dots.p + R, scratch);  // <T1, T0>
-  }
-  const int64_t kmax = (M - 1) / 2;  // need <T_k,T_k> for 2k <= M-1, <T_{k+1},T_k> for 2k+1 <= M-1
-  for (int64_t k = 1; k <= kmax; ++k) {
-    column_reduce(st, 0, n, R, Tcur, R, Tcur, R, nullptr, dots.p + 2 * k * R, scratch);
-    if (2 * k + 1 <= M - 1) {
-      // T_{k+1} = 2 invd A T_k - 2 c invd T_k - T_{k-1}
-      step(Tprev, Tcur, Tnext, -1.0, 2.0 * invd, -2.0 * c * invd);
-      column_reduce(st, 0, n, R, Tnext, R, Tcur, R, nullptr, dots.p + (2 * k + 1) * R, scratch);
-      double *t = Tprev;
-      Tprev = Tcur;
-      Tcur = Tnext;
-      Tnext = t;
+  // dots: for k = 0, 1, ...: <T_{k+1}, T_k> then <T_k, T_k> (R values each)
+  double *Tprev = t0.p, *Tcur = t0.p, *Tnext = t1.p, *Tfree = t2.p;
+  int64_t done = 0;
+  for (int64_t k = 0; k < steps; ++k) {
+    double *slot = partial.p + (k - done) * set;
+    if (2 * k + 1 < M) {
+      if (k == 0)  // T1 = A_hat T0 = invd A T0 - c invd T0 (Q term with coefficient 0)
+        step(Tcur, Tcur, Tnext, 0.0, invd, -c * invd, false);
+      else  // T_{k+1} = 2 invd A T_k - 2 c invd T_k - T_{k-1}
+        step(Tprev, Tcur, Tnext, -1.0, 2.0 * invd, -2.0 * c * invd, k & 1);
+      column_partials(st, 2, n, R, Tnext, R, Tcur, R, nullptr, slot);
+    } else {  // an odd M: the last moment needs <T_k, T_k> only
+      column_partials(st, 2, n, R, Tcur, R, Tcur, R, nullptr, slot);
     }
+    if (k + 1 - done == batch || k + 1 == steps) {
+      column_totals(st, 0, chunks, R, 2 * (k + 1 - done), partial.p, dots.p + 2 * done * R);
+      done = k + 1;
+    }
+    double *t = k == 0 ? Tfree : Tprev;
+    Tprev = Tcur;
+    Tcur = Tnext;
+    Tnext = t;
   }
-  std::vector<double> h((size_t)M * R);
-  SMA_CUDA(cudaMemcpyAsync(h.data(), dots.p, (size_t)M * R * sizeof(double),
-                           cudaMemcpyDeviceToHost, st));
+  std::vector<double> h((size_t)2 * steps * R);
+  SMA_CUDA(cudaMemcpyAsync(h.data(), dots.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   SMA_CUDA(cudaStreamSynchronize(st));
   std::vector<double> pv((size_t)M * R);
   for (int64_t j = 0; j < R; ++j) {
-    const double m0 = h[j], m1 = M > 1 ? h[R + j] : 0.0;
+    const double m0 = h[R + j], m1 = M > 1 ? h[j] : 0.0;
     pv[j] = m0;
     if (M > 1) pv[R + j] = m1;
     for (int64_t q = 2; q < M; ++q) {
-      const double dq = h[q * R + j];
+      const double dq = h[((q ^ 1) * R) + j];  // even: <T_k, T_k>, stored second
       pv[q * R + j] = 2.0 * dq - ((q % 2 == 0) ? m0 : m1);
     }
   }
