@@ -1,5 +1,5 @@
-// The fused CSR Clenshaw step (included by csr_clenshaw_f64.cu and csr_clenshaw_f32.cu, one
-// translation unit per element type).
+// The fused Clenshaw step of CSR matrices and of the matrix-free models (1D Laplacian, 3D
+// Anderson, XXZ chain), included by csr_clenshaw_f{64,32}.cu and model_clenshaw_f{64,32}.cu.
 //
 //   out[i, :] = ck*Q[i, :] + alpha * sum_j A[i,j] B1[j, :] + beta*B1[i, :] - B2[i, :]
 //
@@ -28,8 +28,14 @@
 // it): a CTA reads what no step writes -- its row pointers -- and starts the prefetch of its
 // row of Q, then waits for the previous grid before it touches B1 or B2 or writes anything.
 //
+// A model's CTA first writes the columns of its rows to shared memory, one thread per entry (the
+// work of a whole row in each of its threads -- divisions, a sorting network, 64-80 registers --
+// made the Anderson step 2.4 times slower than the CSR one: 96 us at n = 110592, b = 64 FP64);
+// from there on it is a CSR matrix with one value on the diagonal and one off it.
+//
 // Every configuration accumulates with FMA in ascending column order -- the order of the
-// reference's CSC product on a symmetric matrix -- so all write bit-identical results.
+// reference's CSC product on a symmetric matrix -- so all write bit-identical results
+// (the XXZ model in its bond order).
 #pragma once
 
 #include <algorithm>
@@ -39,7 +45,7 @@
 #include "vec.cuh"
 
 namespace sma {
-namespace csr {
+namespace rows {
 
 constexpr int kThreads = 128;
 constexpr int kPanel = 64;  // vectors of a row in one panel
@@ -49,6 +55,9 @@ template <typename T>
 struct Step {
   const int *rowptr, *colind;
   const T *val;
+  sma_stencil model;  // the models' data, and the kind of operator they make up
+  int kind;
+  uint32_t entries;  // room for a model row's columns in shared memory
   const T *Q, *B1, *B2;
   T *out;
   const T *cseg;      // per-column coefficients (PC), else null
@@ -75,18 +84,35 @@ __device__ __forceinline__ uint64_t row_bytes(uint32_t row, uint64_t ld) {
   return (uint64_t)row * (uint32_t)ld;
 }
 
+// Where a row's entries come from.
+template <typename T>
+struct CsrRow {
+  const int *cols;
+  const T *vals;
+  __device__ __forceinline__ int col(int j) const { return __ldg(cols + j); }
+  __device__ __forceinline__ T val(int j) const { return __ldg(vals + j); }
+};
+template <typename T>
+struct ModelRow {  // entry `dpos` is the diagonal
+  const int *cols;
+  int dpos;
+  T diag, off;
+  __device__ __forceinline__ int col(int j) const { return cols[j]; }
+  __device__ __forceinline__ T val(int j) const { return j == dpos ? diag : off; }
+};
+
 // R consecutive entries from j: all R gathers are issued before the first FMA; FMAs in
 // ascending entry order.
-template <typename T, int V, int R, bool W>
-__device__ __forceinline__ void chunk(const Step<T> &a, int j, const T *B1c, T (&acc)[V]) {
+template <typename T, int V, int R, bool W, typename Row>
+__device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint64_t ldb, T (&acc)[V]) {
   int c[R];
   T x[R][V], v[R];
 #pragma unroll
-  for (int u = 0; u < R; ++u) c[u] = __ldg(a.colind + j + u);
+  for (int u = 0; u < R; ++u) c[u] = row.col(j + u);
 #pragma unroll
-  for (int u = 0; u < R; ++u) ldv<T, V>(at(B1c, row_bytes<W>((uint32_t)c[u], a.ldb)), x[u]);
+  for (int u = 0; u < R; ++u) ldv<T, V>(at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
 #pragma unroll
-  for (int u = 0; u < R; ++u) v[u] = __ldg(a.val + j + u);
+  for (int u = 0; u < R; ++u) v[u] = row.val(j + u);
 #pragma unroll
   for (int u = 0; u < R; ++u)
 #pragma unroll
@@ -95,20 +121,104 @@ __device__ __forceinline__ void chunk(const Step<T> &a, int j, const T *B1c, T (
 
 // acc += the row's entries [j, end): chunks of U, then the r < U remaining entries as ONE chunk
 // of exactly r (a switch over r).
-template <typename T, int V, int U, bool W>
-__device__ __forceinline__ void row_product(const Step<T> &a, int j, int end, const T *B1c,
-                                            T (&acc)[V]) {
-  for (; j + U <= end; j += U) chunk<T, V, U, W>(a, j, B1c, acc);
+template <typename T, int V, int U, bool W, typename Row>
+__device__ __forceinline__ void row_product(const Row &row, int j, int end, const T *B1c,
+                                            uint64_t ldb, T (&acc)[V]) {
+  for (; j + U <= end; j += U) chunk<T, V, U, W>(row, j, B1c, ldb, acc);
   switch (end - j) {
-    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(a, j, B1c, acc); break;
-    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(a, j, B1c, acc); break;
-    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(a, j, B1c, acc); break;
-    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(a, j, B1c, acc); break;
-    case 3: chunk<T, V, 3, W>(a, j, B1c, acc); break;
-    case 2: chunk<T, V, 2, W>(a, j, B1c, acc); break;
-    case 1: chunk<T, V, 1, W>(a, j, B1c, acc); break;
+    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(row, j, B1c, ldb, acc); break;
+    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(row, j, B1c, ldb, acc); break;
+    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(row, j, B1c, ldb, acc); break;
+    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(row, j, B1c, ldb, acc); break;
+    case 3: chunk<T, V, 3, W>(row, j, B1c, ldb, acc); break;
+    case 2: chunk<T, V, 2, W>(row, j, B1c, ldb, acc); break;
+    case 1: chunk<T, V, 1, W>(row, j, B1c, ldb, acc); break;
     default: break;
   }
+}
+
+// ------------------------------------------------------------------ the models' rows
+// Entry u of model row `row`: its place among the row's entries in accumulation order and its
+// column, or place -1 when the row has no such entry.
+struct Entry {
+  int place, col;
+};
+
+// tridiag(-1, 2, -1): u = 0, 1, 2 are the columns row - 1, row, row + 1, evaluated as the
+// reference's lap1d_matblock! (polfed.jl:1209-1219) -x[i-1] + 2 x[i] - x[i+1].
+__device__ __forceinline__ Entry lap1d_entry(uint32_t row, uint32_t n, int u) {
+  const int64_t col = (int64_t)row + u - 1;
+  if (col < 0 || col >= n) return {-1, 0};
+  return {row == 0 ? u - 1 : u, (int)col};
+}
+
+// 3D Anderson model on an L^3 periodic lattice, row i = x + L (y + L z): u = 0 is the diagonal,
+// 1..6 the neighbours x+-1, y+-1, z+-1 (distinct for L >= 3).  An entry's place is the number of
+// smaller columns: the order of the stored matrix's CSR row.
+__device__ __forceinline__ Entry anderson_entry(uint32_t row, uint32_t L, int u) {
+  const uint32_t l2 = L * L, z = row / l2, rem = row - z * l2, y = rem / L, x = rem - y * L;
+  const int r = (int)row, l = (int)L, ll = (int)l2;
+  const int c[7] = {r,
+                    x + 1 == L ? r - (l - 1) : r + 1,      x == 0 ? r + (l - 1) : r - 1,
+                    y + 1 == L ? r - (l - 1) * l : r + l,  y == 0 ? r + (l - 1) * l : r - l,
+                    z + 1 == L ? r - (l - 1) * ll : r + ll, z == 0 ? r + (l - 1) * ll : r - ll};
+  int mine = c[0], place = 0;
+#pragma unroll
+  for (int k = 1; k < 7; ++k) mine = k == u ? c[k] : mine;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) place += c[k] < mine;
+  return {place, mine};
+}
+
+// Random-field XXZ chain of length L in the Sz = 0 sector.  Row r is the basis state s =
+// states[r] (bit i = site i up); its index is its combinatorial rank sum_j C(p_j, j) over its set
+// bits p_1 < p_2 < ... .  u = 0 is the diagonal; u = i + 1 flips the antiparallel bond (i, i + 1),
+// which moves one set bit by one position and the rank by +-C(i, k), k the number of set bits
+// below i; u = L flips the periodic bond (L-1, 0) and ranks the flipped state.  Places in bond
+// order.
+__device__ __forceinline__ Entry xxz_entry(uint32_t row, const sma_stencil &m, int u) {
+  if (u == 0) return {0, (int)row};
+  const unsigned s = __ldg(m.states + row);
+  const int i = u - 1;
+  const unsigned flips = s ^ (s >> 1);  // bit i: bond (i, i + 1) is antiparallel, i < L - 1
+  const unsigned below = (1u << i) - 1u;
+  const int place = 1 + __popc(flips & below);
+  if (u < m.L) {
+    if (!((flips >> i) & 1u)) return {-1, 0};
+    const int d = __ldg(m.binom + i * 17 + __popc(s & below));
+    return {place, (s >> i) & 1u ? (int)row + d : (int)row - d};
+  }
+  if (!(((s >> (m.L - 1)) ^ s) & 1u)) return {-1, 0};
+  unsigned t = s ^ (1u | (1u << (m.L - 1)));
+  int col = 0;
+  for (int j = 1; t; ++j) {
+    col += __ldg(m.binom + (__ffs(t) - 1) * 17 + j);
+    t &= t - 1;
+  }
+  return {place, col};
+}
+
+// The columns of the CTA's rows [row0, row0 + rows) into cols (a.entries each), their number into
+// cnt and the place of the diagonal into dpos: one thread per entry.
+template <typename T>
+__device__ __forceinline__ void model_rows(const Step<T> &a, uint32_t row0, int *cols, int *cnt,
+                                           int *dpos) {
+  const sma_stencil &m = a.model;
+  if (threadIdx.x < a.rows) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < a.rows * a.entries; e += kThreads) {
+    const uint32_t r = e / a.entries, row = row0 + r;
+    const int u = (int)(e - r * a.entries);
+    if (row >= a.n) continue;
+    const Entry x = a.kind == OP_LAP1D      ? lap1d_entry(row, a.n, u)
+                    : a.kind == OP_ANDERSON ? anderson_entry(row, (uint32_t)m.L, u)
+                                            : xxz_entry(row, m, u);
+    if (x.place < 0) continue;
+    cols[r * a.entries + x.place] = x.col;
+    if (x.col == (int)row) dpos[r] = x.place;
+    atomicAdd(cnt + r, 1);
+  }
+  __syncthreads();
 }
 
 // The Q coefficients of the thread's V columns.
@@ -129,8 +239,9 @@ __device__ __forceinline__ void coefficients(const Step<T> &a, uint32_t c0, T (&
 }
 
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W>
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
+  extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const uint32_t r = threadIdx.x * a.divlanes >> 16;
@@ -139,10 +250,14 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   const bool in = r < a.rows && row < a.n && c0 < a.b;
   int start = 0, end = 0;
   if (in) {
-    start = __ldg(a.rowptr + row);
-    end = __ldg(a.rowptr + row + 1);
+    if constexpr (!MODEL) {
+      start = __ldg(a.rowptr + row);
+      end = __ldg(a.rowptr + row + 1);
+    }
     if constexpr (HQ) prefetch_l2(at(a.Q + c0, row * a.ldq));
   }
+  int *cnt = model_smem + a.rows * a.entries, *dpos = cnt + a.rows;
+  if constexpr (MODEL) model_rows(a, bx * a.rows, model_smem, cnt, dpos);
   pdl_wait_then_trigger();
   if (!in) return;
   const uint64_t own = row * a.ldb;
@@ -150,7 +265,13 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   T acc[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = T(0);
-  row_product<T, V, U, W>(a, start, end, a.B1 + c0, acc);
+  if constexpr (MODEL) {
+    const T diag = a.kind == OP_LAP1D ? T(2) : (T)__ldg(a.model.diag + row);
+    const ModelRow<T> mr{model_smem + r * a.entries, dpos[r], diag, (T)a.model.hop};
+    row_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
+  } else {
+    row_product<T, V, U, W>(CsrRow<T>{a.colind, a.val}, start, end, a.B1 + c0, a.ldb, acc);
+  }
   T q[V], s[V], t[V], ck[V], o[V];
   if constexpr (HQ) ldv<T, V, false>(at(a.Q + c0, row * a.ldq), q);
   if constexpr (HB) ldv<T, V, false>(at(a.B2 + c0, own), t);
@@ -162,31 +283,32 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   stv<T, V>(const_cast<T *>(at(a.out + c0, row * a.ldo)), o);
 }
 
-}  // namespace csr
+}  // namespace rows
 }  // namespace sma
 
 #include "csr_bulk.cuh"
 
 namespace sma {
-namespace csr {
+namespace rows {
 
 // ------------------------------------------------------------------ launch
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W>
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
+  if (MODEL) cfg.dynamicSmemBytes = a.rows * (a.entries + 2) * sizeof(int);  // 17.9 KB at most
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = op->ctx->pdl ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W>, a));
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL>, a));
   SMA_CHECK_LAUNCH();
 }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
   const uint32_t vecs = a.b / V;
   // as few panels as keep a row within kPanel vectors, each a multiple of 4 vectors (128 bytes)
@@ -214,8 +336,8 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
-    if (small) launch<T, V, 8, 8, HQ, HS, HB, PC, W>(op, st, a, grid);
-    else launch<T, V, 4, 12, HQ, HS, HB, PC, W>(op, st, a, grid);
+    if (small) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL>(op, st, a, grid);
+    else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL>(op, st, a, grid);
   }
 }
 
@@ -233,7 +355,7 @@ template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
 void launch_config(const sma_op *op, cudaStream_t st, const Step<T> &a, const Config &c) {
   if constexpr (!PC)
     if (c.bulk) return launch_bulk<T, V, HQ, HS, HB>(op, st, a);
-  launch_width<T, V, HQ, HS, HB, PC, false>(op, st, a, c.gathers);
+  launch_width<T, V, HQ, HS, HB, PC, false, false>(op, st, a, c.gathers);
 }
 
 template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
@@ -285,9 +407,11 @@ bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
   return true;
 }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
 void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
-  if (!tuned_step<T, V, HQ, HS, HB, PC>(op, st, a)) launch_width<T, V, HQ, HS, HB, PC, false>(op, st, a);
+  if constexpr (!MODEL)
+    if (tuned_step<T, V, HQ, HS, HB, PC>(op, st, a)) return;
+  launch_width<T, V, HQ, HS, HB, PC, false, MODEL>(op, st, a);
 }
 
 inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
@@ -295,14 +419,21 @@ inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) ==
 // Picks the vector width: the widest that widths, strides and addresses allow, but narrower
 // while the step would not give every SM a CTA (XXZ L = 14, b = 8 FP64: 4.4, 3.3 and 3.1 us a
 // step with 4, 2 and 1 columns a thread).
-template <typename T, bool HQ, bool HS, bool HB, bool PC>
+template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
   require(b < (int64_t)1 << 31, SMA_ERR_ARG, "block too wide");
-  if constexpr (sizeof(T) == 8) a.val = op->val64;
-  else a.val = op->val32;
-  a.rowptr = op->rowptr;
-  a.colind = op->colind;
+  if constexpr (MODEL) {
+    a.model = op->stencil;
+    a.kind = op->kind;
+    if (op->kind == OP_LAP1D) a.model.hop = -1.0;
+    a.entries = op->kind == OP_LAP1D ? 3 : op->kind == OP_ANDERSON ? 7 : (uint32_t)op->stencil.L + 1;
+  } else {
+    if constexpr (sizeof(T) == 8) a.val = op->val64;
+    else a.val = op->val32;
+    a.rowptr = op->rowptr;
+    a.colind = op->colind;
+  }
   a.n = (uint32_t)op->n;
   a.b = (uint32_t)b;
   auto fits = [&](int v) {
@@ -313,21 +444,21 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   };
   const int64_t want = (int64_t)op->ctx->num_sms * kThreads;
   auto take = [&](int v) { return fits(v) && op->n * (b / v) >= want; };
-  if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true>(op, st, a);
+  if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL>(op, st, a);
   if constexpr (sizeof(T) == 4)
-    if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC>(op, st, a);
-  if (take(4)) return launch_rule<T, 4, HQ, HS, HB, PC>(op, st, a);
-  if (take(2)) return launch_rule<T, 2, HQ, HS, HB, PC>(op, st, a);
-  launch_width<T, 1, HQ, HS, HB, PC, false>(op, st, a);
+    if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC, MODEL>(op, st, a);
+  if (take(4)) return launch_rule<T, 4, HQ, HS, HB, PC, MODEL>(op, st, a);
+  if (take(2)) return launch_rule<T, 2, HQ, HS, HB, PC, MODEL>(op, st, a);
+  launch_width<T, 1, HQ, HS, HB, PC, false, MODEL>(op, st, a);
 }
 
-}  // namespace csr
+}  // namespace rows
 
-template <typename T>
-void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
-                       const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                       double alpha, double beta, bool has_self, bool rev) {
-  csr::Step<T> a{};
+template <typename T, bool MODEL>
+void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                   const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
+                   double alpha, double beta, bool has_self, bool rev) {
+  rows::Step<T> a{};
   a.Q = Q;
   a.B1 = B1;
   a.B2 = B2;
@@ -339,31 +470,10 @@ void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
   a.alpha = (T)alpha;
   a.beta = (T)beta;
   a.rev = rev;
-  if (Q && has_self && B2) return csr::step<T, true, true, true, false>(op, st, b, a);
-  if (Q && has_self && !B2) return csr::step<T, true, true, false, false>(op, st, b, a);
-  if (!Q && !has_self && !B2) return csr::step<T, false, false, false, false>(op, st, b, a);
+  if (Q && has_self && B2) return rows::step<T, true, true, true, false, MODEL>(op, st, b, a);
+  if (Q && has_self && !B2) return rows::step<T, true, true, false, false, MODEL>(op, st, b, a);
+  if (!Q && !has_self && !B2) return rows::step<T, false, false, false, false, MODEL>(op, st, b, a);
   throw Error(SMA_ERR_INTERNAL, "unsupported Clenshaw step variant");
 }
 
-// The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
-// cseg[c] when colseg is null; Q, B1 and B2 are all read.
-template <typename T>
-void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
-                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
-                           const T *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  csr::Step<T> a{};
-  a.Q = Q;
-  a.B1 = B1;
-  a.B2 = B2;
-  a.out = out;
-  a.cseg = cseg;
-  a.colseg = colseg;
-  a.ldq = (uint64_t)ldq * sizeof(T);
-  a.ldb = (uint64_t)ldb * sizeof(T);
-  a.ldo = (uint64_t)ldo * sizeof(T);
-  a.alpha = (T)alpha;
-  a.beta = (T)beta;
-  a.rev = rev;
-  csr::step<T, true, true, true, true>(op, st, b, a);
-}
 }  // namespace sma

@@ -1,5 +1,5 @@
 // A second family of the fused CSR step, kept to measure the first against (the tuning table of
-// csr_clenshaw.cuh): whole neighbour rows staged in shared memory by 1D bulk copies.  Measured
+// clenshaw_step.cuh): whole neighbour rows staged in shared memory by 1D bulk copies.  Measured
 // 2 to 4 times slower (Anderson n = 262144, b = 64 FP32: 160-254 us a step): a row of 128-512
 // bytes is too small a copy for the copy engine.
 #pragma once
@@ -8,7 +8,7 @@
 #include "vec.cuh"
 
 namespace sma {
-namespace csr {
+namespace rows {
 
 // BULK family: a CTA of kBulkThreads threads owns RC = kBulkThreads / G rows (G threads of V
 // elements each cover a row in ONE pass, b = G V) and first stages everything its step
@@ -216,5 +216,5 @@ bool bulk_fits(const sma_op *op, const Step<T> &a) {
          200 * 1024;
 }
 
-}  // namespace csr
+}  // namespace rows
 }  // namespace sma

@@ -1,0 +1,14 @@
+// FP64 Clenshaw steps of the matrix-free models (clenshaw_step.cuh).
+#include "clenshaw_step.cuh"
+
+namespace sma {
+
+template <>
+void model_clenshaw_step<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q,
+                                 int64_t ldq, const double *B1, const double *B2, int64_t ldb,
+                                 double *out, int64_t ldo, double ck, double alpha, double beta,
+                                 bool has_self, bool rev) {
+  clenshaw_step<double, true>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
+}
+
+}  // namespace sma

@@ -4,7 +4,7 @@
 // blockIdx.x + gridDim.x, ...; between steps all CTAs meet at a grid barrier.  This removes
 // the per-step launch and the drain/fill of a kernel boundary, which dominate when a step
 // is short (a matrix and block that live in L2: the C2 configuration's steps take
-// ~17 us).  Each step computes exactly what the fused step kernel of csr_clenshaw.cuh
+// ~17 us).  Each step computes exactly what the fused step kernel of clenshaw_step.cuh
 // computes, with the same FMA order, so the results are bit-identical to the step-by-step
 // filter.
 //

@@ -5,7 +5,7 @@
 // windows sorted by filter degree (highest first).  The Clenshaw recurrence runs from the
 // highest degree down; window w's columns join at index K_w, so at every index the active
 // columns are a prefix of the block and one launch of the segmented CSR step
-// (csr_clenshaw.cuh) updates all of them, each column with its own window's coefficient.
+// (clenshaw_step.cuh) updates all of them, each column with its own window's coefficient.
 // The three recurrence blocks start zeroed, which makes a joining window's first step
 // exactly its B1 = c_K Q and its second step exactly the one without B2: every window's
 // filtered block is bit-identical to the single-window filter of filter.cu, while the

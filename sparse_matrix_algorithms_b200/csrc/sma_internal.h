@@ -68,7 +68,7 @@ inline void require(bool ok, int code, const std::string &msg) {
 }
 
 // Timed launches of the CSR step for one (type and vector width, variant, width) of an operator
-// (the tuning table of csr_clenshaw.cuh).
+// (the tuning table of clenshaw_step.cuh).
 struct CsrTune {
   std::vector<cudaEvent_t> events;  // start and stop of each timed launch so far
   int chosen = -1;                  // the configuration kept once all have been timed
@@ -192,7 +192,11 @@ template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
                           double alpha, double beta, bool has_self, bool rev = false);
-// The CSR form of launch_clenshaw_step (csr_clenshaw_f64.cu / csr_clenshaw_f32.cu).
+// The CSR and the model form of launch_clenshaw_step (csr_clenshaw_*.cu, model_clenshaw_*.cu).
+template <typename T>
+void model_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                         const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
+                         double alpha, double beta, bool has_self, bool rev);
 template <typename T>
 void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                        const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
@@ -201,7 +205,7 @@ void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
 // this operator gave up its bounded wait; synchronizes the stream when the family was used.
 void check_bulk_error(const sma_op *op, cudaStream_t st);
 // The segmented CSR step (batched slicing, the POLFED polish): column c uses the coefficient
-// cseg[colseg[c]] (colseg nondecreasing), or cseg[c] when colseg is null (csr_clenshaw.cuh).
+// cseg[colseg[c]] (colseg nondecreasing), or cseg[c] when colseg is null (clenshaw_step.cuh).
 template <typename T>
 void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
