@@ -33,6 +33,24 @@ void ClenshawWork<T>::ensure(const sma_op *op, int64_t n_, int64_t b, cudaStream
 }
 
 template <typename T>
+bool ClenshawWork<T>::fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t st) {
+  try {
+    ensure(op, n_, w, st);
+    if (!q.p) q.alloc(n * bcap, st);
+    return true;
+  } catch (const Error &e) {
+    if (e.code != SMA_ERR_NOMEM) throw;
+    cudaGetLastError();  // the failed allocation is not an error of a later launch
+    b1.release();
+    b2.release();
+    tmp.release();
+    q.release();
+    bcap = 0;
+    return false;
+  }
+}
+
+template <typename T>
 void ClenshawWork<T>::drop_graph() {
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
@@ -41,6 +59,25 @@ void ClenshawWork<T>::drop_graph() {
   g_op = nullptr;
   g_b = -1;
   g_calls = 0;
+}
+
+// The fused step runs on the widest vectors that divide the width.  An odd width leaves 8- or
+// 4-byte accesses, so the recurrence's own blocks (and a staged copy of Q) take the width of
+// least cost: columns times the time of a column relative to 32-byte vectors, measured as 1.18
+// with 16 bytes (FP32 n = 262144, b = 64: 49 against 42.5 us) and 1.6 with 8 (FP64 n = 27000,
+// b = 37: 10.3 us against 6.6 at b = 40); 4-byte accesses are put at 2.5.
+int64_t recurrence_width(int64_t b, int elem_bytes) {
+  const double cost[4] = {1.0, 1.18, 1.6, 2.5};  // 32, 16, 8 and 4 bytes
+  int64_t best = b;
+  double least = 0.0;
+  for (int k = 0, bytes = 32; bytes >= elem_bytes; bytes /= 2, ++k) {
+    const int64_t v = bytes / elem_bytes, w = (b + v - 1) / v * v;
+    if (k == 0 || (double)w * cost[k] < least) {
+      least = (double)w * cost[k];
+      best = w;
+    }
+  }
+  return best;
 }
 
 double clenshaw_step_bytes(const sma_op *op, int64_t b, int elem_bytes) {
@@ -91,11 +128,13 @@ static void matblock_apply(const sma_op *op, cudaStream_t st, const T *X, T *AX,
   }
 }
 
-// The launches of one filter (K >= 1); returns the step count and algorithmic bytes.
+// The launches of one filter (K >= 1) on recurrence blocks of width w >= b (w = b for operators
+// without a fused step; Q is read over w columns but by the last step); returns the step count
+// and algorithmic bytes.
 template <typename T>
 static FilterCount record_filter(const sma_op *op, cudaStream_t st,
                                  const std::vector<double> &coeffs, double smin, double smax,
-                                 const T *Q, int64_t ldq, T *Y, int64_t ldy, int64_t b,
+                                 const T *Q, int64_t ldq, T *Y, int64_t ldy, int64_t b, int64_t w,
                                  ClenshawWork<T> &work) {
   FilterCount fc;
   const int64_t n = op->n;
@@ -107,15 +146,15 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   const bool fused = op->kind != OP_MATBLOCK && op->kind != OP_CSR_HALF;
   const double blk = (double)n * (double)b * sizeof(T);
   T *B1 = work.b1.p, *B2 = work.b2.p, *TMP = work.tmp.p;
-  const int64_t ld = b;
+  const int64_t ld = w;
   // step K+1 of the reference: B1 = c_K Q (its product multiplies zeros)
-  launch_scale_block<T>(st, n, b, Q, ldq, B1, ld, coeffs[K]);
+  launch_scale_block<T>(st, n, w, Q, ldq, B1, ld, coeffs[K]);
   fc.bytes += 2 * blk;
   bool b2_zero = true;
   const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   for (int64_t ci = K - 1; ci >= 1; --ci) {
     if (fused) {
-      launch_clenshaw_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, TMP, ld,
+      launch_clenshaw_step<T>(op, st, w, Q, ldq, B1, b2_zero ? nullptr : B2, ld, TMP, ld,
                               coeffs[ci], alpha, beta, true, ci & 1);
     } else {
       matblock_apply<T>(op, st, B1, work.ax.p, ld, b);
@@ -146,6 +185,7 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
 
 // Filters of degree below this run eagerly (launch overhead is then not the question).
 constexpr int64_t kGraphMinDegree = 32;
+constexpr int64_t kPadMinDegree = 4;
 
 template <typename T>
 static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
@@ -162,16 +202,36 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     fc.bytes += 2.0 * (double)n * (double)b * sizeof(T);
     return fc;
   }
-  work.ensure(op, n, b, st);
-  if (op->kind == OP_CSR && op->ctx->persistent && K >= kGraphMinDegree) {
+  const bool fused = op->kind != OP_MATBLOCK && op->kind != OP_CSR_HALF;
+  const bool persistent = op->kind == OP_CSR && op->ctx->persistent && K >= kGraphMinDegree;
+  int64_t w = b;
+  bool stage = false;  // run on a copy of Q: half a step's time, for a gain with every step
+  if (fused && !persistent && K >= kPadMinDegree) {
+    w = recurrence_width(b, sizeof(T));
+    int64_t vec = 32;  // the access that w allows
+    while ((w * (int64_t)sizeof(T)) % vec) vec /= 2;
+    stage = w != b || (ldq * (int64_t)sizeof(T)) % vec || (uintptr_t)Q % vec;
+    if (stage && !work.fits(op, n, w, st)) {
+      w = b;
+      stage = false;
+    }
+  }
+  work.ensure(op, n, w, st);
+  if (persistent) {
     if (work.coef.count < (size_t)(K + 1)) work.coef.alloc(K + 1, st);
     if (!work.barrier.p) work.barrier.alloc(3, st);
     return persistent_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work.b1.p,
                                 work.b2.p, work.tmp.p, work.coef.p, work.barrier.p);
   }
-  if (op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF || K < kGraphMinDegree ||
-      !op->ctx->filter_graphs)
-    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work);
+  auto eager = [&]() {
+    if (stage) {  // zero columns stay zero through the recurrence
+      if (!work.q.p) work.q.alloc(n * work.bcap, st);
+      launch_pad_block<T, T>(st, n, b, Q, ldq, w, work.q.p, w);
+      return record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, Y, ldy, b, w, work);
+    }
+    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, w, work);
+  };
+  if (!fused || K < kGraphMinDegree || !op->ctx->filter_graphs) return eager();
   // repeated filter -> CUDA graph on the staging blocks
   const bool same = work.g_op == op && work.g_b == b && work.g_smin == smin &&
                     work.g_smax == smax && work.g_coeffs == coeffs;
@@ -184,18 +244,15 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     work.g_coeffs = coeffs;
   }
   work.g_calls += 1;
-  if (work.g_calls == 1)  // first call: eager, a graph pays from its second use
-    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work);
-  if (!work.q.p) {
-    work.q.alloc(n * work.bcap, st);
-    work.y.alloc(n * work.bcap, st);
-  }
-  launch_copy_block<T, T>(st, n, b, Q, ldq, work.q.p, b);
+  if (work.g_calls == 1) return eager();  // a graph pays from its second use
+  if (!work.q.p) work.q.alloc(n * work.bcap, st);
+  if (!work.y.p) work.y.alloc(n * work.bcap, st);
+  launch_pad_block<T, T>(st, n, b, Q, ldq, w, work.q.p, w);
   if (!work.exec) {
     const int64_t l0 = g_kernel_launches.load();
     SMA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
-      fc = record_filter<T>(op, st, coeffs, smin, smax, work.q.p, b, work.y.p, b, b, work);
+      fc = record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, work.y.p, w, w, w, work);
     } catch (...) {
       cudaGraph_t g = nullptr;
       cudaStreamEndCapture(st, &g);
@@ -216,7 +273,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
   SMA_CUDA(cudaGraphLaunch(work.exec, st));
   g_kernel_launches.fetch_add(work.g_launches);
   work.replays += 1;
-  launch_copy_block<T, T>(st, n, b, work.y.p, b, Y, ldy);
+  launch_copy_block<T, T>(st, n, b, work.y.p, w, Y, ldy);
   return fc;
 }
 

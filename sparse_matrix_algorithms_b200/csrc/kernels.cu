@@ -22,41 +22,42 @@ std::atomic<int64_t> g_kernel_launches{0};
 namespace {
 
 // ------------------------------------------------------------------ elementwise block ops
-template <typename T>
-__global__ void scale_block_kernel(int64_t n, int64_t b, const T *__restrict__ Q, int64_t ldq,
+// Element t of an n x b block is (t / b, t % b).  I: the index type; 32-bit divisions, where the
+// block allows them, are a quarter of the 64-bit ones that made these kernels slower than memory.
+template <typename T, typename I>
+__global__ void scale_block_kernel(I total, I b, const T *__restrict__ Q, int64_t ldq,
                                    T *__restrict__ out, int64_t ldo, T ck) {
-  const int64_t total = n * b;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / b, j = t % b;
-    out[i * ldo + j] = mul_rn(ck, Q[i * ldq + j]);
+  const I stride = (I)gridDim.x * blockDim.x;
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const I i = (I)t / b, j = (I)t - i * b;
+    out[(int64_t)i * ldo + j] = mul_rn(ck, Q[(int64_t)i * ldq + j]);
   }
 }
 
-template <typename T>
-__global__ void clenshaw_axpy_kernel(int64_t n, int64_t b, const T *__restrict__ Q, int64_t ldq,
+template <typename T, typename I>
+__global__ void clenshaw_axpy_kernel(I total, I b, const T *__restrict__ Q, int64_t ldq,
                                      const T *__restrict__ AX, int64_t ldax,
                                      const T *__restrict__ B1, const T *__restrict__ B2,
                                      int64_t ldb, T *__restrict__ out, int64_t ldo, T ck, T alpha,
                                      T beta) {
-  const int64_t total = n * b;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / b, j = t % b;
+  const I stride = (I)gridDim.x * blockDim.x;
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const I r = (I)t / b;
+    const int64_t i = r, j = (I)t - r * b;
     const T q = Q[i * ldq + j], a = AX[i * ldax + j], s = B1[i * ldb + j];
     out[i * ldo + j] = B2 ? clenshaw_combine<true, true, true>(a, q, s, B2[i * ldb + j], ck, alpha, beta)
                           : clenshaw_combine<true, true, false>(a, q, s, T(0), ck, alpha, beta);
   }
 }
 
-template <typename TS, typename TD>
-__global__ void copy_block_kernel(int64_t n, int64_t b, const TS *__restrict__ src, int64_t lds,
+// dst (n x w) <- src (n x b), w >= b, the columns past b zero
+template <typename TS, typename TD, typename I>
+__global__ void copy_block_kernel(I total, I w, I b, const TS *__restrict__ src, int64_t lds,
                                   TD *__restrict__ dst, int64_t ldd) {
-  const int64_t total = n * b;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / b, j = t % b;
-    dst[i * ldd + j] = (TD)src[i * lds + j];
+  const I stride = (I)gridDim.x * blockDim.x;
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const I i = (I)t / w, j = (I)t - i * w;
+    dst[(int64_t)i * ldd + j] = j < b ? (TD)src[(int64_t)i * lds + j] : TD(0);
   }
 }
 
@@ -333,8 +334,13 @@ void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T 
 template <typename T>
 void launch_scale_block(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq, T *out,
                         int64_t ldo, double ck) {
-  if (n * b == 0) return;
-  scale_block_kernel<T><<<grid_for(n * b), 256, 0, st>>>(n, b, Q, ldq, out, ldo, (T)ck);
+  const int64_t total = n * b;
+  if (total == 0) return;
+  if (total >> 32)
+    scale_block_kernel<T, uint64_t><<<grid_for(total), 256, 0, st>>>(total, b, Q, ldq, out, ldo, (T)ck);
+  else
+    scale_block_kernel<T, uint32_t><<<grid_for(total), 256, 0, st>>>((uint32_t)total, (uint32_t)b, Q,
+                                                                     ldq, out, ldo, (T)ck);
   SMA_CHECK_LAUNCH();
 }
 
@@ -342,20 +348,40 @@ template <typename T>
 void launch_clenshaw_axpy(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq,
                           const T *AX, int64_t ldax, const T *B1, const T *B2, int64_t ldb,
                           T *out, int64_t ldo, double ck, double alpha, double beta) {
-  if (n * b == 0) return;
-  clenshaw_axpy_kernel<T><<<grid_for(n * b), 256, 0, st>>>(n, b, Q, ldq, AX, ldax, B1, B2, ldb,
-                                                           out, ldo, (T)ck, (T)alpha, (T)beta);
+  const int64_t total = n * b;
+  if (total == 0) return;
+  if (total >> 32)
+    clenshaw_axpy_kernel<T, uint64_t><<<grid_for(total), 256, 0, st>>>(
+        total, b, Q, ldq, AX, ldax, B1, B2, ldb, out, ldo, (T)ck, (T)alpha, (T)beta);
+  else
+    clenshaw_axpy_kernel<T, uint32_t><<<grid_for(total), 256, 0, st>>>(
+        (uint32_t)total, (uint32_t)b, Q, ldq, AX, ldax, B1, B2, ldb, out, ldo, (T)ck, (T)alpha, (T)beta);
+  SMA_CHECK_LAUNCH();
+}
+
+template <typename TS, typename TD>
+void launch_pad_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int64_t lds, int64_t w,
+                      TD *dst, int64_t ldd) {
+  const int64_t total = n * w;
+  if (total == 0) return;
+  if (total >> 32)
+    copy_block_kernel<TS, TD, uint64_t><<<grid_for(total), 256, 0, st>>>(total, w, b, src, lds, dst, ldd);
+  else
+    copy_block_kernel<TS, TD, uint32_t><<<grid_for(total), 256, 0, st>>>(
+        (uint32_t)total, (uint32_t)w, (uint32_t)b, src, lds, dst, ldd);
   SMA_CHECK_LAUNCH();
 }
 
 template <typename TS, typename TD>
 void launch_copy_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int64_t lds, TD *dst,
                        int64_t ldd) {
-  if (n * b == 0) return;
-  copy_block_kernel<TS, TD><<<grid_for(n * b), 256, 0, st>>>(n, b, src, lds, dst, ldd);
-  SMA_CHECK_LAUNCH();
+  launch_pad_block<TS, TD>(st, n, b, src, lds, b, dst, ldd);
 }
 
+template void launch_pad_block<double, double>(cudaStream_t, int64_t, int64_t, const double *,
+                                               int64_t, int64_t, double *, int64_t);
+template void launch_pad_block<float, float>(cudaStream_t, int64_t, int64_t, const float *, int64_t,
+                                             int64_t, float *, int64_t);
 template void launch_clenshaw_step<double>(const sma_op *, cudaStream_t, int64_t, const double *,
                                            int64_t, const double *, const double *, int64_t,
                                            double *, int64_t, double, double, double, bool, bool);

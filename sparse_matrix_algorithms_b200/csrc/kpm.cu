@@ -31,12 +31,12 @@ __global__ void rademacher_kernel(int64_t n, int64_t R, uint64_t seed, double *_
                                   int64_t ld) {
   const uint64_t s = seed ^ 0x2545F4914F6CDD1DULL;
   const uint64_t golden = 0x9E3779B97F4A7C15ULL;
-  const int64_t total = n * R;
+  const int64_t total = n * ld;  // columns R..ld-1 are zero
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / R, j = t % R;
+    const int64_t i = t / ld, j = t % ld;
     const uint64_t k = (uint64_t)i + (uint64_t)j * (uint64_t)n;
-    out[i * ld + j] = (kpm_mix64(s + (k + 1) * golden) >> 63) ? -1.0 : 1.0;
+    out[t] = j >= R ? 0.0 : (kpm_mix64(s + (k + 1) * golden) >> 63) ? -1.0 : 1.0;
   }
 }
 
@@ -53,21 +53,22 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
   // dots of one step: <T_{k+1}, T_k> and <T_k, T_k>, chunks x R partials each; the partials of
   // `batch` steps are summed by one launch
+  const bool product_then_axpy = op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF;
+  const int64_t w = product_then_axpy ? R : recurrence_width(R, sizeof(double));
   const int64_t chunks = column_chunks(n, R), set = 2 * chunks * R;
   const int64_t steps = (M + 1) / 2;
   const int64_t batch = std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
-  DevBuf<double> t0(n * R, st), t1(n * R, st), t2(n * R, st), dots(2 * steps * R, st),
+  DevBuf<double> t0(n * w, st), t1(n * w, st), t2(n * w, st), dots(2 * steps * R, st),
       partial(batch * set, st);
   {
-    const int64_t total = n * R;
+    const int64_t total = n * w;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    rademacher_kernel<<<std::max(grid, 1u), 256, 0, st>>>(n, R, seed, t0.p, R);
+    rademacher_kernel<<<std::max(grid, 1u), 256, 0, st>>>(n, R, seed, t0.p, w);
     SMA_CHECK_LAUNCH();
   }
   // out = ck Q + alpha A B1 + beta B1: the fused step for device operators, the caller's
   // block product followed by the axpy kernel for callback operators
   DevBuf<double> ax;
-  const bool product_then_axpy = op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF;
   if (product_then_axpy) ax.alloc(n * R, st);
   auto step = [&](const double *Q, const double *B1, double *out, double ck, double alpha,
                   double beta, bool rev) {
@@ -75,7 +76,7 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
       op_apply(op, st, B1, R, ax.p, R, R);
       launch_clenshaw_axpy<double>(st, n, R, Q, R, ax.p, R, B1, nullptr, R, out, R, ck, alpha, beta);
     } else {
-      launch_clenshaw_step<double>(op, st, R, Q, R, B1, nullptr, R, out, R, ck, alpha, beta, true, rev);
+      launch_clenshaw_step<double>(op, st, w, Q, w, B1, nullptr, w, out, w, ck, alpha, beta, true, rev);
     }
   };
   // dots: for k = 0, 1, ...: <T_{k+1}, T_k> then <T_k, T_k> (R values each)
@@ -88,9 +89,9 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
         step(Tcur, Tcur, Tnext, 0.0, invd, -c * invd, false);
       else  // T_{k+1} = 2 invd A T_k - 2 c invd T_k - T_{k-1}
         step(Tprev, Tcur, Tnext, -1.0, 2.0 * invd, -2.0 * c * invd, k & 1);
-      column_partials(st, 2, n, R, Tnext, R, Tcur, R, nullptr, slot);
+      column_partials(st, 2, n, R, Tnext, w, Tcur, w, nullptr, slot);
     } else {  // an odd M: the last moment needs <T_k, T_k> only
-      column_partials(st, 2, n, R, Tcur, R, Tcur, R, nullptr, slot);
+      column_partials(st, 2, n, R, Tcur, w, Tcur, w, nullptr, slot);
     }
     if (k + 1 - done == batch || k + 1 == steps) {
       column_totals(st, 0, chunks, R, 2 * (k + 1 - done), partial.p, dots.p + 2 * done * R);

@@ -239,6 +239,10 @@ void column_totals(cudaStream_t st, int mode, int64_t chunks, int64_t k, int64_t
 template <typename TS, typename TD>
 void launch_copy_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int64_t lds, TD *dst,
                        int64_t ldd);
+// The same into the first b columns of an n x w block, the columns past b zeroed.
+template <typename TS, typename TD>
+void launch_pad_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int64_t lds, int64_t w,
+                      TD *dst, int64_t ldd);
 // dst column-major n x k (ld n) <- src row-major n x k (ld lds)
 void launch_rowmajor_to_colmajor(cudaStream_t st, int64_t n, int64_t k, const double *src,
                                  int64_t lds, double *dst);
@@ -287,7 +291,7 @@ std::vector<double> build_coeffs(int64_t degree, double smin, double smax, doubl
 
 // ------------------------------------------------------------------ filter (filter.cu)
 // Work space of the block Clenshaw recurrence: three n x b blocks (+ AX for matrix-free),
-// and the CUDA graph of a repeated filter: from the second call with the same operator,
+// (their width padded, filter.cu), and the CUDA graph of a repeated filter: from the second call with the same operator,
 // width, coefficients and bounds, the whole recurrence (on staging blocks q -> y at fixed
 // addresses) is replayed from a graph instead of launched step by step.
 template <typename T>
@@ -304,6 +308,8 @@ struct ClenshawWork {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   void ensure(const sma_op *op, int64_t n_, int64_t b, cudaStream_t st);
+  // ensure() and the staging block of Q; false, with nothing held, when memory does not allow it
+  bool fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t st);
   void drop_graph();
   ClenshawWork() = default;
   ClenshawWork(const ClenshawWork &) = delete;
@@ -340,6 +346,10 @@ void half_product(const sma_op *op, cudaStream_t st, const T *X, int64_t ldx, T 
 // AX = A X for FP64 blocks (any operator kind)
 void op_apply(const sma_op *op, cudaStream_t st, const double *X, int64_t ldx, double *Y,
               int64_t ldy, int64_t b);
+
+// Width of a recurrence's own blocks for b columns of elem_bytes (filter.cu): b, or b padded to a
+// width that wider vectors divide.
+int64_t recurrence_width(int64_t b, int elem_bytes);
 
 // Algorithmic bytes of one fused Clenshaw step over b columns
 double clenshaw_step_bytes(const sma_op *op, int64_t b, int elem_bytes);

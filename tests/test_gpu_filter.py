@@ -247,3 +247,61 @@ def test_autotuned_filter_bit_identical_to_untuned(lib_built, monkeypatch, capfd
     monkeypatch.setenv("SMA_AUTOTUNE", "0")
     plain = S.apply_poly_block(S.SparseOperator(A, S.Context(0)), Q, c, smin, smax, precision=precision)
     np.testing.assert_array_equal(tuned, plain)
+
+
+@pytest.mark.parametrize("precision,rtol", [("fp64", 1e-12), ("fp32", 2e-4)])
+@pytest.mark.parametrize("b,ldq,shift", [
+    (1, 1, 0), (3, 3, 0), (5, 7, 1), (9, 9, 0), (13, 16, 0), (31, 31, 0), (33, 40, 1),
+    (64, 65, 0), (64, 64, 1), (66, 66, 0), (127, 128, 0), (260, 260, 0), (517, 517, 0)])
+def test_filter_ragged_widths_and_strides(lib_built, precision, rtol, b, ldq, shift):
+    """Widths around the vector, CTA and panel edges of the step kernel (1, 2, 4 or 8 columns a
+    thread, panels beyond 64 vectors), strides and addresses that forbid wide accesses, degrees on
+    both sides of the staging threshold; every column equal to the filter of that column alone at
+    the oracle's tolerance, and nothing written past the block."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    A = _ragged(333, 4)
+    n = A.shape[0]
+    smin, smax = _bounds(A)
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    Qh = M.splitmix_normal(b, n, b)
+    store = torch.full((n * ldq + shift + 8,), 7.0, dtype=dt, device="cuda")
+    Q = store[shift:shift + n * ldq].view(n, ldq)
+    Q[:, :b] = torch.as_tensor(Qh, device="cuda").to(dt)
+    op = S.SparseOperator(A)
+    for K in (1, 3, 4, 45):
+        c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+        Y = torch.full((n, b + 3), 3.0, dtype=dt, device="cuda")
+        torch.cuda.synchronize()
+        L.check(L.load().sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, Q.data_ptr(),
+                                                  ldq, Y.data_ptr(), b + 3, b, L.PRECISIONS[precision]))
+        ref = O.apply_poly_block(A, Qh, c, smin, smax)
+        got = Y.cpu().numpy()
+        assert np.abs(got[:, :b] - ref).max() <= rtol * max(np.abs(ref).max(), np.abs(Qh).max())
+        assert np.all(got[:, b:] == 3.0)
+
+
+@pytest.mark.parametrize("stencil", ["lap1d", "anderson", "xxz"])
+@pytest.mark.parametrize("b", [1, 3, 8, 31, 200])
+def test_model_steps_equal_the_stored_matrix(lib_built, stencil, b):
+    """The models' entries are built per CTA: first and last rows, wrapped neighbours and the
+    periodic bond, at one and at many rows a CTA.  Bit for bit for the models whose entries are
+    accumulated in the stored matrix's order."""
+    import sparse_matrix_algorithms_b200 as S
+
+    if stencil == "lap1d":
+        op, A = S.Lap1dOperator(1001), M.lap1d(1001)
+    elif stencil == "anderson":
+        op, A = S.AndersonOperator(7, 16.5, 5), M.anderson3d(7, 16.5, 5)
+    else:
+        op, A = S.XXZOperator(10, 5.0, 1), M.xxz_sz0(10, 5.0, 1)
+    smin, smax = _bounds(A)
+    c = O.build_coeffs(40, smin, smax, 0.1, -0.4, 0.3, "step", True)
+    Q = M.splitmix_normal(b, A.shape[0], b)
+    got, ref = S.apply_poly_block(op, Q, c, smin, smax), S.apply_poly_block(A, Q, c, smin, smax)
+    if stencil == "xxz":
+        assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
+    else:
+        np.testing.assert_array_equal(got, ref)
