@@ -6,7 +6,7 @@
 #include <cstdlib>
 #include <string>
 
-#include "sma_internal.h"
+#include "solver_common.h"
 
 namespace sma {
 sma_result *cheb_solve(sma_op *op, double emin, double emax, const sma_cheb_opts &o);
@@ -200,11 +200,16 @@ int sma_op_create_csc(sma_ctx *ctx, int64_t n, int64_t nnz, const int64_t *colpt
     op->kind = OP_CSR;
     op->n = n;
     op->nnz = nnz;
+    int64_t uneven = 0;
+    for (int64_t i = 1; i < n; ++i) uneven += rp[i + 1] - rp[i] != rp[i] - rp[i - 1];
+    op->ragged = uneven > n / 10;
     try {
       cudaStream_t st = ctx->stream;
       SMA_CUDA(cudaMalloc((void **)&op->rowptr, (n + 1) * sizeof(int)));
-      SMA_CUDA(cudaMalloc((void **)&op->colind, std::max<int64_t>(nnz, 1) * sizeof(int)));
-      SMA_CUDA(cudaMalloc((void **)&op->val64, std::max<int64_t>(nnz, 1) * sizeof(double)));
+      SMA_CUDA(cudaMalloc((void **)&op->colind, (nnz + kRowPad) * sizeof(int)));
+      SMA_CUDA(cudaMalloc((void **)&op->val64, (nnz + kRowPad) * sizeof(double)));
+      SMA_CUDA(cudaMemsetAsync(op->colind + nnz, 0, kRowPad * sizeof(int), st));
+      SMA_CUDA(cudaMemsetAsync(op->val64 + nnz, 0, kRowPad * sizeof(double), st));
       SMA_CUDA(cudaMemcpyAsync(op->rowptr, rp.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
       if (nnz) {
         SMA_CUDA(cudaMemcpyAsync(op->colind, ci.data(), nnz * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -424,10 +429,7 @@ int sma_apply_poly_block_dev(sma_op *op, const double *coeffs, int64_t K, double
       SMA_CUDA(cudaStreamSynchronize(st));
     } else {
       require(op->kind != OP_MATBLOCK, SMA_ERR_ARG, "FP32 filtering needs a device operator");
-      if ((op->kind == OP_CSR || op->kind == OP_CSR_HALF) && !op->val32) {
-        SMA_CUDA(cudaMalloc((void **)&op->val32, std::max<int64_t>(op->nnz, 1) * sizeof(float)));
-        launch_copy_block<double, float>(st, op->nnz, 1, op->val64, 1, op->val32, 1);
-      }
+      detail::ensure_fp32_values(op);
       ClenshawWork<float> w;
       apply_poly_block<float>(op, st, c, smin, smax, (const float *)Q_dev, ldq, (float *)Y_dev, ldy,
                               b, w);
@@ -467,10 +469,7 @@ int sma_apply_poly_block_percol_dev(sma_op *op, const double *coeffs, int64_t K,
     if (precision == SMA_PREC_FP64) {
       run(0.0);
     } else {
-      if ((op->kind == OP_CSR || op->kind == OP_CSR_HALF) && !op->val32) {
-        SMA_CUDA(cudaMalloc((void **)&op->val32, std::max<int64_t>(op->nnz, 1) * sizeof(float)));
-        launch_copy_block<double, float>(st, op->nnz, 1, op->val64, 1, op->val32, 1);
-      }
+      detail::ensure_fp32_values(op);
       run(0.0f);
     }
   });

@@ -137,6 +137,34 @@ __device__ __forceinline__ void row_product(const Row &row, int j, int end, cons
   }
 }
 
+// The same for rows of unequal lengths: chunks of U whose accesses past the row's end are
+// predicated off (the entry arrays are readable that far, kRowPad).  The rows of a warp then walk
+// one code path; with the exact chunks above each remainder is a path of its own, and the warp
+// waits for the gathers of all of them in turn (XXZ L = 16, b = 32: 5.3 -> 4.0 us a step FP64,
+// 4.1 -> 3.1 FP32; L = 18 13.2 -> 12.3).  An absent entry adds 0 * 0.
+template <typename T, int V, int U, bool W, typename Row>
+__device__ __forceinline__ void ragged_product(const Row &row, int j, int end, const T *B1c,
+                                               uint64_t ldb, T (&acc)[V]) {
+  for (; j < end; j += U) {
+    int c[U];
+    T x[U][V], v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = row.col(j + u);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      ldv_if<T, V>(j + u < end, at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      v[u] = row.val(j + u);
+      if (j + u >= end) v[u] = T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = fma(v[u], x[u][i], acc[i]);
+  }
+}
+
 // ------------------------------------------------------------------ the models' rows
 // Entry u of model row `row`: its place among the row's entries in accumulation order and its
 // column, or place -1 when the row has no such entry.
@@ -239,7 +267,8 @@ __device__ __forceinline__ void coefficients(const Step<T> &a, uint32_t c0, T (&
 }
 
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
+          bool RAGGED>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
@@ -268,9 +297,12 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   if constexpr (MODEL) {
     const T diag = a.kind == OP_LAP1D ? T(2) : (T)__ldg(a.model.diag + row);
     const ModelRow<T> mr{model_smem + r * a.entries, dpos[r], diag, (T)a.model.hop};
-    row_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
+    if constexpr (RAGGED) ragged_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
+    else row_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
   } else {
-    row_product<T, V, U, W>(CsrRow<T>{a.colind, a.val}, start, end, a.B1 + c0, a.ldb, acc);
+    const CsrRow<T> cr{a.colind, a.val};
+    if constexpr (RAGGED) ragged_product<T, V, U, W>(cr, start, end, a.B1 + c0, a.ldb, acc);
+    else row_product<T, V, U, W>(cr, start, end, a.B1 + c0, a.ldb, acc);
   }
   T q[V], s[V], t[V], ck[V], o[V];
   if constexpr (HQ) ldv<T, V, false>(at(a.Q + c0, row * a.ldq), q);
@@ -292,21 +324,24 @@ namespace sma {
 namespace rows {
 
 // ------------------------------------------------------------------ launch
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
+          bool RAGGED>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
-  if (MODEL) cfg.dynamicSmemBytes = a.rows * (a.entries + 2) * sizeof(int);  // 17.9 KB at most
+  if (MODEL) cfg.dynamicSmemBytes = (a.rows * (a.entries + 2) + kRowPad) * sizeof(int);  // 18 KB at most
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = op->ctx->pdl ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL>, a));
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED>, a));
   SMA_CHECK_LAUNCH();
 }
+
+inline bool ragged(const sma_op *op) { return op->kind == OP_XXZ || op->ragged; }
 
 template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
@@ -317,12 +352,14 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
   const uint32_t gx = (a.n + a.rows - 1) / a.rows;
-  // Fewer than six waves of 8-CTA residency: a step is then a latency, not a stream, and twice
-  // the gathers in flight at half the occupancy is the faster kernel (Anderson L = 20, b = 64
-  // FP64: 3.7 us against 5.0; XXZ L = 18, b = 32: 13.5 against 14.2; with 2 M threads 43.8
-  // against 42.5).
-  const bool small = gathers ? gathers == 8
-                             : (int64_t)a.n * vecs < 6LL * 8 * kThreads * op->ctx->num_sms;
+  // Fewer than six waves of 8-CTA residency: a step is then a latency, not a stream, and more
+  // gathers in flight at a lower occupancy are the faster kernel (Anderson L = 20, b = 64
+  // FP64: 3.7 us against 5.0; with 2 M threads 43.8 against 42.5; ragged rows, U = 6 against 4:
+  // XXZ L = 18, b = 32 12.3 against 13.6, with 1.5 M threads 51.0 against 48.0), for ragged rows
+  // once more below one wave (U = 8 against 6: XXZ L = 16, b = 32 4.0 against 5.2, L = 18 12.6
+  // against 12.3).
+  const int64_t wave = 8LL * kThreads * op->ctx->num_sms, threads = (int64_t)a.n * vecs;
+  if (gathers == 0) gathers = threads >= 6 * wave ? 4 : !ragged(op) || threads < wave ? 8 : 6;
   constexpr uint32_t kGridY = 65535;
   const uint32_t ny = (vecs + a.lanes - 1) / a.lanes;
   const uint32_t span = kGridY * a.lanes * V, width = a.b;
@@ -336,8 +373,14 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
-    if (small) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL>(op, st, a, grid);
-    else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL>(op, st, a, grid);
+    if (ragged(op)) {
+      if (gathers == 8) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
+      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
+    } else {
+      if (gathers == 8) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false>(op, st, a, grid);
+    }
   }
 }
 
@@ -417,8 +460,8 @@ void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
 inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
 
 // Picks the vector width: the widest that widths, strides and addresses allow, but narrower
-// while the step would not give every SM a CTA (XXZ L = 14, b = 8 FP64: 4.4, 3.3 and 3.1 us a
-// step with 4, 2 and 1 columns a thread).
+// while the step would not give every SM a CTA (Anderson L = 12, b = 8), or with ragged rows half
+// a CTA (XXZ L = 14, b = 8 FP64: 2.6 and 2.1 us a step with 4 and 2 columns a thread).
 template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
@@ -442,7 +485,7 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
            aligned(a.out, bytes) && (!HQ || (a.ldq % bytes == 0 && aligned(a.Q, bytes))) &&
            (!HB || aligned(a.B2, bytes)) && (!PC || a.colseg || aligned(a.cseg, bytes));
   };
-  const int64_t want = (int64_t)op->ctx->num_sms * kThreads;
+  const int64_t want = (int64_t)op->ctx->num_sms * kThreads / (ragged(op) ? 2 : 1);
   auto take = [&](int v) { return fits(v) && op->n * (b / v) >= want; };
   if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL>(op, st, a);
   if constexpr (sizeof(T) == 4)

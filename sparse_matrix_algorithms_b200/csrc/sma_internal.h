@@ -123,12 +123,13 @@ struct sma_op {
   int64_t n = 0, nnz = 0;
   // CSR (== CSC of the symmetric matrix), 0-based, int32 indices
   int *rowptr = nullptr;
-  int *colind = nullptr;
+  int *colind = nullptr;  // kRowPad zeros follow the arrays of OP_CSR
   double *val64 = nullptr;
   float *val32 = nullptr;  // created on first FP32 use
   // Gershgorin bounds, computed on upload
   double gersh_min = 0, gersh_max = 0;
   bool has_gersh = false;
+  bool ragged = false;  // CSR: more than a tenth of the rows differ in length from the row before
   int sym_state = 0;  // 0 unknown, 1 A == A^T, 2 not symmetric
   // caller callback
   sma_matblock_fn fn = nullptr;
@@ -145,6 +146,10 @@ struct sma_op {
 };
 
 namespace sma {
+
+// Entries past the last that colind, val64 and val32 of a CSR operator hold (zeros): the step
+// kernel reads ragged rows in whole chunks.
+constexpr int kRowPad = 8;
 
 // ------------------------------------------------------------------ device buffers
 // Stream-ordered device allocation owned by one solve.

@@ -49,6 +49,32 @@ __device__ __forceinline__ void ldv(const T *__restrict__ p, T (&f)[V]) {
   memcpy(f, w, sizeof(w));
 }
 
+// ldv where ok, else zeros: the access itself is predicated, nothing branches.
+template <typename T, int V>
+__device__ __forceinline__ void ldv_if(bool ok, const T *__restrict__ p, T (&f)[V]) {
+  constexpr int kBytes = V * (int)sizeof(T);
+  unsigned w[kBytes / 4];
+#pragma unroll
+  for (int i = 0; i < kBytes / 4; ++i) w[i] = 0u;
+  if constexpr (kBytes == 32)
+    asm("{\n .reg .pred p;\n setp.ne.u32 p, %9, 0;\n"
+        " @p ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]),
+          "+r"(w[7])
+        : "l"(p), "r"((unsigned)ok));
+  else if constexpr (kBytes == 16)
+    asm("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n"
+        " @p ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n}"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]) : "l"(p), "r"((unsigned)ok));
+  else if constexpr (kBytes == 8)
+    asm("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.global.nc.v2.b32 {%0, %1}, [%2];\n}"
+        : "+r"(w[0]), "+r"(w[1]) : "l"(p), "r"((unsigned)ok));
+  else
+    asm("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.global.nc.b32 %0, [%1];\n}"
+        : "+r"(w[0]) : "l"(p), "r"((unsigned)ok));
+  memcpy(f, w, sizeof(w));
+}
+
 template <typename T, int V>
 __device__ __forceinline__ void stv(T *__restrict__ p, const T (&f)[V]) {
   constexpr int kBytes = V * (int)sizeof(T);
