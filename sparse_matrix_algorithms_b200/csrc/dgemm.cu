@@ -8,15 +8,20 @@
 //           X: n x m row-major (ldx); B: m x p given as a column-major C (B = C, ldc) or as
 //           the transpose of one (B = C^T, C p x m column-major, ldc).
 //
-// Both stage their operand tiles in shared memory with cp.async (16-byte copies, double
-// buffered) and run mma.sync.aligned.m8n8k4.row.col.f64 on the tiles: a warp owns a 32 x 32
-// (update) or 32 x 16 (gram) piece of the CTA's 64 x 64 / 128 x 64 output tile and keeps its
-// accumulators in registers.  The gram splits n over the grid; every CTA writes its 64 x 64
-// partial product to a workspace and a second kernel sums the partials in a fixed order,
-// so results are deterministic (the same bits every run).  The update owns whole rows of Y:
-// with beta = 0 it may write in place over X when p <= 64 (X <- X B, the triangular solve of
-// CholQR written as a product with R^-1), since a CTA reads all of its rows of X before it
-// writes them.
+// Both run mma.sync.aligned.m8n8k4.row.col.f64 on operand tiles that cp.async brings to shared
+// memory, three chunks of 16 in flight and one barrier a chunk: a warp owns a 32 x 32 piece of the
+// CTA's 64 x 64 output tile (smaller ones for narrow products), keeps its accumulators in
+// registers and reads the next four indices' fragments while it multiplies.  The gram splits n
+// over the grid so that the tiles fill whole waves of three CTAs an SM; every CTA writes its
+// partial tile to a workspace and a second kernel sums the partials in a fixed order, so results
+// are deterministic (the same bits every run).  The update owns whole rows of Y: with beta = 0 it
+// may write in place over X when p <= 64 (X <- X B, the triangular solve of CholQR written as a
+// product with R^-1), since a CTA reads all of its rows of X before it writes them.
+//
+// What bounds it: the FP64 tensor pipe, 37.1 TFLOP/s measured from registers.  Four warps a CTA
+// and three CTAs an SM keep it busier than eight and two (35.7 against 34.7 TFLOP/s at p = 512),
+// and the copies' addresses are pointers that advance: recomputed for every chunk they cost as
+// much as the barriers (31.3 TFLOP/s).
 //
 // DMMA fragment layout of m8n8k4 (PTX ISA, "Matrix Fragments for mma.m8n8k4 with .f64"):
 // lane = 4 g + t (g = groupID 0..7, t = thread in group 0..3);
@@ -29,6 +34,9 @@
 namespace sma {
 namespace dmma {
 
+constexpr int kThreads = 128;  // four warps
+constexpr int kDepth = 16;     // summation indices of a chunk
+
 __device__ __forceinline__ void mma_8x8x4(double (&d)[2], double a, double b) {
   asm volatile(
       "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
@@ -36,245 +44,361 @@ __device__ __forceinline__ void mma_8x8x4(double (&d)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
+// BYTES (8 or 16) from global to shared memory, zeros where !ok (the source is then not read).
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *smem, const void *gmem, bool ok) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+  const int n = ok ? BYTES : 0;
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// ------------------------------------------------------------------ update
-// CTA tile: 128 rows x 64 columns of Y; 8 warps as 4 (rows) x 2 (columns), warp tile
-// 32 x 32 = 4 x 4 fragments.  K chunk 16 (four k-steps of 4), two stages.
-constexpr int UM = 128, UN = 64, UK = 16;
-constexpr int UA = UK + 4;  // padded row of the A stage (doubles)
-constexpr int UB = UK + 4;  // padded row of the B stage, stored [column][k]
-constexpr int kUpdateThreads = 256;
-
-struct UpdateSmem {
-  double a[2][UM][UA];
-  double b[2][UN][UB];
+// A CTA tile of WM x WN warps, each MT x NT fragments of 8 x 8; chunks in flight and CTAs an SM.
+template <int WM_, int WN_, int MT_, int NT_, int STAGES_ = 3, int CTAS_ = 3>
+struct Tile {
+  static constexpr int WM = WM_, WN = WN_, MT = MT_, NT = NT_, kStages = STAGES_, kCtas = CTAS_;
+  static constexpr int M = WM * MT * 8, N = WN * NT * 8;
+  static_assert(WM * WN * 32 == kThreads, "four warps");
+  static_assert(M % 16 == 0 && N % 16 == 0, "whole passes of 16-byte copies");
 };
 
-// B(i, j) for the update: TB = false -> C[i + j ldc] (column-major m x p);
-// TB = true -> C[j + i ldc] (the transpose of a column-major p x m).
-template <bool TB>
-__global__ void __launch_bounds__(kUpdateThreads)
+// acc += A B over one chunk: a(k, i) and b(k, j) give this lane's element of fragment i (j) at
+// summation index k; the fragments of k + 4 are read before those of k are multiplied.
+template <typename T, typename A, typename B>
+__device__ __forceinline__ void multiply(double (&acc)[T::MT][T::NT][2], const A &a, const B &b) {
+  double fa[2][T::MT], fb[2][T::NT];
+#pragma unroll
+  for (int i = 0; i < T::MT; ++i) fa[0][i] = a(0, i);
+#pragma unroll
+  for (int j = 0; j < T::NT; ++j) fb[0][j] = b(0, j);
+#pragma unroll
+  for (int k = 0; k < kDepth; k += 4) {
+    const int cur = (k / 4) & 1;
+    if (k + 4 < kDepth) {
+#pragma unroll
+      for (int i = 0; i < T::MT; ++i) fa[cur ^ 1][i] = a(k + 4, i);
+#pragma unroll
+      for (int j = 0; j < T::NT; ++j) fb[cur ^ 1][j] = b(k + 4, j);
+    }
+#pragma unroll
+    for (int i = 0; i < T::MT; ++i)
+#pragma unroll
+      for (int j = 0; j < T::NT; ++j) mma_8x8x4(acc[i][j], fa[cur][i], fb[cur][j]);
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void clear(double (&acc)[T::MT][T::NT][2]) {
+#pragma unroll
+  for (int i = 0; i < T::MT; ++i)
+#pragma unroll
+    for (int j = 0; j < T::NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+}
+
+// The chunks 0..nk-1 through the stages: load(stage, chunk) issues copies, use(stage) computes.
+template <int kStages, typename Load, typename Use>
+__device__ __forceinline__ void pipeline(int nk, const Load &load, const Use &use) {
+#pragma unroll
+  for (int c = 0; c < kStages - 1; ++c) {
+    if (c < nk) load(c, c);
+    cp_async_commit();
+  }
+  int stage = 0;
+  for (int c = 0; c < nk; ++c) {
+    cp_async_wait<kStages - 2>();  // chunk c has landed (this thread's part of it)
+    __syncthreads();               // everybody's; and chunk c - 1 is consumed: its stage is free
+    const int next = c + kStages - 1;
+    if (next < nk) load(stage == 0 ? kStages - 1 : stage - 1, next);
+    cp_async_commit();
+    use(stage);
+    stage = stage + 1 == kStages ? 0 : stage + 1;
+  }
+}
+
+// ------------------------------------------------------------------ update
+constexpr int kPad = kDepth + 4;  // shared rows of 20 doubles: conflict-free fragment reads
+
+template <typename T>
+struct UpdateSmem {
+  double a[T::kStages][T::M][kPad];
+  double b[T::kStages][T::N][kPad];  // stored [column][k]
+};
+
+// B(i, j): TB = false -> C[i + j ldc] (column-major m x p); TB = true -> C[j + i ldc] (the
+// transpose of a column-major p x m).  vecx, vecc, vecy: 16-byte accesses of X, C (TB = false), Y.
+template <bool TB, typename T>
+__global__ void __launch_bounds__(kThreads, T::kCtas)
 update_kernel(int64_t n, int m, int p, const double *X, int64_t ldx,  // Y may alias X
               const double *__restrict__ C, int64_t ldc, double *Y, int64_t ldy, double alpha,
-              double beta, bool vec16) {
+              double beta, int coltiles, bool vecx, bool vecc, bool vecy) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  UpdateSmem &sm = *reinterpret_cast<UpdateSmem *>(smem_raw);
+  UpdateSmem<T> &sm = *reinterpret_cast<UpdateSmem<T> *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wr = (warp & 3) * 32, wc = (warp >> 2) * 32;
-  const int64_t row0 = (int64_t)blockIdx.x * UM;
-  const int col0 = blockIdx.y * UN;
-  double acc[4][4][2];
+  const int wr = warp % T::WM * T::MT * 8, wc = warp / T::WM * T::NT * 8;
+  // column tiles next to each other: they read the same rows of X
+  const int64_t row0 = (int64_t)(blockIdx.x / coltiles) * T::M;
+  const int col0 = blockIdx.x % coltiles * T::N;
+  double acc[T::MT][T::NT][2];
+  clear<T>(acc);
+  // This thread's 16-byte copies of a whole chunk: rows r of X (columns of C), two indices from c
+  // on; the pointers advance with the chunks.
+  constexpr int kPerRow = kDepth / 2, PA = T::M * kPerRow / kThreads, PB = T::N * kPerRow / kThreads;
+  static_assert(T::M * kPerRow % kThreads == 0 && T::N * kPerRow % kThreads == 0, "whole passes");
+  const int r = tid / kPerRow, c = tid % kPerRow * 2;
+  constexpr int kStep = kThreads / kPerRow;  // rows between two copies of a thread
+  const double *px[PA], *pc[PB];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < PA; ++i)
+    px[i] = row0 + r + i * kStep < n ? X + (row0 + r + i * kStep) * ldx + c : nullptr;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int nk = (m + UK - 1) / UK;  // m = 0: Y = beta Y
-  // stage loader: A rows row0.., k chunk kc; B k chunk kc, columns col0..
-  auto load = [&](int stage, int kc) {
-    const int k0 = kc * UK;
-    // A: 128 x 16 doubles; with 16-byte copies 8 per row
-    if (vec16 && k0 + UK <= m) {
-      for (int e = tid; e < UM * (UK / 2); e += kUpdateThreads) {
-        const int r = e / (UK / 2), c2 = (e % (UK / 2)) * 2;
-        const int64_t gr = row0 + r;
-        double *dst = &sm.a[stage][r][c2];
-        if (gr < n) cp_async16(dst, X + gr * ldx + k0 + c2);
-        else { dst[0] = 0.0; dst[1] = 0.0; }
+  for (int i = 0; i < PB; ++i)
+    pc[i] = !TB && col0 + r + i * kStep < p ? C + (int64_t)(col0 + r + i * kStep) * ldc + c : nullptr;
+  auto load = [&](int stage, int chunk) {
+    const int k0 = chunk * kDepth;
+    const bool whole = k0 + kDepth <= m;
+    if (vecx && whole) {
+#pragma unroll
+      for (int i = 0; i < PA; ++i) {
+        cp_async<16>(&sm.a[stage][r + i * kStep][c], px[i] ? px[i] : X, px[i] != nullptr);
+        if (px[i]) px[i] += kDepth;
       }
     } else {
-      for (int e = tid; e < UM * UK; e += kUpdateThreads) {
-        const int r = e / UK, c = e % UK;
-        const int64_t gr = row0 + r;
-        double *dst = &sm.a[stage][r][c];
-        if (gr < n && k0 + c < m) cp_async8(dst, X + gr * ldx + k0 + c);
-        else *dst = 0.0;
+      for (int e = tid; e < T::M * kDepth; e += kThreads) {
+        const int rr = e / kDepth, cc = e % kDepth;
+        const bool ok = row0 + rr < n && k0 + cc < m;
+        cp_async<8>(&sm.a[stage][rr][cc], X + (ok ? (row0 + rr) * ldx + k0 + cc : 0), ok);
       }
     }
-    // B: 16 (k) x 64 (columns), stored [column][k]
-    for (int e = tid; e < UN * UK; e += kUpdateThreads) {
-      int j, kk;
-      if (TB) { kk = e / UN; j = e % UN; }   // consecutive threads: consecutive columns
-      else { j = e / UK; kk = e % UK; }      // consecutive threads: consecutive k
-      const int gk = k0 + kk, gj = col0 + j;
-      double *dst = &sm.b[stage][j][kk];
-      if (gk < m && gj < p) cp_async8(dst, TB ? C + gj + (int64_t)gk * ldc : C + gk + (int64_t)gj * ldc);
-      else *dst = 0.0;
+    if (!TB && vecc && whole) {
+#pragma unroll
+      for (int i = 0; i < PB; ++i) {
+        cp_async<16>(&sm.b[stage][r + i * kStep][c], pc[i] ? pc[i] : C, pc[i] != nullptr);
+        if (pc[i]) pc[i] += kDepth;
+      }
+    } else {
+      for (int e = tid; e < T::N * kDepth; e += kThreads) {
+        const int j = TB ? e % T::N : e / kDepth, kk = TB ? e / T::N : e % kDepth;
+        const int gk = k0 + kk, gj = col0 + j;
+        const bool ok = gk < m && gj < p;
+        cp_async<8>(&sm.b[stage][j][kk], C + (!ok ? 0 : TB ? gj + (int64_t)gk * ldc : gk + (int64_t)gj * ldc), ok);
+      }
     }
-    cp_async_commit();
   };
-  if (nk > 0) load(0, 0);
-  for (int kc = 0; kc < nk; ++kc) {
-    const int stage = kc & 1;
-    if (kc + 1 < nk) {
-      load(stage ^ 1, kc + 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+  pipeline<T::kStages>((m + kDepth - 1) / kDepth, load, [&](int stage) {  // m = 0: Y = beta Y
+    const double *a = &sm.a[stage][wr + g][t], *b = &sm.b[stage][wc + g][t];
+    multiply<T>(acc, [&](int k, int i) { return a[i * 8 * kPad + k]; },
+                [&](int k, int j) { return b[j * 8 * kPad + k]; });
+  });
+  // Y = alpha acc + beta Y (Y not read when beta == 0)
 #pragma unroll
-    for (int ks = 0; ks < UK; ks += 4) {
-      double a[4], b[4];
+  for (int i = 0; i < T::MT; ++i) {
+    const int64_t yr = row0 + wr + i * 8 + g;
+    if (yr >= n) continue;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = sm.a[stage][wr + i * 8 + g][ks + t];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = sm.b[stage][wc + j * 8 + g][ks + t];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) mma_8x8x4(acc[i][j], a[i], b[j]);
-    }
-    __syncthreads();
-  }
-  // epilogue: Y = alpha acc + beta Y (Y not read when beta == 0)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t r = row0 + wr + i * 8 + g;
-    if (r >= n) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = col0 + wc + j * 8 + 2 * t;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (c + h < p) {
-          double *y = Y + r * ldy + c + h;
-          *y = beta == 0.0 ? alpha * acc[i][j][h] : alpha * acc[i][j][h] + beta * *y;
+    for (int j = 0; j < T::NT; ++j) {
+      const int yc = col0 + wc + j * 8 + 2 * t;
+      double *y = Y + yr * ldy + yc;
+      double v0 = alpha * acc[i][j][0], v1 = alpha * acc[i][j][1];
+      if (vecy && yc + 1 < p) {
+        double2 *y2 = reinterpret_cast<double2 *>(y);
+        if (beta != 0.0) {
+          const double2 o = *y2;
+          v0 += beta * o.x;
+          v1 += beta * o.y;
         }
+        *y2 = make_double2(v0, v1);
+      } else {
+        if (yc < p) y[0] = beta == 0.0 ? v0 : v0 + beta * y[0];
+        if (yc + 1 < p) y[1] = beta == 0.0 ? v1 : v1 + beta * y[1];
       }
     }
   }
 }
 
 // ------------------------------------------------------------------ gram
-// Output tile 64 (m) x 64 (k) per CTA; the CTA sums rows [r0, r1) of n in chunks of 16.
-// 8 warps as 2 (m) x 4 (k): warp tile 32 x 16 = 4 x 2 fragments.
-constexpr int GM = 64, GN = 64, GK = 16;
-constexpr int GP = 64 + 4;  // padded stage rows (doubles)
-constexpr int kGramThreads = 256;
-
+template <typename T>
 struct GramSmem {
-  double x[2][GK][GP];
-  double y[2][GK][GP];
+  double x[T::kStages][kDepth][T::M + 4];
+  double y[T::kStages][kDepth][T::N + 4];
 };
 
-__global__ void __launch_bounds__(kGramThreads)
+// Whether the tile at (m0, k0) lies below the diagonal.
+template <typename T>
+__host__ __device__ __forceinline__ bool below(int m0, int k0) { return m0 >= k0 + T::N; }
+
+// Tile (blockIdx.x, blockIdx.y) of X^T Y over the rows of split blockIdx.z; its partial product
+// column-major into the workspace.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, T::kCtas)
 gram_partial_kernel(int64_t n, int m, int k, const double *__restrict__ X, int64_t ldx,
                     const double *__restrict__ Y, int64_t ldy, int64_t rows_per_split,
                     double *__restrict__ part, bool vec16, bool upper) {
-  if (upper && blockIdx.x > blockIdx.y) return;  // a tile below the diagonal (no barrier yet)
+  const int m0 = blockIdx.x * T::M, k0 = blockIdx.y * T::N;
+  if (upper && below<T>(m0, k0)) return;  // no barrier yet
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  GramSmem &sm = *reinterpret_cast<GramSmem *>(smem_raw);
+  GramSmem<T> &sm = *reinterpret_cast<GramSmem<T> *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = (warp & 1) * 32, wk = (warp >> 1) * 16;
-  const int m0 = blockIdx.x * GM, k0 = blockIdx.y * GN;
+  const int wm = warp % T::WM * T::MT * 8, wk = warp / T::WM * T::NT * 8;
   const int64_t r0 = (int64_t)blockIdx.z * rows_per_split;
   const int64_t r1 = min(n, r0 + rows_per_split);
-  double acc[4][2][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  double acc[T::MT][T::NT][2];
+  clear<T>(acc);
   const int64_t nrows = r1 > r0 ? r1 - r0 : 0;
-  const int nc = (int)((nrows + GK - 1) / GK);
-  auto load = [&](int stage, int c) {
-    const int64_t rb = r0 + (int64_t)c * GK;
-    if (vec16 && m0 + GM <= m && k0 + GN <= k) {
-      for (int e = tid; e < GK * (GM / 2); e += kGramThreads) {
-        const int r = e / (GM / 2), c2 = (e % (GM / 2)) * 2;
-        const int64_t gr = rb + r;
-        double *dx = &sm.x[stage][r][c2];
-        double *dy = &sm.y[stage][r][c2];
-        if (gr < r1) {
-          cp_async16(dx, X + gr * ldx + m0 + c2);
-          cp_async16(dy, Y + gr * ldy + k0 + c2);
-        } else {
-          dx[0] = dx[1] = 0.0;
-          dy[0] = dy[1] = 0.0;
-        }
-      }
-    } else {
-      for (int e = tid; e < GK * GM; e += kGramThreads) {
-        const int r = e / GM, c1 = e % GM;
-        const int64_t gr = rb + r;
-        double *dx = &sm.x[stage][r][c1];
-        double *dy = &sm.y[stage][r][c1];
-        if (gr < r1 && m0 + c1 < m) cp_async8(dx, X + gr * ldx + m0 + c1);
-        else *dx = 0.0;
-        if (gr < r1 && k0 + c1 < k) cp_async8(dy, Y + gr * ldy + k0 + c1);
-        else *dy = 0.0;
-      }
+  // This thread's 16-byte copies of a whole chunk: rows rx + i * .. of X (ry of Y) at columns cx
+  // (cy); the pointers advance with the chunks.
+  constexpr int WX = T::M / 2, WY = T::N / 2;  // copies of a row
+  constexpr int SX = kThreads / WX, SY = kThreads / WY, PX = kDepth / SX, PY = kDepth / SY;
+  const int rx = tid / WX, cx = tid % WX * 2, ry = tid / WY, cy = tid % WY * 2;
+  const bool wholex = vec16 && m0 + T::M <= m, wholey = vec16 && k0 + T::N <= k;
+  const double *px = X + (r0 + rx) * ldx + m0 + cx, *py = Y + (r0 + ry) * ldy + k0 + cy;
+  const int64_t stepx = SX * ldx, stepy = SY * ldy;
+  auto slow = [&](double *dst, int pitch, int W, const double *src, int64_t ld, int c0, int cols,
+                  int64_t rb) {
+    for (int e = tid; e < kDepth * W; e += kThreads) {
+      const int rr = e / W, cc = e % W;
+      const bool ok = rb + rr < r1 && c0 + cc < cols;
+      cp_async<8>(dst + rr * pitch + cc, src + (ok ? (rb + rr) * ld + c0 + cc : 0), ok);
     }
-    cp_async_commit();
   };
-  if (nc > 0) load(0, 0);
-  for (int c = 0; c < nc; ++c) {
-    const int stage = c & 1;
-    if (c + 1 < nc) {
-      load(stage ^ 1, c + 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+  auto load = [&](int stage, int chunk) {
+    const int64_t rb = r0 + (int64_t)chunk * kDepth;
+    const bool whole = rb + kDepth <= r1;
+    if (wholex && whole) {
 #pragma unroll
-    for (int ks = 0; ks < GK; ks += 4) {
-      double a[4], b[2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = sm.x[stage][ks + t][wm + i * 8 + g];  // A = X^T
-#pragma unroll
-      for (int j = 0; j < 2; ++j) b[j] = sm.y[stage][ks + t][wk + j * 8 + g];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) mma_8x8x4(acc[i][j], a[i], b[j]);
-    }
-    __syncthreads();
-  }
-  // partial tile, column-major 64 x 64 within this CTA's slot
-  double *pt = part + (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * (GM * GN);
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int ii = wm + i * 8 + g, jj = wk + j * 8 + 2 * t + h;
-        pt[ii + jj * GM] = acc[i][j][h];
+      for (int i = 0; i < PX; ++i) {
+        cp_async<16>(&sm.x[stage][rx + i * SX][cx], px, true);
+        px += stepx;
       }
+    } else {
+      slow(&sm.x[stage][0][0], T::M + 4, T::M, X, ldx, m0, m, rb);
+    }
+    if (wholey && whole) {
+#pragma unroll
+      for (int i = 0; i < PY; ++i) {
+        cp_async<16>(&sm.y[stage][ry + i * SY][cy], py, true);
+        py += stepy;
+      }
+    } else {
+      slow(&sm.y[stage][0][0], T::N + 4, T::N, Y, ldy, k0, k, rb);
+    }
+  };
+  pipeline<T::kStages>((int)((nrows + kDepth - 1) / kDepth), load, [&](int stage) {
+    const double *a = &sm.x[stage][t][wm + g], *b = &sm.y[stage][t][wk + g];  // A = X^T
+    multiply<T>(acc, [&](int kk, int i) { return a[kk * (T::M + 4) + i * 8]; },
+                [&](int kk, int j) { return b[kk * (T::N + 4) + j * 8]; });
+  });
+  double *pt = part + (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * (T::M * T::N);
+#pragma unroll
+  for (int i = 0; i < T::MT; ++i)
+#pragma unroll
+    for (int j = 0; j < T::NT; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        pt[wm + i * 8 + g + (wk + j * 8 + 2 * t + h) * T::M] = acc[i][j][h];
 }
 
-// C[i + j ldc] = alpha * sum_s part_s(i, j) + beta * C[i + j ldc], splits summed in order.
-__global__ void gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits,
-                                   const double *__restrict__ part, double *C, int64_t ldc,
-                                   double alpha, double beta, bool upper) {
+// C[i + j ldc] = alpha * sum_s part_s(i, j) + beta * C[i + j ldc]: a CTA takes 32 elements, its
+// eight warps a share of the splits each (one thread per element took 18 us for the 79 partials of
+// a 32 x 32 product), summed in a fixed order.
+template <typename T>
+__global__ void __launch_bounds__(256)
+gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
+                   double *C, int64_t ldc, double alpha, double beta, bool upper) {
+  __shared__ double sh[8][33];
+  const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int64_t total = (int64_t)m * k;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t e0 = (int64_t)blockIdx.x * 32; e0 < total; e0 += (int64_t)gridDim.x * 32) {
+    const int64_t e = e0 + cl;
     const int i = (int)(e % m), j = (int)(e / m);
-    const int bx = i / GM, by = j / GN, ii = i % GM, jj = j % GN;
-    if (upper && bx > by) continue;  // its partials were never written
+    const int bx = i / T::M, by = j / T::N;
+    // partials below the diagonal were never written
+    const bool ok = e < total && !(upper && below<T>(bx * T::M, by * T::N));
     double s = 0.0;
-    for (int z = 0; z < splits; ++z)
-      s += part[(((int64_t)z * tiles_k + by) * tiles_m + bx) * (GM * GN) + ii + jj * GM];
-    double *c = C + i + (int64_t)j * ldc;
-    *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
+    if (ok) {
+      const int64_t stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
+      const double *p = part + ((int64_t)by * tiles_m + bx) * (T::M * T::N) + i % T::M + j % T::N * T::M;
+#pragma unroll 4
+      for (int z = rl; z < splits; z += 8) s += p[z * stride];
+    }
+    sh[rl][cl] = s;
+    __syncthreads();
+    if (rl == 0 && ok) {
+      s = 0.0;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) s += sh[r][cl];
+      double *c = C + i + (int64_t)j * ldc;
+      *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
+    }
+    __syncthreads();
   }
 }
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
+
+template <bool TB, typename T>
+void launch_update(cudaStream_t st, int64_t n, int64_t m, int64_t p, const double *X, int64_t ldx,
+                   const double *C, int64_t ldc, double *Y, int64_t ldy, double alpha, double beta) {
+  const int64_t coltiles = (p + T::N - 1) / T::N, grid = (n + T::M - 1) / T::M * coltiles;
+  require(grid < (int64_t)1 << 31, SMA_ERR_ARG, "product too large");
+  const size_t smem = sizeof(UpdateSmem<T>);
+  SMA_CUDA(cudaFuncSetAttribute(update_kernel<TB, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  update_kernel<TB, T><<<(unsigned)grid, kThreads, smem, st>>>(
+      n, (int)m, (int)p, X, ldx, C, ldc, Y, ldy, alpha, beta, (int)coltiles,
+      aligned16(X) && ldx % 2 == 0, aligned16(C) && ldc % 2 == 0, aligned16(Y) && ldy % 2 == 0);
+  SMA_CHECK_LAUNCH();
+}
+
+template <typename T>
+void launch_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, const double *X,
+                 int64_t ldx, const double *Y, int64_t ldy, double *C, int64_t ldc, double alpha,
+                 double beta, DevBuf<double> &work, bool upper) {
+  const int tm = (int)((m + T::M - 1) / T::M), tk = (int)((k + T::N - 1) / T::N);
+  int64_t tiles = (int64_t)tm * tk;
+  if (upper) {
+    tiles = 0;
+    for (int x = 0; x < tm; ++x)
+      for (int y = 0; y < tk; ++y) tiles += !below<T>(x * T::M, y * T::N);
+  }
+  // The number of splits (of at least 256 rows) with the least time: the multiplications at the
+  // share of the last wave that is filled, plus the partials' way to memory and back.
+  const int64_t slots = (int64_t)T::kCtas * num_sms, most = std::max<int64_t>(1, (n + 255) / 256);
+  int64_t splits = 1;
+  double least = 1e300;
+  for (int64_t s = 1; s <= std::min(most, std::max<int64_t>(8, 4 * slots / tiles)); ++s) {
+    const int64_t waves = (tiles * s + slots - 1) / slots;
+    const double t = (double)n / s * waves * (2.0 * T::M * T::N * slots / 35e12) +
+                     (double)(tiles * s) * (T::M * T::N * 16 / 6e12);
+    if (t < least) {
+      least = t;
+      splits = s;
+    }
+  }
+  const int64_t rows = (n + splits - 1) / splits;
+  const size_t need = (size_t)splits * tm * tk * T::M * T::N;
+  if (work.count < need) work.alloc(need, st);
+  const bool vec16 = aligned16(X) && aligned16(Y) && ldx % 2 == 0 && ldy % 2 == 0;
+  const size_t smem = sizeof(GramSmem<T>);
+  SMA_CUDA(cudaFuncSetAttribute(gram_partial_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gram_partial_kernel<T><<<dim3(tm, tk, (unsigned)splits), kThreads, smem, st>>>(
+      n, (int)m, (int)k, X, ldx, Y, ldy, rows, work.p, vec16, upper);
+  SMA_CHECK_LAUNCH();
+  const int blocks = (int)std::min<int64_t>((m * k + 31) / 32, 8LL * num_sms);
+  gram_reduce_kernel<T><<<blocks, 256, 0, st>>>((int)m, (int)k, tm, tk, (int)splits, work.p, C, ldc,
+                                                alpha, beta, upper);
+  SMA_CHECK_LAUNCH();
+}
+
+using Wide = Tile<2, 2, 4, 4>;         // 64 x 64
+using Short = Tile<2, 2, 4, 4, 2, 4>;  // the same for a short summation: more CTAs to hide its ends
+using Narrow = Tile<4, 1, 2, 4>;  // 64 x 32
+using Small = Tile<2, 2, 2, 2>;   // 32 x 32
 
 }  // namespace dmma
 
@@ -284,20 +408,17 @@ void dgemm_update(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t p,
   using namespace dmma;
   if (n == 0 || p == 0) return;
   require(m <= INT32_MAX && p <= INT32_MAX, SMA_ERR_ARG, "product too wide");
-  const bool vec16 = aligned16(X) && ldx % 2 == 0;
-  const dim3 grid((unsigned)((n + UM - 1) / UM), (unsigned)((p + UN - 1) / UN));
-  const size_t smem = sizeof(UpdateSmem);
-  if (transC) {
-    SMA_CUDA(cudaFuncSetAttribute(update_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    update_kernel<true><<<grid, kUpdateThreads, smem, st>>>(n, (int)m, (int)p, X, ldx, C, ldc, Y,
-                                                           ldy, alpha, beta, vec16);
-  } else {
-    SMA_CUDA(cudaFuncSetAttribute(update_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    update_kernel<false><<<grid, kUpdateThreads, smem, st>>>(n, (int)m, (int)p, X, ldx, C, ldc, Y,
-                                                            ldy, alpha, beta, vec16);
-  }
-  SMA_CHECK_LAUNCH();
   (void)num_sms;
+  if (p <= 32) {  // half of a wide tile would be padding
+    if (transC) launch_update<true, Narrow>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    else launch_update<false, Narrow>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+  } else if (m <= 128) {
+    if (transC) launch_update<true, Short>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    else launch_update<false, Short>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+  } else {
+    if (transC) launch_update<true, Wide>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    else launch_update<false, Wide>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+  }
 }
 
 void dgemm_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, const double *X,
@@ -306,24 +427,13 @@ void dgemm_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, c
   using namespace dmma;
   if (m == 0 || k == 0) return;
   require(m <= INT32_MAX && k <= INT32_MAX, SMA_ERR_ARG, "product too wide");
-  const int tm = (int)((m + GM - 1) / GM), tk = (int)((k + GN - 1) / GN);
-  // about two CTAs per SM over the whole grid, each summing at least 256 rows
-  const int64_t want = std::max<int64_t>(1, (2LL * num_sms) / ((int64_t)tm * tk));
-  const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(want, (n + 255) / 256));
-  const int64_t rows = (n + splits - 1) / splits;
-  const size_t need = (size_t)splits * tm * tk * GM * GN;
-  if (work.count < need) work.alloc(need, st);
-  const bool vec16 = aligned16(X) && aligned16(Y) && ldx % 2 == 0 && ldy % 2 == 0;
-  const size_t smem = sizeof(GramSmem);
-  SMA_CUDA(cudaFuncSetAttribute(gram_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gram_partial_kernel<<<dim3(tm, tk, (unsigned)splits), kGramThreads, smem, st>>>(
-      n, (int)m, (int)k, X, ldx, Y, ldy, rows, work.p, vec16, upper && m == k);
-  SMA_CHECK_LAUNCH();
-  const int64_t total = m * k;
-  const int blocks = (int)std::min<int64_t>((total + 255) / 256, 4LL * num_sms);
-  gram_reduce_kernel<<<blocks, 256, 0, st>>>((int)m, (int)k, tm, tk, (int)splits, work.p, C, ldc,
-                                             alpha, beta, upper && m == k);
-  SMA_CHECK_LAUNCH();
+  upper = upper && m == k;
+  if (m <= 32 && k <= 32)
+    launch_gram<Small>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
+  else if (k <= 32)
+    launch_gram<Narrow>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
+  else
+    launch_gram<Wide>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
 }
 
 }  // namespace sma
