@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const uint32_t r = threadIdx.x * a.divlanes >> 16;
-  const uint32_t row = bx * a.rows + r;
-  const uint32_t c0 = (by * a.lanes + threadIdx.x - r * a.lanes) * V;
+  uint32_t row = bx * a.rows + r;
+  uint32_t c0 = (by * a.lanes + threadIdx.x - r * a.lanes) * V;
   const bool in = r < a.rows && row < a.n && c0 < a.b;
   int start = 0, end = 0;
   if (in) {
@@ -289,6 +289,8 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   if constexpr (MODEL) model_rows(a, bx * a.rows, model_smem, cnt, dpos);
   pdl_wait_then_trigger();
   if (!in) return;
+  if constexpr (MODEL) row = after_wait(row);  // B1's places come from shared memory
+  else c0 = after_wait(c0);
   const uint64_t own = row * a.ldb;
   if constexpr (HB) prefetch_l2(at(a.B2 + c0, own));
   T acc[V];
@@ -352,14 +354,19 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
   const uint32_t gx = (a.n + a.rows - 1) / a.rows;
-  // Fewer than six waves of 8-CTA residency: a step is then a latency, not a stream, and more
-  // gathers in flight at a lower occupancy are the faster kernel (Anderson L = 20, b = 64
-  // FP64: 3.7 us against 5.0; with 2 M threads 43.8 against 42.5; ragged rows, U = 6 against 4:
-  // XXZ L = 18, b = 32 12.3 against 13.6, with 1.5 M threads 51.0 against 48.0), for ragged rows
-  // once more below one wave (U = 8 against 6: XXZ L = 16, b = 32 4.0 against 5.2, L = 18 12.6
-  // against 12.3).
+  // Waves of 8-CTA residency decide what a step's time is.  Six and more: a stream, which wants
+  // every warp it can get.  Below, more and more a latency, which wants more gathers in flight at
+  // less occupancy -- unless a row has no more than four.  Us a step, step after step:
+  //   Anderson L = 20, b = 64 FP64 (0.85 waves)  exact U = 8 4.0, U = 4 5.6
+  //   Anderson L = 64, b = 64 FP32 (14)          exact U = 8 43.8, U = 4 42.5
+  //   1D Laplacian n = 20000, b = 32 FP32 (0.5)  exact U = 8 3.2, U = 4 2.9
+  //   XXZ L = 16, b = 32 FP64 (0.7)              ragged U = 8 4.5, U = 6 5.7, U = 4 5.5
+  //   XXZ L = 18, b = 32 FP64 (2.6)              ragged U = 8 13.4, U = 6 13.1, U = 4 13.6
+  //   XXZ L = 20, b = 64 FP32 (9.8)              ragged U = 6 51.0, U = 4 48.0
   const int64_t wave = 8LL * kThreads * op->ctx->num_sms, threads = (int64_t)a.n * vecs;
-  if (gathers == 0) gathers = threads >= 6 * wave ? 4 : !ragged(op) || threads < wave ? 8 : 6;
+  const bool uneven = ragged(op);
+  if (gathers == 0)
+    gathers = threads >= 6 * wave || op->nnz <= 4 * op->n ? 4 : uneven && threads >= 2 * wave ? 6 : 8;
   constexpr uint32_t kGridY = 65535;
   const uint32_t ny = (vecs + a.lanes - 1) / a.lanes;
   const uint32_t span = kGridY * a.lanes * V, width = a.b;
@@ -373,7 +380,7 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
-    if (ragged(op)) {
+    if (uneven) {
       if (gathers == 8) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
       else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
       else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
@@ -459,9 +466,10 @@ void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
 
 inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
 
-// Picks the vector width: the widest that widths, strides and addresses allow, but narrower
-// while the step would not give every SM a CTA (Anderson L = 12, b = 8), or with ragged rows half
-// a CTA (XXZ L = 14, b = 8 FP64: 2.6 and 2.1 us a step with 4 and 2 columns a thread).
+// Picks the vector width: the widest that widths, strides and addresses allow, but half of it
+// below 40000 threads, and less while the step would not give every SM half a CTA (us a step:
+// Anderson L = 16, b = 32 FP64, 32768 threads 2.6, 65536 2.4; L = 20, b = 64 FP32, 64000 threads
+// 2.9, 128000 3.2; XXZ L = 14, b = 32 FP64, 27456 threads 3.1, 54912 2.8).
 template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
@@ -485,8 +493,13 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
            aligned(a.out, bytes) && (!HQ || (a.ldq % bytes == 0 && aligned(a.Q, bytes))) &&
            (!HB || aligned(a.B2, bytes)) && (!PC || a.colseg || aligned(a.cseg, bytes));
   };
-  const int64_t want = (int64_t)op->ctx->num_sms * kThreads / (ragged(op) ? 2 : 1);
-  auto take = [&](int v) { return fits(v) && op->n * (b / v) >= want; };
+  int widest = 32 / (int)sizeof(T);
+  while (widest > 1 && !fits(widest)) widest /= 2;
+  auto take = [&](int v) {
+    const int64_t threads = op->n * (b / v);
+    return v < widest ? fits(v) && threads >= 64LL * op->ctx->num_sms
+                      : v == widest && threads >= 40000;
+  };
   if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL>(op, st, a);
   if constexpr (sizeof(T) == 4)
     if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC, MODEL>(op, st, a);

@@ -49,6 +49,13 @@ __device__ __forceinline__ void ldv(const T *__restrict__ p, T (&f)[V]) {
   memcpy(f, w, sizeof(w));
 }
 
+// An index through which every address after the wait for the previous kernel is formed: ties the
+// loads there, which the compiler could otherwise hoist past the wait.
+__device__ __forceinline__ uint32_t after_wait(uint32_t i) {
+  asm volatile("" : "+r"(i)::"memory");
+  return i;
+}
+
 // ldv where ok, else zeros: the access itself is predicated, nothing branches.
 template <typename T, int V>
 __device__ __forceinline__ void ldv_if(bool ok, const T *__restrict__ p, T (&f)[V]) {

@@ -305,3 +305,31 @@ def test_model_steps_equal_the_stored_matrix(lib_built, stencil, b):
         assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
     else:
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("rows", ["equal", "short", "ragged"])
+@pytest.mark.parametrize("b", [32, 64])
+@pytest.mark.parametrize("threads", [9472, 40000, 303104, 909312])
+def test_filter_at_the_edges_of_the_step_rule(lib_built, rows, b, threads):
+    """The step's gathers in flight and columns a thread follow the number of threads (n b / 4 and
+    n b / 2 for FP64): one row below and exactly at each line of the rule, for rows of one length,
+    of at most four entries and of all lengths, against the oracle."""
+    import sparse_matrix_algorithms_b200 as S
+
+    at = threads * (2 if threads == 9472 else 4) // b
+    for n in (at - 1, at):
+        if rows == "ragged":
+            d = np.where(np.arange(n) % 3 == 0, 1.0, 0.0)  # a third of the rows has far entries
+            off = [sp.diags([d[:n - k] * d[k:] * 0.1], [k]) for k in (3, 6, 9, 12, 15)]
+            A = M._canonical((sum(off) + sum(off).T + 0.5 * M.lap1d(n)).tocsr())
+        elif rows == "equal":
+            off = [sp.diags([np.full(n - k, -1.0 / k)], [k]) for k in (1, 7, 50)]
+            A = M._canonical((sum(off) + sum(off).T + sp.diags([np.cos(np.arange(n))], [0])).tocsr())
+        else:
+            A = M.lap1d(n)
+        smin, smax = _bounds(A)
+        Q = M.splitmix_normal(b, n, b)
+        c = O.build_coeffs(5, smin, smax, 0.1, -0.4, 0.3, "step", True)
+        ref = O.apply_poly_block(A, Q, c, smin, smax)
+        got = S.apply_poly_block(A, Q, c, smin, smax)
+        assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
