@@ -118,3 +118,40 @@ def test_update_in_place_triangular_inverse(lib_built):
     got = Xd.cpu().numpy()
     ref = X @ Rinv
     assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("m,p", [(1, 1), (31, 32), (33, 31), (128, 33), (129, 64), (127, 32), (200, 65)])
+def test_products_at_the_edges_of_their_tiles(lib_built, m, p):
+    """Tile choices change at 32 columns and at 128 summands: both sides, with an aligned and an
+    odd leading dimension, n one off a multiple of the tile; tolerances as above."""
+    import sparse_matrix_algorithms_b200 as S
+
+    ctx = S.context()
+    rng = np.random.default_rng(m + p)
+    for n in (63, 64, 4097):
+        for pad in (m % 2, 1 - m % 2):
+            X, B = rng.standard_normal((n, m + pad)), rng.standard_normal((m, p))
+            Y0 = rng.standard_normal((n, p + pad))
+            Y = _update(ctx, X, np.ascontiguousarray(B.T), p, False, Y0, 0.5, -2.0, m)
+            ref = 0.5 * X[:, :m] @ B - 2.0 * Y0[:, :p]
+            assert np.abs(Y[:, :p] - ref).max() <= 1e-13 * max((np.abs(X[:, :m]) @ np.abs(B)).max(), 8.0)
+            assert np.array_equal(Y[:, p:], Y0[:, p:])
+            C = _gram(ctx, X, Y0, m, p)
+            scale = (np.abs(X[:, :m]).T @ np.abs(Y0[:, :p])).max()
+            assert np.abs(C.T - X[:, :m].T @ Y0[:, :p]).max() <= 1e-13 * max(scale, 1.0)
+
+
+@pytest.mark.parametrize("k", [1, 31, 32, 33, 64])
+def test_update_in_place_of_every_width(lib_built, k):
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    rng = np.random.default_rng(k)
+    n = 1000
+    X, B = rng.standard_normal((n, k)), rng.standard_normal((k, k))
+    Xd, Cd = _dev(X), _dev(B.T)
+    torch.cuda.synchronize()
+    L.check(L.load().sma_dense_update_dev(S.context().handle, n, k, k, Xd.data_ptr(), k, Cd.data_ptr(),
+                                          k, 0, Xd.data_ptr(), k, 1.0, 0.0))
+    assert np.abs(Xd.cpu().numpy() - X @ B).max() <= 1e-13 * max((np.abs(X) @ np.abs(B)).max(), 1.0)

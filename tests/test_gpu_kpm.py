@@ -64,3 +64,17 @@ def test_kpm_count_tracks_dense_count(lib_built):
         exact = int(np.sum((lam >= a) & (lam <= b)))
         est = S.kpm_count(mu, A.shape[0], smin, smax, a, b)
         assert abs(est - exact) <= 0.1 * exact + 4, (a, b, est, exact)
+
+
+@pytest.mark.parametrize("n", [64, 1331])
+@pytest.mark.parametrize("R", [1, 3, 16, 33])
+@pytest.mark.parametrize("M_", [3, 34])
+def test_kpm_moments_of_ragged_blocks(lib_built, n, R, M_):
+    """Blocks of odd widths (the recurrence runs on padded rows), few rows and odd moment counts."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.lap1d(n) if n == 64 else M.anderson3d(11, 16.5, 1)
+    smin, smax = O.gershgorin_bounds(A)
+    _, pv = S.kpm_moments(A, M_, R, smin=smin, smax=smax, seed=2, per_vector=True)
+    _, pvo = O.kpm_moments(A, M_, R, 2, smin, smax, per_vector=True)
+    np.testing.assert_allclose(pv, pvo, rtol=0, atol=1e-11)
