@@ -62,8 +62,9 @@ struct Step {
   T *out;
   const T *cseg;      // per-column coefficients (PC), else null
   const int *colseg;  // PC: the coefficient of column c is cseg[colseg[c]], or cseg[c] when null
+  const T *topseg;    // PC: the highest coefficients, like cseg
   uint64_t ldq, ldb, ldo;
-  T ck, alpha, beta;
+  T ck, top, alpha, beta;
   uint32_t n, b;      // rows, columns
   uint32_t lanes;     // vectors of a row in one panel
   uint32_t rows;      // rows of a CTA (rows * lanes <= kThreads)
@@ -101,10 +102,23 @@ struct ModelRow {  // entry `dpos` is the diagonal
   __device__ __forceinline__ T val(int j) const { return j == dpos ? diag : off; }
 };
 
+// What the gathered rows are multiplied with before they enter the product: nothing, or in the
+// first step of a recurrence the highest coefficient (rounded like the block c_K Q it replaces).
+struct Unscaled {
+  template <typename T>
+  __device__ __forceinline__ T operator()(T x, int) const { return x; }
+};
+template <typename T, int V>
+struct Scaled {
+  const T (&c)[V];
+  __device__ __forceinline__ T operator()(T x, int i) const { return mul_rn(c[i], x); }
+};
+
 // R consecutive entries from j: all R gathers are issued before the first FMA; FMAs in
 // ascending entry order.
-template <typename T, int V, int R, bool W, typename Row>
-__device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint64_t ldb, T (&acc)[V]) {
+template <typename T, int V, int R, bool W, typename Row, typename F>
+__device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint64_t ldb, T (&acc)[V],
+                                      F f) {
   int c[R];
   T x[R][V], v[R];
 #pragma unroll
@@ -116,23 +130,23 @@ __device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint6
 #pragma unroll
   for (int u = 0; u < R; ++u)
 #pragma unroll
-    for (int i = 0; i < V; ++i) acc[i] = fma(v[u], x[u][i], acc[i]);
+    for (int i = 0; i < V; ++i) acc[i] = fma(v[u], f(x[u][i], i), acc[i]);
 }
 
 // acc += the row's entries [j, end): chunks of U, then the r < U remaining entries as ONE chunk
 // of exactly r (a switch over r).
-template <typename T, int V, int U, bool W, typename Row>
+template <typename T, int V, int U, bool W, typename Row, typename F>
 __device__ __forceinline__ void row_product(const Row &row, int j, int end, const T *B1c,
-                                            uint64_t ldb, T (&acc)[V]) {
-  for (; j + U <= end; j += U) chunk<T, V, U, W>(row, j, B1c, ldb, acc);
+                                            uint64_t ldb, T (&acc)[V], F f) {
+  for (; j + U <= end; j += U) chunk<T, V, U, W>(row, j, B1c, ldb, acc, f);
   switch (end - j) {
-    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(row, j, B1c, ldb, acc); break;
-    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(row, j, B1c, ldb, acc); break;
-    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(row, j, B1c, ldb, acc); break;
-    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(row, j, B1c, ldb, acc); break;
-    case 3: chunk<T, V, 3, W>(row, j, B1c, ldb, acc); break;
-    case 2: chunk<T, V, 2, W>(row, j, B1c, ldb, acc); break;
-    case 1: chunk<T, V, 1, W>(row, j, B1c, ldb, acc); break;
+    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(row, j, B1c, ldb, acc, f); break;
+    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(row, j, B1c, ldb, acc, f); break;
+    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(row, j, B1c, ldb, acc, f); break;
+    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(row, j, B1c, ldb, acc, f); break;
+    case 3: chunk<T, V, 3, W>(row, j, B1c, ldb, acc, f); break;
+    case 2: chunk<T, V, 2, W>(row, j, B1c, ldb, acc, f); break;
+    case 1: chunk<T, V, 1, W>(row, j, B1c, ldb, acc, f); break;
     default: break;
   }
 }
@@ -142,9 +156,9 @@ __device__ __forceinline__ void row_product(const Row &row, int j, int end, cons
 // one code path; with the exact chunks above each remainder is a path of its own, and the warp
 // waits for the gathers of all of them in turn (XXZ L = 16, b = 32: 5.3 -> 4.0 us a step FP64,
 // 4.1 -> 3.1 FP32; L = 18 13.2 -> 12.3).  An absent entry adds 0 * 0.
-template <typename T, int V, int U, bool W, typename Row>
+template <typename T, int V, int U, bool W, typename Row, typename F>
 __device__ __forceinline__ void ragged_product(const Row &row, int j, int end, const T *B1c,
-                                               uint64_t ldb, T (&acc)[V]) {
+                                               uint64_t ldb, T (&acc)[V], F f) {
   for (; j < end; j += U) {
     int c[U];
     T x[U][V], v[U];
@@ -161,7 +175,7 @@ __device__ __forceinline__ void ragged_product(const Row &row, int j, int end, c
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < V; ++i) acc[i] = fma(v[u], x[u][i], acc[i]);
+      for (int i = 0; i < V; ++i) acc[i] = fma(v[u], f(x[u][i], i), acc[i]);
   }
 }
 
@@ -249,26 +263,31 @@ __device__ __forceinline__ void model_rows(const Step<T> &a, uint32_t row0, int 
   __syncthreads();
 }
 
-// The Q coefficients of the thread's V columns.
+// The coefficients of the thread's V columns: c in all, or from cseg.
 template <typename T, int V, bool PC>
-__device__ __forceinline__ void coefficients(const Step<T> &a, uint32_t c0, T (&ck)[V]) {
+__device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cseg, uint32_t c0,
+                                             T (&ck)[V]) {
   if constexpr (!PC) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) ck[i] = a.ck;
+    for (int i = 0; i < V; ++i) ck[i] = c;
   } else if (a.colseg == nullptr) {  // one polynomial per column: its coefficients side by side
-    ldv<T, V>(a.cseg + c0, ck);
+    ldv<T, V>(cseg + c0, ck);
   } else {  // segments are runs of columns: equal ends, one coefficient
     const int s0 = __ldg(a.colseg + c0), s1 = __ldg(a.colseg + c0 + V - 1);
-    ck[0] = __ldg(a.cseg + s0);
+    ck[0] = __ldg(cseg + s0);
 #pragma unroll
     for (int i = 1; i < V; ++i)
-      ck[i] = s0 == s1 ? ck[0] : __ldg(a.cseg + __ldg(a.colseg + c0 + i));
+      ck[i] = s0 == s1 ? ck[0] : __ldg(cseg + __ldg(a.colseg + c0 + i));
   }
 }
 
+// Where in a recurrence a step stands.  B1 = c_K Q, the block that it starts from, is never
+// written: the first step gathers it from Q, and the second, whose B2 it is, has Q's row anyway.
+enum Place { INNER, FIRST, SECOND };
+
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
-          bool RAGGED>
+          bool RAGGED, Place P>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
@@ -292,25 +311,36 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   if constexpr (MODEL) row = after_wait(row);  // B1's places come from shared memory
   else c0 = after_wait(c0);
   const uint64_t own = row * a.ldb;
-  if constexpr (HB) prefetch_l2(at(a.B2 + c0, own));
-  T acc[V];
+  if constexpr (HB && P != SECOND) prefetch_l2(at(a.B2 + c0, own));
+  T acc[V], top[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = T(0);
+  if constexpr (P == FIRST) coefficients<T, V, PC>(a, a.top, a.topseg, c0, top);
+  auto product = [&](const auto &row, int j, int end, auto f) {
+    if constexpr (RAGGED) ragged_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, f);
+    else row_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, f);
+  };
+  auto gather = [&](const auto &row, int j, int end) {
+    if constexpr (P == FIRST) product(row, j, end, Scaled<T, V>{top});
+    else product(row, j, end, Unscaled{});
+  };
   if constexpr (MODEL) {
     const T diag = a.kind == OP_LAP1D ? T(2) : (T)__ldg(a.model.diag + row);
-    const ModelRow<T> mr{model_smem + r * a.entries, dpos[r], diag, (T)a.model.hop};
-    if constexpr (RAGGED) ragged_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
-    else row_product<T, V, U, W>(mr, 0, cnt[r], a.B1 + c0, a.ldb, acc);
+    gather(ModelRow<T>{model_smem + r * a.entries, dpos[r], diag, (T)a.model.hop}, 0, cnt[r]);
   } else {
-    const CsrRow<T> cr{a.colind, a.val};
-    if constexpr (RAGGED) ragged_product<T, V, U, W>(cr, start, end, a.B1 + c0, a.ldb, acc);
-    else row_product<T, V, U, W>(cr, start, end, a.B1 + c0, a.ldb, acc);
+    gather(CsrRow<T>{a.colind, a.val}, start, end);
   }
   T q[V], s[V], t[V], ck[V], o[V];
   if constexpr (HQ) ldv<T, V, false>(at(a.Q + c0, row * a.ldq), q);
-  if constexpr (HB) ldv<T, V, false>(at(a.B2 + c0, own), t);
-  if constexpr (HS) ldv<T, V>(at(a.B1 + c0, own), s);
-  if constexpr (HQ) coefficients<T, V, PC>(a, c0, ck);
+  if constexpr (HB && P != SECOND) ldv<T, V, false>(at(a.B2 + c0, own), t);
+  if constexpr (HS && P != FIRST) ldv<T, V>(at(a.B1 + c0, own), s);
+  if constexpr (HQ) coefficients<T, V, PC>(a, a.ck, a.cseg, c0, ck);
+  if constexpr (P == SECOND) coefficients<T, V, PC>(a, a.top, a.topseg, c0, top);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    if constexpr (P == FIRST) s[i] = mul_rn(top[i], q[i]);
+    if constexpr (P == SECOND) t[i] = mul_rn(top[i], q[i]);
+  }
 #pragma unroll
   for (int i = 0; i < V; ++i)
     o[i] = clenshaw_combine<HQ, HS, HB>(acc[i], q[i], s[i], t[i], ck[i], a.alpha, a.beta);
@@ -327,7 +357,7 @@ namespace rows {
 
 // ------------------------------------------------------------------ launch
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
-          bool RAGGED>
+          bool RAGGED, Place P>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -338,14 +368,16 @@ void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = op->ctx->pdl ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED>, a));
+  // the first step gathers the caller's Q, which the grid before may have read and written in
+  // place: it starts after that grid has ended, with nothing of it in L1
+  cfg.numAttrs = op->ctx->pdl && P != FIRST ? 1 : 0;
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED, P>, a));
   SMA_CHECK_LAUNCH();
 }
 
 inline bool ragged(const sma_op *op) { return op->kind == OP_XXZ || op->ragged; }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL, Place P>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
   const uint32_t vecs = a.b / V;
   // as few panels as keep a row within kPanel vectors, each a multiple of 4 vectors (128 bytes)
@@ -376,17 +408,20 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
       a.out += span;
       if (HQ) a.Q += span;
       if (HB) a.B2 += span;
-      if (PC) { if (a.colseg) a.colseg += span; else a.cseg += span; }
+      if (PC) { if (a.colseg) a.colseg += span; else { a.cseg += span; if (P != INNER) a.topseg += span; } }
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
-    if (uneven) {
-      if (gathers == 8) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
-      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
-      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true>(op, st, a, grid);
+    if constexpr (P == FIRST) {  // the coefficients take registers too, and it is one step
+      if (uneven) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+      else launch<T, V, 4, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
+    } else if (uneven) {
+      if (gathers == 8) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
     } else {
-      if (gathers == 8) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false>(op, st, a, grid);
-      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false>(op, st, a, grid);
+      if (gathers == 8) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
     }
   }
 }
@@ -405,7 +440,7 @@ template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
 void launch_config(const sma_op *op, cudaStream_t st, const Step<T> &a, const Config &c) {
   if constexpr (!PC)
     if (c.bulk) return launch_bulk<T, V, HQ, HS, HB>(op, st, a);
-  launch_width<T, V, HQ, HS, HB, PC, false, false>(op, st, a, c.gathers);
+  launch_width<T, V, HQ, HS, HB, PC, false, false, INNER>(op, st, a, c.gathers);
 }
 
 template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
@@ -457,11 +492,11 @@ bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
   return true;
 }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool MODEL, Place P>
 void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
-  if constexpr (!MODEL)
+  if constexpr (!MODEL && P == INNER)
     if (tuned_step<T, V, HQ, HS, HB, PC>(op, st, a)) return;
-  launch_width<T, V, HQ, HS, HB, PC, false, MODEL>(op, st, a);
+  launch_width<T, V, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
 }
 
 inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
@@ -470,7 +505,7 @@ inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) ==
 // below 40000 threads, and less while the step would not give every SM half a CTA (us a step:
 // Anderson L = 16, b = 32 FP64, 32768 threads 2.6, 65536 2.4; L = 20, b = 64 FP32, 64000 threads
 // 2.9, 128000 3.2; XXZ L = 14, b = 32 FP64, 27456 threads 3.1, 54912 2.8).
-template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL>
+template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL, Place P = INNER>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
   require(b < (int64_t)1 << 31, SMA_ERR_ARG, "block too wide");
@@ -491,7 +526,8 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
     const int bytes = v * (int)sizeof(T);
     return b % v == 0 && a.ldb % bytes == 0 && a.ldo % bytes == 0 && aligned(a.B1, bytes) &&
            aligned(a.out, bytes) && (!HQ || (a.ldq % bytes == 0 && aligned(a.Q, bytes))) &&
-           (!HB || aligned(a.B2, bytes)) && (!PC || a.colseg || aligned(a.cseg, bytes));
+           (!HB || P == SECOND || aligned(a.B2, bytes)) &&
+           (!PC || a.colseg || (aligned(a.cseg, bytes) && (P == INNER || aligned(a.topseg, bytes))));
   };
   int widest = 32 / (int)sizeof(T);
   while (widest > 1 && !fits(widest)) widest /= 2;
@@ -500,20 +536,19 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
     return v < widest ? fits(v) && threads >= 64LL * op->ctx->num_sms
                       : v == widest && threads >= 40000;
   };
-  if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL>(op, st, a);
+  if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL, P>(op, st, a);
   if constexpr (sizeof(T) == 4)
-    if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC, MODEL>(op, st, a);
-  if (take(4)) return launch_rule<T, 4, HQ, HS, HB, PC, MODEL>(op, st, a);
-  if (take(2)) return launch_rule<T, 2, HQ, HS, HB, PC, MODEL>(op, st, a);
-  launch_width<T, 1, HQ, HS, HB, PC, false, MODEL>(op, st, a);
+    if (take(8)) return launch_rule<T, 8, HQ, HS, HB, PC, MODEL, P>(op, st, a);
+  if (take(4)) return launch_rule<T, 4, HQ, HS, HB, PC, MODEL, P>(op, st, a);
+  if (take(2)) return launch_rule<T, 2, HQ, HS, HB, PC, MODEL, P>(op, st, a);
+  launch_width<T, 1, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
 }
 
 }  // namespace rows
 
-template <typename T, bool MODEL>
-void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
-                   const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                   double alpha, double beta, bool has_self, bool rev) {
+template <typename T>
+rows::Step<T> clenshaw_arguments(const T *Q, int64_t ldq, const T *B1, const T *B2, int64_t ldb, T *out,
+                                 int64_t ldo, double alpha, double beta, bool rev) {
   rows::Step<T> a{};
   a.Q = Q;
   a.B1 = B1;
@@ -522,14 +557,35 @@ void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int
   a.ldq = (uint64_t)ldq * sizeof(T);
   a.ldb = (uint64_t)ldb * sizeof(T);
   a.ldo = (uint64_t)ldo * sizeof(T);
-  a.ck = (T)ck;
   a.alpha = (T)alpha;
   a.beta = (T)beta;
   a.rev = rev;
+  return a;
+}
+
+template <typename T, bool MODEL>
+void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                   const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
+                   double alpha, double beta, bool has_self, bool rev) {
+  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
+  a.ck = (T)ck;
   if (Q && has_self && B2) return rows::step<T, true, true, true, false, MODEL>(op, st, b, a);
   if (Q && has_self && !B2) return rows::step<T, true, true, false, false, MODEL>(op, st, b, a);
   if (!Q && !has_self && !B2) return rows::step<T, false, false, false, false, MODEL>(op, st, b, a);
   throw Error(SMA_ERR_INTERNAL, "unsupported Clenshaw step variant");
+}
+
+// The first step of a recurrence (B1 null: it is c_top Q) and the second (B2 is c_top Q).
+template <typename T, bool MODEL>
+void clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
+                    int64_t ldb, T *out, int64_t ldo, double top, double ck, double alpha, double beta,
+                    bool rev) {
+  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1 ? B1 : Q, nullptr, B1 ? ldb : ldq, out, ldo, alpha,
+                                          beta, rev);
+  a.ck = (T)ck;
+  a.top = (T)top;
+  if (B1) rows::step<T, true, true, true, false, MODEL, rows::SECOND>(op, st, b, a);
+  else rows::step<T, true, true, false, false, MODEL, rows::FIRST>(op, st, b, a);
 }
 
 }  // namespace sma

@@ -11,26 +11,37 @@ void csr_clenshaw_step<double>(const sma_op *op, cudaStream_t st, int64_t b, con
   clenshaw_step<double, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
 }
 
+template <>
+void csr_clenshaw_start<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
+                                const double *B1, int64_t ldb, double *out, int64_t ldo, double top,
+                                double ck, double alpha, double beta, bool rev) {
+  clenshaw_start<double, false>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
+}
+
 // The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
 // cseg[c] when colseg is null; Q, B1 and B2 are all read.
 template <>
 void csr_clenshaw_step_seg<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
                            const double *B1, const double *B2, int64_t ldb, double *out, int64_t ldo,
                            const double *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  rows::Step<double> a{};
-  a.Q = Q;
-  a.B1 = B1;
-  a.B2 = B2;
-  a.out = out;
+  rows::Step<double> a = clenshaw_arguments<double>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
   a.cseg = cseg;
   a.colseg = colseg;
-  a.ldq = (uint64_t)ldq * sizeof(double);
-  a.ldb = (uint64_t)ldb * sizeof(double);
-  a.ldo = (uint64_t)ldo * sizeof(double);
-  a.alpha = (double)alpha;
-  a.beta = (double)beta;
-  a.rev = rev;
   rows::step<double, true, true, true, true, false>(op, st, b, a);
+}
+
+// Its first step (B1 null) and second, topseg the highest coefficients.
+template <>
+void csr_clenshaw_start_seg<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
+                            const double *B1, int64_t ldb, double *out, int64_t ldo, const double *topseg,
+                            const double *cseg, const int *colseg, double alpha, double beta, bool rev) {
+  rows::Step<double> a = clenshaw_arguments<double>(Q, ldq, B1 ? B1 : Q, nullptr, B1 ? ldb : ldq, out, ldo,
+                                                alpha, beta, rev);
+  a.topseg = topseg;
+  a.cseg = cseg;
+  a.colseg = colseg;
+  if (B1) rows::step<double, true, true, true, true, false, rows::SECOND>(op, st, b, a);
+  else rows::step<double, true, true, false, true, false, rows::FIRST>(op, st, b, a);
 }
 
 }  // namespace sma

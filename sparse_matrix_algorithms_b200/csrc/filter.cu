@@ -145,17 +145,45 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   const double beta = -2.0 * c * invd;
   const bool fused = op->kind != OP_MATBLOCK && op->kind != OP_CSR_HALF;
   const double blk = (double)n * (double)b * sizeof(T);
+  const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   T *B1 = work.b1.p, *B2 = work.b2.p, *TMP = work.tmp.p;
   const int64_t ld = w;
-  // step K+1 of the reference: B1 = c_K Q (its product multiplies zeros)
-  launch_scale_block<T>(st, n, w, Q, ldq, B1, ld, coeffs[K]);
-  fc.bytes += 2 * blk;
-  bool b2_zero = true;
-  const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
-  for (int64_t ci = K - 1; ci >= 1; --ci) {
+  auto rotate = [&]() {  // B1, B2, TMP = TMP, B1, B2
+    T *t = B2;
+    B2 = B1;
+    B1 = TMP;
+    TMP = t;
+  };
+  // Step K+1 of the reference is B1 = c_K Q (its product multiplies zeros).  With a fused step the
+  // next two form it from Q, which they read anyhow: two passes over a block and a launch less
+  // (Anderson L = 64: FP32 b = 768, K = 16 10.0 -> 9.56 ms; per-column b = 496, K = 24, whose zero
+  // blocks and first product are gone too, 10.57 -> 10.02 ms).  A first step
+  // that is also the last could write to the Q that it gathers (Y = Q): it takes the block.
+  const bool fold = fused && K >= 2;
+  int64_t ci = K - 1;
+  if (fold) {
+    launch_clenshaw_start<T>(op, st, w, Q, ldq, nullptr, ld, TMP, ld, coeffs[K], coeffs[ci], alpha, beta,
+                             ci & 1);
+    fc.steps += 1;
+    fc.bytes += mat_bytes + 2 * blk;
+    B1 = TMP;
+    TMP = work.b1.p;
+    --ci;
+    if (ci >= 1) {
+      launch_clenshaw_start<T>(op, st, w, Q, ldq, B1, ld, TMP, ld, coeffs[K], coeffs[ci], alpha, beta, ci & 1);
+      fc.steps += 1;
+      fc.bytes += mat_bytes + 3 * blk;
+      rotate();
+      --ci;
+    }
+  } else {
+    launch_scale_block<T>(st, n, w, Q, ldq, B1, ld, coeffs[K]);
+    fc.bytes += 2 * blk;
+  }
+  bool b2_zero = !fold;
+  for (; ci >= 1; --ci) {
     if (fused) {
-      launch_clenshaw_step<T>(op, st, w, Q, ldq, B1, b2_zero ? nullptr : B2, ld, TMP, ld,
-                              coeffs[ci], alpha, beta, true, ci & 1);
+      launch_clenshaw_step<T>(op, st, w, Q, ldq, B1, B2, ld, TMP, ld, coeffs[ci], alpha, beta, true, ci & 1);
     } else {
       matblock_apply<T>(op, st, B1, work.ax.p, ld, b);
       launch_clenshaw_axpy<T>(st, n, b, Q, ldq, work.ax.p, ld, B1, b2_zero ? nullptr : B2, ld,
@@ -163,14 +191,14 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
     }
     fc.steps += 1;
     fc.bytes += mat_bytes + (b2_zero ? 3 : 4) * blk;
-    T *t = B2;  // B1, B2, TMP = TMP, B1, B2
-    B2 = B1;
-    B1 = TMP;
-    TMP = t;
+    rotate();
     b2_zero = false;
   }
   // final step: Y = c_0 Q + invd*A B1 - c*invd*B1 - B2
-  if (fused) {
+  if (fold && K == 2) {
+    launch_clenshaw_start<T>(op, st, b, Q, ldq, B1, ld, Y, ldy, coeffs[K], coeffs[0], invd, -(c * invd));
+    b2_zero = true;  // not read
+  } else if (fused) {
     launch_clenshaw_step<T>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, ld, Y, ldy, coeffs[0],
                             invd, -(c * invd), true, false);
   } else {
@@ -268,7 +296,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     const double blk = (double)n * (double)b * sizeof(T);
     const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
     fc.steps = K;
-    fc.bytes = 2 * blk + (mat_bytes + 3 * blk) + (double)(K - 1) * (mat_bytes + 4 * blk);
+    fc.bytes = (mat_bytes + 2 * blk) + (mat_bytes + 3 * blk) + (double)(K - 2) * (mat_bytes + 4 * blk);
   }
   SMA_CUDA(cudaGraphLaunch(work.exec, st));
   g_kernel_launches.fetch_add(work.g_launches);

@@ -332,6 +332,20 @@ void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T 
 }
 
 template <typename T>
+void launch_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                           const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,
+                           double alpha, double beta, bool rev) {
+  if (op->n == 0 || b == 0) return;
+  if (op->kind == OP_CSR) {
+    csr_clenshaw_start<T>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
+  } else if (op->kind == OP_LAP1D || op->kind == OP_ANDERSON || op->kind == OP_XXZ) {
+    model_clenshaw_start<T>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
+  } else {
+    throw Error(SMA_ERR_INTERNAL, "fused Clenshaw step needs a device operator");
+  }
+}
+
+template <typename T>
 void launch_scale_block(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq, T *out,
                         int64_t ldo, double ck) {
   const int64_t total = n * b;
@@ -388,6 +402,12 @@ template void launch_clenshaw_step<double>(const sma_op *, cudaStream_t, int64_t
 template void launch_clenshaw_step<float>(const sma_op *, cudaStream_t, int64_t, const float *,
                                           int64_t, const float *, const float *, int64_t, float *,
                                           int64_t, double, double, double, bool, bool);
+template void launch_clenshaw_start<double>(const sma_op *, cudaStream_t, int64_t, const double *,
+                                            int64_t, const double *, int64_t, double *, int64_t, double,
+                                            double, double, double, bool);
+template void launch_clenshaw_start<float>(const sma_op *, cudaStream_t, int64_t, const float *,
+                                           int64_t, const float *, int64_t, float *, int64_t, double,
+                                           double, double, double, bool);
 template void launch_scale_block<double>(cudaStream_t, int64_t, int64_t, const double *, int64_t,
                                          double *, int64_t, double);
 template void launch_scale_block<float>(cudaStream_t, int64_t, int64_t, const float *, int64_t,

@@ -11,4 +11,11 @@ void model_clenshaw_step<double>(const sma_op *op, cudaStream_t st, int64_t b, c
   clenshaw_step<double, true>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
 }
 
+template <>
+void model_clenshaw_start<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q,
+                                  int64_t ldq, const double *B1, int64_t ldb, double *out, int64_t ldo,
+                                  double top, double ck, double alpha, double beta, bool rev) {
+  clenshaw_start<double, true>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
+}
+
 }  // namespace sma

@@ -95,19 +95,37 @@ void filter_noalloc(sma_op *op, const double *coeffs, int64_t K, double smin, do
   if (K == 0) {
     launch_scale_block<double>(st, n, b, Q, ldq, Y, ldy, coeffs[0]);
   } else {
-    launch_scale_block<double>(st, n, b, Q, ldq, B1, b, coeffs[K]);
-    bool b2_zero = true;
-    for (int64_t ci = K - 1; ci >= 1; --ci) {
-      launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, b, TMP, b,
-                                   coeffs[ci], alpha, beta, true, ci & 1);
+    auto rotate = [&]() {
       double *t = B2;
       B2 = B1;
       B1 = TMP;
       TMP = t;
-      b2_zero = false;
+    };
+    int64_t ci = K - 1;
+    const bool fold = K >= 2;  // B1 = c_K Q is never written (record_filter)
+    if (fold) {
+      launch_clenshaw_start<double>(op, st, b, Q, ldq, nullptr, b, TMP, b, coeffs[K], coeffs[ci], alpha,
+                                    beta, ci & 1);
+      std::swap(B1, TMP);
+      if (--ci >= 1) {
+        launch_clenshaw_start<double>(op, st, b, Q, ldq, B1, b, TMP, b, coeffs[K], coeffs[ci], alpha,
+                                      beta, ci & 1);
+        rotate();
+        --ci;
+      }
+    } else {
+      launch_scale_block<double>(st, n, b, Q, ldq, B1, b, coeffs[K]);
     }
-    launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, b2_zero ? nullptr : B2, b, Y, ldy,
-                                 coeffs[0], invd, -(c * invd), true, false);
+    for (; ci >= 1; --ci) {
+      launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, B2, b, TMP, b, coeffs[ci], alpha, beta, true,
+                                   ci & 1);
+      rotate();
+    }
+    if (K == 2)
+      launch_clenshaw_start<double>(op, st, b, Q, ldq, B1, b, Y, ldy, coeffs[K], coeffs[0], invd, -(c * invd));
+    else
+      launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, fold ? B2 : nullptr, b, Y, ldy, coeffs[0], invd,
+                                   -(c * invd), true, false);
   }
   SMA_CUDA(cudaStreamSynchronize(st));
   check_bulk_error(op, st);  // a bulk-copy step reports a wait that gave up

@@ -98,8 +98,9 @@ int grid_of(int64_t total) {
 // Y = q(A_hat) Q where column j of the n x b blocks (ld = b) runs its own polynomial with
 // coefficients coef[m * b + j], m = 0..K (row-major (K+1) x b table, FP32 or FP64 like
 // the blocks).  B1, B2, TMP (and AX for operators without a fused step) are n x b work
-// blocks.  The recurrence starts from zero
-// blocks, so its first product multiplies zeros (one extra step out of K+1).
+// blocks.  The recurrence starts from zero blocks, so its first product multiplies zeros (one
+// extra step out of K+1); with the fused step and K >= 2 it starts from c_K Q, which the next two
+// steps form from Q (record_filter in filter.cu): neither that step nor the zero blocks are there.
 template <typename T>
 FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int64_t K,
                           double smin, double smax, const T *Q, T *Y, int64_t b, T *B1, T *B2,
@@ -109,10 +110,7 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
   require(op->kind != OP_MATBLOCK, SMA_ERR_ARG, "the per-column filter needs a device operator");
   const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
   const double alpha = 2.0 * invd, beta = -2.0 * c * invd;
-  const size_t bytes = (size_t)(n * b) * sizeof(T);
-  SMA_CUDA(cudaMemsetAsync(B1, 0, bytes, st));
-  SMA_CUDA(cudaMemsetAsync(B2, 0, bytes, st));
-  const bool fused = op->kind == OP_CSR;
+  const bool fused = op->kind == OP_CSR, fold = fused && K >= 2;
   auto step = [&](const T *crow, T *out, double al, double be, bool rev) {
     if (fused) {
       csr_clenshaw_step_seg<T>(op, st, b, Q, b, B1, B2, b, out, b, crow, nullptr, al, be, rev);
@@ -128,17 +126,40 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
   };
   const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   const double blk = (double)n * (double)b * sizeof(T);
-  for (int64_t k = K; k >= 1; --k) {
-    step(coef + k * b, TMP, alpha, beta, k & 1);
-    T *t = B2;  // B1, B2, TMP = TMP, B1, B2
+  auto rotate = [&]() {  // B1, B2, TMP = TMP, B1, B2
+    T *t = B2;
     B2 = B1;
     B1 = TMP;
     TMP = t;
+  };
+  auto start = [&](int64_t k, const T *b1, T *out, double al, double be) {
+    csr_clenshaw_start_seg<T>(op, st, b, Q, b, b1, b, out, b, coef + K * b, coef + k * b, nullptr, al, be,
+                              k & 1);
+  };
+  int64_t k = K;
+  if (fold) {
+    start(--k, nullptr, TMP, alpha, beta);
+    std::swap(B1, TMP);
+    if (--k >= 1) {
+      start(k--, B1, TMP, alpha, beta);
+      rotate();
+    }
+    fc.steps = K;
+    fc.bytes = (double)K * (mat_bytes + 4 * blk) - 3 * blk;
+  } else {
+    const size_t bytes = (size_t)(n * b) * sizeof(T);
+    SMA_CUDA(cudaMemsetAsync(B1, 0, bytes, st));
+    SMA_CUDA(cudaMemsetAsync(B2, 0, bytes, st));
+    fc.steps = K + 1;
+    fc.bytes = (double)(K + 1) * (mat_bytes + 4 * blk);
   }
-  step(coef, Y, invd, -(c * invd), false);
+  for (; k >= 1; --k) {
+    step(coef + k * b, TMP, alpha, beta, k & 1);
+    rotate();
+  }
+  if (fold && K == 2) start(0, B1, Y, invd, -(c * invd));
+  else step(coef, Y, invd, -(c * invd), false);
   check_bulk_error(op, st);
-  fc.steps = K + 1;
-  fc.bytes = (double)(K + 1) * (mat_bytes + 4 * blk);
   return fc;
 }
 

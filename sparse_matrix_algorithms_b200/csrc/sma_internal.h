@@ -197,7 +197,21 @@ template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
                           double alpha, double beta, bool has_self, bool rev = false);
-// The CSR and the model form of launch_clenshaw_step (csr_clenshaw_*.cu, model_clenshaw_*.cu).
+// The first two steps of a recurrence, whose block c_top Q is not written: B1 = c_top Q (B1 null),
+// and B2 = c_top Q.  The first must not write to Q.
+template <typename T>
+void launch_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                           const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,
+                           double alpha, double beta, bool rev = false);
+// The CSR and the model form of both (csr_clenshaw_*.cu, model_clenshaw_*.cu).
+template <typename T>
+void model_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                          const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,
+                          double alpha, double beta, bool rev);
+template <typename T>
+void csr_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                        const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,
+                        double alpha, double beta, bool rev);
 template <typename T>
 void model_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                          const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
@@ -215,6 +229,11 @@ template <typename T>
 void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
                            const T *cseg, const int *colseg, double alpha, double beta, bool rev);
+// Its first step (B1 null) and second, topseg the highest coefficients.
+template <typename T>
+void csr_clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                            const T *B1, int64_t ldb, T *out, int64_t ldo, const T *topseg,
+                            const T *cseg, const int *colseg, double alpha, double beta, bool rev);
 // out = ck * Q
 template <typename T>
 void launch_scale_block(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq, T *out,

@@ -333,3 +333,42 @@ def test_filter_at_the_edges_of_the_step_rule(lib_built, rows, b, threads):
         ref = O.apply_poly_block(A, Q, c, smin, smax)
         got = S.apply_poly_block(A, Q, c, smin, smax)
         assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
+
+
+@pytest.mark.parametrize("kind", ["csr", "anderson", "xxz"])
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+@pytest.mark.parametrize("b", [1, 5, 24])
+def test_first_steps_of_every_recurrence(lib_built, kind, K, b):
+    """The block c_K Q is folded into the first two steps: the degrees at which those are also the
+    last, in place (Y = Q) and not, through the block, the allocation-free and the per-column
+    entry."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    op, A = {"csr": lambda: (S.SparseOperator(_ragged(333, 4)), _ragged(333, 4)),
+             "anderson": lambda: (S.AndersonOperator(7, 16.5, 5), M.anderson3d(7, 16.5, 5)),
+             "xxz": lambda: (S.XXZOperator(10, 5.0, 1), M.xxz_sz0(10, 5.0, 1))}[kind]()
+    n = A.shape[0]
+    smin, smax = _bounds(A)
+    Q = M.splitmix_normal(K, n, b)
+    c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+    ref = O.apply_poly_block(A, Q, c, smin, smax)
+    table = np.ascontiguousarray(np.repeat(c[:, None], b, axis=1))
+    lib, scale = L.load(), max(np.abs(ref).max(), np.abs(Q).max())
+    for in_place in (False, True):
+        for entry in ("block", "noalloc", "percol"):
+            dQ = _device(Q)
+            dY = dQ if in_place else torch.full_like(dQ, 7.0)
+            torch.cuda.synchronize()
+            if entry == "block":
+                rc = lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, dQ.data_ptr(), b,
+                                                  dY.data_ptr(), b, b, 0)
+            elif entry == "noalloc":
+                rc = lib.sma_apply_poly_block_noalloc(op.handle, c.ctypes.data, K, smin, smax,
+                                                      dQ.data_ptr(), b, dY.data_ptr(), b, b)
+            else:
+                rc = lib.sma_apply_poly_block_percol_dev(op.handle, table.ctypes.data, K, smin, smax,
+                                                         dQ.data_ptr(), dY.data_ptr(), b, 0)
+            L.check(rc)
+            assert np.abs(dY.cpu().numpy() - ref).max() <= 1e-12 * scale, (entry, in_place)
