@@ -44,4 +44,19 @@ void csr_clenshaw_start_seg<double>(const sma_op *op, cudaStream_t st, int64_t b
   else rows::step<double, true, true, false, true, false, rows::FIRST>(op, st, b, a);
 }
 
+void csr_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                       double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                       double *dots, int64_t plane) {
+  clenshaw_dots<false>(op, st, b, Q, B1, out, ck, alpha, beta, rev, cols, dots, plane);
+}
+
+// The CTAs of a DOTS step, 0 where a pass of its own is as good: a CTA's sums are 2 / rows of a
+// block, written once and read once, against the two blocks of the pass.
+int64_t clenshaw_dot_chunks(const sma_op *op, int64_t b) {
+  if (op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF) return 0;
+  const int v = rows::vector_width<double>(op, b, [&](int w) { return b % w == 0; });
+  const int64_t rows = rows::kThreads / (b / v);
+  return b / v <= 16 ? (op->n + rows - 1) / rows : 0;
+}
+
 }  // namespace sma

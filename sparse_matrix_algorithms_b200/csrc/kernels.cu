@@ -345,6 +345,16 @@ void launch_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T
   }
 }
 
+void launch_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                          double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                          double *dots, int64_t plane) {
+  if (op->n == 0 || b == 0) return;
+  if (op->kind == OP_CSR)
+    csr_clenshaw_dots(op, st, b, Q, B1, out, ck, alpha, beta, rev, cols, dots, plane);
+  else
+    model_clenshaw_dots(op, st, b, Q, B1, out, ck, alpha, beta, rev, cols, dots, plane);
+}
+
 template <typename T>
 void launch_scale_block(cudaStream_t st, int64_t n, int64_t b, const T *Q, int64_t ldq, T *out,
                         int64_t ldo, double ck) {

@@ -9,7 +9,10 @@
 // T_{k+1} = 2 A_hat T_k - T_{k-1} is the fused Clenshaw step of the filter with
 // Q = T_{k-1} and coefficient -1; the doubling identities
 //   mu_{2k} = 2 <T_k, T_k> - mu_0,   mu_{2k+1} = 2 <T_{k+1}, T_k> - mu_1
-// give two moments per sparse product, so M moments take ceil(M/2) products.
+// give two moments per sparse product, so M moments take ceil(M/2) products.  The step sums both
+// dots itself where it can (DOTS in clenshaw_step.cuh): us for 256 moments, with a pass over the two
+// blocks after each step and without, Anderson L = 20 R = 16 1105 and 379, L = 64 R = 32 10695 and
+// 7863, XXZ L = 20 R = 16 5428 and 4384.
 #include <cmath>
 
 #include "sma_internal.h"
@@ -55,11 +58,18 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   // `batch` steps are summed by one launch
   const bool product_then_axpy = op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF;
   const int64_t w = product_then_axpy ? R : recurrence_width(R, sizeof(double));
-  const int64_t chunks = column_chunks(n, R), set = 2 * chunks * R;
-  const int64_t steps = (M + 1) / 2;
+  // The step's own sums where a set of them is small (256 MB), in kGroup chunks to a first sum,
+  // zeros after the last; else a pass over the two blocks.
+  constexpr int64_t kGroup = 64;
+  int64_t chunks = (clenshaw_dot_chunks(op, w) + kGroup - 1) / kGroup * kGroup;
+  const bool fused = chunks > 0 && 2 * chunks * R <= int64_t(32) << 20;
+  if (!fused) chunks = column_chunks(n, R);
+  const int64_t set = 2 * chunks * R;
+  const int64_t steps = (M + 1) / 2, fused_steps = fused ? M / 2 : 0;
   const int64_t batch = std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
   DevBuf<double> t0(n * w, st), t1(n * w, st), t2(n * w, st), dots(2 * steps * R, st),
-      partial(batch * set, st);
+      partial(batch * set, st), sums(fused ? batch * 2 * (chunks / kGroup) * R : 0, st);
+  if (fused) SMA_CUDA(cudaMemsetAsync(partial.p, 0, (size_t)(batch * set) * sizeof(double), st));
   {
     const int64_t total = n * w;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16);
@@ -68,16 +78,19 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   }
   // out = ck Q + alpha A B1 + beta B1: the fused step for device operators, the caller's
   // block product followed by the axpy kernel for callback operators
-  DevBuf<double> ax;
+  DevBuf<double> ax, last;
   if (product_then_axpy) ax.alloc(n * R, st);
   auto step = [&](const double *Q, const double *B1, double *out, double ck, double alpha,
-                  double beta, bool rev) {
+                  double beta, bool rev, double *slot) {
+    if (fused)
+      return launch_clenshaw_dots(op, st, w, Q, B1, out, ck, alpha, beta, rev, R, slot, chunks * R);
     if (product_then_axpy) {
       op_apply(op, st, B1, R, ax.p, R, R);
       launch_clenshaw_axpy<double>(st, n, R, Q, R, ax.p, R, B1, nullptr, R, out, R, ck, alpha, beta);
     } else {
       launch_clenshaw_step<double>(op, st, w, Q, w, B1, nullptr, w, out, w, ck, alpha, beta, true, rev);
     }
+    column_partials(st, 2, n, R, out, w, B1, w, nullptr, slot);
   };
   // dots: for k = 0, 1, ...: <T_{k+1}, T_k> then <T_k, T_k> (R values each)
   double *Tprev = t0.p, *Tcur = t0.p, *Tnext = t1.p, *Tfree = t2.p;
@@ -86,15 +99,24 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
     double *slot = partial.p + (k - done) * set;
     if (2 * k + 1 < M) {
       if (k == 0)  // T1 = A_hat T0 = invd A T0 - c invd T0 (Q term with coefficient 0)
-        step(Tcur, Tcur, Tnext, 0.0, invd, -c * invd, false);
+        step(Tcur, Tcur, Tnext, 0.0, invd, -c * invd, false, slot);
       else  // T_{k+1} = 2 invd A T_k - 2 c invd T_k - T_{k-1}
-        step(Tprev, Tcur, Tnext, -1.0, 2.0 * invd, -2.0 * c * invd, k & 1);
-      column_partials(st, 2, n, R, Tnext, w, Tcur, w, nullptr, slot);
-    } else {  // an odd M: the last moment needs <T_k, T_k> only
+        step(Tprev, Tcur, Tnext, -1.0, 2.0 * invd, -2.0 * c * invd, k & 1, slot);
+    } else if (fused) {  // an odd M: the last moment needs <T_k, T_k> only
+      column_reduce(st, 0, n, R, Tcur, w, Tcur, w, nullptr, dots.p + (2 * k + 1) * R, last);
+    } else {
       column_partials(st, 2, n, R, Tcur, w, Tcur, w, nullptr, slot);
     }
-    if (k + 1 - done == batch || k + 1 == steps) {
-      column_totals(st, 0, chunks, R, 2 * (k + 1 - done), partial.p, dots.p + 2 * done * R);
+    if (fused ? k + 1 <= fused_steps && (k + 1 - done == batch || k + 1 == fused_steps)
+              : k + 1 - done == batch || k + 1 == steps) {
+      const int64_t groups = 2 * (k + 1 - done);
+      double *out = dots.p + 2 * done * R;
+      if (fused) {
+        column_totals(st, 0, kGroup, R, groups * (chunks / kGroup), partial.p, sums.p);
+        column_totals(st, 0, chunks / kGroup, R, groups, sums.p, out);
+      } else {
+        column_totals(st, 0, chunks, R, groups, partial.p, out);
+      }
       done = k + 1;
     }
     double *t = k == 0 ? Tfree : Tprev;

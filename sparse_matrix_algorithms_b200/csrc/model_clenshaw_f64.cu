@@ -18,4 +18,10 @@ void model_clenshaw_start<double>(const sma_op *op, cudaStream_t st, int64_t b, 
   clenshaw_start<double, true>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
 }
 
+void model_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                         double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                         double *dots, int64_t plane) {
+  clenshaw_dots<true>(op, st, b, Q, B1, out, ck, alpha, beta, rev, cols, dots, plane);
+}
+
 }  // namespace sma

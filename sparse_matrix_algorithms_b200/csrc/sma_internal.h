@@ -203,7 +203,20 @@ template <typename T>
 void launch_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,
                            double alpha, double beta, bool rev = false);
-// The CSR and the model form of both (csr_clenshaw_*.cu, model_clenshaw_*.cu).
+// out = ck Q + alpha A B1 + beta B1 on n x b blocks (ld = b), and per CTA the sums of out B1 over
+// its rows in the first `cols` columns: dots[chunk cols + col], `plane` later those of B1 B1.
+// clenshaw_dot_chunks: the number of CTAs, 0 where this step is not to be used.
+int64_t clenshaw_dot_chunks(const sma_op *op, int64_t b);
+void launch_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                          double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                          double *dots, int64_t plane);
+void csr_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                       double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                       double *dots, int64_t plane);
+void model_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
+                         double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
+                         double *dots, int64_t plane);
+// The CSR and the model form of the others (csr_clenshaw_*.cu, model_clenshaw_*.cu).
 template <typename T>
 void model_clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, int64_t ldb, T *out, int64_t ldo, double top, double ck,

@@ -78,3 +78,20 @@ def test_kpm_moments_of_ragged_blocks(lib_built, n, R, M_):
     _, pv = S.kpm_moments(A, M_, R, smin=smin, smax=smax, seed=2, per_vector=True)
     _, pvo = O.kpm_moments(A, M_, R, 2, smin, smax, per_vector=True)
     np.testing.assert_allclose(pv, pvo, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("R", [2, 12, 20, 40, 64, 72])
+@pytest.mark.parametrize("kind", ["csr", "anderson", "xxz"])
+def test_kpm_dots_of_every_row_layout(lib_built, kind, R):
+    """The step sums its own dots per CTA where 16 or fewer threads make a row (in shuffles, or a
+    tree for other counts than powers of two), else a pass of its own does: a last CTA with rows
+    missing, more CTAs than one group of the second stage, an odd number of moments."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.xxz_sz0(14, 5.0, 1) if kind == "xxz" else M.anderson3d(15, 16.5, 1)
+    op = {"csr": lambda: S.SparseOperator(A), "anderson": lambda: S.AndersonOperator(15, 16.5, 1),
+          "xxz": lambda: S.XXZOperator(14, 5.0, 1)}[kind]()
+    smin, smax = O.gershgorin_bounds(A)
+    _, pv = S.kpm_moments(op, 21, R, smin=smin, smax=smax, seed=3, per_vector=True)
+    _, pvo = O.kpm_moments(A, 21, R, 3, smin, smax, per_vector=True)
+    np.testing.assert_allclose(pv, pvo, rtol=0, atol=1e-11)
