@@ -203,6 +203,7 @@ int sma_op_create_csc(sma_ctx *ctx, int64_t n, int64_t nnz, const int64_t *colpt
     int64_t uneven = 0;
     for (int64_t i = 1; i < n; ++i) uneven += rp[i + 1] - rp[i] != rp[i] - rp[i - 1];
     op->ragged = uneven > n / 10;
+    op->band = banded_width(n, rp, ci);
     try {
       cudaStream_t st = ctx->stream;
       SMA_CUDA(cudaMalloc((void **)&op->rowptr, (n + 1) * sizeof(int)));
@@ -316,6 +317,7 @@ int sma_op_create_lap1d(sma_ctx *ctx, int64_t n, sma_op **out) {
     op->kind = OP_LAP1D;
     op->n = n;
     op->nnz = 3 * n - 2;
+    op->band = n > 2 ? 1 : 0;
     op->sym_state = 1;
     *out = op;
   });

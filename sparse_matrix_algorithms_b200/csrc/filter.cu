@@ -29,14 +29,16 @@ void ClenshawWork<T>::ensure(const sma_op *op, int64_t n_, int64_t b, cudaStream
   tmp.alloc(n * b, st);
   q.release();
   y.release();
+  b3.release();
   if (op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF) ax.alloc(n * b, st);
 }
 
 template <typename T>
-bool ClenshawWork<T>::fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t st) {
+bool ClenshawWork<T>::fits_with(DevBuf<T> &extra, const sma_op *op, int64_t n_, int64_t w,
+                                cudaStream_t st) {
   try {
     ensure(op, n_, w, st);
-    if (!q.p) q.alloc(n * bcap, st);
+    if (!extra.p) extra.alloc(n * bcap, st);
     return true;
   } catch (const Error &e) {
     if (e.code != SMA_ERR_NOMEM) throw;
@@ -45,6 +47,7 @@ bool ClenshawWork<T>::fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t
     b2.release();
     tmp.release();
     q.release();
+    b3.release();
     bcap = 0;
     return false;
   }
@@ -234,6 +237,10 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
   const bool persistent = op->kind == OP_CSR && op->ctx->persistent && K >= kGraphMinDegree;
   int64_t w = b;
   bool stage = false;  // run on a copy of Q: half a step's time, for a gain with every step
+  if (!persistent && banded_fits(op, K, Q, ldq, Y, ldy, b) && work.fits_with(work.b3, op, n, b, st)) {
+    T *const buf[4] = {work.b1.p, work.b2.p, work.tmp.p, work.b3.p};
+    return banded_filter<T>(op, st, &coeffs, nullptr, K, smin, smax, Q, ldq, Y, ldy, b, buf);
+  }
   if (fused && !persistent && K >= kPadMinDegree) {
     w = recurrence_width(b, sizeof(T));
     int64_t vec = 32;  // the access that w allows

@@ -111,6 +111,20 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
   const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
   const double alpha = 2.0 * invd, beta = -2.0 * c * invd;
   const bool fused = op->kind == OP_CSR, fold = fused && K >= 2;
+  if (banded_fits(op, K, Q, b, Y, b, b)) {
+    DevBuf<T> fourth;
+    try {
+      fourth.alloc(n * b, st);
+    } catch (const Error &e) {  // no memory for it: a step a launch
+      if (e.code != SMA_ERR_NOMEM) throw;
+      cudaGetLastError();
+      fourth.count = 0;
+    }
+    if (fourth.p) {
+      T *const buf[4] = {B1, B2, TMP, fourth.p};
+      return banded_filter<T>(op, st, nullptr, coef, K, smin, smax, Q, b, Y, b, b, buf);
+    }
+  }
   auto step = [&](const T *crow, T *out, double al, double be, bool rev) {
     if (fused) {
       csr_clenshaw_step_seg<T>(op, st, b, Q, b, B1, B2, b, out, b, crow, nullptr, al, be, rev);

@@ -123,6 +123,7 @@ struct sma_op {
   int64_t n = 0, nnz = 0;
   // CSR (== CSC of the symmetric matrix), 0-based, int32 indices
   int *rowptr = nullptr;
+  int band = 0;  // rows hold exactly the entries |i - j| <= band (1 or 2, else 0; banded.cu)
   int *colind = nullptr;  // kRowPad zeros follow the arrays of OP_CSR
   double *val64 = nullptr;
   float *val32 = nullptr;  // created on first FP32 use
@@ -334,6 +335,7 @@ std::vector<double> build_coeffs(int64_t degree, double smin, double smax, doubl
 template <typename T>
 struct ClenshawWork {
   DevBuf<T> b1, b2, tmp, ax, q, y, coef;
+  DevBuf<T> b3;                // banded filter: a fourth block
   DevBuf<unsigned> barrier;  // persistent filter: arrival count, generation, error flag
   int64_t n = 0, bcap = 0;
   // graph cache
@@ -346,7 +348,8 @@ struct ClenshawWork {
   cudaGraphExec_t exec = nullptr;
   void ensure(const sma_op *op, int64_t n_, int64_t b, cudaStream_t st);
   // ensure() and the staging block of Q; false, with nothing held, when memory does not allow it
-  bool fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t st);
+  bool fits(const sma_op *op, int64_t n_, int64_t w, cudaStream_t st) { return fits_with(q, op, n_, w, st); }
+  bool fits_with(DevBuf<T> &extra, const sma_op *op, int64_t n_, int64_t w, cudaStream_t st);
   void drop_graph();
   ClenshawWork() = default;
   ClenshawWork(const ClenshawWork &) = delete;
@@ -371,6 +374,16 @@ FilterCount persistent_filter(const sma_op *op, cudaStream_t st, const std::vect
                               double smin, double smax, const T *Q, int64_t ldq, T *Y, int64_t ldy,
                               int64_t b, T *buf0, T *buf1, T *buf2, T *coeff_dev,
                               unsigned *barrier_words);
+
+// The filter of an operator with op->band > 0, many steps a launch (banded.cu), where banded_fits:
+// coeffs, or the (K+1) x b table of a per-column filter.  buf: four n x b blocks.
+template <typename T>
+bool banded_fits(const sma_op *op, int64_t K, const T *Q, int64_t ldq, const T *Y, int64_t ldy, int64_t b);
+template <typename T>
+FilterCount banded_filter(const sma_op *op, cudaStream_t st, const std::vector<double> *coeffs,
+                          const T *table, int64_t K, double smin, double smax, const T *Q, int64_t ldq,
+                          T *Y, int64_t ldy, int64_t b, T *const buf[4]);
+int banded_width(int64_t n, const std::vector<int> &rowptr, const std::vector<int> &cols);
 
 // persistent.cu: the bounded grid barrier with a missing CTA; SMA_ERR_TIMEOUT expected
 int barrier_selftest(sma_ctx *ctx);

@@ -372,3 +372,70 @@ def test_first_steps_of_every_recurrence(lib_built, kind, K, b):
                                                          dQ.data_ptr(), dY.data_ptr(), b, 0)
             L.check(rc)
             assert np.abs(dY.cpu().numpy() - ref).max() <= 1e-12 * scale, (entry, in_place)
+
+
+def _band(n, w, seed):
+    rng = np.random.default_rng(seed)
+    off = [sp.diags([rng.uniform(0.5, 1.0, n - k)], [k]) for k in range(1, w + 1)]
+    return M._canonical((sum(off) + sum(off).T + sp.diags([rng.uniform(-1, 1, n)], [0])).tocsr())
+
+
+@pytest.mark.parametrize("w,n", [(1, 3), (1, 257), (1, 1500), (2, 5), (2, 130), (2, 1111)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("b", [1, 7, 8, 9, 40])
+def test_banded_filter_equals_the_step_by_step_one(lib_built, w, n, precision, b):
+    """Operators with a full narrow band take many steps a launch, halo rows recomputed; in place
+    they take one (other CTAs still read Q).  Bit for bit the same, for numbers of steps around
+    those of a launch, and equal to the oracle; so is the per-column filter, whose columns differ."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    A = _band(n, w, n + b)
+    smin, smax = _bounds(A)
+    op, lib = S.SparseOperator(A), L.load()
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    rtol = 1e-12 if precision == "fp64" else 2e-4
+    Q = torch.zeros((n, b + 3), dtype=dt, device="cuda")
+    Q[:, :b] = torch.as_tensor(M.splitmix_normal(b, n, b), device="cuda").to(dt)
+    Qh = Q[:, :b].double().cpu().numpy()
+    for K in (1, 2, 7, 8, 9, 16, 33, 70):
+        c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+        ref = O.apply_poly_block(A, Qh, c, smin, smax)
+        Y = torch.full((n, b + 1), 3.0, dtype=dt, device="cuda")
+        Z = Q.clone()
+        P, R = Q[:, :b].contiguous(), torch.empty((n, b), dtype=dt, device="cuda")
+        torch.cuda.synchronize()
+        for src, out in ((Q, Y), (Z, Z)):
+            L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, src.data_ptr(),
+                                                 b + 3, out.data_ptr(), out.shape[1], b,
+                                                 L.PRECISIONS[precision]))
+        table = np.ascontiguousarray(c[:, None] * np.linspace(1.0, 2.0, b)[None, :])
+        L.check(lib.sma_apply_poly_block_percol_dev(op.handle, table.ctypes.data, K, smin, smax,
+                                                    P.data_ptr(), R.data_ptr(), b, L.PRECISIONS[precision]))
+        scale = max(np.abs(ref).max(), np.abs(Qh).max())
+        assert torch.equal(Y[:, :b], Z[:, :b]), K
+        assert bool((Y[:, b:] == 3.0).all())
+        assert np.abs(Y[:, :b].double().cpu().numpy() - ref).max() <= rtol * scale
+        assert np.abs(R.double().cpu().numpy() / np.linspace(1.0, 2.0, b) - ref).max() <= rtol * scale
+
+
+def test_band_of_the_laplacian_stencil_and_of_other_matrices(lib_built):
+    """The 1D Laplacian stencil equals its stored matrix; a periodic chain, a band with a missing
+    entry and a wider one keep the step kernel."""
+    import sparse_matrix_algorithms_b200 as S
+
+    n = 700
+    ring = sp.lil_matrix(M.lap1d(n))
+    ring[0, n - 1] = ring[n - 1, 0] = -1.0
+    hole = sp.lil_matrix(M.lap1d(n))
+    hole[350, 351] = hole[351, 350] = 0.0
+    for op, A in ((S.Lap1dOperator(n), M.lap1d(n)), (None, ring), (None, hole), (None, _band(n, 3, 1))):
+        A = M._canonical(sp.csr_matrix(A))
+        A.eliminate_zeros()
+        smin, smax = _bounds(A)
+        c = O.build_coeffs(50, smin, smax, 0.1, -0.4, 0.3, "step", True)
+        Q = M.splitmix_normal(3, n, 12)
+        ref = O.apply_poly_block(A, Q, c, smin, smax)
+        got = S.apply_poly_block(A if op is None else op, Q, c, smin, smax)
+        assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
