@@ -459,13 +459,36 @@ int sma_apply_poly_block_percol_dev(sma_op *op, const double *coeffs, int64_t K,
     cudaStream_t st = op->ctx->stream;
     auto run = [&](auto zero) {
       using T = decltype(zero);
-      std::vector<T> ch((K + 1) * b);
-      for (int64_t i = 0; i < (K + 1) * b; ++i) ch[i] = (T)coeffs[i];
-      DevBuf<T> coef(ch.size(), st), B1(n * b, st), B2(n * b, st), TMP(n * b, st), AX;
-      if (op->kind != OP_CSR) AX.alloc(n * b, st);
+      // a width that wide accesses divide, Q copied, as in apply_poly_block; without the memory, b
+      const int64_t w = op->kind == OP_CSR_HALF || op->band ? b : recurrence_width(b, sizeof(T));
+      DevBuf<T> coef, B1, B2, TMP, AX, Qw;
+      auto allocate = [&](int64_t width) {
+        coef.alloc((K + 1) * width, st);
+        B1.alloc(n * width, st);
+        B2.alloc(n * width, st);
+        TMP.alloc(n * width, st);
+        if (op->kind == OP_CSR_HALF) AX.alloc(n * width, st);
+        if (width != b) Qw.alloc(n * width, st);
+      };
+      int64_t width = K >= 4 ? w : b;  // below, the copy costs what it gains
+      try {
+        allocate(width);
+      } catch (const Error &e) {
+        if (e.code != SMA_ERR_NOMEM || width == b) throw;
+        cudaGetLastError();
+        Qw.release();
+        allocate(width = b);
+      }
+      std::vector<T> ch((K + 1) * width, T(0));
+      for (int64_t k = 0; k <= K; ++k)
+        for (int64_t j = 0; j < b; ++j) ch[k * width + j] = (T)coeffs[k * b + j];
       SMA_CUDA(cudaMemcpyAsync(coef.p, ch.data(), ch.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-      percol_filter<T>(op, st, coef.p, K, smin, smax, (const T *)Q_dev, (T *)Y_dev, b, B1.p, B2.p,
-                       TMP.p, AX.p);
+      const T *Q = (const T *)Q_dev;
+      if (width != b) {
+        launch_pad_block<T, T>(st, n, b, Q, b, width, Qw.p, width);
+        Q = Qw.p;
+      }
+      percol_filter<T>(op, st, coef.p, K, smin, smax, Q, (T *)Y_dev, width, B1.p, B2.p, TMP.p, AX.p, b);
       SMA_CUDA(cudaStreamSynchronize(st));
     };
     if (precision == SMA_PREC_FP64) {

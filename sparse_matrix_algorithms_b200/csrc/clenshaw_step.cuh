@@ -649,6 +649,32 @@ void clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, in
   else rows::step<T, true, true, false, false, MODEL, rows::FIRST>(op, st, b, a);
 }
 
+// The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
+// cseg[c] when colseg is null; Q, B1 and B2 are all read.
+template <typename T, bool MODEL>
+void clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
+                       const T *B2, int64_t ldb, T *out, int64_t ldo, const T *cseg, const int *colseg,
+                       double alpha, double beta, bool rev) {
+  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
+  a.cseg = cseg;
+  a.colseg = colseg;
+  rows::step<T, true, true, true, true, MODEL>(op, st, b, a);
+}
+
+// Its first step (B1 null) and second, topseg the highest coefficients.
+template <typename T, bool MODEL>
+void clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
+                        int64_t ldb, T *out, int64_t ldo, const T *topseg, const T *cseg, const int *colseg,
+                        double alpha, double beta, bool rev) {
+  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1 ? B1 : Q, nullptr, B1 ? ldb : ldq, out, ldo, alpha,
+                                          beta, rev);
+  a.topseg = topseg;
+  a.cseg = cseg;
+  a.colseg = colseg;
+  if (B1) rows::step<T, true, true, true, true, MODEL, rows::SECOND>(op, st, b, a);
+  else rows::step<T, true, true, false, true, MODEL, rows::FIRST>(op, st, b, a);
+}
+
 // out = ck Q + alpha A B1 + beta B1, with the sums of a DOTS step (n x b blocks, ld = b).
 template <bool MODEL>
 void clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,

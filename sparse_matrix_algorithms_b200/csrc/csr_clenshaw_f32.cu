@@ -18,30 +18,18 @@ void csr_clenshaw_start<float>(const sma_op *op, cudaStream_t st, int64_t b, con
   clenshaw_start<float, false>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
 }
 
-// The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
-// cseg[c] when colseg is null; Q, B1 and B2 are all read.
 template <>
 void csr_clenshaw_step_seg<float>(const sma_op *op, cudaStream_t st, int64_t b, const float *Q, int64_t ldq,
                            const float *B1, const float *B2, int64_t ldb, float *out, int64_t ldo,
                            const float *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  rows::Step<float> a = clenshaw_arguments<float>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
-  a.cseg = cseg;
-  a.colseg = colseg;
-  rows::step<float, true, true, true, true, false>(op, st, b, a);
+  clenshaw_step_seg<float, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, cseg, colseg, alpha, beta, rev);
 }
 
-// Its first step (B1 null) and second, topseg the highest coefficients.
 template <>
 void csr_clenshaw_start_seg<float>(const sma_op *op, cudaStream_t st, int64_t b, const float *Q, int64_t ldq,
                             const float *B1, int64_t ldb, float *out, int64_t ldo, const float *topseg,
                             const float *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  rows::Step<float> a = clenshaw_arguments<float>(Q, ldq, B1 ? B1 : Q, nullptr, B1 ? ldb : ldq, out, ldo,
-                                                alpha, beta, rev);
-  a.topseg = topseg;
-  a.cseg = cseg;
-  a.colseg = colseg;
-  if (B1) rows::step<float, true, true, true, true, false, rows::SECOND>(op, st, b, a);
-  else rows::step<float, true, true, false, true, false, rows::FIRST>(op, st, b, a);
+  clenshaw_start_seg<float, false>(op, st, b, Q, ldq, B1, ldb, out, ldo, topseg, cseg, colseg, alpha, beta, rev);
 }
 
 }  // namespace sma

@@ -18,30 +18,18 @@ void csr_clenshaw_start<double>(const sma_op *op, cudaStream_t st, int64_t b, co
   clenshaw_start<double, false>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
 }
 
-// The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
-// cseg[c] when colseg is null; Q, B1 and B2 are all read.
 template <>
 void csr_clenshaw_step_seg<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
                            const double *B1, const double *B2, int64_t ldb, double *out, int64_t ldo,
                            const double *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  rows::Step<double> a = clenshaw_arguments<double>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
-  a.cseg = cseg;
-  a.colseg = colseg;
-  rows::step<double, true, true, true, true, false>(op, st, b, a);
+  clenshaw_step_seg<double, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, cseg, colseg, alpha, beta, rev);
 }
 
-// Its first step (B1 null) and second, topseg the highest coefficients.
 template <>
 void csr_clenshaw_start_seg<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
                             const double *B1, int64_t ldb, double *out, int64_t ldo, const double *topseg,
                             const double *cseg, const int *colseg, double alpha, double beta, bool rev) {
-  rows::Step<double> a = clenshaw_arguments<double>(Q, ldq, B1 ? B1 : Q, nullptr, B1 ? ldb : ldq, out, ldo,
-                                                alpha, beta, rev);
-  a.topseg = topseg;
-  a.cseg = cseg;
-  a.colseg = colseg;
-  if (B1) rows::step<double, true, true, true, true, false, rows::SECOND>(op, st, b, a);
-  else rows::step<double, true, true, false, true, false, rows::FIRST>(op, st, b, a);
+  clenshaw_start_seg<double, false>(op, st, b, Q, ldq, B1, ldb, out, ldo, topseg, cseg, colseg, alpha, beta, rev);
 }
 
 void csr_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,

@@ -18,4 +18,18 @@ void model_clenshaw_start<float>(const sma_op *op, cudaStream_t st, int64_t b, c
   clenshaw_start<float, true>(op, st, b, Q, ldq, B1, ldb, out, ldo, top, ck, alpha, beta, rev);
 }
 
+template <>
+void model_clenshaw_step_seg<float>(const sma_op *op, cudaStream_t st, int64_t b, const float *Q, int64_t ldq,
+                           const float *B1, const float *B2, int64_t ldb, float *out, int64_t ldo,
+                           const float *cseg, const int *colseg, double alpha, double beta, bool rev) {
+  clenshaw_step_seg<float, true>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, cseg, colseg, alpha, beta, rev);
+}
+
+template <>
+void model_clenshaw_start_seg<float>(const sma_op *op, cudaStream_t st, int64_t b, const float *Q, int64_t ldq,
+                            const float *B1, int64_t ldb, float *out, int64_t ldo, const float *topseg,
+                            const float *cseg, const int *colseg, double alpha, double beta, bool rev) {
+  clenshaw_start_seg<float, true>(op, st, b, Q, ldq, B1, ldb, out, ldo, topseg, cseg, colseg, alpha, beta, rev);
+}
+
 }  // namespace sma

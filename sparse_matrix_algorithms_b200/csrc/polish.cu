@@ -72,8 +72,8 @@ __global__ void combine_kernel(int64_t n, int64_t k, const double *__restrict__ 
   }
 }
 
-// out = crow[j] Q + alpha AX + beta B1 - B2 (per-column coefficient; operators without a
-// fused step: the model stencils and half storage).
+// out = crow[j] Q + alpha AX + beta B1 - B2 (per-column coefficient; half storage, which has no
+// fused step).
 template <typename T>
 __global__ void percol_axpy_kernel(int64_t n, int64_t b, const T *__restrict__ Q,
                                    const T *__restrict__ AX, const T *__restrict__ B1,
@@ -101,17 +101,19 @@ int grid_of(int64_t total) {
 // blocks.  The recurrence starts from zero blocks, so its first product multiplies zeros (one
 // extra step out of K+1); with the fused step and K >= 2 it starts from c_K Q, which the next two
 // steps form from Q (record_filter in filter.cu): neither that step nor the zero blocks are there.
+// Y has the first yb columns (b by default; fewer where a caller padded the others).
 template <typename T>
 FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int64_t K,
                           double smin, double smax, const T *Q, T *Y, int64_t b, T *B1, T *B2,
-                          T *TMP, T *AX) {
+                          T *TMP, T *AX, int64_t yb) {
   FilterCount fc;
+  if (yb == 0) yb = b;
   const int64_t n = op->n;
   require(op->kind != OP_MATBLOCK, SMA_ERR_ARG, "the per-column filter needs a device operator");
   const double c = 0.5 * (smin + smax), invd = 2.0 / (smax - smin);
   const double alpha = 2.0 * invd, beta = -2.0 * c * invd;
-  const bool fused = op->kind == OP_CSR, fold = fused && K >= 2;
-  if (banded_fits(op, K, Q, b, Y, b, b)) {
+  const bool fused = op->kind != OP_CSR_HALF, fold = fused && K >= 2;
+  if (yb == b && banded_fits(op, K, Q, b, Y, b, b)) {
     DevBuf<T> fourth;
     try {
       fourth.alloc(n * b, st);
@@ -125,14 +127,13 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
       return banded_filter<T>(op, st, nullptr, coef, K, smin, smax, Q, b, Y, b, b, buf);
     }
   }
-  auto step = [&](const T *crow, T *out, double al, double be, bool rev) {
+  auto *const seg = op->kind == OP_CSR ? csr_clenshaw_step_seg<T> : model_clenshaw_step_seg<T>;
+  auto *const start_seg = op->kind == OP_CSR ? csr_clenshaw_start_seg<T> : model_clenshaw_start_seg<T>;
+  auto step = [&](const T *crow, T *out, int64_t w, double al, double be, bool rev) {
     if (fused) {
-      csr_clenshaw_step_seg<T>(op, st, b, Q, b, B1, B2, b, out, b, crow, nullptr, al, be, rev);
+      seg(op, st, w, Q, b, B1, B2, b, out, w, crow, nullptr, al, be, rev);
     } else {
-      if (op->kind == OP_CSR_HALF)
-        half_product<T>(op, st, B1, b, AX, b, b);
-      else
-        launch_clenshaw_step<T>(op, st, b, nullptr, 0, B1, nullptr, b, AX, b, 0.0, 1.0, 0.0, false);
+      half_product<T>(op, st, B1, b, AX, b, b);
       percol_axpy_kernel<T><<<grid_of(n * b), 256, 0, st>>>(n, b, Q, AX, B1, B2, out, b, crow,
                                                            (T)al, (T)be);
       SMA_CHECK_LAUNCH();
@@ -146,16 +147,15 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
     B1 = TMP;
     TMP = t;
   };
-  auto start = [&](int64_t k, const T *b1, T *out, double al, double be) {
-    csr_clenshaw_start_seg<T>(op, st, b, Q, b, b1, b, out, b, coef + K * b, coef + k * b, nullptr, al, be,
-                              k & 1);
+  auto start = [&](int64_t k, const T *b1, T *out, int64_t w, double al, double be) {
+    start_seg(op, st, w, Q, b, b1, b, out, w, coef + K * b, coef + k * b, nullptr, al, be, k & 1);
   };
   int64_t k = K;
   if (fold) {
-    start(--k, nullptr, TMP, alpha, beta);
+    start(--k, nullptr, TMP, b, alpha, beta);
     std::swap(B1, TMP);
     if (--k >= 1) {
-      start(k--, B1, TMP, alpha, beta);
+      start(k--, B1, TMP, b, alpha, beta);
       rotate();
     }
     fc.steps = K;
@@ -168,21 +168,21 @@ FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int6
     fc.bytes = (double)(K + 1) * (mat_bytes + 4 * blk);
   }
   for (; k >= 1; --k) {
-    step(coef + k * b, TMP, alpha, beta, k & 1);
+    step(coef + k * b, TMP, b, alpha, beta, k & 1);
     rotate();
   }
-  if (fold && K == 2) start(0, B1, Y, invd, -(c * invd));
-  else step(coef, Y, invd, -(c * invd), false);
+  if (fold && K == 2) start(0, B1, Y, yb, invd, -(c * invd));
+  else step(coef, Y, yb, invd, -(c * invd), false);
   check_bulk_error(op, st);
   return fc;
 }
 
 template FilterCount percol_filter<float>(const sma_op *, cudaStream_t, const float *, int64_t,
                                           double, double, const float *, float *, int64_t,
-                                          float *, float *, float *, float *);
+                                          float *, float *, float *, float *, int64_t);
 template FilterCount percol_filter<double>(const sma_op *, cudaStream_t, const double *, int64_t,
                                            double, double, const double *, double *, int64_t,
-                                           double *, double *, double *, double *);
+                                           double *, double *, double *, double *, int64_t);
 
 // Coefficients e_0..e_{K-1} of q_t (p's divided difference at t) and p(t), from the
 // Clenshaw intermediates of p at t.
@@ -247,7 +247,7 @@ PolishOut polish_mixed(const sma_op *op, const PolishCoeffs &coeffs_of, int64_t 
     B2.alloc(n * kap, st);
     TMP.alloc(n * kap, st);
     coef32.alloc(Kmax * kap, st);
-    if (op->kind != OP_CSR) AX32.alloc(n * kap, st);
+    if (op->kind == OP_CSR_HALF) AX32.alloc(n * kap, st);
   };
   DevBuf<int> act_d(kpad, st), slot_d(k, st);
   // Rayleigh-Ritz with A on span(V) (V n x k, orthonormalized in place): X = V E,

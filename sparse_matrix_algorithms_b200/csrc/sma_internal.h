@@ -237,15 +237,23 @@ void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
 // Throws SMA_ERR_TIMEOUT (and clears the flag) when a BULK-family launch of the CSR step on
 // this operator gave up its bounded wait; synchronizes the stream when the family was used.
 void check_bulk_error(const sma_op *op, cudaStream_t st);
-// The segmented CSR step (batched slicing, the POLFED polish): column c uses the coefficient
-// cseg[colseg[c]] (colseg nondecreasing), or cseg[c] when colseg is null (clenshaw_step.cuh).
+// The segmented step (batched slicing, the POLFED polish): column c uses the coefficient
+// cseg[colseg[c]] (colseg nondecreasing), or cseg[c] when colseg is null (clenshaw_step.cuh); its
+// first step (B1 null) and second, topseg the highest coefficients.  csr_, model_: their forms.
 template <typename T>
 void csr_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                            const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
                            const T *cseg, const int *colseg, double alpha, double beta, bool rev);
-// Its first step (B1 null) and second, topseg the highest coefficients.
 template <typename T>
 void csr_clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                            const T *B1, int64_t ldb, T *out, int64_t ldo, const T *topseg,
+                            const T *cseg, const int *colseg, double alpha, double beta, bool rev);
+template <typename T>
+void model_clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
+                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo,
+                           const T *cseg, const int *colseg, double alpha, double beta, bool rev);
+template <typename T>
+void model_clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                             const T *B1, int64_t ldb, T *out, int64_t ldo, const T *topseg,
                             const T *cseg, const int *colseg, double alpha, double beta, bool rev);
 // out = ck * Q
@@ -453,7 +461,7 @@ int64_t orthonormalize(sma_ctx *ctx, int64_t n, int64_t k, double *X, int64_t ld
 template <typename T>
 FilterCount percol_filter(const sma_op *op, cudaStream_t st, const T *coef, int64_t K,
                           double smin, double smax, const T *Q, T *Y, int64_t b, T *B1, T *B2,
-                          T *TMP, T *AX);
+                          T *TMP, T *AX, int64_t yb = 0);
 // e[0..K-1]: Chebyshev coefficients of (p(s) - p(t)) / (s - t) for p = sum c_m T_m; *pt = p(t).
 void divided_difference(const std::vector<double> &c, double t, double *e, double *pt);
 struct PolishOut {

@@ -119,3 +119,24 @@ def test_residual_form_in_fp32_reaches_fp64_accuracy(lib_built):
     err_32 = np.abs(Y32 - Y_ref).max() / np.abs(Y_ref).max()
     assert err_res <= 1e-11
     assert err_32 >= 1e3 * err_res  # the direct FP32 filter is far less accurate
+
+
+@pytest.mark.parametrize("kind", ["csr", "anderson", "xxz"])
+@pytest.mark.parametrize("precision,rtol", [("fp64", 1e-12), ("fp32", 2e-4)])
+@pytest.mark.parametrize("b", [9, 37, 101])
+def test_percol_filter_of_odd_widths(lib_built, kind, precision, rtol, b):
+    """Odd widths run on padded blocks with zero coefficients in the columns beyond; the models take
+    the same fused step as a stored matrix."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.xxz_sz0(10, 5.0, 1) if kind == "xxz" else M.anderson3d(7, 16.5, 5)
+    op = {"csr": lambda: S.SparseOperator(A), "anderson": lambda: S.AndersonOperator(7, 16.5, 5),
+          "xxz": lambda: S.XXZOperator(10, 5.0, 1)}[kind]()
+    smin, smax = O.gershgorin_bounds(A)
+    Q = M.splitmix_normal(b, A.shape[0], b)
+    scale = np.linspace(1.0, 2.0, b)
+    for K in (3, 4, 20):
+        c = O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True)
+        Y = _percol(op, np.ascontiguousarray(c[:, None] * scale[None, :]), smin, smax, Q, precision)
+        ref = O.apply_poly_block(A, Q, c, smin, smax)
+        assert np.abs(Y / scale - ref).max() <= rtol * max(np.abs(ref).max(), np.abs(Q).max())
