@@ -435,12 +435,31 @@ void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
 
 inline bool ragged(const sma_op *op) { return op->kind == OP_XXZ || op->ragged; }
 
+// Vectors of a panel: the whole row up to kPanel; else a multiple of 4 (128 bytes), with as few
+// panels as need be, or up to twice as many if more of a CTA's threads then have work (a CTA takes
+// whole rows of a panel, so 48 lanes leave a quarter idle: 96 vectors in 3 panels instead of 2, us
+// a step, Anderson L = 64 FP32 598 -> 582, XXZ L = 18 FP64 150 -> 141; 66 in 3 124 -> 117).  A
+// row that fits one panel stays in one: in two, 43 vectors took 114 -> 122 us (Anderson L = 48).
+inline uint32_t panel_lanes(uint32_t vecs) {
+  if (vecs <= kPanel) return vecs;
+  const uint32_t fewest = (vecs + kPanel - 1) / kPanel;
+  uint32_t best = 0;
+  double most = 0.0;
+  for (uint32_t p = fewest; p <= 2 * fewest; ++p) {
+    const uint32_t lanes = ((vecs + p - 1) / p + 3) / 4 * 4;
+    const double work = (double)(kThreads / lanes * lanes) * vecs / ((vecs + lanes - 1) / lanes * lanes);
+    if (work > 1.02 * most) {
+      most = work;
+      best = lanes;
+    }
+  }
+  return best;
+}
+
 template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL, Form P>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
   const uint32_t vecs = a.b / V;
-  // as few panels as keep a row within kPanel vectors, each a multiple of 4 vectors (128 bytes)
-  const uint32_t panels = (vecs + kPanel - 1) / kPanel;
-  a.lanes = panels == 1 ? vecs : ((vecs + panels - 1) / panels + 3) / 4 * 4;
+  a.lanes = panel_lanes(vecs);
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
   const uint32_t gx = (a.n + a.rows - 1) / a.rows;
