@@ -61,6 +61,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // A CTA tile of WM x WN warps, each MT x NT fragments of 8 x 8; chunks in flight and CTAs an SM.
 template <int WM_, int WN_, int MT_, int NT_, int STAGES_ = 3, int CTAS_ = 3>
 struct Tile {
+  using Self = Tile;
   static constexpr int WM = WM_, WN = WN_, MT = MT_, NT = NT_, kStages = STAGES_, kCtas = CTAS_;
   static constexpr int M = WM * MT * 8, N = WN * NT * 8;
   static_assert(WM * WN * 32 == kThreads, "four warps");
@@ -238,7 +239,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, T::kCtas)
 gram_partial_kernel(int64_t n, int m, int k, const double *__restrict__ X, int64_t ldx,
                     const double *__restrict__ Y, int64_t ldy, int64_t rows_per_split,
-                    double *__restrict__ part, bool vec16, bool upper) {
+                    double *__restrict__ part, bool vecx, bool vecy, bool upper) {
   const int m0 = blockIdx.x * T::M, k0 = blockIdx.y * T::N;
   if (upper && below<T>(m0, k0)) return;  // no barrier yet
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -256,7 +257,7 @@ gram_partial_kernel(int64_t n, int m, int k, const double *__restrict__ X, int64
   constexpr int WX = T::M / 2, WY = T::N / 2;  // copies of a row
   constexpr int SX = kThreads / WX, SY = kThreads / WY, PX = kDepth / SX, PY = kDepth / SY;
   const int rx = tid / WX, cx = tid % WX * 2, ry = tid / WY, cy = tid % WY * 2;
-  const bool wholex = vec16 && m0 + T::M <= m, wholey = vec16 && k0 + T::N <= k;
+  const bool wholex = vecx && m0 + T::M <= m, wholey = vecy && k0 + T::N <= k;
   const double *px = X + (r0 + rx) * ldx + m0 + cx, *py = Y + (r0 + ry) * ldy + k0 + cy;
   const int64_t stepx = SX * ldx, stepy = SY * ldy;
   auto slow = [&](double *dst, int pitch, int W, const double *src, int64_t ld, int c0, int cols,
@@ -304,17 +305,19 @@ gram_partial_kernel(int64_t n, int m, int k, const double *__restrict__ X, int64
         pt[wm + i * 8 + g + (wk + j * 8 + 2 * t + h) * T::M] = acc[i][j][h];
 }
 
-// C[i + j ldc] = alpha * sum_s part_s(i, j) + beta * C[i + j ldc]: a CTA takes 32 elements, its
-// eight warps a share of the splits each (one thread per element took 18 us for the 79 partials of
-// a 32 x 32 product), summed in a fixed order.
-template <typename T>
+// C[i + j ldc] = alpha * sum_s part_s(i, j) + beta * C[i + j ldc]: a CTA takes LANES elements, its
+// 256 / LANES groups of threads a share of the splits each, summed in a fixed order.  Few elements
+// with hundreds of splits take LANES = 8 (32 x 32, 391 splits: 16.0 -> 8.5 us; 480 x 32, 55 splits:
+// 5.4 us with 32, 10.4 with 8).
+template <typename T, int LANES>
 __global__ void __launch_bounds__(256)
 gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
                    double *C, int64_t ldc, double alpha, double beta, bool upper) {
-  __shared__ double sh[8][33];
-  const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
+  constexpr int kGroups = 256 / LANES;
+  __shared__ double sh[kGroups][LANES + 1];
+  const int cl = threadIdx.x % LANES, rl = threadIdx.x / LANES;
   const int64_t total = (int64_t)m * k;
-  for (int64_t e0 = (int64_t)blockIdx.x * 32; e0 < total; e0 += (int64_t)gridDim.x * 32) {
+  for (int64_t e0 = (int64_t)blockIdx.x * LANES; e0 < total; e0 += (int64_t)gridDim.x * LANES) {
     const int64_t e = e0 + cl;
     const int i = (int)(e % m), j = (int)(e / m);
     const int bx = i / T::M, by = j / T::N;
@@ -324,15 +327,15 @@ gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const dou
     if (ok) {
       const int64_t stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
       const double *p = part + ((int64_t)by * tiles_m + bx) * (T::M * T::N) + i % T::M + j % T::N * T::M;
-#pragma unroll 4
-      for (int z = rl; z < splits; z += 8) s += p[z * stride];
+#pragma unroll 8
+      for (int z = rl; z < splits; z += kGroups) s += p[z * stride];
     }
     sh[rl][cl] = s;
     __syncthreads();
     if (rl == 0 && ok) {
       s = 0.0;
 #pragma unroll
-      for (int r = 0; r < 8; ++r) s += sh[r][cl];
+      for (int r = 0; r < kGroups; ++r) s += sh[r][cl];
       double *c = C + i + (int64_t)j * ldc;
       *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
     }
@@ -358,47 +361,74 @@ void launch_update(cudaStream_t st, int64_t n, int64_t m, int64_t p, const doubl
 template <typename T>
 void launch_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, const double *X,
                  int64_t ldx, const double *Y, int64_t ldy, double *C, int64_t ldc, double alpha,
-                 double beta, DevBuf<double> &work, bool upper) {
+                 double beta, DevBuf<double> &work, bool upper, int64_t splits) {
   const int tm = (int)((m + T::M - 1) / T::M), tk = (int)((k + T::N - 1) / T::N);
-  int64_t tiles = (int64_t)tm * tk;
-  if (upper) {
-    tiles = 0;
-    for (int x = 0; x < tm; ++x)
-      for (int y = 0; y < tk; ++y) tiles += !below<T>(x * T::M, y * T::N);
-  }
-  // The number of splits (of at least 256 rows) with the least time: the multiplications at the
-  // share of the last wave that is filled, plus the partials' way to memory and back.
-  const int64_t slots = (int64_t)T::kCtas * num_sms, most = std::max<int64_t>(1, (n + 255) / 256);
-  int64_t splits = 1;
-  double least = 1e300;
-  for (int64_t s = 1; s <= std::min(most, std::max<int64_t>(8, 4 * slots / tiles)); ++s) {
-    const int64_t waves = (tiles * s + slots - 1) / slots;
-    const double t = (double)n / s * waves * (2.0 * T::M * T::N * slots / 35e12) +
-                     (double)(tiles * s) * (T::M * T::N * 16 / 6e12);
-    if (t < least) {
-      least = t;
-      splits = s;
-    }
-  }
   const int64_t rows = (n + splits - 1) / splits;
   const size_t need = (size_t)splits * tm * tk * T::M * T::N;
   if (work.count < need) work.alloc(need, st);
-  const bool vec16 = aligned16(X) && aligned16(Y) && ldx % 2 == 0 && ldy % 2 == 0;
+  const bool vecx = aligned16(X) && ldx % 2 == 0, vecy = aligned16(Y) && ldy % 2 == 0;
   const size_t smem = sizeof(GramSmem<T>);
   SMA_CUDA(cudaFuncSetAttribute(gram_partial_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   gram_partial_kernel<T><<<dim3(tm, tk, (unsigned)splits), kThreads, smem, st>>>(
-      n, (int)m, (int)k, X, ldx, Y, ldy, rows, work.p, vec16, upper);
+      n, (int)m, (int)k, X, ldx, Y, ldy, rows, work.p, vecx, vecy, upper);
   SMA_CHECK_LAUNCH();
-  const int blocks = (int)std::min<int64_t>((m * k + 31) / 32, 8LL * num_sms);
-  gram_reduce_kernel<T><<<blocks, 256, 0, st>>>((int)m, (int)k, tm, tk, (int)splits, work.p, C, ldc,
-                                                alpha, beta, upper);
+  auto reduce = [&](auto kernel, int lanes) {
+    const int blocks = (int)std::min<int64_t>((m * k + lanes - 1) / lanes, 8LL * num_sms);
+    kernel<<<blocks, 256, 0, st>>>((int)m, (int)k, tm, tk, (int)splits, work.p, C, ldc, alpha, beta, upper);
+  };
+  if (m * k <= 4096) reduce(gram_reduce_kernel<T, 8>, 8);
+  else reduce(gram_reduce_kernel<T, 32>, 32);
   SMA_CHECK_LAUNCH();
 }
 
 using Wide = Tile<2, 2, 4, 4>;         // 64 x 64
 using Short = Tile<2, 2, 4, 4, 2, 4>;  // the same for a short summation: more CTAs to hide its ends
-using Narrow = Tile<4, 1, 2, 4>;  // 64 x 32
-using Small = Tile<2, 2, 2, 2>;   // 32 x 32
+using Narrow = Tile<4, 1, 2, 4>;       // 64 x 32
+using Small = Tile<2, 2, 2, 2, 3, 6>;  // 32 x 32
+
+// The time of a product's tiles in us, from what a chunk takes: `shared`, its share of a busy SM
+// (the tensor pipe and what a size of tile loses beside it), and `alone`, the latency of a CTA that
+// has the SM for itself.  Measured with one tile against another at 60 shapes, n = 3000 to 262144:
+// large tiles win only where they are full and make many waves (262144 x 1024 x 64: update 1042 us
+// with 64 x 64, 1101 with 32 x 32; 30000 x 1024 x 64: 198 and 142; 262144 x 160 x 160: gram 672 and
+// 444; 20000 x 32 x 32: gram 15 with 79 splits of 32 x 32, 12 with 313).
+struct Rate {
+  double shared, alone;
+  int ctas;
+};
+constexpr Rate kWide{0.585, 1.05, Wide::kCtas}, kShort{0.60, 1.05, Short::kCtas},
+    kNarrow{0.305, 0.75, Narrow::kCtas}, kSmall{0.160, 0.52, Small::kCtas};
+
+inline double tiles_time(const Rate &r, int64_t tiles, int64_t chunks, int sms) {
+  auto wave = [&](int64_t each) { return (chunks + 2) * std::max(r.alone, each * r.shared); };
+  const int64_t slots = (int64_t)r.ctas * sms, rest = tiles % slots;
+  return (tiles / slots) * wave(r.ctas) + (rest ? wave((rest + sms - 1) / sms) : 0.0);
+}
+
+// The gram's splits of n, at least 64 rows each, at most 512: whole waves or whole rounds of the
+// SMs, against the partials' way to memory and back and their sum.
+struct Splits {
+  double time;
+  int64_t count;
+};
+template <typename T>
+Splits gram_splits(const Rate &r, int64_t n, int64_t m, int64_t k, bool upper, int sms) {
+  int64_t tiles = 0;
+  for (int64_t x = 0; x < m; x += T::M)
+    for (int64_t y = 0; y < k; y += T::N) tiles += !(upper && below<T>((int)x, (int)y));
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(512, n / 64));
+  const double ragged = m % T::M || k % T::N ? 1.08 : 1.0;  // tiles that stick out copy 8 bytes a time
+  Splits best{1e300, 1};
+  auto consider = [&](int64_t s) {
+    s = std::max<int64_t>(1, std::min(s, most));
+    const double t = ragged * tiles_time(r, tiles * s, ((n + s - 1) / s + kDepth - 1) / kDepth, sms) +
+                     (double)(tiles * s) * (T::M * T::N * 16 / 12e6) + 0.01 * s;
+    if (t < best.time) best = {t, s};
+  };
+  consider(most);
+  for (int64_t w = 1; w <= 4 * r.ctas; ++w) consider(w * sms / tiles);
+  return best;
+}
 
 }  // namespace dmma
 
@@ -408,16 +438,27 @@ void dgemm_update(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t p,
   using namespace dmma;
   if (n == 0 || p == 0) return;
   require(m <= INT32_MAX && p <= INT32_MAX, SMA_ERR_ARG, "product too wide");
-  (void)num_sms;
+  auto run = [&](auto tile) {
+    using T = typename decltype(tile)::Self;
+    if (transC) launch_update<true, T>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    else launch_update<false, T>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+  };
+  auto time = [&](auto tile, const Rate &r) {
+    using T = typename decltype(tile)::Self;
+    return tiles_time(r, (n + T::M - 1) / T::M * ((p + T::N - 1) / T::N), (m + kDepth - 1) / kDepth, num_sms);
+  };
+  // in place one CTA has to read a row of X before it is written: no tile narrower than p
+  const bool in_place = (uintptr_t)X < (uintptr_t)(Y + n * ldy) && (uintptr_t)Y < (uintptr_t)(X + n * ldx);
+  const double small = in_place && p > 32 ? 1e300 : time(Small{}, kSmall);
   if (p <= 32) {  // half of a wide tile would be padding
-    if (transC) launch_update<true, Narrow>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
-    else launch_update<false, Narrow>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    if (small <= time(Narrow{}, kNarrow)) run(Small{});
+    else run(Narrow{});
   } else if (m <= 128) {
-    if (transC) launch_update<true, Short>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
-    else launch_update<false, Short>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    if (small <= time(Short{}, kShort)) run(Small{});
+    else run(Short{});
   } else {
-    if (transC) launch_update<true, Wide>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
-    else launch_update<false, Wide>(st, n, m, p, X, ldx, C, ldc, Y, ldy, alpha, beta);
+    if (small <= time(Wide{}, kWide)) run(Small{});
+    else run(Wide{});
   }
 }
 
@@ -428,12 +469,20 @@ void dgemm_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, c
   if (m == 0 || k == 0) return;
   require(m <= INT32_MAX && k <= INT32_MAX, SMA_ERR_ARG, "product too wide");
   upper = upper && m == k;
-  if (m <= 32 && k <= 32)
-    launch_gram<Small>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
-  else if (k <= 32)
-    launch_gram<Narrow>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
-  else
-    launch_gram<Wide>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper);
+  auto run = [&](auto tile, int64_t splits) {
+    using T = typename decltype(tile)::Self;
+    launch_gram<T>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper, splits);
+  };
+  const Splits small = gram_splits<Small>(kSmall, n, m, k, upper, num_sms);
+  if (k <= 32) {
+    const Splits narrow = gram_splits<Narrow>(kNarrow, n, m, k, upper, num_sms);
+    if (small.time <= narrow.time) run(Small{}, small.count);
+    else run(Narrow{}, narrow.count);
+  } else {
+    const Splits wide = gram_splits<Wide>(kWide, n, m, k, upper, num_sms);
+    if (small.time <= wide.time) run(Small{}, small.count);
+    else run(Wide{}, wide.count);
+  }
 }
 
 }  // namespace sma
