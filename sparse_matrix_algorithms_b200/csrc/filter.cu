@@ -10,10 +10,11 @@
 // (chebyshev_subspace_iteration.jl:562-565).
 //
 // The reference zero-fills B1 and B2 and runs K+1 sparse products.  The first step
-// multiplies zeros, so here it is the scaling B1 = c_K Q (bit-identical: every
-// dropped term is an exact zero), and the second step reads no B2.  Each remaining
-// step is ONE fused kernel launch (kernels.cu) for device operators; caller-supplied
-// operators get the product from their callback followed by the axpy kernel.
+// multiplies zeros and gives B1 = c_K Q (bit-identical: every dropped term is an exact
+// zero), which the next two steps form from Q themselves.  Each step is ONE fused kernel
+// launch (clenshaw_step.cuh) for device operators, for full narrow bands many steps are one
+// (banded.cu); caller-supplied operators get the product from their callback followed by the
+// axpy kernel, and a scaled block to start from.
 #include "sma_internal.h"
 
 namespace sma {
