@@ -417,3 +417,18 @@ def test_filter_graph_replay_is_bit_identical(lib_built, monkeypatch):
     np.testing.assert_array_equal(X, X0)
     # the same kernels, plus the staging copies in and out of each replay
     assert st["kernel_launches"] == st0["kernel_launches"] + 2 * 7
+
+
+@pytest.mark.parametrize("s", [1, 5, 63, 64, 65])
+def test_polfed_blocks_around_the_one_kernel_factorization(lib_built, s):
+    """Blocks of at most 64 columns are factorized and inverted by one kernel, wider ones by the
+    library: the Laplacian's eigenvalues either way, at the tolerance of the solve."""
+    import sparse_matrix_algorithms_b200 as S
+
+    n = 900
+    exact = 2.0 - 2.0 * np.cos(np.pi * np.arange(1, n + 1) / (n + 1))
+    lo, hi = 0.5 * (exact[399] + exact[400]), 0.5 * (exact[419] + exact[420])
+    lam, X, res = S.polfed(M.lap1d(n), 20, 400, s=s, smin=0.0, smax=4.0, sigma=0.5 * (lo + hi), emin=lo,
+                           emax=hi, tol=1e-10, window_type="delta", mmax=max(4, 160 // s), seed=1)
+    np.testing.assert_allclose(np.sort(lam), exact[400:420], rtol=0, atol=1e-9)
+    assert np.abs(X.T @ X - np.eye(X.shape[1])).max() <= 1e-10
