@@ -71,7 +71,7 @@ struct Step {
   uint32_t n, b;      // rows, columns
   uint32_t lanes;     // vectors of a row in one panel
   uint32_t rows;      // rows of a CTA (rows * lanes <= kThreads)
-  uint32_t divlanes;  // ceil(2^16 / lanes): tid / lanes = tid * divlanes >> 16 for tid < 128
+  uint32_t divlanes;  // ceil(2^16 / lanes): i / lanes = i * divlanes >> 16 for i < 192
   int rev;
 };
 
@@ -291,16 +291,23 @@ __device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cse
 enum Form { INNER, FIRST, SECOND, DOTS };
 
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
+// FLAT: a CTA does not take whole rows, its threads go on in the next row where the CTA before ended.
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
-          bool RAGGED, Form P>
+          bool RAGGED, Form P, bool FLAT>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  const uint32_t r = threadIdx.x * a.divlanes >> 16;
-  uint32_t row = bx * a.rows + r;
-  uint32_t c0 = (by * a.lanes + threadIdx.x - r * a.lanes) * V;
-  const bool in = r < a.rows && row < a.n && c0 < a.b;
+  static_assert(!FLAT || !(MODEL || P == DOTS), "these need whole rows");
+  uint32_t row0 = bx * a.rows, i = threadIdx.x;
+  if constexpr (FLAT) {
+    row0 = bx * kThreads / a.lanes;
+    i += bx * kThreads - row0 * a.lanes;
+  }
+  const uint32_t r = i * a.divlanes >> 16;
+  uint32_t row = row0 + r;
+  uint32_t c0 = (by * a.lanes + i - r * a.lanes) * V;
+  const bool in = (FLAT || r < a.rows) && row < a.n && c0 < a.b;
   int start = 0, end = 0;
   if (in) {
     if constexpr (!MODEL) {
@@ -415,7 +422,7 @@ namespace rows {
 
 // ------------------------------------------------------------------ launch
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
-          bool RAGGED, Form P>
+          bool RAGGED, Form P, bool FLAT = false>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -429,7 +436,7 @@ void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   // the first step gathers the caller's Q, which the grid before may have read and written in
   // place: it starts after that grid has ended, with nothing of it in L1
   cfg.numAttrs = op->ctx->pdl && P != FIRST ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED, P>, a));
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED, P, FLAT>, a));
   SMA_CHECK_LAUNCH();
 }
 
@@ -462,7 +469,6 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   a.lanes = panel_lanes(vecs);
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
-  const uint32_t gx = (a.n + a.rows - 1) / a.rows;
   // Waves of 8-CTA residency decide what a step's time is.  Six and more: a stream, which wants
   // every warp it can get.  Below, more and more a latency, which wants more gathers in flight at
   // less occupancy -- unless a row has no more than four.  Us a step, step after step:
@@ -476,6 +482,17 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   const bool uneven = ragged(op);
   if (gathers == 0)
     gathers = threads >= 6 * wave || op->nnz <= 4 * op->n ? 4 : uneven && threads >= 2 * wave ? 6 : 8;
+  // Whole rows leave threads idle where lanes do not divide 128.  Going on in the next row instead
+  // takes a division per CTA and lets warps straddle rows: the better way for streams, unless whole
+  // warps are idle or a few threads of long rows (us a step, whole rows and flat, Anderson L = 48:
+  // 13 lanes 34.1 and 32.6, 22 55.8 and 52.0, 43 117 and 107, 50 143 and 128; 48 120 and 121, 60
+  // 152 and 155).
+  constexpr bool kFlat = !(MODEL || P == DOTS || P == FIRST);
+  const uint32_t used = a.rows * a.lanes;
+  const bool flat = kFlat && gathers != 8 && used % 32 != 0 && (a.lanes <= 40 || kThreads - used >= 16) &&
+                    (uint64_t)a.n * a.lanes < (uint64_t)1 << 32;
+  const uint32_t gx = flat ? (uint32_t)(((uint64_t)a.n * a.lanes + kThreads - 1) / kThreads)
+                           : (a.n + a.rows - 1) / a.rows;
   constexpr uint32_t kGridY = 65535;
   const uint32_t ny = (vecs + a.lanes - 1) / a.lanes;
   const uint32_t span = kGridY * a.lanes * V, width = a.b;
@@ -492,13 +509,17 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
     if constexpr (P == FIRST) {  // the coefficients take registers too, and it is one step
       if (uneven) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
       else launch<T, V, 4, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
-    } else if (uneven) {
-      if (gathers == 8) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+    } else if (gathers == 8) {
+      if (uneven) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+      else launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
+    } else if (flat) {
+      if (!uneven) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P, kFlat>(op, st, a, grid);
+      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
+    } else {
+      if (!uneven) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
       else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
       else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
-    } else {
-      if (gathers == 8) launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
-      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
     }
   }
 }

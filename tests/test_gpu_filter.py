@@ -439,3 +439,22 @@ def test_band_of_the_laplacian_stencil_and_of_other_matrices(lib_built):
         ref = O.apply_poly_block(A, Q, c, smin, smax)
         got = S.apply_poly_block(A if op is None else op, Q, c, smin, smax)
         assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
+
+
+@pytest.mark.parametrize("n,b", [(30011, 52), (75001, 52), (45013, 88), (75001, 172)])
+@pytest.mark.parametrize("rows", ["equal", "ragged"])
+def test_filter_where_ctas_end_within_rows(lib_built, n, b, rows):
+    """Thread counts a row that do not divide a CTA's (13, 22, 43): large blocks go on in the next
+    row, the last CTA beyond the last; against the oracle."""
+    import sparse_matrix_algorithms_b200 as S
+
+    d = np.where(np.arange(n) % 3 == 0, 1.0, 0.0) if rows == "ragged" else np.ones(n)
+    off = [sp.diags([d[:n - k] * d[k:] * 0.1], [k]) for k in (3, 6, 9, 12)]
+    A = M._canonical((sum(off) + sum(off).T + 0.5 * M.lap1d(n)).tocsr())
+    A.eliminate_zeros()
+    smin, smax = _bounds(A)
+    Q = M.splitmix_normal(b, n, b)
+    c = np.ascontiguousarray(O.build_coeffs(4, smin, smax, 0.1, -0.4, 0.3, "step", True))
+    ref = O.apply_poly_block(A, Q, c, smin, smax)
+    got = S.apply_poly_block(A, Q, c, smin, smax)
+    assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
