@@ -51,10 +51,7 @@ __global__ void __launch_bounds__(kMaxThreads) kernel(const __grid_constant__ Ar
   __shared__ T edge[2][2 * W][kMaxThreads];  // per strip its first W rows, then its last W
   const int tid = threadIdx.x, strip = tid / a.columns, lane = tid - strip * a.columns;
   const bool below = tid >= a.columns, above = tid + a.columns < (int)blockDim.x;
-  const int64_t c = (int64_t)blockIdx.y * a.columns + lane;
   const int64_t out0 = (int64_t)blockIdx.x * a.rows, r0 = out0 - a.halo + (int64_t)strip * S;
-  // most threads own rows that are all there, with all entries: nothing of theirs is predicated
-  const bool whole = r0 >= 0 && r0 + S <= a.n && c < a.b;
   T v[S][2 * W + 1];
   if (r0 >= W && r0 + S <= a.n - W) {
     const T *p = a.val ? a.val + __ldg(a.rowptr + r0) : nullptr;
@@ -78,6 +75,11 @@ __global__ void __launch_bounds__(kMaxThreads) kernel(const __grid_constant__ Ar
     }
   }
   pdl_wait_then_trigger();
+  // every address in the blocks has c in it: none of their loads, which the compiler may take for
+  // loads of constants, can move above the wait for the launch that wrote them
+  const int64_t c = after_wait((int64_t)blockIdx.y * a.columns + lane);
+  // most threads own rows that are all there, with all entries: nothing of theirs is predicated
+  const bool whole = r0 >= 0 && r0 + S <= a.n && c < a.b;
   auto read = [&](const T *block, int64_t ld, T (&to)[S]) {
     const T *p = block + r0 * ld + c;
     if (whole) {

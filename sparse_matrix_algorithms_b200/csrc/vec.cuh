@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstring>
 
 namespace sma {
@@ -53,6 +54,10 @@ __device__ __forceinline__ void ldv(const T *__restrict__ p, T (&f)[V]) {
 // loads there, which the compiler could otherwise hoist past the wait.
 __device__ __forceinline__ uint32_t after_wait(uint32_t i) {
   asm volatile("" : "+r"(i)::"memory");
+  return i;
+}
+__device__ __forceinline__ int64_t after_wait(int64_t i) {
+  asm volatile("" : "+l"(i)::"memory");
   return i;
 }
 

@@ -458,3 +458,34 @@ def test_filter_where_ctas_end_within_rows(lib_built, n, b, rows):
     ref = O.apply_poly_block(A, Q, c, smin, smax)
     got = S.apply_poly_block(A, Q, c, smin, smax)
     assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Q).max())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n,b", [(600, 8), (20000, 8), (20000, 64)])
+def test_banded_launches_wait_for_the_one_before(lib_built, precision, n, b):
+    """Many launches of the banded filter in a row, each started while the one before still runs: its
+    blocks may be read only after the wait.  The same bits, over and over, as the step kernel's, which
+    an in-place call takes, for the stored matrix and the stencil."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    lib, K = L.load(), 400
+    c = np.ascontiguousarray(O.build_coeffs(K, 0.0, 4.0, 1.7, 1.6, 1.8, "step", True))
+    Q = torch.as_tensor(M.splitmix_normal(3, n, b), device="cuda")
+    Q = Q.to(torch.float64 if precision == "fp64" else torch.float32)
+
+    def run(op, q, y):
+        torch.cuda.synchronize()
+        L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, 0.0, 4.0, q.data_ptr(), b, y.data_ptr(),
+                                             b, b, L.PRECISIONS[precision]))
+        return y
+
+    ops = S.SparseOperator(M.lap1d(n)), S.Lap1dOperator(n)
+    Z = Q.clone()
+    ref = run(ops[0], Z, Z)
+    Z = Q.clone()
+    assert torch.equal(run(ops[1], Z, Z), ref)
+    for _ in range(5):
+        for op in ops:
+            assert torch.equal(run(op, Q, torch.empty_like(Q)), ref)
