@@ -12,9 +12,9 @@
 // memory, three chunks of 16 in flight and one barrier a chunk: a warp owns a 32 x 32 piece of the
 // CTA's 64 x 64 output tile (smaller ones for narrow products), keeps its accumulators in
 // registers and reads the next four indices' fragments while it multiplies.  The gram splits n
-// over the grid so that the tiles fill whole waves of three CTAs an SM; every CTA writes its
-// partial tile to a workspace and a second kernel sums the partials in a fixed order, so results
-// are deterministic (the same bits every run).  The update owns whole rows of Y: with beta = 0 it
+// over the grid; every CTA writes its partial tile to a workspace and a second kernel sums the
+// partials one after the other, so results are deterministic (the same bits every run, and with
+// every tile).  The update owns whole rows of Y: with beta = 0 it
 // may write in place over X when p <= 64 (X <- X B, the triangular solve of CholQR written as a
 // product with R^-1), since a CTA reads all of its rows of X before it writes them.
 //
@@ -305,41 +305,71 @@ gram_partial_kernel(int64_t n, int m, int k, const double *__restrict__ X, int64
         pt[wm + i * 8 + g + (wk + j * 8 + 2 * t + h) * T::M] = acc[i][j][h];
 }
 
-// C[i + j ldc] = alpha * sum_s part_s(i, j) + beta * C[i + j ldc]: a CTA takes LANES elements, its
-// 256 / LANES groups of threads a share of the splits each, summed in a fixed order.  Few elements
-// with hundreds of splits take LANES = 8 (32 x 32, 391 splits: 16.0 -> 8.5 us; 480 x 32, 55 splits:
-// 5.4 us with 32, 10.4 with 8).
-template <typename T, int LANES>
+// Element e of C = alpha * sum_z part_z + beta C: its place in the partials of split 0, or -1 where
+// those below the diagonal were never written.
+template <typename T>
+__device__ __forceinline__ int64_t partial_place(int64_t e, int m, int tiles_m, bool upper) {
+  const int i = (int)(e % m), j = (int)(e / m), bx = i / T::M, by = j / T::N;
+  if (upper && below<T>(bx * T::M, by * T::N)) return -1;
+  return ((int64_t)by * tiles_m + bx) * (T::M * T::N) + i % T::M + j % T::N * T::M;
+}
+__device__ __forceinline__ void finish(double *C, int64_t ldc, int64_t e, int m, double s, double alpha,
+                                       double beta) {
+  double *c = C + e % m + e / m * ldc;
+  *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
+}
+
+// Both sum the splits one after the other, whatever the tiles were.  With few splits a thread takes
+// an element.  With many, the chain of loads would be the time: a CTA takes LANES elements, its
+// 256 / LANES groups of threads bring a share of the splits each to shared memory, and one of them
+// adds those up.
+template <typename T>
 __global__ void __launch_bounds__(256)
 gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
                    double *C, int64_t ldc, double alpha, double beta, bool upper) {
-  constexpr int kGroups = 256 / LANES;
-  __shared__ double sh[kGroups][LANES + 1];
-  const int cl = threadIdx.x % LANES, rl = threadIdx.x / LANES;
-  const int64_t total = (int64_t)m * k;
-  for (int64_t e0 = (int64_t)blockIdx.x * LANES; e0 < total; e0 += (int64_t)gridDim.x * LANES) {
-    const int64_t e = e0 + cl;
-    const int i = (int)(e % m), j = (int)(e / m);
-    const int bx = i / T::M, by = j / T::N;
-    // partials below the diagonal were never written
-    const bool ok = e < total && !(upper && below<T>(bx * T::M, by * T::N));
+  const int64_t total = (int64_t)m * k, stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t at = partial_place<T>(e, m, tiles_m, upper);
+    if (at < 0) continue;
     double s = 0.0;
-    if (ok) {
-      const int64_t stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
-      const double *p = part + ((int64_t)by * tiles_m + bx) * (T::M * T::N) + i % T::M + j % T::N * T::M;
 #pragma unroll 8
-      for (int z = rl; z < splits; z += kGroups) s += p[z * stride];
-    }
-    sh[rl][cl] = s;
-    __syncthreads();
-    if (rl == 0 && ok) {
-      s = 0.0;
+    for (int z = 0; z < splits; ++z) s += part[at + z * stride];
+    finish(C, ldc, e, m, s, alpha, beta);
+  }
+}
+
+template <typename T, int LANES>
+__global__ void __launch_bounds__(256)
+gram_reduce_many_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
+                        double *C, int64_t ldc, double alpha, double beta, bool upper) {
+  constexpr int kGroups = 256 / LANES, kEach = 8;  // splits of a group in one round
+  __shared__ double sh[kGroups * kEach][LANES + 1];
+  const int cl = threadIdx.x % LANES, rl = threadIdx.x / LANES;
+  const int64_t total = (int64_t)m * k, stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
+  for (int64_t e0 = (int64_t)blockIdx.x * LANES; e0 < total; e0 += (int64_t)gridDim.x * LANES) {
+    const int64_t e = e0 + cl, at = e < total ? partial_place<T>(e, m, tiles_m, upper) : -1;
+    double s = 0.0;
+    for (int z0 = 0; z0 < splits; z0 += kGroups * kEach) {
+      const int count = min(kGroups * kEach, splits - z0);
+      if (at >= 0) {
+        double v[kEach];
 #pragma unroll
-      for (int r = 0; r < kGroups; ++r) s += sh[r][cl];
-      double *c = C + i + (int64_t)j * ldc;
-      *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
+        for (int u = 0; u < kEach; ++u) {
+          const int z = rl + u * kGroups;
+          v[u] = z < count ? part[at + (z0 + z) * stride] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) sh[rl + u * kGroups][cl] = v[u];
+      }
+      __syncthreads();
+      if (rl == 0 && at >= 0) {
+#pragma unroll 8
+        for (int z = 0; z < count; ++z) s += sh[z][cl];
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    if (rl == 0 && at >= 0) finish(C, ldc, e, m, s, alpha, beta);
   }
 }
 
@@ -372,12 +402,13 @@ void launch_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, 
   gram_partial_kernel<T><<<dim3(tm, tk, (unsigned)splits), kThreads, smem, st>>>(
       n, (int)m, (int)k, X, ldx, Y, ldy, rows, work.p, vecx, vecy, upper);
   SMA_CHECK_LAUNCH();
-  auto reduce = [&](auto kernel, int lanes) {
-    const int blocks = (int)std::min<int64_t>((m * k + lanes - 1) / lanes, 8LL * num_sms);
+  auto reduce = [&](auto kernel, int elements) {
+    const int blocks = (int)std::min<int64_t>((m * k + elements - 1) / elements, 8LL * num_sms);
     kernel<<<blocks, 256, 0, st>>>((int)m, (int)k, tm, tk, (int)splits, work.p, C, ldc, alpha, beta, upper);
   };
-  if (m * k <= 4096) reduce(gram_reduce_kernel<T, 8>, 8);
-  else reduce(gram_reduce_kernel<T, 32>, 32);
+  if (splits <= 32) reduce(gram_reduce_kernel<T>, 256);
+  else if (m * k <= 4096) reduce(gram_reduce_many_kernel<T, 8>, 8);
+  else reduce(gram_reduce_many_kernel<T, 32>, 32);
   SMA_CHECK_LAUNCH();
 }
 
@@ -385,13 +416,17 @@ using Wide = Tile<2, 2, 4, 4>;         // 64 x 64
 using Short = Tile<2, 2, 4, 4, 2, 4>;  // the same for a short summation: more CTAs to hide its ends
 using Narrow = Tile<4, 1, 2, 4>;       // 64 x 32
 using Small = Tile<2, 2, 2, 2, 3, 6>;  // 32 x 32
+using Tiny = Tile<2, 2, 1, 1, 3, 8>;   // 16 x 16, gram only
 
 // The time of a product's tiles in us, from what a chunk takes: `shared`, its share of a busy SM
 // (the tensor pipe and what a size of tile loses beside it), and `alone`, the latency of a CTA that
 // has the SM for itself.  Measured with one tile against another at 60 shapes, n = 3000 to 262144:
 // large tiles win only where they are full and make many waves (262144 x 1024 x 64: update 1042 us
-// with 64 x 64, 1101 with 32 x 32; 30000 x 1024 x 64: 198 and 142; 262144 x 160 x 160: gram 672 and
-// 444; 20000 x 32 x 32: gram 15 with 79 splits of 32 x 32, 12 with 313).
+// with 64 x 64, 1101 with 32 x 32; 30000 x 1024 x 64: 198 and 142).  Of the gram, whose tiles below
+// the diagonal leave gaps, whole calls in us with 64 x 64, 64 x 32, 32 x 32 and 16 x 16:
+//   262144 x 1024 x 64   1060, 1143, 1148, 1744     262144 x 480 x 32   579, 305, 323, 432
+//   262144 x 160 x 160    694,  727,  497,  685      20000 x 32 x 32     36,  30,  25,  24
+//   262144 x 200 x 16     313,  209,  227,  141       3000 x 16 x 8      38,  33,  30,  25
 struct Rate {
   double shared, alone;
   int ctas;
@@ -405,29 +440,24 @@ inline double tiles_time(const Rate &r, int64_t tiles, int64_t chunks, int sms) 
   return (tiles / slots) * wave(r.ctas) + (rest ? wave((rest + sms - 1) / sms) : 0.0);
 }
 
-// The gram's splits of n, at least 64 rows each, at most 512: whole waves or whole rounds of the
-// SMs, against the partials' way to memory and back and their sum.
-struct Splits {
-  double time;
-  int64_t count;
-};
+// The gram's splits of n: two CTAs an SM if the tiles were 64 x 64, at least 256 rows each.  They and
+// the order in which they are summed fix the result's last bits, so they follow from the shape alone
+// and not from the tile: a solve that keeps an unconverged pair carries a last bit of its basis to the
+// sixth digit of that pair.
+int64_t gram_splits(int64_t n, int64_t m, int64_t k, int sms) {
+  const int64_t want = 2LL * sms / (((m + 63) / 64) * ((k + 63) / 64));
+  return std::max<int64_t>(1, std::min<int64_t>(want, (n + 255) / 256));
+}
+
+// Its CTAs are long: those past the first wave start as others end, with no gap between.
 template <typename T>
-Splits gram_splits(const Rate &r, int64_t n, int64_t m, int64_t k, bool upper, int sms) {
+double gram_time(const Rate &r, int64_t n, int64_t m, int64_t k, bool upper, int64_t splits, int sms) {
   int64_t tiles = 0;
   for (int64_t x = 0; x < m; x += T::M)
     for (int64_t y = 0; y < k; y += T::N) tiles += !(upper && below<T>((int)x, (int)y));
-  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(512, n / 64));
-  const double ragged = m % T::M || k % T::N ? 1.08 : 1.0;  // tiles that stick out copy 8 bytes a time
-  Splits best{1e300, 1};
-  auto consider = [&](int64_t s) {
-    s = std::max<int64_t>(1, std::min(s, most));
-    const double t = ragged * tiles_time(r, tiles * s, ((n + s - 1) / s + kDepth - 1) / kDepth, sms) +
-                     (double)(tiles * s) * (T::M * T::N * 16 / 12e6) + 0.01 * s;
-    if (t < best.time) best = {t, s};
-  };
-  consider(most);
-  for (int64_t w = 1; w <= 4 * r.ctas; ++w) consider(w * sms / tiles);
-  return best;
+  const int64_t ctas = tiles * splits, chunks = ((n + splits - 1) / splits + kDepth - 1) / kDepth;
+  const double each = ctas <= r.ctas * sms ? (double)((ctas + sms - 1) / sms) : (double)ctas / sms;
+  return (chunks + 2) * std::max(r.alone, each * r.shared);
 }
 
 }  // namespace dmma
@@ -469,19 +499,24 @@ void dgemm_gram(cudaStream_t st, int num_sms, int64_t n, int64_t m, int64_t k, c
   if (m == 0 || k == 0) return;
   require(m <= INT32_MAX && k <= INT32_MAX, SMA_ERR_ARG, "product too wide");
   upper = upper && m == k;
-  auto run = [&](auto tile, int64_t splits) {
+  const int64_t splits = gram_splits(n, m, k, num_sms);
+  auto run = [&](auto tile) {
     using T = typename decltype(tile)::Self;
     launch_gram<T>(st, num_sms, n, m, k, X, ldx, Y, ldy, C, ldc, alpha, beta, work, upper, splits);
   };
-  const Splits small = gram_splits<Small>(kSmall, n, m, k, upper, num_sms);
-  if (k <= 32) {
-    const Splits narrow = gram_splits<Narrow>(kNarrow, n, m, k, upper, num_sms);
-    if (small.time <= narrow.time) run(Small{}, small.count);
-    else run(Narrow{}, narrow.count);
+  auto time = [&](auto tile, const Rate &r) {
+    using T = typename decltype(tile)::Self;
+    return gram_time<T>(r, n, m, k, upper, splits, num_sms);
+  };
+  const double small = time(Small{}, kSmall);
+  if (k <= 16) {
+    run(Tiny{});
+  } else if (k <= 32) {
+    if (small <= time(Narrow{}, kNarrow)) run(Small{});
+    else run(Narrow{});
   } else {
-    const Splits wide = gram_splits<Wide>(kWide, n, m, k, upper, num_sms);
-    if (small.time <= wide.time) run(Small{}, small.count);
-    else run(Wide{}, wide.count);
+    if (small <= time(Wide{}, kWide)) run(Small{});
+    else run(Wide{});
   }
 }
 

@@ -155,3 +155,62 @@ def test_update_in_place_of_every_width(lib_built, k):
     L.check(L.load().sma_dense_update_dev(S.context().handle, n, k, k, Xd.data_ptr(), k, Cd.data_ptr(),
                                           k, 0, Xd.data_ptr(), k, 1.0, 0.0))
     assert np.abs(Xd.cpu().numpy() - X @ B).max() <= 1e-13 * max((np.abs(X) @ np.abs(B)).max(), 1.0)
+
+
+def _gram_of_ones_in_order(x, m, k):
+    """X^T 1 as the Gram sums it: rows in order within a split, the splits one after the other; the
+    splits follow from the shape as the kernel states it (148 SMs)."""
+    n = x.shape[0]
+    splits = max(1, min(2 * 148 // (-(-m // 64) * -(-k // 64)), -(-n // 256)))
+    rows = -(-n // splits)
+    total = np.zeros(x.shape[1])
+    for r in range(0, n, rows):
+        total = total + np.add.accumulate(x[r:r + rows], axis=0)[-1]
+    return total, rows
+
+
+@pytest.mark.parametrize("n,m,k", [(20000, 32, 32), (262144, 16, 8), (9999, 100, 64), (3000, 300, 13), (5001, 17, 17),
+                                   (100000, 15, 1), (40000, 130, 130), (262144, 192, 64), (200, 3, 3)])
+def test_gram_sums_in_the_order_of_the_shape(lib_built, n, m, k):
+    """The order of a Gram's sums is part of its result (an unconverged pair of a solve shows it): ones
+    and, in every column, pairs of +-2^70 that swallow the ones summed between them, so that the total
+    tells which rows were summed with which.  Exact, whatever the tile: the 2^70 go first and last in a
+    group of four rows, within which the order does not matter then."""
+    import sparse_matrix_algorithms_b200 as S
+
+    rng = np.random.default_rng(n + m)
+    x = np.ones((n, m))
+    _, rows = _gram_of_ones_in_order(x[:, :1], m, k)
+    for c in range(m):
+        a, b = np.sort(rng.choice(n // 8 - 1, 2, replace=False)) * 8 if n >= 64 else (0, 8)
+        a, b = [r // rows * rows + r % rows // 4 * 4 for r in (int(a), int(b))]  # groups start with their split
+        b = min(b + 3, b // rows * rows + rows - 1, n - 1)
+        if b % rows % 4 == 3 and b > a:
+            x[a, c], x[b, c] = 2.0 ** 70, -(2.0 ** 70)
+    ref, _ = _gram_of_ones_in_order(x, m, k)
+    assert n < 1000 or np.unique(ref).size > min(m, 8)
+    C = _gram(S.context(), x, np.ones((n, k)), m, k)
+    np.testing.assert_array_equal(C, np.broadcast_to(ref, (k, m)))
+
+
+def test_gram_of_a_wide_block_with_little_memory_left(lib_built):
+    """The workspace of the partial products stays small where the tiles alone fill the GPU: 1896
+    columns with 1.5 GB of device memory left."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    n, k = 131072, 1896
+    ctx = S.context()
+    X = torch.randn(n, k, dtype=torch.float64, device="cuda")
+    C = torch.empty(k, k, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - 3 * 2 ** 29, dtype=torch.uint8, device="cuda")
+    try:
+        L.check(L.load().sma_dense_gram_dev(ctx.handle, n, k, k, X.data_ptr(), k, X.data_ptr(), k, C.data_ptr(), k,
+                                            1.0, 0.0))
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert (C - X.T @ X).abs().max().item() <= 1e-13 * n
