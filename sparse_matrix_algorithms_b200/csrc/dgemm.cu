@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "sma_internal.h"
+#include "vec.cuh"
 
 namespace sma {
 namespace dmma {
@@ -196,7 +197,7 @@ update_kernel(int64_t n, int m, int p, const double *X, int64_t ldx,  // Y may a
     multiply<T>(acc, [&](int k, int i) { return a[i * 8 * kPad + k]; },
                 [&](int k, int j) { return b[j * 8 * kPad + k]; });
   });
-  // Y = alpha acc + beta Y (Y not read when beta == 0)
+  // Y = alpha acc + beta Y (Y not read when beta == 0), the first product and the sum rounded once
 #pragma unroll
   for (int i = 0; i < T::MT; ++i) {
     const int64_t yr = row0 + wr + i * 8 + g;
@@ -205,18 +206,16 @@ update_kernel(int64_t n, int m, int p, const double *X, int64_t ldx,  // Y may a
     for (int j = 0; j < T::NT; ++j) {
       const int yc = col0 + wc + j * 8 + 2 * t;
       double *y = Y + yr * ldy + yc;
-      double v0 = alpha * acc[i][j][0], v1 = alpha * acc[i][j][1];
+      auto result = [&](double sum, const double &old) {
+        return beta == 0.0 ? alpha * sum : fma(alpha, sum, mul_rn(beta, old));
+      };
       if (vecy && yc + 1 < p) {
         double2 *y2 = reinterpret_cast<double2 *>(y);
-        if (beta != 0.0) {
-          const double2 o = *y2;
-          v0 += beta * o.x;
-          v1 += beta * o.y;
-        }
-        *y2 = make_double2(v0, v1);
+        const double2 o = beta == 0.0 ? make_double2(0.0, 0.0) : *y2;
+        *y2 = make_double2(result(acc[i][j][0], o.x), result(acc[i][j][1], o.y));
       } else {
-        if (yc < p) y[0] = beta == 0.0 ? v0 : v0 + beta * y[0];
-        if (yc + 1 < p) y[1] = beta == 0.0 ? v1 : v1 + beta * y[1];
+        if (yc < p) y[0] = result(acc[i][j][0], y[0]);
+        if (yc + 1 < p) y[1] = result(acc[i][j][1], y[1]);
       }
     }
   }

@@ -214,3 +214,21 @@ def test_gram_of_a_wide_block_with_little_memory_left(lib_built):
         del held
         torch.cuda.empty_cache()
     assert (C - X.T @ X).abs().max().item() <= 1e-13 * n
+
+
+@pytest.mark.parametrize("p", [1, 2, 33, 64])
+@pytest.mark.parametrize("odd", [0, 1])
+def test_update_rounds_its_epilogue_once(lib_built, p, odd):
+    """alpha acc + beta Y is one fused multiply-add on the rounded product beta Y, by the 16-byte path
+    and the 8-byte one (an odd leading dimension): one product of one summand, exactly."""
+    from fractions import Fraction
+    import sparse_matrix_algorithms_b200 as S
+
+    rng = np.random.default_rng(p)
+    n, alpha, beta = 130, 0.37, 1.3
+    X, B, Y = rng.standard_normal((n, 1)), rng.standard_normal((p, 1)), rng.standard_normal((n, p + odd))
+    got = _update(S.context(), X, B, p, False, Y, alpha, beta, 1)
+    acc, by = X * B.T, beta * Y[:, :p]
+    ref = [[float(Fraction(alpha) * Fraction(a) + Fraction(b)) for a, b in zip(*r)] for r in zip(acc, by)]
+    np.testing.assert_array_equal(got[:, :p], np.array(ref))
+    np.testing.assert_array_equal(got[:, p:], Y[:, p:])
