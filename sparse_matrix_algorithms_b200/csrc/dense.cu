@@ -92,56 +92,6 @@ bool Dense::sygvd(int64_t k, double *A, int64_t lda, double *B, int64_t ldb, dou
 
 namespace {
 
-// Upper Cholesky G = R^T R of a k x k column-major G, k <= 64, in its upper triangle, with R^{-1}
-// (k x k, zeros below), out = R's diagonal and the 1-based index of the first pivot that is not
-// positive (then nothing else is written), else 0.  One CTA, everything in shared memory: a step
-// of the elimination takes a row of [G | I] off the rows below it, so that L^{-1} = R^{-T} is there
-// when R is.  A chain of k square roots and divisions bounds it; the library's
-// factorization, identity and triangular solve took 30 us and a second wait of the host (POLFED of
-// the 1D Laplacian, s = 32 n = 20000 23.9 -> 22.6 ms, s = 16 n = 6000 8.7 -> 7.5 ms).
-constexpr int kCholMax = 64, kCholThreads = 512;
-__global__ void __launch_bounds__(kCholThreads)
-chol_inverse_kernel(int k, double *G, int64_t ldg, double *__restrict__ Rinv, double *__restrict__ out) {
-  __shared__ double M[kCholMax][kCholMax + 1];  // R's rows; below the diagonal those of L^{-1}
-  __shared__ double dinv[kCholMax];
-  constexpr int kGroups = kCholThreads / kCholMax;
-  const int l = threadIdx.x % kCholMax, g = threadIdx.x / kCholMax;
-  if (l < k)
-    for (int c = g; c < k; c += kGroups) M[l][c] = l <= c ? G[l + c * ldg] : 0.0;
-  __syncthreads();
-  for (int j = 0; j < k; ++j) {
-    const double p = M[j][j];
-    if (!(p > 0.0)) {
-      if (threadIdx.x == 0) out[k] = j + 1;
-      return;
-    }
-    const double r = sqrt(p), inv = 1.0 / r;
-    __syncthreads();
-    if (g == 0 && l < k) {
-      if (l == j) {
-        M[j][j] = r;
-        dinv[j] = inv;
-      } else {
-        M[j][l] *= inv;
-      }
-    }
-    __syncthreads();
-    if (l < k) {
-      const double row = l == j ? inv : M[j][l];
-      for (int i = j + 1 + g; i < k; i += kGroups)
-        if (l <= j || l >= i) M[i][l] = fma(-M[j][i], row, M[i][l]);
-    }
-    __syncthreads();
-  }
-  if (l < k)
-    for (int c = g; c < k; c += kGroups) {
-      if (l <= c) G[l + c * ldg] = M[l][c];
-      Rinv[l + (int64_t)c * k] = l < c ? M[c][l] : l == c ? dinv[c] : 0.0;
-    }
-  if (g == 0 && l < k) out[l] = M[l][l];
-  if (threadIdx.x == 0) out[k] = 0.0;
-}
-
 // Upper Cholesky of the k x k column-major G in place. Returns cuSOLVER's info.
 int potrf_upper(sma_ctx *ctx, int64_t k, double *G, int64_t ldg) {
   int lwork = 0;
@@ -249,21 +199,8 @@ bool cholqr_pass(sma_ctx *ctx, int64_t n, int64_t k, double *X, int64_t ldx, dou
   if (G.count < (size_t)(k * k)) G.alloc(k * k, ctx->stream);
   dn.gram(n, k, k, X, ldx, X, ldx, G.p, k);
   if (shift > 0.0) launch_add_diagonal(ctx->stream, k, G.p, k, shift);
-  const bool small = k <= kCholMax && !ctx->cublas_dense;  // beyond, R^{-1} is a product's size too
-  DevBuf<double> Rinv, out;
-  std::vector<double> d;
-  if (small) {
-    Rinv.alloc(k * k, ctx->stream);
-    out.alloc(k + 1, ctx->stream);
-    chol_inverse_kernel<<<1, kCholThreads, 0, ctx->stream>>>((int)k, G.p, k, Rinv.p, out.p);
-    SMA_CHECK_LAUNCH();
-    d = to_host(ctx, out.p, k + 1);
-    if (d[k] != 0.0) return false;
-    d.pop_back();
-  } else {
-    if (potrf_upper(ctx, k, G.p, k) != 0) return false;
-    d = diag_to_host(ctx, G.p, k);
-  }
+  if (potrf_upper(ctx, k, G.p, k) != 0) return false;
+  std::vector<double> d = diag_to_host(ctx, G.p, k);
   double dmax = 0.0, dmin = INFINITY;
   for (double v : d) {
     if (!(std::isfinite(v) && v > 0.0)) return false;
@@ -271,10 +208,7 @@ bool cholqr_pass(sma_ctx *ctx, int64_t n, int64_t k, double *X, int64_t ldx, dou
     dmin = std::min(dmin, v);
   }
   if (max_spread > 0.0 && dmax / dmin > max_spread) return false;
-  if (small)
-    dgemm_update(ctx->stream, ctx->num_sms, n, k, k, X, ldx, Rinv.p, k, false, X, ldx, 1.0, 0.0);
-  else
-    trsm_right_upper(ctx, n, k, G.p, k, X, ldx);
+  trsm_right_upper(ctx, n, k, G.p, k, X, ldx);
   F.push(G.p, d);
   return true;
 }
