@@ -29,6 +29,7 @@
 //   C/D (8 x 8):     c0 = C[g][2t], c1 = C[g][2t + 1].
 #include <algorithm>
 
+#include "ordered_sum.cuh"
 #include "sma_internal.h"
 #include "vec.cuh"
 
@@ -318,10 +319,8 @@ __device__ __forceinline__ void finish(double *C, int64_t ldc, int64_t e, int m,
   *c = beta == 0.0 ? alpha * s : alpha * s + beta * *c;
 }
 
-// Both sum the splits one after the other, whatever the tiles were.  With few splits a thread takes
-// an element.  With many, the chain of loads would be the time: a CTA takes LANES elements, its
-// 256 / LANES groups of threads bring a share of the splits each to shared memory, and one of them
-// adds those up.
+// Both sum the splits one after the other, whatever the tiles were: with few splits a thread an
+// element, with many a CTA LANES elements at a time.
 template <typename T>
 __global__ void __launch_bounds__(256)
 gram_reduce_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
@@ -342,33 +341,12 @@ template <typename T, int LANES>
 __global__ void __launch_bounds__(256)
 gram_reduce_many_kernel(int m, int k, int tiles_m, int tiles_k, int splits, const double *__restrict__ part,
                         double *C, int64_t ldc, double alpha, double beta, bool upper) {
-  constexpr int kGroups = 256 / LANES, kEach = 8;  // splits of a group in one round
-  __shared__ double sh[kGroups * kEach][LANES + 1];
-  const int cl = threadIdx.x % LANES, rl = threadIdx.x / LANES;
+  __shared__ OrderedSum<LANES, 8> sum;
   const int64_t total = (int64_t)m * k, stride = (int64_t)tiles_k * tiles_m * (T::M * T::N);
   for (int64_t e0 = (int64_t)blockIdx.x * LANES; e0 < total; e0 += (int64_t)gridDim.x * LANES) {
-    const int64_t e = e0 + cl, at = e < total ? partial_place<T>(e, m, tiles_m, upper) : -1;
-    double s = 0.0;
-    for (int z0 = 0; z0 < splits; z0 += kGroups * kEach) {
-      const int count = min(kGroups * kEach, splits - z0);
-      if (at >= 0) {
-        double v[kEach];
-#pragma unroll
-        for (int u = 0; u < kEach; ++u) {
-          const int z = rl + u * kGroups;
-          v[u] = z < count ? part[at + (z0 + z) * stride] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < kEach; ++u) sh[rl + u * kGroups][cl] = v[u];
-      }
-      __syncthreads();
-      if (rl == 0 && at >= 0) {
-#pragma unroll 8
-        for (int z = 0; z < count; ++z) s += sh[z][cl];
-      }
-      __syncthreads();
-    }
-    if (rl == 0 && at >= 0) finish(C, ldc, e, m, s, alpha, beta);
+    const int64_t e = e0 + threadIdx.x % LANES, at = e < total ? partial_place<T>(e, m, tiles_m, upper) : -1;
+    const double s = sum(at < 0 ? nullptr : part + at, stride, splits);
+    if (threadIdx.x < LANES && at >= 0) finish(C, ldc, e, m, s, alpha, beta);
   }
 }
 

@@ -8,6 +8,7 @@
 // (chebyshev_subspace_iteration.jl:573-582, polfed.jl:483-492); AX never reaches memory.
 // It lives in clenshaw_step.cuh; this file holds its dispatcher and the small kernels around
 // the solvers.
+#include "ordered_sum.cuh"
 #include "sma_internal.h"
 #include "vec.cuh"
 
@@ -93,14 +94,61 @@ __global__ void randn_kernel(int64_t n, int64_t m, uint64_t seed, double *__rest
 }
 
 // ------------------------------------------------------------------ column reductions
-// Stage 1: a CTA sums one chunk of rows of up to 32 columns.  The 2^lc threads of a row group
-// sit on consecutive columns, so that narrow blocks (k = 16 of the KPM vectors) still use every
-// lane; 256 >> lc rows are in flight per pass.  mode 2 forms sum X Y and, `plane` further on, sum
-// Y Y from one read of both blocks.
+// mode 0: sum X Y down every column; mode 1: sum (Y - lam X)^2.  The order of the sums is part of
+// the result (a mixed-precision solve scales residuals with these norms before it rounds them to
+// FP32): a chunk of rows in eight interleaved groups, the groups one after the other, then the chunks.
+// Stage 1: the 2^lc threads of a row group sit on consecutive columns, so that narrow blocks use
+// every lane; a CTA takes 32 >> lc chunks of up to 32 columns.
 __global__ void __launch_bounds__(256)
 colred_stage1(int mode, int lc, int64_t n, int64_t k, const double *__restrict__ X, int64_t ldx,
               const double *__restrict__ Y, int64_t ldy, const double *__restrict__ lam,
-              double *__restrict__ partial, int64_t rows_per_chunk, int64_t plane) {
+              double *__restrict__ partial, int64_t chunks, int64_t rows_per_chunk) {
+  __shared__ double sh[256];
+  const int tid = threadIdx.x, cl = tid & ((1 << lc) - 1), rl = tid >> lc;
+  const int64_t col = ((int64_t)blockIdx.y << lc) + cl;
+  const int64_t chunk = (int64_t)blockIdx.x * (32 >> lc) + rl / 8;
+  const int64_t r0 = chunk * rows_per_chunk, r1 = min(n, r0 + rows_per_chunk);
+  double s = 0.0;
+  if (col < k && chunk < chunks) {
+    const double l = mode == 1 ? lam[col] : 0.0;
+#pragma unroll 4
+    for (int64_t i = r0 + rl % 8; i < r1; i += 8) {
+      const double x = X[i * ldx + col];
+      const double y = Y[i * ldy + col];
+      if (mode == 0) {
+        s = fma(x, y, s);
+      } else {
+        const double d = fma(-l, x, y);
+        s = fma(d, d, s);
+      }
+    }
+  }
+  sh[tid] = s;
+  __syncthreads();
+  if (rl % 8 == 0 && col < k && chunk < chunks) {
+    double t = 0.0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) t += sh[tid + (r << lc)];
+    partial[chunk * k + col] = t;
+  }
+}
+
+constexpr int kSumLanes = 4;
+__global__ void __launch_bounds__(256)
+colred_stage2(int mode, int64_t chunks, int64_t k, const double *__restrict__ partial, double *__restrict__ out) {
+  __shared__ OrderedSum<kSumLanes, 16> sum;
+  const int64_t col = (int64_t)blockIdx.x * kSumLanes + threadIdx.x % kSumLanes;
+  const double t = sum(col < k ? partial + col : nullptr, k, chunks);
+  if (threadIdx.x < kSumLanes && col < k) out[col] = mode == 1 ? sqrt(t) : t;
+}
+
+// The sums of a KPM step, sum X Y and, `plane` further on, sum Y Y from one read of both blocks, whose
+// order is free.  Stage 1: a CTA sums one chunk of rows of up to 32 columns; 256 >> lc rows are in
+// flight per pass.
+__global__ void __launch_bounds__(256)
+dots_stage1(int lc, int64_t n, int64_t k, const double *__restrict__ X, int64_t ldx,
+            const double *__restrict__ Y, int64_t ldy, double *__restrict__ partial,
+            int64_t rows_per_chunk, int64_t plane) {
   __shared__ double sh[2][256];
   const int tid = threadIdx.x, cl = tid & ((1 << lc) - 1), rl = tid >> lc, R = 256 >> lc;
   const int64_t col = ((int64_t)blockIdx.y << lc) + cl;
@@ -108,18 +156,12 @@ colred_stage1(int mode, int lc, int64_t n, int64_t k, const double *__restrict__
   const int64_t r1 = min(n, r0 + rows_per_chunk);
   double s = 0.0, s2 = 0.0;
   if (col < k) {
-    const double l = mode == 1 ? lam[col] : 0.0;
 #pragma unroll 4
     for (int64_t i = r0 + rl; i < r1; i += R) {
       const double x = X[i * ldx + col];
       const double y = Y[i * ldy + col];
-      if (mode == 1) {
-        const double d = y - l * x;
-        s = fma(d, d, s);
-      } else {
-        s = fma(x, y, s);
-        s2 = fma(y, y, s2);
-      }
+      s = fma(x, y, s);
+      s2 = fma(y, y, s2);
     }
   }
   sh[0][tid] = s;
@@ -133,7 +175,7 @@ colred_stage1(int mode, int lc, int64_t n, int64_t k, const double *__restrict__
   }
   if (rl == 0 && col < k) {
     partial[(int64_t)blockIdx.x * k + col] = sh[0][tid];
-    if (mode == 2) partial[plane + (int64_t)blockIdx.x * k + col] = sh[1][tid];
+    partial[plane + (int64_t)blockIdx.x * k + col] = sh[1][tid];
   }
 }
 
@@ -141,8 +183,8 @@ colred_stage1(int mode, int lc, int64_t n, int64_t k, const double *__restrict__
 // after the other), eight row groups of a CTA sharing the chunks: a serial sum of the 1184
 // partials of a KPM reduction took 80 of its 90 us.
 __global__ void __launch_bounds__(256)
-colred_stage2(int mode, int64_t chunks, int64_t k, int64_t total, const double *__restrict__ partial,
-              double *__restrict__ out) {
+dots_stage2(int64_t chunks, int64_t k, int64_t total, const double *__restrict__ partial,
+            double *__restrict__ out) {
   __shared__ double sh[8][33];
   const int cl = threadIdx.x % 32, rl = threadIdx.x / 32;
   const int64_t e = (int64_t)blockIdx.x * 32 + cl;
@@ -158,7 +200,7 @@ colred_stage2(int mode, int64_t chunks, int64_t k, int64_t total, const double *
     t = 0.0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) t += sh[r][cl];
-    out[e] = mode == 1 ? sqrt(t) : t;
+    out[e] = t;
   }
 }
 
@@ -443,29 +485,33 @@ void launch_randn(cudaStream_t st, int64_t n, int64_t m, uint64_t seed, double *
   SMA_CHECK_LAUNCH();
 }
 
-void column_partials(cudaStream_t st, int mode, int64_t n, int64_t k, const double *X, int64_t ldx,
-                     const double *Y, int64_t ldy, const double *lam, double *partial) {
+// 2^lc columns of a CTA: up to 32
+static int column_lanes(int64_t k) {
   int lc = 0;
   while (lc < 5 && (1 << lc) < k) ++lc;
-  const int64_t ctiles = (k + (1 << lc) - 1) >> lc;
-  const int64_t chunks = column_chunks(n, k);
-  const dim3 grid((unsigned)chunks, (unsigned)ctiles);
-  colred_stage1<<<grid, 256, 0, st>>>(mode, lc, n, k, X, ldx, Y, ldy, lam, partial,
-                                      (n + chunks - 1) / chunks, chunks * k);
+  return lc;
+}
+
+void column_dots(cudaStream_t st, int64_t n, int64_t k, const double *X, int64_t ldx, const double *Y,
+                 int64_t ldy, double *partial) {
+  const int lc = column_lanes(k);
+  const int64_t chunks = column_dot_chunks(n, k);
+  const dim3 grid((unsigned)chunks, (unsigned)((k + (1 << lc) - 1) >> lc));
+  dots_stage1<<<grid, 256, 0, st>>>(lc, n, k, X, ldx, Y, ldy, partial, (n + chunks - 1) / chunks, chunks * k);
   SMA_CHECK_LAUNCH();
 }
 
 // Chunks of rows: four CTAs an SM over the whole grid, each thread summing at least eight rows.
-int64_t column_chunks(int64_t n, int64_t k) {
+int64_t column_dot_chunks(int64_t n, int64_t k) {
   const int64_t ctiles = (k + 31) / 32;
   const int64_t rows = k >= 32 ? 64 : 8 * (256 / std::max<int64_t>(k, 1));
   return std::max<int64_t>(1, std::min<int64_t>((n + rows - 1) / rows, (148 * 4 + ctiles - 1) / ctiles));
 }
 
-void column_totals(cudaStream_t st, int mode, int64_t chunks, int64_t k, int64_t groups,
-                   const double *partial, double *out) {
+void column_dot_totals(cudaStream_t st, int64_t chunks, int64_t k, int64_t groups, const double *partial,
+                       double *out) {
   const int64_t total = groups * k;
-  colred_stage2<<<(unsigned)((total + 31) / 32), 256, 0, st>>>(mode, chunks, k, total, partial, out);
+  dots_stage2<<<(unsigned)((total + 31) / 32), 256, 0, st>>>(chunks, k, total, partial, out);
   SMA_CHECK_LAUNCH();
 }
 
@@ -473,10 +519,17 @@ void column_reduce(cudaStream_t st, int mode, int64_t n, int64_t k, const double
                    const double *Y, int64_t ldy, const double *lam, double *out,
                    DevBuf<double> &scratch) {
   if (k == 0) return;
-  const int64_t chunks = column_chunks(n, k);
+  const int64_t tiles = (k + 31) / 32;
+  int64_t chunks = std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, (148 * 8 + tiles - 1) / tiles));
+  const int64_t rows = (n + chunks - 1) / chunks;
+  chunks = rows ? (n + rows - 1) / rows : 1;
   if (scratch.count < (size_t)(chunks * k)) scratch.alloc(chunks * k, st);
-  column_partials(st, mode, n, k, X, ldx, Y, ldy, lam, scratch.p);
-  column_totals(st, mode, chunks, k, 1, scratch.p, out);
+  const int lc = column_lanes(k), each = 32 >> lc;
+  const dim3 grid((unsigned)((chunks + each - 1) / each), (unsigned)((k + (1 << lc) - 1) >> lc));
+  colred_stage1<<<grid, 256, 0, st>>>(mode, lc, n, k, X, ldx, Y, ldy, lam, scratch.p, chunks, rows);
+  SMA_CHECK_LAUNCH();
+  colred_stage2<<<(unsigned)((k + kSumLanes - 1) / kSumLanes), 256, 0, st>>>(mode, chunks, k, scratch.p, out);
+  SMA_CHECK_LAUNCH();
 }
 
 static void transpose(cudaStream_t st, int64_t R, int64_t C, const double *in, int64_t ldi,

@@ -63,7 +63,7 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   constexpr int64_t kGroup = 64;
   int64_t chunks = (clenshaw_dot_chunks(op, w) + kGroup - 1) / kGroup * kGroup;
   const bool fused = chunks > 0 && 2 * chunks * R <= int64_t(32) << 20;
-  if (!fused) chunks = column_chunks(n, R);
+  if (!fused) chunks = column_dot_chunks(n, R);
   const int64_t set = 2 * chunks * R;
   const int64_t steps = (M + 1) / 2, fused_steps = fused ? M / 2 : 0;
   const int64_t batch = std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
@@ -90,7 +90,7 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
     } else {
       launch_clenshaw_step<double>(op, st, w, Q, w, B1, nullptr, w, out, w, ck, alpha, beta, true, rev);
     }
-    column_partials(st, 2, n, R, out, w, B1, w, nullptr, slot);
+    column_dots(st, n, R, out, w, B1, w, slot);
   };
   // dots: for k = 0, 1, ...: <T_{k+1}, T_k> then <T_k, T_k> (R values each)
   double *Tprev = t0.p, *Tcur = t0.p, *Tnext = t1.p, *Tfree = t2.p;
@@ -105,17 +105,17 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
     } else if (fused) {  // an odd M: the last moment needs <T_k, T_k> only
       column_reduce(st, 0, n, R, Tcur, w, Tcur, w, nullptr, dots.p + (2 * k + 1) * R, last);
     } else {
-      column_partials(st, 2, n, R, Tcur, w, Tcur, w, nullptr, slot);
+      column_dots(st, n, R, Tcur, w, Tcur, w, slot);
     }
     if (fused ? k + 1 <= fused_steps && (k + 1 - done == batch || k + 1 == fused_steps)
               : k + 1 - done == batch || k + 1 == steps) {
       const int64_t groups = 2 * (k + 1 - done);
       double *out = dots.p + 2 * done * R;
       if (fused) {
-        column_totals(st, 0, kGroup, R, groups * (chunks / kGroup), partial.p, sums.p);
-        column_totals(st, 0, chunks / kGroup, R, groups, sums.p, out);
+        column_dot_totals(st, kGroup, R, groups * (chunks / kGroup), partial.p, sums.p);
+        column_dot_totals(st, chunks / kGroup, R, groups, sums.p, out);
       } else {
-        column_totals(st, 0, chunks, R, groups, partial.p, out);
+        column_dot_totals(st, chunks, R, groups, partial.p, out);
       }
       done = k + 1;
     }

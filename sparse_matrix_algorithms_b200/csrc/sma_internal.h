@@ -274,13 +274,13 @@ void launch_randn(cudaStream_t st, int64_t n, int64_t m, uint64_t seed, double *
 void column_reduce(cudaStream_t st, int mode, int64_t n, int64_t k, const double *X, int64_t ldx,
                    const double *Y, int64_t ldy, const double *lam, double *out,
                    DevBuf<double> &scratch);
-// Its two stages apart, so that many reductions can share one second stage: chunks x k partials
-// (mode 2: those of mode 0, then those of sum Y Y) and the sums of `groups` such sets.
-int64_t column_chunks(int64_t n, int64_t k);
-void column_partials(cudaStream_t st, int mode, int64_t n, int64_t k, const double *X, int64_t ldx,
-                     const double *Y, int64_t ldy, const double *lam, double *partial);
-void column_totals(cudaStream_t st, int mode, int64_t chunks, int64_t k, int64_t groups,
-                   const double *partial, double *out);
+// The sums of KPM steps: chunks x k partials of sum X Y, then as many of sum Y Y, and the sums of
+// `groups` sets of chunks x k partials (one launch for many steps).
+int64_t column_dot_chunks(int64_t n, int64_t k);
+void column_dots(cudaStream_t st, int64_t n, int64_t k, const double *X, int64_t ldx, const double *Y,
+                 int64_t ldy, double *partial);
+void column_dot_totals(cudaStream_t st, int64_t chunks, int64_t k, int64_t groups, const double *partial,
+                       double *out);
 // dst (row-major n x b, ldd) <- src (row-major, lds); optional type conversion
 template <typename TS, typename TD>
 void launch_copy_block(cudaStream_t st, int64_t n, int64_t b, const TS *src, int64_t lds, TD *dst,
