@@ -101,7 +101,8 @@ int sma_ctx_create(int device, sma_ctx **out) {
     auto *ctx = new sma_ctx();
     ctx->device = device;
     const char *at = std::getenv("SMA_AUTOTUNE"), *av = std::getenv("SMA_AUTOTUNE_VERBOSE");
-    ctx->tune = av && std::string(av) == "1" && !(at && std::string(at) == "0");
+    ctx->tune = at && std::string(at) == "1";
+    ctx->tune_verbose = av && std::string(av) == "1" && !(at && std::string(at) == "0");
     const char *fg = std::getenv("SMA_FILTER_GRAPHS");
     ctx->filter_graphs = !(fg && std::string(fg) == "0");
     const char *pe = std::getenv("SMA_PERSISTENT");

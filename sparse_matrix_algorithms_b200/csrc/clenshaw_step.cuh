@@ -40,6 +40,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "sma_internal.h"
 #include "vec.cuh"
@@ -73,6 +74,7 @@ struct Step {
   uint32_t rows;      // rows of a CTA (rows * lanes <= kThreads)
   uint32_t divlanes;  // ceil(2^16 / lanes): i / lanes = i * divlanes >> 16 for i < 192
   int rev;
+  bool tune;          // host: the step may be one of the autotuner's trials
 };
 
 template <typename T>
@@ -463,8 +465,9 @@ inline uint32_t panel_lanes(uint32_t vecs) {
   return best;
 }
 
+// Where not 0 or negative, `gathers` and `flat` take the place of the rules for them.
 template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL, Form P>
-void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0) {
+void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0, int flat_wanted = -1) {
   const uint32_t vecs = a.b / V;
   a.lanes = panel_lanes(vecs);
   a.rows = kThreads / a.lanes;
@@ -489,8 +492,8 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   // 152 and 155).
   constexpr bool kFlat = !(MODEL || P == DOTS || P == FIRST);
   const uint32_t used = a.rows * a.lanes;
-  const bool flat = kFlat && gathers != 8 && used % 32 != 0 && (a.lanes <= 40 || kThreads - used >= 16) &&
-                    (uint64_t)a.n * a.lanes < (uint64_t)1 << 32;
+  const bool flat = kFlat && gathers != 8 && used < kThreads && (uint64_t)a.n * a.lanes < (uint64_t)1 << 32 &&
+                    (flat_wanted < 0 ? used % 32 != 0 && (a.lanes <= 40 || kThreads - used >= 16) : flat_wanted > 0);
   const uint32_t gx = flat ? (uint32_t)(((uint64_t)a.n * a.lanes + kThreads - 1) / kThreads)
                            : (a.n + a.rows - 1) / a.rows;
   constexpr uint32_t kGridY = 65535;
@@ -524,44 +527,74 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0)
   }
 }
 
-// ------------------------------------------------------------------ the tuning table
-// With SMA_AUTOTUNE_VERBOSE=1 in the environment (and SMA_AUTOTUNE not 0) the first launches of
-// each shape of an operator with n >= 20000 run every configuration in turn, four times, on the
-// real steps, bracketed by events; then the table is printed and the fastest kept.  A check of
-// the rules above: without the variable they alone choose.
+// ------------------------------------------------------------------ the autotuner
+// With SMA_AUTOTUNE=1 the first launches of each shape of an operator with n >= 20000 run every
+// configuration in turn, four times, on the real steps, bracketed by events, and the fastest is kept:
+// for matrices that the rules, which were measured on lattices, chains and rings of up to 100 entries
+// a row, may not fit.  SMA_AUTOTUNE_VERBOSE=1 does the same and prints the table, as a check of the
+// rules: what it found is kept only with SMA_AUTOTUNE=1.  With neither the rules alone choose.
 struct Config {
   bool bulk;
-  int V, gathers;
+  int V, gathers, flat;
 };
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
+template <typename T, bool HQ, bool HS, bool HB, bool PC>
 void launch_config(const sma_op *op, cudaStream_t st, const Step<T> &a, const Config &c) {
-  if constexpr (!PC)
-    if (c.bulk) return launch_bulk<T, V, HQ, HS, HB>(op, st, a);
-  launch_width<T, V, HQ, HS, HB, PC, false, false, INNER>(op, st, a, c.gathers);
+  auto with = [&](auto width) {
+    constexpr int V = decltype(width)::value;
+    if constexpr (!PC)
+      if (c.bulk) return launch_bulk<T, V, HQ, HS, HB>(op, st, a);
+    launch_width<T, V, HQ, HS, HB, PC, false, false, INNER>(op, st, a, c.gathers, c.flat);
+  };
+  if constexpr (sizeof(T) == 4)
+    if (c.V == 8) return with(std::integral_constant<int, 8>{});
+  if (c.V == 4) return with(std::integral_constant<int, 4>{});
+  if (c.V == 2) return with(std::integral_constant<int, 2>{});
+  with(std::integral_constant<int, 1>{});
 }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC>
-bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
-  if (!op->ctx->tune || op->n < 20000) return false;
-  cudaStreamCaptureStatus cap;
-  SMA_CUDA(cudaStreamIsCapturing(st, &cap));
-  CsrTune &t = const_cast<sma_op *>(op)->tuned[{(int64_t)sizeof(T) * 8 + V, HQ * 8 + HS * 4 + HB * 2 + PC, a.b}];
-  std::vector<Config> cfg = {{false, V, 8}, {false, V, 4}};
-  if constexpr (!PC) {
-    if (bulk_fits<T, V, HQ, HS, HB>(op, a)) {
-      if (!op->bulk_err && cap == cudaStreamCaptureStatusNone) {
-        SMA_CUDA(cudaMalloc((void **)&const_cast<sma_op *>(op)->bulk_err, sizeof(int)));
-        SMA_CUDA(cudaMemset(op->bulk_err, 0, sizeof(int)));
-      }
-      if (op->bulk_err) cfg.push_back({true, V, 0});
+// Whole rows and flat ones, with every number of gathers that there is, at the widest vectors and at
+// half of them; the BULK family where it fits.
+template <typename T, bool HQ, bool HS, bool HB, bool PC>
+std::vector<Config> configs(const sma_op *op, const Step<T> &a, int widest) {
+  std::vector<Config> all;
+  for (int v = widest; v >= 1 && 2 * v >= widest; v /= 2) {
+    const uint32_t lanes = panel_lanes(a.b / v);
+    for (int gathers : {8, 6, 4}) {
+      if (gathers == 6 && !ragged(op)) continue;
+      all.push_back({false, v, gathers, 0});
+      if (gathers != 8 && kThreads % lanes) all.push_back({false, v, gathers, 1});
     }
   }
-  if (t.chosen >= 0) {
-    launch_config<T, V, HQ, HS, HB, PC>(op, st, a, cfg[std::min(t.chosen, (int)cfg.size() - 1)]);
+  if constexpr (!PC) {
+    bool fits = widest == 4 ? bulk_fits<T, 4, HQ, HS, HB>(op, a) : widest == 2 ? bulk_fits<T, 2, HQ, HS, HB>(op, a)
+                                                                              : false;
+    if constexpr (sizeof(T) == 4) fits = widest == 8 ? bulk_fits<T, 8, HQ, HS, HB>(op, a) : fits;
+    if (fits) all.push_back({true, widest, 0, 0});
+  }
+  return all;
+}
+
+// v: the rule's vector width.
+template <typename T, bool HQ, bool HS, bool HB, bool PC>
+bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a, int widest, int v) {
+  const sma_ctx *ctx = op->ctx;
+  if (!(ctx->tune || ctx->tune_verbose) || !a.tune || op->n < 20000) return false;
+  cudaStreamCaptureStatus cap;
+  SMA_CUDA(cudaStreamIsCapturing(st, &cap));
+  const std::vector<Config> cfg = configs<T, HQ, HS, HB, PC>(op, a, widest);
+  CsrTune &t = const_cast<sma_op *>(op)->tuned[{(int64_t)sizeof(T) * 16 + widest,
+                                                cfg.back().bulk * 16 + HQ * 8 + HS * 4 + HB * 2 + PC, a.b}];
+  if (t.done && !ctx->tune) return false;
+  if (t.done) {
+    launch_config<T, HQ, HS, HB, PC>(op, st, a, cfg[t.fastest]);
     return true;
   }
   if (cap != cudaStreamCaptureStatusNone) return false;
+  if (cfg.back().bulk && !op->bulk_err) {
+    SMA_CUDA(cudaMalloc((void **)&const_cast<sma_op *>(op)->bulk_err, sizeof(int)));
+    SMA_CUDA(cudaMemset(op->bulk_err, 0, sizeof(int)));
+  }
   cudaEvent_t e[2];
   const size_t i = t.events.size() / 2;
   for (cudaEvent_t &x : e) {
@@ -569,7 +602,7 @@ bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
     t.events.push_back(x);
   }
   SMA_CUDA(cudaEventRecord(e[0], st));
-  launch_config<T, V, HQ, HS, HB, PC>(op, st, a, cfg[i % cfg.size()]);
+  launch_config<T, HQ, HS, HB, PC>(op, st, a, cfg[i % cfg.size()]);
   SMA_CUDA(cudaEventRecord(e[1], st));
   if (i + 1 < 4 * cfg.size()) return true;
   SMA_CUDA(cudaEventSynchronize(e[1]));
@@ -580,33 +613,32 @@ bool tuned_step(const sma_op *op, cudaStream_t st, const Step<T> &a) {
     best[k % cfg.size()] = std::min(best[k % cfg.size()], ms);
   }
   t.release();
-  t.chosen = (int)(std::min_element(best.begin(), best.end()) - best.begin());
-  fprintf(stderr, "sma autotune: %s n=%lld b=%lld variant=%d%d%d ->", sizeof(T) == 8 ? "fp64" : "fp32",
-          (long long)op->n, (long long)a.b, (int)HQ, (int)HS, (int)HB);
+  t.fastest = (int)(std::min_element(best.begin(), best.end()) - best.begin());
+  t.done = true;
+  if (!ctx->tune_verbose) return true;
+  fprintf(stderr, "sma autotune: %s n=%lld b=%lld variant=%d%d%d%d, the rule has V%d ->", sizeof(T) == 8 ? "fp64" : "fp32",
+          (long long)op->n, (long long)a.b, (int)HQ, (int)HS, (int)HB, (int)PC, v);
   for (size_t k = 0; k < cfg.size(); ++k)
-    fprintf(stderr, " %s%s/V%d/U%d=%.1fus", (int)k == t.chosen ? "*" : "",
-            cfg[k].bulk ? "bulk" : "rows", V, cfg[k].gathers, 1e3 * best[k]);
+    fprintf(stderr, " %s%s/V%d/U%d=%.1fus", (int)k == t.fastest ? "*" : "",
+            cfg[k].bulk ? "bulk" : cfg[k].flat ? "flat" : "rows", cfg[k].V, cfg[k].gathers, 1e3 * best[k]);
   fprintf(stderr, "\n");
   return true;
 }
 
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool MODEL, Form P>
-void launch_rule(const sma_op *op, cudaStream_t st, const Step<T> &a) {
-  if constexpr (!MODEL && P == INNER)
-    if (tuned_step<T, V, HQ, HS, HB, PC>(op, st, a)) return;
-  launch_width<T, V, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
-}
-
 inline bool aligned(const void *p, int bytes) { return ((uintptr_t)p % bytes) == 0; }
 
-// Picks the vector width: the widest that widths, strides and addresses allow (fits), but half of
-// it below 40000 threads, and less while the step would not give every SM half a CTA (us a step:
+template <typename T, typename Fits>
+int widest_vector(Fits fits) {
+  int v = 32 / (int)sizeof(T);
+  while (v > 1 && !fits(v)) v /= 2;
+  return v;
+}
+
+// The vector width: the widest that widths, strides and addresses allow, but half of it below 40000
+// threads, and less while the step would not give every SM half a CTA (us a step:
 // Anderson L = 16, b = 32 FP64, 32768 threads 2.6, 65536 2.4; L = 20, b = 64 FP32, 64000 threads
 // 2.9, 128000 3.2; XXZ L = 14, b = 32 FP64, 27456 threads 3.1, 54912 2.8).
-template <typename T, typename Fits>
-int vector_width(const sma_op *op, int64_t b, Fits fits) {
-  int widest = 32 / (int)sizeof(T);
-  while (widest > 1 && !fits(widest)) widest /= 2;
+inline int vector_width(const sma_op *op, int64_t b, int widest) {
   for (int v = widest; v > 1; v /= 2)
     if (op->n * (b / v) >= (v == widest ? 40000 : 64LL * op->ctx->num_sms)) return v;
   return 1;
@@ -637,11 +669,13 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
            (!PC || a.colseg || (aligned(a.cseg, bytes) && (P == INNER || aligned(a.topseg, bytes))));
   };
   if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL, P>(op, st, a);
-  const int v = vector_width<T>(op, b, fits);
+  const int widest = widest_vector<T>(fits), v = vector_width(op, b, widest);
+  if constexpr (!MODEL && P == INNER)
+    if (tuned_step<T, HQ, HS, HB, PC>(op, st, a, widest, v)) return;
   if constexpr (sizeof(T) == 4)
-    if (v == 8) return launch_rule<T, 8, HQ, HS, HB, PC, MODEL, P>(op, st, a);
-  if (v == 4) return launch_rule<T, 4, HQ, HS, HB, PC, MODEL, P>(op, st, a);
-  if (v == 2) return launch_rule<T, 2, HQ, HS, HB, PC, MODEL, P>(op, st, a);
+    if (v == 8) return launch_width<T, 8, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
+  if (v == 4) return launch_width<T, 4, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
+  if (v == 2) return launch_width<T, 2, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
   launch_width<T, 1, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
 }
 
@@ -649,7 +683,7 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
 
 template <typename T>
 rows::Step<T> clenshaw_arguments(const T *Q, int64_t ldq, const T *B1, const T *B2, int64_t ldb, T *out,
-                                 int64_t ldo, double alpha, double beta, bool rev) {
+                                 int64_t ldo, double alpha, double beta, bool rev, bool tune = true) {
   rows::Step<T> a{};
   a.Q = Q;
   a.B1 = B1;
@@ -661,14 +695,15 @@ rows::Step<T> clenshaw_arguments(const T *Q, int64_t ldq, const T *B1, const T *
   a.alpha = (T)alpha;
   a.beta = (T)beta;
   a.rev = rev;
+  a.tune = tune;
   return a;
 }
 
 template <typename T, bool MODEL>
 void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                    const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                   double alpha, double beta, bool has_self, bool rev) {
-  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev);
+                   double alpha, double beta, bool has_self, bool rev, bool tune = false) {
+  rows::Step<T> a = clenshaw_arguments<T>(Q, ldq, B1, B2, ldb, out, ldo, alpha, beta, rev, tune);
   a.ck = (T)ck;
   if (Q && has_self && B2) return rows::step<T, true, true, true, false, MODEL>(op, st, b, a);
   if (Q && has_self && !B2) return rows::step<T, true, true, false, false, MODEL>(op, st, b, a);

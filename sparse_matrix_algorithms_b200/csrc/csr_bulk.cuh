@@ -1,5 +1,4 @@
-// A second family of the fused CSR step, kept to measure the first against (the tuning table of
-// clenshaw_step.cuh): whole neighbour rows staged in shared memory by 1D bulk copies.  Measured
+// A second family of the fused CSR step, one of the autotuner's candidates (clenshaw_step.cuh): whole neighbour rows staged in shared memory by 1D bulk copies.  Measured
 // 2 to 4 times slower (Anderson n = 262144, b = 64 FP32: 160-254 us a step): a row of 128-512
 // bytes is too small a copy for the copy engine.
 #pragma once

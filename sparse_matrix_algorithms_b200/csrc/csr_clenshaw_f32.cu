@@ -7,8 +7,8 @@ template <>
 void csr_clenshaw_step<float>(const sma_op *op, cudaStream_t st, int64_t b, const float *Q, int64_t ldq,
                                const float *B1, const float *B2, int64_t ldb, float *out,
                                int64_t ldo, double ck, double alpha, double beta, bool has_self,
-                               bool rev) {
-  clenshaw_step<float, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
+                               bool rev, bool tune) {
+  clenshaw_step<float, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev, tune);
 }
 
 template <>

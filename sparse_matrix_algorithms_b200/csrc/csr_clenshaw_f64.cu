@@ -7,8 +7,8 @@ template <>
 void csr_clenshaw_step<double>(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, int64_t ldq,
                                const double *B1, const double *B2, int64_t ldb, double *out,
                                int64_t ldo, double ck, double alpha, double beta, bool has_self,
-                               bool rev) {
-  clenshaw_step<double, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
+                               bool rev, bool tune) {
+  clenshaw_step<double, false>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev, tune);
 }
 
 template <>
@@ -42,7 +42,7 @@ void csr_clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const doubl
 // block, written once and read once, against the two blocks of the pass.
 int64_t clenshaw_dot_chunks(const sma_op *op, int64_t b) {
   if (op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF) return 0;
-  const int v = rows::vector_width<double>(op, b, [&](int w) { return b % w == 0; });
+  const int v = rows::vector_width(op, b, rows::widest_vector<double>([&](int w) { return b % w == 0; }));
   const int64_t rows = rows::kThreads / (b / v);
   return b / v <= 16 ? (op->n + rows - 1) / rows : 0;
 }

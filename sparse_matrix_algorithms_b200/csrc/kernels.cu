@@ -362,10 +362,10 @@ __global__ void check_csr_kernel(int64_t n, const int *__restrict__ rowptr,
 template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                          double alpha, double beta, bool has_self, bool rev) {
+                          double alpha, double beta, bool has_self, bool rev, bool tune) {
   if (op->n == 0 || b == 0) return;
   if (op->kind == OP_CSR) {
-    csr_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
+    csr_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev, tune);
   } else if (op->kind == OP_LAP1D || op->kind == OP_ANDERSON || op->kind == OP_XXZ) {
     model_clenshaw_step<T>(op, st, b, Q, ldq, B1, B2, ldb, out, ldo, ck, alpha, beta, has_self, rev);
   } else {
@@ -450,10 +450,10 @@ template void launch_pad_block<float, float>(cudaStream_t, int64_t, int64_t, con
                                              int64_t, float *, int64_t);
 template void launch_clenshaw_step<double>(const sma_op *, cudaStream_t, int64_t, const double *,
                                            int64_t, const double *, const double *, int64_t,
-                                           double *, int64_t, double, double, double, bool, bool);
+                                           double *, int64_t, double, double, double, bool, bool, bool);
 template void launch_clenshaw_step<float>(const sma_op *, cudaStream_t, int64_t, const float *,
                                           int64_t, const float *, const float *, int64_t, float *,
-                                          int64_t, double, double, double, bool, bool);
+                                          int64_t, double, double, double, bool, bool, bool);
 template void launch_clenshaw_start<double>(const sma_op *, cudaStream_t, int64_t, const double *,
                                             int64_t, const double *, int64_t, double *, int64_t, double,
                                             double, double, double, bool);

@@ -13,14 +13,16 @@
 //    3 * 2^21 * 8 bytes = 48 MiB, held on every device where it is loaded until the process
 //    exits;
 //  * every call on a device uses the same array, which keeps the contents of the last call.
-//    The recurrence writes each block before reading it (B1 = c_K Q first; B2 is first read
-//    after being written), so nothing has to start at zero.  Calls whose work overlaps on
+//    The recurrence writes each block before reading it (its first step gathers c_K Q from Q,
+//    or for K = 1 from a copy), so nothing has to start at zero.  Calls whose work overlaps on
 //    the GPU -- different streams, contexts or threads on the same device -- race on the
 //    array; callers serialize them;
 //  * the first call on a device looks the array's device address up (cudaGetSymbolAddress
 //    with that device current) and caches it; make that first call before any stream
 //    capture.  cudaDeviceReset ends every context of this library on that device, this
-//    cached address included.
+//    cached address included;
+//  * the steps are the rules' (clenshaw_step.cuh): no trials of the autotuner, which create
+//    events and may allocate.
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -118,17 +120,16 @@ void filter_noalloc(sma_op *op, const double *coeffs, int64_t K, double smin, do
     }
     for (; ci >= 1; --ci) {
       launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, B2, b, TMP, b, coeffs[ci], alpha, beta, true,
-                                   ci & 1);
+                                   ci & 1, false);
       rotate();
     }
     if (K == 2)
       launch_clenshaw_start<double>(op, st, b, Q, ldq, B1, b, Y, ldy, coeffs[K], coeffs[0], invd, -(c * invd));
     else
       launch_clenshaw_step<double>(op, st, b, Q, ldq, B1, fold ? B2 : nullptr, b, Y, ldy, coeffs[0], invd,
-                                   -(c * invd), true, false);
+                                   -(c * invd), true, false, false);
   }
   SMA_CUDA(cudaStreamSynchronize(st));
-  check_bulk_error(op, st);  // a bulk-copy step reports a wait that gave up
 }
 
 }  // namespace

@@ -68,10 +68,11 @@ inline void require(bool ok, int code, const std::string &msg) {
 }
 
 // Timed launches of the CSR step for one (type and vector width, variant, width) of an operator
-// (the tuning table of clenshaw_step.cuh).
+// (the autotuner of clenshaw_step.cuh).
 struct CsrTune {
   std::vector<cudaEvent_t> events;  // start and stop of each timed launch so far
-  int chosen = -1;                  // the configuration kept once all have been timed
+  bool done = false;                // all have been timed
+  int fastest = -1;                 // the configuration that was
   CsrTune() = default;
   CsrTune(const CsrTune &) = delete;
   CsrTune &operator=(const CsrTune &) = delete;
@@ -91,7 +92,8 @@ struct sma_ctx {
   cublasHandle_t cublas = nullptr;
   cusolverDnHandle_t cusolver = nullptr;
   int num_sms = 148;
-  bool tune = false;  // SMA_AUTOTUNE_VERBOSE=1 and SMA_AUTOTUNE not 0: time the CSR step's kernels
+  bool tune = false;          // SMA_AUTOTUNE=1: time the CSR step's kernels and keep the fastest
+  bool tune_verbose = false;  // SMA_AUTOTUNE_VERBOSE=1, SMA_AUTOTUNE not 0: time them and print the times
   // SMA_FILTER_GRAPHS=0 turns off the CUDA-graph replay of repeated filters (filter.cu)
   bool filter_graphs = true;
   // SMA_PERSISTENT=1: CSR filters run as one persistent cooperative launch (persistent.cu)
@@ -135,7 +137,7 @@ struct sma_op {
   // caller callback
   sma_matblock_fn fn = nullptr;
   void *user = nullptr;
-  // the tuning table of the CSR step; for its BULK family the most CSR entries any CTA of RC rows
+  // the autotuner of the CSR step; for its BULK family the most CSR entries any CTA of RC rows
   // holds, per RC (from a host copy of the row pointers), and the device flag its bounded wait
   // sets when it gives up
   std::map<std::array<int64_t, 3>, sma::CsrTune> tuned;
@@ -193,11 +195,12 @@ struct Block {
 // ------------------------------------------------------------------ kernels (kernels.cu)
 // out = ck*Q + alpha*(A*B1) + beta*B1 - B2 over b columns (one Clenshaw step).
 // Q may be null (ck ignored), B2 may be null, has_self=false drops the beta*B1 term.  rev: the
-// rows are walked from the last to the first; a recurrence alternates it from step to step.
+// rows are walked from the last to the first; a recurrence alternates it from step to step.  tune =
+// false: no trial of the autotuner (nothing is allocated, no event created).
 template <typename T>
 void launch_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                           const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                          double alpha, double beta, bool has_self, bool rev = false);
+                          double alpha, double beta, bool has_self, bool rev = false, bool tune = true);
 // The first two steps of a recurrence, whose block c_top Q is not written: B1 = c_top Q (B1 null),
 // and B2 = c_top Q.  The first must not write to Q.
 template <typename T>
@@ -233,7 +236,7 @@ void model_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *
 template <typename T>
 void csr_clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                        const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
-                       double alpha, double beta, bool has_self, bool rev);
+                       double alpha, double beta, bool has_self, bool rev, bool tune = true);
 // Throws SMA_ERR_TIMEOUT (and clears the flag) when a BULK-family launch of the CSR step on
 // this operator gave up its bounded wait; synchronizes the stream when the family was used.
 void check_bulk_error(const sma_op *op, cudaStream_t st);

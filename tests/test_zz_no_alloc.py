@@ -105,3 +105,31 @@ def test_noalloc_filter_size_limit(lib_built):
     rc = L.load().sma_apply_poly_block_noalloc(half.handle, c.ctypes.data, len(c) - 1, 0.0, 4.0,
                                                Q.data_ptr(), b, Q.data_ptr(), b, b)
     assert rc == L.SMA_ERR_ARG
+
+
+@pytest.mark.parametrize("autotune,verbose", [(None, "1"), ("1", "1"), ("1", None)])
+def test_noalloc_filter_makes_no_trials_of_the_autotuner(lib_built, monkeypatch, capfd, autotune, verbose):
+    """The autotuner's trials create events and allocate; the allocation-free entry takes the rule's
+    step whatever the environment asks for, also of an operator that the regular entry has tuned."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+
+    for name, value in (("SMA_AUTOTUNE", autotune), ("SMA_AUTOTUNE_VERBOSE", verbose)):
+        monkeypatch.delenv(name, raising=False)
+        if value:
+            monkeypatch.setenv(name, value)
+    A = M.anderson3d(30, 16.5, 9)  # n = 27000: large enough to be tuned
+    n, b = A.shape[0], 32
+    op = S.SparseOperator(A, S.Context(0))
+    smin, smax = O.gershgorin_bounds(A)
+    c = np.ascontiguousarray(O.build_coeffs(200, smin, smax, 0.1, -0.4, 0.3, "step", True))
+    Q = torch.as_tensor(M.splitmix_normal(5, n, b), device="cuda")
+    Y = torch.empty_like(Q)
+    first = _run("sma_apply_poly_block_noalloc", op, c, smin, smax, Q, b, Y, b, b)
+    free = torch.cuda.mem_get_info()[0]
+    assert np.array_equal(_run("sma_apply_poly_block_noalloc", op, c, smin, smax, Q, b, Y, b, b), first)
+    assert torch.cuda.mem_get_info()[0] == free
+    assert "sma autotune" not in capfd.readouterr().err
+    assert np.array_equal(_run("sma_apply_poly_block_dev", op, c, smin, smax, Q, b, Y, b, b), first)
+    assert ("sma autotune" in capfd.readouterr().err) == (verbose is not None)
+    assert np.array_equal(_run("sma_apply_poly_block_noalloc", op, c, smin, smax, Q, b, Y, b, b), first)
