@@ -57,18 +57,36 @@ void kpm_moments(const sma_op *op, int64_t M, int64_t R, uint64_t seed, double s
   // dots of one step: <T_{k+1}, T_k> and <T_k, T_k>, chunks x R partials each; the partials of
   // `batch` steps are summed by one launch
   const bool product_then_axpy = op->kind == OP_MATBLOCK || op->kind == OP_CSR_HALF;
-  const int64_t w = product_then_axpy ? R : recurrence_width(R, sizeof(double));
   // The step's own sums where a set of them is small (256 MB), in kGroup chunks to a first sum,
   // zeros after the last; else a pass over the two blocks.
   constexpr int64_t kGroup = 64;
-  int64_t chunks = (clenshaw_dot_chunks(op, w) + kGroup - 1) / kGroup * kGroup;
-  const bool fused = chunks > 0 && 2 * chunks * R <= int64_t(32) << 20;
-  if (!fused) chunks = column_dot_chunks(n, R);
-  const int64_t set = 2 * chunks * R;
-  const int64_t steps = (M + 1) / 2, fused_steps = fused ? M / 2 : 0;
-  const int64_t batch = std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
-  DevBuf<double> t0(n * w, st), t1(n * w, st), t2(n * w, st), dots(2 * steps * R, st),
-      partial(batch * set, st), sums(fused ? batch * 2 * (chunks / kGroup) * R : 0, st);
+  const int64_t steps = (M + 1) / 2;
+  int64_t w, chunks, set, batch, fused_steps;
+  bool fused;
+  DevBuf<double> t0, t1, t2, dots, partial, sums;
+  auto allocate = [&](bool spare) {  // spare: the least memory, unpadded blocks and one step's partials
+    w = product_then_axpy || spare ? R : recurrence_width(R, sizeof(double));
+    chunks = spare ? 0 : (clenshaw_dot_chunks(op, w) + kGroup - 1) / kGroup * kGroup;
+    fused = chunks > 0 && 2 * chunks * R <= int64_t(32) << 20;
+    if (!fused) chunks = column_dot_chunks(n, R);
+    set = 2 * chunks * R;
+    fused_steps = fused ? M / 2 : 0;
+    batch = spare ? 1 : std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t(4) << 20) / set));
+    t0.alloc(n * w, st);
+    t1.alloc(n * w, st);
+    t2.alloc(n * w, st);
+    dots.alloc(2 * steps * R, st);
+    partial.alloc(batch * set, st);
+    if (fused) sums.alloc(batch * 2 * (chunks / kGroup) * R, st);
+  };
+  try {
+    allocate(false);
+  } catch (const Error &e) {
+    if (e.code != SMA_ERR_NOMEM) throw;
+    cudaGetLastError();  // the failed allocation is not an error of a later launch
+    for (DevBuf<double> *x : {&t0, &t1, &t2, &dots, &partial, &sums}) x->release();
+    allocate(true);
+  }
   if (fused) SMA_CUDA(cudaMemsetAsync(partial.p, 0, (size_t)(batch * set) * sizeof(double), st));
   {
     const int64_t total = n * w;

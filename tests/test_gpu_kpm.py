@@ -95,3 +95,38 @@ def test_kpm_dots_of_every_row_layout(lib_built, kind, R):
     _, pv = S.kpm_moments(op, 21, R, smin=smin, smax=smax, seed=3, per_vector=True)
     _, pvo = O.kpm_moments(A, 21, R, 3, smin, smax, per_vector=True)
     np.testing.assert_allclose(pv, pvo, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("L,M_,R", [(84, 32, 16), (24, 279, 80)])
+def test_kpm_partials_in_many_batches(lib_built, L, M_, R):
+    """More steps than the partials of one batch, which their number does not divide: the step's own
+    sums (six steps a batch) and the pass over the blocks (132), an even and an odd number of moments."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.anderson3d(L, 16.5, 1)
+    smin, smax = O.gershgorin_bounds(A)
+    _, pv = S.kpm_moments(A, M_, R, smin=smin, smax=smax, seed=3, per_vector=True)
+    _, pvo = O.kpm_moments(A, M_, R, 3, smin, smax, per_vector=True)
+    np.testing.assert_allclose(pv, pvo, rtol=0, atol=1e-11)
+
+
+def test_kpm_with_little_memory_left(lib_built):
+    """Three unpadded blocks and the sums of one step are all that a call needs: 13 columns, which run
+    padded to 16 where there is room for them (1.04 GB of blocks, 0.85 GB unpadded).  In a process of
+    its own: the library keeps the memory that it has had."""
+    import subprocess
+
+    code = """if True:
+        import sys, numpy as np, torch
+        import sparse_matrix_algorithms_b200 as S
+        op = S.AndersonOperator(140, 16.5, 1)
+        moments = lambda: S.kpm_moments(op, 9, 13, smin=-15.0, smax=15.0, seed=3, per_vector=True)[1]
+        torch.cuda.init()
+        held = torch.empty(torch.cuda.mem_get_info()[0] - 960 * 10 ** 6, dtype=torch.uint8, device="cuda")
+        got = moments()
+        del held
+        torch.cuda.empty_cache()
+        np.testing.assert_allclose(got, moments(), rtol=0, atol=1e-13)
+    """
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, cwd=ROOT, timeout=300)
+    assert out.returncode == 0, out.stderr.decode()[-2000:]
