@@ -132,15 +132,30 @@ static void matblock_apply(const sma_op *op, cudaStream_t st, const T *X, T *AX,
   }
 }
 
-// The launches of one filter (K >= 1) on recurrence blocks of width w >= b (w = b for operators
-// without a fused step; Q is read over w columns but by the last step); returns the step count
-// and algorithmic bytes.
+// Whether a filter's first two steps form the block c_K Q themselves (record_filter).
+static bool folds(const sma_op *op, int64_t K) {
+  return op->kind != OP_MATBLOCK && op->kind != OP_CSR_HALF && K >= 2;
+}
+
+// Steps and algorithmic bytes of a filter of b columns, whatever width its blocks are padded to: Q,
+// B1, B2 read and one block written a step, without B1 and B2 in the first and B2 in the second of a
+// folded one, else a scaled block to start from, and no B2 in the first step.
 template <typename T>
-static FilterCount record_filter(const sma_op *op, cudaStream_t st,
-                                 const std::vector<double> &coeffs, double smin, double smax,
-                                 const T *Q, int64_t ldq, T *Y, int64_t ldy, int64_t b, int64_t w,
-                                 ClenshawWork<T> &work) {
+static FilterCount count_filter(const sma_op *op, int64_t K, int64_t b) {
   FilterCount fc;
+  fc.steps = K;
+  fc.bytes = (double)K * clenshaw_step_bytes(op, 0, sizeof(T)) +
+             (double)(4 * K + (folds(op, K) ? -3 : 1)) * (double)op->n * (double)b * sizeof(T);
+  return fc;
+}
+
+// The launches of one filter (K >= 1) on recurrence blocks of width w >= b (w = b for operators
+// without a fused step; Q is read over w columns but by the last step).
+template <typename T>
+static void record_filter(const sma_op *op, cudaStream_t st,
+                          const std::vector<double> &coeffs, double smin, double smax,
+                          const T *Q, int64_t ldq, T *Y, int64_t ldy, int64_t b, int64_t w,
+                          ClenshawWork<T> &work) {
   const int64_t n = op->n;
   const int64_t K = (int64_t)coeffs.size() - 1;
   const double c = 0.5 * (smin + smax);
@@ -148,8 +163,6 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   const double alpha = 2.0 * invd;
   const double beta = -2.0 * c * invd;
   const bool fused = op->kind != OP_MATBLOCK && op->kind != OP_CSR_HALF;
-  const double blk = (double)n * (double)b * sizeof(T);
-  const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
   T *B1 = work.b1.p, *B2 = work.b2.p, *TMP = work.tmp.p;
   const int64_t ld = w;
   auto rotate = [&]() {  // B1, B2, TMP = TMP, B1, B2
@@ -163,26 +176,21 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
   // (Anderson L = 64: FP32 b = 768, K = 16 10.0 -> 9.56 ms; per-column b = 496, K = 24, whose zero
   // blocks and first product are gone too, 10.57 -> 10.02 ms).  A first step
   // that is also the last could write to the Q that it gathers (Y = Q): it takes the block.
-  const bool fold = fused && K >= 2;
+  const bool fold = folds(op, K);
   int64_t ci = K - 1;
   if (fold) {
     launch_clenshaw_start<T>(op, st, w, Q, ldq, nullptr, ld, TMP, ld, coeffs[K], coeffs[ci], alpha, beta,
                              ci & 1);
-    fc.steps += 1;
-    fc.bytes += mat_bytes + 2 * blk;
     B1 = TMP;
     TMP = work.b1.p;
     --ci;
     if (ci >= 1) {
       launch_clenshaw_start<T>(op, st, w, Q, ldq, B1, ld, TMP, ld, coeffs[K], coeffs[ci], alpha, beta, ci & 1);
-      fc.steps += 1;
-      fc.bytes += mat_bytes + 3 * blk;
       rotate();
       --ci;
     }
   } else {
     launch_scale_block<T>(st, n, w, Q, ldq, B1, ld, coeffs[K]);
-    fc.bytes += 2 * blk;
   }
   bool b2_zero = !fold;
   for (; ci >= 1; --ci) {
@@ -193,8 +201,6 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
       launch_clenshaw_axpy<T>(st, n, b, Q, ldq, work.ax.p, ld, B1, b2_zero ? nullptr : B2, ld,
                               TMP, ld, coeffs[ci], alpha, beta);
     }
-    fc.steps += 1;
-    fc.bytes += mat_bytes + (b2_zero ? 3 : 4) * blk;
     rotate();
     b2_zero = false;
   }
@@ -210,9 +216,6 @@ static FilterCount record_filter(const sma_op *op, cudaStream_t st,
     launch_clenshaw_axpy<T>(st, n, b, Q, ldq, work.ax.p, ld, B1, b2_zero ? nullptr : B2, ld, Y,
                             ldy, coeffs[0], invd, -(c * invd));
   }
-  fc.steps += 1;
-  fc.bytes += mat_bytes + (b2_zero ? 3 : 4) * blk;
-  return fc;
 }
 
 // Filters of degree below this run eagerly (launch overhead is then not the question).
@@ -259,13 +262,16 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     return persistent_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, work.b1.p,
                                 work.b2.p, work.tmp.p, work.coef.p, work.barrier.p);
   }
+  fc = count_filter<T>(op, K, b);
   auto eager = [&]() {
     if (stage) {  // zero columns stay zero through the recurrence
       if (!work.q.p) work.q.alloc(n * work.bcap, st);
       launch_pad_block<T, T>(st, n, b, Q, ldq, w, work.q.p, w);
-      return record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, Y, ldy, b, w, work);
+      record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, Y, ldy, b, w, work);
+    } else {
+      record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, w, work);
     }
-    return record_filter<T>(op, st, coeffs, smin, smax, Q, ldq, Y, ldy, b, w, work);
+    return fc;
   };
   if (!fused || K < kGraphMinDegree || !op->ctx->filter_graphs) return eager();
   // repeated filter -> CUDA graph on the staging blocks
@@ -288,7 +294,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     const int64_t l0 = g_kernel_launches.load();
     SMA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
-      fc = record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, work.y.p, w, w, w, work);
+      record_filter<T>(op, st, coeffs, smin, smax, work.q.p, w, work.y.p, w, w, w, work);
     } catch (...) {
       cudaGraph_t g = nullptr;
       cudaStreamEndCapture(st, &g);
@@ -299,12 +305,6 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     SMA_CUDA(cudaGraphInstantiate(&work.exec, work.graph, 0));
     work.g_launches = g_kernel_launches.load() - l0;
     g_kernel_launches.fetch_sub(work.g_launches);  // counted when the graph runs
-  } else {
-    // step and byte counts of the recorded filter
-    const double blk = (double)n * (double)b * sizeof(T);
-    const double mat_bytes = clenshaw_step_bytes(op, 0, sizeof(T));
-    fc.steps = K;
-    fc.bytes = (mat_bytes + 2 * blk) + (mat_bytes + 3 * blk) + (double)(K - 2) * (mat_bytes + 4 * blk);
   }
   SMA_CUDA(cudaGraphLaunch(work.exec, st));
   g_kernel_launches.fetch_add(work.g_launches);

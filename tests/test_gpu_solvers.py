@@ -432,3 +432,22 @@ def test_polfed_blocks_around_the_one_kernel_factorization(lib_built, s):
                            emax=hi, tol=1e-10, window_type="delta", mmax=max(4, 160 // s), seed=1)
     np.testing.assert_allclose(np.sort(lam), exact[400:420], rtol=0, atol=1e-9)
     assert np.abs(X.T @ X - np.eye(X.shape[1])).max() <= 1e-10
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_filter_bytes_count_the_columns_asked_for(lib_built, monkeypatch, precision):
+    """37 columns run on blocks padded to 40: the algorithmic bytes are those of 37, the same in the
+    call that records the CUDA graph, in its replays and without a graph."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.anderson3d(10, 16.5, 3)
+    smin, smax = O.gershgorin_bounds(A)
+    b, K, its, size = 37, 40, 4, 8 if precision == "fp64" else 4
+    step = A.nnz * (size + 4) + 4 * (A.shape[0] + 1)
+    for graphs in ("1", "0"):
+        monkeypatch.setenv("SMA_FILTER_GRAPHS", graphs)
+        st = {}
+        S.chebyshev_poly_real_symm_sparse(S.SparseOperator(A, S.Context(0)), -0.5, 0.5, smin=smin, smax=smax, m0=b,
+                                          degree=K, maxiter=its, precision=precision, stats=st)
+        assert st["graph_replays"] == (its - 1 if graphs == "1" else 0)
+        assert st["filter_bytes"] == its * (K * step + (4 * K - 3) * A.shape[0] * b * size)
