@@ -287,8 +287,14 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
   }
   work.g_calls += 1;
   if (work.g_calls == 1) return eager();  // a graph pays from its second use
-  if (!work.q.p) work.q.alloc(n * work.bcap, st);
-  if (!work.y.p) work.y.alloc(n * work.bcap, st);
+  try {
+    if (!work.q.p) work.q.alloc(n * work.bcap, st);
+    if (!work.y.p) work.y.alloc(n * work.bcap, st);
+  } catch (const Error &e) {  // no memory for the staging blocks: step by step
+    if (e.code != SMA_ERR_NOMEM) throw;
+    cudaGetLastError();  // the failed allocation is not an error of a later launch
+    return eager();
+  }
   launch_pad_block<T, T>(st, n, b, Q, ldq, w, work.q.p, w);
   if (!work.exec) {
     const int64_t l0 = g_kernel_launches.load();

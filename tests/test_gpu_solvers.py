@@ -451,3 +451,33 @@ def test_filter_bytes_count_the_columns_asked_for(lib_built, monkeypatch, precis
                                           degree=K, maxiter=its, precision=precision, stats=st)
         assert st["graph_replays"] == (its - 1 if graphs == "1" else 0)
         assert st["filter_bytes"] == its * (K * step + (4 * K - 3) * A.shape[0] * b * size)
+
+
+def test_repeated_filter_with_little_memory_left(lib_built):
+    """The staging blocks of a repeated filter's graph are a convenience: a solve of 13 columns, padded
+    to 16, of 2.7 million rows runs with 2.45 GB left, step by step (five padded blocks and the solver's
+    own take 2.6 GB, five unpadded 2.3).  In a process of its own: the library keeps the memory that it
+    has had."""
+    import os
+    import subprocess
+    import sys
+
+    code = """if True:
+        import torch
+        import sparse_matrix_algorithms_b200 as S
+        op = S.AndersonOperator(140, 16.5, 1)
+        def replays():
+            st = {}
+            S.chebyshev_poly_real_symm_sparse(S.MatrixFreeRealSymOp(op.n, None, op), -1e-3, 1e-3, smin=-15.0, smax=15.0,
+                                              m0=13, degree=40, maxiter=3, two_hit=False, stats=st)
+            return st["graph_replays"]
+        torch.cuda.init()
+        held = torch.empty(torch.cuda.mem_get_info()[0] - 2450 * 10 ** 6, dtype=torch.uint8, device="cuda")
+        assert replays() == 0
+        del held
+        torch.cuda.empty_cache()
+        assert replays() == 2
+    """
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, cwd=root, timeout=300)
+    assert out.returncode == 0, out.stderr.decode()[-2000:]
