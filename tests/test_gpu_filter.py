@@ -472,7 +472,7 @@ def test_banded_launches_wait_for_the_one_before(lib_built, precision, n, b):
 
     lib, K = L.load(), 400
     c = np.ascontiguousarray(O.build_coeffs(K, 0.0, 4.0, 1.7, 1.6, 1.8, "step", True))
-    Q = torch.as_tensor(M.splitmix_normal(3, n, b), device="cuda")
+    Q = _device(M.splitmix_normal(3, n, b))
     Q = Q.to(torch.float64 if precision == "fp64" else torch.float32)
 
     def run(op, q, y):
@@ -489,3 +489,63 @@ def test_banded_launches_wait_for_the_one_before(lib_built, precision, n, b):
     for _ in range(5):
         for op in ops:
             assert torch.equal(run(op, Q, torch.empty_like(Q)), ref)
+
+
+@pytest.mark.parametrize("b", [32, 64])
+@pytest.mark.parametrize("threads", [9472, 40000, 303104, 909312])
+def test_step_rule_for_short_rows_that_are_no_band(lib_built, b, threads):
+    """The rule's line for rows of at most four entries, on a ring, which the banded filter does not
+    take: one launch a step, one row below and exactly at each line, against the oracle."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    lib, K = L.load(), 5
+    at = threads * (2 if threads == 9472 else 4) // b
+    for n in (at - 1, at):
+        far = sp.coo_matrix((np.ones(1), ([0], [n - 1])), shape=(n, n))
+        A = M._canonical((M.lap1d(n) - far - far.T).tocsr())
+        op = S.SparseOperator(A)
+        smin, smax = _bounds(A)
+        Qh = M.splitmix_normal(b, n, b)
+        Q = _device(Qh)
+        Y = torch.empty_like(Q)
+        c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+        torch.cuda.synchronize()
+        before = lib.sma_kernel_launch_count()
+        L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, Q.data_ptr(), b, Y.data_ptr(),
+                                             b, b, 0))
+        assert lib.sma_kernel_launch_count() - before == K
+        ref = O.apply_poly_block(A, Qh, c, smin, smax)
+        assert np.abs(Y.cpu().numpy() - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Qh).max())
+
+
+@pytest.mark.parametrize("n", [2, 3, 130, 1001])
+@pytest.mark.parametrize("b", [1, 3, 8, 31, 200])
+def test_lap1d_stencil_on_the_step_kernel(lib_built, n, b):
+    """The 1D Laplacian's rows as the step kernel builds them, which in-place calls take (one launch a
+    step): against the oracle, and bit for bit the stored matrix's and, for n >= 3, the banded filter's."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    lib, K = L.load(), 20
+    A = M.lap1d(n)
+    c = np.ascontiguousarray(O.build_coeffs(K, 0.0, 4.0, 1.7, 1.3, 2.1, "step", True))
+    Qh = M.splitmix_normal(b, n, b)
+    ref = O.apply_poly_block(A, Qh, c, 0.0, 4.0)
+    out = []
+    for op in (S.Lap1dOperator(n), S.SparseOperator(A)):
+        for in_place in (True, False):
+            Q = _device(Qh)
+            Y = Q if in_place else torch.empty_like(Q)
+            torch.cuda.synchronize()
+            before = lib.sma_kernel_launch_count()
+            L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, 0.0, 4.0, Q.data_ptr(), b,
+                                                 Y.data_ptr(), b, b, 0))
+            launches = lib.sma_kernel_launch_count() - before
+            assert launches >= K if in_place or n < 3 else launches < K
+            out.append(Y.cpu().numpy())
+    assert np.abs(out[0] - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Qh).max())
+    for got in out[1:]:
+        np.testing.assert_array_equal(got, out[0])

@@ -123,7 +123,7 @@ def test_noalloc_filter_makes_no_trials_of_the_autotuner(lib_built, monkeypatch,
     op = S.SparseOperator(A, S.Context(0))
     smin, smax = O.gershgorin_bounds(A)
     c = np.ascontiguousarray(O.build_coeffs(200, smin, smax, 0.1, -0.4, 0.3, "step", True))
-    Q = torch.as_tensor(M.splitmix_normal(5, n, b), device="cuda")
+    Q = torch.as_tensor(M.splitmix_normal(5, n, b), device="cuda").contiguous()
     Y = torch.empty_like(Q)
     first = _run("sma_apply_poly_block_noalloc", op, c, smin, smax, Q, b, Y, b, b)
     free = torch.cuda.mem_get_info()[0]
