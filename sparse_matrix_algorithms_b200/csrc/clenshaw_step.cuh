@@ -31,7 +31,8 @@
 // A model's CTA first writes the columns of its rows to shared memory, one thread per entry (the
 // work of a whole row in each of its threads -- divisions, a sorting network, 64-80 registers --
 // made the Anderson step 2.4 times slower than the CSR one: 96 us at n = 110592, b = 64 FP64);
-// from there on it is a CSR matrix with one value on the diagonal and one off it.
+// from there on it is a CSR matrix with one value on the diagonal and one off it.  XXZ rows of few
+// threads are walked bit by bit instead, by each of those.
 //
 // Every configuration accumulates with FMA in ascending column order -- the order of the
 // reference's CSC product on a symmetric matrix -- so all write bit-identical results
@@ -268,6 +269,58 @@ __device__ __forceinline__ void model_rows(const Step<T> &a, uint32_t row0, int 
   __syncthreads();
 }
 
+// An XXZ row walked bit by bit by each thread that takes columns of it, for rows of few threads: in
+// shared memory the L + 1 places of such a row are filled by about as many threads as then read them.
+struct Walk {
+  unsigned state, todo;  // bit i of todo: bond (i, i + 1) still to come, the periodic one is bit L - 1
+  uint32_t periodic;     // its column
+};
+
+__device__ __forceinline__ Walk xxz_walk(const sma_stencil &m, uint32_t row) {
+  const unsigned s = __ldg(m.states + row);
+  const Entry p = xxz_entry(row, m, m.L);
+  const unsigned bonds = (s ^ (s >> 1)) & ((1u << (m.L - 1)) - 1u);
+  return {s, bonds | (p.place < 0 ? 0u : 1u << (m.L - 1)), (uint32_t)p.col};
+}
+
+// acc += the walked row: the diagonal and the bonds in ascending order (the places of xxz_entry), U at
+// a time, the last of them predicated like ragged rows.
+template <typename T, int V, int U, bool W, typename F>
+__device__ __forceinline__ void walk_product(const sma_stencil &m, Walk w, uint32_t row, T diag, T off,
+                                             const T *B1c, uint64_t ldb, T (&acc)[V], F f) {
+  const unsigned last = 1u << (m.L - 1);
+  bool first = true;
+  do {
+    T x[U][V], v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      uint32_t col = row;
+      bool there = true;
+      v[u] = off;
+      if (u == 0 && first) {
+        v[u] = diag;
+      } else {
+        there = w.todo != 0;
+        const unsigned bit = w.todo & -w.todo;
+        w.todo ^= bit;
+        if (bit == last) {
+          col = w.periodic;
+        } else if (there) {
+          const int d = __ldg(m.binom + (__ffs(bit) - 1) * 17 + __popc(w.state & (bit - 1u)));
+          col = w.state & bit ? row + d : row - d;
+        }
+        if (!there) v[u] = T(0);
+      }
+      ldv_if<T, V>(there, at(B1c, row_bytes<W>(col, ldb)), x[u]);
+    }
+    first = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = fma(v[u], f(x[u][i], i), acc[i]);
+  } while (w.todo);
+}
+
 // The coefficients of the thread's V columns: c in all, or from cseg.
 template <typename T, int V, bool PC>
 __device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cseg, uint32_t c0,
@@ -292,15 +345,18 @@ __device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cse
 // it holds both factors.
 enum Form { INNER, FIRST, SECOND, DOTS };
 
+// Where the rows' entries come from: a stored matrix, a model's columns in shared memory, or walked.
+enum Rows { STORED, SHARED, WALKED };
+
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
 // FLAT: a CTA does not take whole rows, its threads go on in the next row where the CTA before ended.
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL,
           bool RAGGED, Form P, bool FLAT>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  static_assert(!FLAT || !(MODEL || P == DOTS), "these need whole rows");
+  static_assert(!FLAT || !(MODEL != STORED || P == DOTS), "these need whole rows");
   uint32_t row0 = bx * a.rows, i = threadIdx.x;
   if constexpr (FLAT) {
     row0 = bx * kThreads / a.lanes;
@@ -312,21 +368,24 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   const bool in = (FLAT || r < a.rows) && row < a.n && c0 < a.b;
   int start = 0, end = 0;
   if (in) {
-    if constexpr (!MODEL) {
+    if constexpr (MODEL == STORED) {
       start = __ldg(a.rowptr + row);
       end = __ldg(a.rowptr + row + 1);
     }
     if constexpr (HQ) prefetch_l2(at(a.Q + c0, row * a.ldq));
   }
   int *cnt = model_smem + a.rows * a.entries, *dpos = cnt + a.rows;
-  if constexpr (MODEL) model_rows(a, bx * a.rows, model_smem, cnt, dpos);
+  if constexpr (MODEL == SHARED) model_rows(a, bx * a.rows, model_smem, cnt, dpos);
+  Walk walk{};
+  if constexpr (MODEL == WALKED)
+    if (in) walk = xxz_walk(a.model, row);
   pdl_wait_then_trigger();
   if constexpr (P != DOTS) {
     if (!in) return;
   }
   T dot[P == DOTS ? 2 * V : 1] = {};
   if (P != DOTS || in) {
-    if constexpr (MODEL) row = after_wait(row);  // B1's places come from shared memory
+    if constexpr (MODEL == SHARED) row = after_wait(row);  // B1's places come from shared memory
     else c0 = after_wait(c0);
     const uint64_t own = row * a.ldb;
     if constexpr (HB && P != SECOND) prefetch_l2(at(a.B2 + c0, own));
@@ -342,7 +401,13 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
       if constexpr (P == FIRST) product(row, j, end, Scaled<T, V>{top});
       else product(row, j, end, Unscaled{});
     };
-    if constexpr (MODEL) {
+    if constexpr (MODEL == WALKED) {
+      const T diag = (T)__ldg(a.model.diag + row), off = (T)a.model.hop;
+      if constexpr (P == FIRST)
+        walk_product<T, V, U, W>(a.model, walk, row, diag, off, a.B1 + c0, a.ldb, acc, Scaled<T, V>{top});
+      else
+        walk_product<T, V, U, W>(a.model, walk, row, diag, off, a.B1 + c0, a.ldb, acc, Unscaled{});
+    } else if constexpr (MODEL == SHARED) {
       const T diag = a.kind == OP_LAP1D ? T(2) : (T)__ldg(a.model.diag + row);
       gather(ModelRow<T>{model_smem + r * a.entries, dpos[r], diag, (T)a.model.hop}, 0, cnt[r]);
     } else {
@@ -423,13 +488,13 @@ namespace sma {
 namespace rows {
 
 // ------------------------------------------------------------------ launch
-template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL,
+template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL,
           bool RAGGED, Form P, bool FLAT = false>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
-  if (MODEL) cfg.dynamicSmemBytes = (a.rows * (a.entries + 2) + kRowPad) * sizeof(int);  // 18 KB at most
+  if (MODEL == SHARED) cfg.dynamicSmemBytes = (a.rows * (a.entries + 2) + kRowPad) * sizeof(int);  // 18 KB at most
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -465,13 +530,23 @@ inline uint32_t panel_lanes(uint32_t vecs) {
   return best;
 }
 
+// XXZ rows are walked where few threads share one: at most 6, or 16 in a stream of a wave and more
+// (us a step, places in shared memory and walked: L = 16, b = 1 FP64 17.8 and 4.4, b = 6 6.0 and 4.6;
+// L = 20, b = 8 45.5 and 16.8, b = 32 67.9 and 57.2; L = 22, b = 64 530 and 517; on the other side
+// L = 14, b = 32 3.3 and 4.7; L = 16, b = 32 6.2 and 6.9; L = 20, b = 128 224 and 238).
+inline bool walked(const sma_op *op, uint32_t lanes, int64_t threads) {
+  return op->kind == OP_XXZ && (lanes <= 6 || (lanes <= 16 && threads >= 8LL * kThreads * op->ctx->num_sms));
+}
+
 // Where not 0 or negative, `gathers` and `flat` take the place of the rules for them.
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, bool MODEL, Form P>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL, Form P>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0, int flat_wanted = -1) {
   const uint32_t vecs = a.b / V;
   a.lanes = panel_lanes(vecs);
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
+  if constexpr (MODEL == SHARED)
+    if (walked(op, a.lanes, (int64_t)a.n * vecs)) return launch_width<T, V, HQ, HS, HB, PC, W, WALKED, P>(op, st, a);
   // Waves of 8-CTA residency decide what a step's time is.  Six and more: a stream, which wants
   // every warp it can get.  Below, more and more a latency, which wants more gathers in flight at
   // less occupancy -- unless a row has no more than four.  Us a step, step after step:
@@ -490,7 +565,7 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0,
   // warps are idle or a few threads of long rows (us a step, whole rows and flat, Anderson L = 48:
   // 13 lanes 34.1 and 32.6, 22 55.8 and 52.0, 43 117 and 107, 50 143 and 128; 48 120 and 121, 60
   // 152 and 155).
-  constexpr bool kFlat = !(MODEL || P == DOTS || P == FIRST);
+  constexpr bool kFlat = !(MODEL != STORED || P == DOTS || P == FIRST);
   const uint32_t used = a.rows * a.lanes;
   const bool flat = kFlat && gathers != 8 && used < kThreads && (uint64_t)a.n * a.lanes < (uint64_t)1 << 32 &&
                     (flat_wanted < 0 ? used % 32 != 0 && (a.lanes <= 40 || kThreads - used >= 16) : flat_wanted > 0);
@@ -509,20 +584,27 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0,
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
-    if constexpr (P == FIRST) {  // the coefficients take registers too, and it is one step
+    // A walked row holds its state beside the gathers: two at a time of 16-byte FP64 and of 32-byte
+    // vectors, whose four spill (L = 22, b = 8 FP64 63.5 us against 87), four of the others.
+    if constexpr (MODEL == WALKED) {
+      constexpr bool kTwo = V * sizeof(T) == 32 || (sizeof(T) == 8 && V == 2);
+      constexpr int kCtas = !kTwo || P == FIRST || P == DOTS ? 8 : 12;
+      launch<T, V, kTwo ? 2 : 4, kCtas, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+    } else if constexpr (P == FIRST) {  // the coefficients take registers too, and it is one step
       if (uneven) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
       else launch<T, V, 4, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
     } else if (gathers == 8) {
       if (uneven) launch<T, V, 8, 6, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
       else launch<T, V, 8, 8, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
-    } else if (flat) {
-      if (!uneven) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P, kFlat>(op, st, a, grid);
-      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
-      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
-    } else {
-      if (!uneven) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
-      else if (gathers == 6) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+    } else if (gathers == 6 && uneven) {
+      if (flat) launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
+      else launch<T, V, 6, 8, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+    } else if (uneven) {
+      if (flat) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P, kFlat>(op, st, a, grid);
       else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, true, P>(op, st, a, grid);
+    } else {
+      if (flat) launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P, kFlat>(op, st, a, grid);
+      else launch<T, V, 4, 12, HQ, HS, HB, PC, W, MODEL, false, P>(op, st, a, grid);
     }
   }
 }
@@ -644,11 +726,11 @@ inline int vector_width(const sma_op *op, int64_t b, int widest) {
   return 1;
 }
 
-template <typename T, bool HQ, bool HS, bool HB, bool PC, bool MODEL, Form P = INNER>
+template <typename T, bool HQ, bool HS, bool HB, bool PC, int MODEL, Form P = INNER>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
   require(b < (int64_t)1 << 31, SMA_ERR_ARG, "block too wide");
-  if constexpr (MODEL) {
+  if constexpr (MODEL != STORED) {
     a.model = op->stencil;
     a.kind = op->kind;
     if (op->kind == OP_LAP1D) a.model.hop = -1.0;
@@ -670,7 +752,7 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   };
   if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL, P>(op, st, a);
   const int widest = widest_vector<T>(fits), v = vector_width(op, b, widest);
-  if constexpr (!MODEL && P == INNER)
+  if constexpr (MODEL == STORED && P == INNER)
     if (tuned_step<T, HQ, HS, HB, PC>(op, st, a, widest, v)) return;
   if constexpr (sizeof(T) == 4)
     if (v == 8) return launch_width<T, 8, HQ, HS, HB, PC, false, MODEL, P>(op, st, a);
@@ -699,7 +781,7 @@ rows::Step<T> clenshaw_arguments(const T *Q, int64_t ldq, const T *B1, const T *
   return a;
 }
 
-template <typename T, bool MODEL>
+template <typename T, int MODEL>
 void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq,
                    const T *B1, const T *B2, int64_t ldb, T *out, int64_t ldo, double ck,
                    double alpha, double beta, bool has_self, bool rev, bool tune = false) {
@@ -712,7 +794,7 @@ void clenshaw_step(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int
 }
 
 // The first step of a recurrence (B1 null: it is c_top Q) and the second (B2 is c_top Q).
-template <typename T, bool MODEL>
+template <typename T, int MODEL>
 void clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
                     int64_t ldb, T *out, int64_t ldo, double top, double ck, double alpha, double beta,
                     bool rev) {
@@ -726,7 +808,7 @@ void clenshaw_start(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, in
 
 // The segmented step: column c takes the coefficient cseg[colseg[c]], colseg nondecreasing, or
 // cseg[c] when colseg is null; Q, B1 and B2 are all read.
-template <typename T, bool MODEL>
+template <typename T, int MODEL>
 void clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
                        const T *B2, int64_t ldb, T *out, int64_t ldo, const T *cseg, const int *colseg,
                        double alpha, double beta, bool rev) {
@@ -737,7 +819,7 @@ void clenshaw_step_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q,
 }
 
 // Its first step (B1 null) and second, topseg the highest coefficients.
-template <typename T, bool MODEL>
+template <typename T, int MODEL>
 void clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q, int64_t ldq, const T *B1,
                         int64_t ldb, T *out, int64_t ldo, const T *topseg, const T *cseg, const int *colseg,
                         double alpha, double beta, bool rev) {
@@ -751,7 +833,7 @@ void clenshaw_start_seg(const sma_op *op, cudaStream_t st, int64_t b, const T *Q
 }
 
 // out = ck Q + alpha A B1 + beta B1, with the sums of a DOTS step (n x b blocks, ld = b).
-template <bool MODEL>
+template <int MODEL>
 void clenshaw_dots(const sma_op *op, cudaStream_t st, int64_t b, const double *Q, const double *B1,
                    double *out, double ck, double alpha, double beta, bool rev, int64_t cols,
                    double *dots, int64_t plane) {

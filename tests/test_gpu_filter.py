@@ -549,3 +549,36 @@ def test_lap1d_stencil_on_the_step_kernel(lib_built, n, b):
     assert np.abs(out[0] - ref).max() <= 1e-12 * max(np.abs(ref).max(), np.abs(Qh).max())
     for got in out[1:]:
         np.testing.assert_array_equal(got, out[0])
+
+
+@pytest.mark.parametrize("precision,rtol", [("fp64", 1e-12), ("fp32", 2e-4)])
+@pytest.mark.parametrize("L_", [4, 10, 14, 16])
+def test_xxz_rows_walked_and_in_shared_memory(lib_built, L_, precision, rtol):
+    """XXZ rows of few threads are walked by each of them, the others' entries go through shared
+    memory: every column has the same bits at every width, on both sides of the rule's lines (6 and 16
+    threads a row, a wave of threads), by the block and the per-column entry; against the oracle."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    op, A = S.XXZOperator(L_, 5.0, 1), M.xxz_sz0(L_, 5.0, 1)
+    n, K, lib = A.shape[0], 5, L.load()
+    smin, smax = _bounds(A)
+    c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    Qh = M.splitmix_normal(L_, n, 128)
+    ref = O.apply_poly_block(A, Qh, c, smin, smax)
+    full = None
+    for b in (128, 64, 52, 32, 24, 16, 8, 6, 5, 3, 2, 1):
+        Q = _device(Qh[:, :b]).to(dt)
+        Y, P = torch.empty_like(Q), torch.empty_like(Q)
+        table = np.ascontiguousarray(np.repeat(c[:, None], b, axis=1))
+        torch.cuda.synchronize()
+        L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, Q.data_ptr(), b, Y.data_ptr(), b,
+                                             b, L.PRECISIONS[precision]))
+        L.check(lib.sma_apply_poly_block_percol_dev(op.handle, table.ctypes.data, K, smin, smax, Q.data_ptr(),
+                                                    P.data_ptr(), b, L.PRECISIONS[precision]))
+        if full is None:
+            full = Y
+            assert np.abs(Y.double().cpu().numpy() - ref).max() <= rtol * max(np.abs(ref).max(), np.abs(Qh).max())
+        assert torch.equal(Y, full[:, :b]) and torch.equal(P, Y), b
