@@ -120,17 +120,52 @@ struct Scaled {
   __device__ __forceinline__ T operator()(T x, int i) const { return mul_rn(c[i], x); }
 };
 
+// The V columns of a thread, from the one that its pointers are at: next to each other, in one
+// access; or (STRIDED) a row's threads apart, V accesses of one element, those past the row left out.
+template <typename T, int V, bool STRIDED>
+struct Columns {
+  uint32_t step;  // STRIDED: between two columns
+  int count;      // STRIDED: those that there are
+  static constexpr bool kStrided = STRIDED;
+  template <bool KEEP = true>
+  __device__ __forceinline__ void load(const T *p, T (&f)[V]) const {
+    if constexpr (STRIDED) load_if(true, p, f);
+    else ldv<T, V, KEEP>(p, f);
+  }
+  __device__ __forceinline__ void load_if(bool ok, const T *p, T (&f)[V]) const {
+    if constexpr (STRIDED) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        T x[1];
+        ldv_if<T, 1>(ok && i < count, p + (uint64_t)i * step, x);
+        f[i] = x[0];
+      }
+    } else {
+      ldv_if<T, V>(ok, p, f);
+    }
+  }
+  __device__ __forceinline__ void store(T *p, const T (&f)[V]) const {
+    if constexpr (STRIDED) {
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        if (i < count) p[(uint64_t)i * step] = f[i];
+    } else {
+      stv<T, V>(p, f);
+    }
+  }
+};
+
 // R consecutive entries from j: all R gathers are issued before the first FMA; FMAs in
 // ascending entry order.
-template <typename T, int V, int R, bool W, typename Row, typename F>
+template <typename T, int V, int R, bool W, typename Row, typename C, typename F>
 __device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint64_t ldb, T (&acc)[V],
-                                      F f) {
+                                      const C &cols, F f) {
   int c[R];
   T x[R][V], v[R];
 #pragma unroll
   for (int u = 0; u < R; ++u) c[u] = row.col(j + u);
 #pragma unroll
-  for (int u = 0; u < R; ++u) ldv<T, V>(at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
+  for (int u = 0; u < R; ++u) cols.load(at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
 #pragma unroll
   for (int u = 0; u < R; ++u) v[u] = row.val(j + u);
 #pragma unroll
@@ -141,18 +176,18 @@ __device__ __forceinline__ void chunk(const Row &row, int j, const T *B1c, uint6
 
 // acc += the row's entries [j, end): chunks of U, then the r < U remaining entries as ONE chunk
 // of exactly r (a switch over r).
-template <typename T, int V, int U, bool W, typename Row, typename F>
+template <typename T, int V, int U, bool W, typename Row, typename C, typename F>
 __device__ __forceinline__ void row_product(const Row &row, int j, int end, const T *B1c,
-                                            uint64_t ldb, T (&acc)[V], F f) {
-  for (; j + U <= end; j += U) chunk<T, V, U, W>(row, j, B1c, ldb, acc, f);
+                                            uint64_t ldb, T (&acc)[V], const C &cols, F f) {
+  for (; j + U <= end; j += U) chunk<T, V, U, W>(row, j, B1c, ldb, acc, cols, f);
   switch (end - j) {
-    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(row, j, B1c, ldb, acc, f); break;
-    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(row, j, B1c, ldb, acc, f); break;
-    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(row, j, B1c, ldb, acc, f); break;
-    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(row, j, B1c, ldb, acc, f); break;
-    case 3: chunk<T, V, 3, W>(row, j, B1c, ldb, acc, f); break;
-    case 2: chunk<T, V, 2, W>(row, j, B1c, ldb, acc, f); break;
-    case 1: chunk<T, V, 1, W>(row, j, B1c, ldb, acc, f); break;
+    case 7: if constexpr (U > 7) chunk<T, V, 7, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 6: if constexpr (U > 6) chunk<T, V, 6, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 5: if constexpr (U > 5) chunk<T, V, 5, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 4: if constexpr (U > 4) chunk<T, V, 4, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 3: chunk<T, V, 3, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 2: chunk<T, V, 2, W>(row, j, B1c, ldb, acc, cols, f); break;
+    case 1: chunk<T, V, 1, W>(row, j, B1c, ldb, acc, cols, f); break;
     default: break;
   }
 }
@@ -162,9 +197,9 @@ __device__ __forceinline__ void row_product(const Row &row, int j, int end, cons
 // one code path; with the exact chunks above each remainder is a path of its own, and the warp
 // waits for the gathers of all of them in turn (XXZ L = 16, b = 32: 5.3 -> 4.0 us a step FP64,
 // 4.1 -> 3.1 FP32; L = 18 13.2 -> 12.3).  An absent entry adds 0 * 0.
-template <typename T, int V, int U, bool W, typename Row, typename F>
+template <typename T, int V, int U, bool W, typename Row, typename C, typename F>
 __device__ __forceinline__ void ragged_product(const Row &row, int j, int end, const T *B1c,
-                                               uint64_t ldb, T (&acc)[V], F f) {
+                                               uint64_t ldb, T (&acc)[V], const C &cols, F f) {
   for (; j < end; j += U) {
     int c[U];
     T x[U][V], v[U];
@@ -172,7 +207,7 @@ __device__ __forceinline__ void ragged_product(const Row &row, int j, int end, c
     for (int u = 0; u < U; ++u) c[u] = row.col(j + u);
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      ldv_if<T, V>(j + u < end, at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
+      cols.load_if(j + u < end, at(B1c, row_bytes<W>((uint32_t)c[u], ldb)), x[u]);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       v[u] = row.val(j + u);
@@ -322,20 +357,22 @@ __device__ __forceinline__ void walk_product(const sma_stencil &m, Walk w, uint3
 }
 
 // The coefficients of the thread's V columns: c in all, or from cseg.
-template <typename T, int V, bool PC>
-__device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cseg, uint32_t c0,
+template <typename T, int V, bool PC, typename C>
+__device__ __forceinline__ void coefficients(const Step<T> &a, T c, const T *cseg, uint32_t c0, const C &cols,
                                              T (&ck)[V]) {
   if constexpr (!PC) {
 #pragma unroll
     for (int i = 0; i < V; ++i) ck[i] = c;
   } else if (a.colseg == nullptr) {  // one polynomial per column: its coefficients side by side
-    ldv<T, V>(cseg + c0, ck);
+    cols.load(cseg + c0, ck);
   } else {  // segments are runs of columns: equal ends, one coefficient
-    const int s0 = __ldg(a.colseg + c0), s1 = __ldg(a.colseg + c0 + V - 1);
+    const uint32_t step = C::kStrided ? cols.step : 1;
+    const int count = C::kStrided ? cols.count : V;
+    const int s0 = __ldg(a.colseg + c0), s1 = __ldg(a.colseg + c0 + (count - 1) * step);
     ck[0] = __ldg(cseg + s0);
 #pragma unroll
     for (int i = 1; i < V; ++i)
-      ck[i] = s0 == s1 ? ck[0] : __ldg(cseg + __ldg(a.colseg + c0 + i));
+      ck[i] = s0 == s1 || i >= count ? ck[0] : __ldg(cseg + __ldg(a.colseg + c0 + i * step));
   }
 }
 
@@ -351,12 +388,13 @@ enum Rows { STORED, SHARED, WALKED };
 // HQ, HS, HB: whether the terms with Q, B1's own row and B2 are there.  CTAS: CTAs an SM holds.
 // FLAT: a CTA does not take whole rows, its threads go on in the next row where the CTA before ended.
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL,
-          bool RAGGED, Form P, bool FLAT>
+          bool RAGGED, Form P, bool FLAT, bool STRIDED>
 __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   extern __shared__ int model_smem[];  // a.rows x a.entries columns, then counts and places
   const uint32_t bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const uint32_t by = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   static_assert(!FLAT || !(MODEL != STORED || P == DOTS), "these need whole rows");
+  static_assert(!STRIDED || !(MODEL == WALKED || P == DOTS), "not with these");
   uint32_t row0 = bx * a.rows, i = threadIdx.x;
   if constexpr (FLAT) {
     row0 = bx * kThreads / a.lanes;
@@ -365,14 +403,17 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
   const uint32_t r = i * a.divlanes >> 16;
   uint32_t row = row0 + r;
   uint32_t c0 = (by * a.lanes + i - r * a.lanes) * V;
+  if constexpr (STRIDED) c0 = by * a.lanes * V + i - r * a.lanes;
   const bool in = (FLAT || r < a.rows) && row < a.n && c0 < a.b;
+  Columns<T, V, STRIDED> cols{};
+  if constexpr (STRIDED) cols = {a.lanes, in ? (int)min((uint32_t)V, (a.b - c0 + a.lanes - 1) / a.lanes) : 0};
   int start = 0, end = 0;
   if (in) {
     if constexpr (MODEL == STORED) {
       start = __ldg(a.rowptr + row);
       end = __ldg(a.rowptr + row + 1);
     }
-    if constexpr (HQ) prefetch_l2(at(a.Q + c0, row * a.ldq));
+    if constexpr (HQ && !STRIDED) prefetch_l2(at(a.Q + c0, row * a.ldq));
   }
   int *cnt = model_smem + a.rows * a.entries, *dpos = cnt + a.rows;
   if constexpr (MODEL == SHARED) model_rows(a, bx * a.rows, model_smem, cnt, dpos);
@@ -388,14 +429,14 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
     if constexpr (MODEL == SHARED) row = after_wait(row);  // B1's places come from shared memory
     else c0 = after_wait(c0);
     const uint64_t own = row * a.ldb;
-    if constexpr (HB && P != SECOND) prefetch_l2(at(a.B2 + c0, own));
+    if constexpr (HB && P != SECOND && !STRIDED) prefetch_l2(at(a.B2 + c0, own));
     T acc[V], top[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) acc[i] = T(0);
-    if constexpr (P == FIRST) coefficients<T, V, PC>(a, a.top, a.topseg, c0, top);
+    if constexpr (P == FIRST) coefficients<T, V, PC>(a, a.top, a.topseg, c0, cols, top);
     auto product = [&](const auto &row, int j, int end, auto f) {
-      if constexpr (RAGGED) ragged_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, f);
-      else row_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, f);
+      if constexpr (RAGGED) ragged_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, cols, f);
+      else row_product<T, V, U, W>(row, j, end, a.B1 + c0, a.ldb, acc, cols, f);
     };
     auto gather = [&](const auto &row, int j, int end) {
       if constexpr (P == FIRST) product(row, j, end, Scaled<T, V>{top});
@@ -414,11 +455,11 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
       gather(CsrRow<T>{a.colind, a.val}, start, end);
     }
     T q[V], s[V], t[V], ck[V], o[V];
-    if constexpr (HQ) ldv<T, V, false>(at(a.Q + c0, row * a.ldq), q);
-    if constexpr (HB && P != SECOND) ldv<T, V, false>(at(a.B2 + c0, own), t);
-    if constexpr (HS && P != FIRST) ldv<T, V>(at(a.B1 + c0, own), s);
-    if constexpr (HQ) coefficients<T, V, PC>(a, a.ck, a.cseg, c0, ck);
-    if constexpr (P == SECOND) coefficients<T, V, PC>(a, a.top, a.topseg, c0, top);
+    if constexpr (HQ) cols.template load<false>(at(a.Q + c0, row * a.ldq), q);
+    if constexpr (HB && P != SECOND) cols.template load<false>(at(a.B2 + c0, own), t);
+    if constexpr (HS && P != FIRST) cols.load(at(a.B1 + c0, own), s);
+    if constexpr (HQ) coefficients<T, V, PC>(a, a.ck, a.cseg, c0, cols, ck);
+    if constexpr (P == SECOND) coefficients<T, V, PC>(a, a.top, a.topseg, c0, cols, top);
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       if constexpr (P == FIRST) s[i] = mul_rn(top[i], q[i]);
@@ -427,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) step_kernel(const Step<T> a) {
 #pragma unroll
     for (int i = 0; i < V; ++i)
       o[i] = clenshaw_combine<HQ, HS, HB>(acc[i], q[i], s[i], t[i], ck[i], a.alpha, a.beta);
-    stv<T, V>(const_cast<T *>(at(a.out + c0, row * a.ldo)), o);
+    cols.store(const_cast<T *>(at(a.out + c0, row * a.ldo)), o);
     if constexpr (P == DOTS) {
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -489,7 +530,7 @@ namespace rows {
 
 // ------------------------------------------------------------------ launch
 template <typename T, int V, int U, int CTAS, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL,
-          bool RAGGED, Form P, bool FLAT = false>
+          bool RAGGED, Form P, bool FLAT = false, bool STRIDED = false>
 void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -503,7 +544,7 @@ void launch(const sma_op *op, cudaStream_t st, const Step<T> &a, dim3 grid) {
   // the first step gathers the caller's Q, which the grid before may have read and written in
   // place: it starts after that grid has ended, with nothing of it in L1
   cfg.numAttrs = op->ctx->pdl && P != FIRST ? 1 : 0;
-  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED, P, FLAT>, a));
+  SMA_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<T, V, U, CTAS, HQ, HS, HB, PC, W, MODEL, RAGGED, P, FLAT, STRIDED>, a));
   SMA_CHECK_LAUNCH();
 }
 
@@ -539,13 +580,16 @@ inline bool walked(const sma_op *op, uint32_t lanes, int64_t threads) {
 }
 
 // Where not 0 or negative, `gathers` and `flat` take the place of the rules for them.
-template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL, Form P>
+template <typename T, int V, bool HQ, bool HS, bool HB, bool PC, bool W, int MODEL, Form P, bool STRIDED = false>
 void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0, int flat_wanted = -1) {
-  const uint32_t vecs = a.b / V;
+  const uint32_t vecs = (a.b + V - 1) / V;
   a.lanes = panel_lanes(vecs);
+  // FP64 rows of 4 and 5 such threads take one more, three columns each: b = 15 and 17 at n = 50000,
+  // 41.0 -> 38.3 and 43.5 -> 42.3 us (three steps, five entries a row), b = 13 33.5 either way
+  if (STRIDED && sizeof(T) == 8 && (vecs == 4 || vecs == 5)) ++a.lanes;
   a.rows = kThreads / a.lanes;
   a.divlanes = (65536 + a.lanes - 1) / a.lanes;
-  if constexpr (MODEL == SHARED)
+  if constexpr (MODEL == SHARED && !STRIDED)
     if (walked(op, a.lanes, (int64_t)a.n * vecs)) return launch_width<T, V, HQ, HS, HB, PC, W, WALKED, P>(op, st, a);
   // Waves of 8-CTA residency decide what a step's time is.  Six and more: a stream, which wants
   // every warp it can get.  Below, more and more a latency, which wants more gathers in flight at
@@ -565,7 +609,7 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0,
   // warps are idle or a few threads of long rows (us a step, whole rows and flat, Anderson L = 48:
   // 13 lanes 34.1 and 32.6, 22 55.8 and 52.0, 43 117 and 107, 50 143 and 128; 48 120 and 121, 60
   // 152 and 155).
-  constexpr bool kFlat = !(MODEL != STORED || P == DOTS || P == FIRST);
+  constexpr bool kFlat = !(MODEL != STORED || P == DOTS || P == FIRST || STRIDED);
   const uint32_t used = a.rows * a.lanes;
   const bool flat = kFlat && gathers != 8 && used < kThreads && (uint64_t)a.n * a.lanes < (uint64_t)1 << 32 &&
                     (flat_wanted < 0 ? used % 32 != 0 && (a.lanes <= 40 || kThreads - used >= 16) : flat_wanted > 0);
@@ -584,6 +628,11 @@ void launch_width(const sma_op *op, cudaStream_t st, Step<T> a, int gathers = 0,
     }
     a.b = width - p * a.lanes * V;
     const dim3 grid(gx, std::min(kGridY, ny - p));
+    if constexpr (STRIDED) {  // four addresses a gather
+      if (uneven) launch<T, V, 4, 8, HQ, HS, HB, PC, W, MODEL, true, P, false, true>(op, st, a, grid);
+      else launch<T, V, 4, 8, HQ, HS, HB, PC, W, MODEL, false, P, false, true>(op, st, a, grid);
+      continue;
+    }
     // A walked row holds its state beside the gathers: two at a time of 16-byte FP64 and of 32-byte
     // vectors, whose four spill (L = 22, b = 8 FP64 63.5 us against 87), four of the others.
     if constexpr (MODEL == WALKED) {
@@ -726,6 +775,21 @@ inline int vector_width(const sma_op *op, int64_t b, int widest) {
   return 1;
 }
 
+// Where widths, strides or addresses allow accesses of one element only (odd widths in the
+// allocation-free entry, below the degree that a padded copy pays for, and where that does not fit), a
+// thread takes four columns of a row all the same, a row's threads apart: the row's pointers, columns
+// and values serve four, and four times the gathers are in flight.  Us of three steps, one column a
+// thread and four: 1D Laplacian n = 400000, b = 31 FP64 410 and 216, FP32 351 and 160; b = 3 48 and
+// 34; Anderson L = 80, b = 15 324 and 254.  Not below 48000 threads (Anderson L = 20, b = 17, 40000:
+// 22.5 and 24.6; b = 25, 56000: 25.4 and 24.8), for ragged rows not below 8 threads a row (XXZ L = 18,
+// b = 15 48 and 57; b = 31 72 and 64), for a model's rows of one thread only in large operators
+// (Anderson L = 37, b = 3 32.1 and 33.6; L = 50 45.3 and 43.6).
+inline bool strided(const sma_op *op, int64_t b, int widest) {
+  const int64_t vecs = (b + 3) / 4;
+  return widest == 1 && op->kind != OP_XXZ && b >= 3 && op->n * vecs >= 48000 && (!ragged(op) || vecs >= 8) &&
+         (vecs > 1 || op->kind == OP_CSR || op->n >= 100000);
+}
+
 template <typename T, bool HQ, bool HS, bool HB, bool PC, int MODEL, Form P = INNER>
 void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   if (op->n == 0 || b == 0) return;
@@ -752,6 +816,8 @@ void step(const sma_op *op, cudaStream_t st, int64_t b, Step<T> a) {
   };
   if (a.ldb >> 32) return launch_width<T, 1, HQ, HS, HB, PC, true, MODEL, P>(op, st, a);
   const int widest = widest_vector<T>(fits), v = vector_width(op, b, widest);
+  if constexpr (P != DOTS)
+    if (strided(op, b, widest)) return launch_width<T, 4, HQ, HS, HB, PC, false, MODEL, P, true>(op, st, a);
   if constexpr (MODEL == STORED && P == INNER)
     if (tuned_step<T, HQ, HS, HB, PC>(op, st, a, widest, v)) return;
   if constexpr (sizeof(T) == 4)

@@ -582,3 +582,55 @@ def test_xxz_rows_walked_and_in_shared_memory(lib_built, L_, precision, rtol):
             full = Y
             assert np.abs(Y.double().cpu().numpy() - ref).max() <= rtol * max(np.abs(ref).max(), np.abs(Qh).max())
         assert torch.equal(Y, full[:, :b]) and torch.equal(P, Y), b
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind,n,widths", [("csr", 50653, (3, 5, 13, 15, 17, 19, 31)), ("anderson", 50653, (5, 13, 31)),
+                                           ("ring", 3100, (61, 253, 257, 261)), ("ragged", 6100, (29, 31, 61))])
+def test_filter_of_columns_a_row_apart(lib_built, precision, kind, n, widths):
+    """Blocks that allow accesses of one element only, wide enough for four columns a thread: at every
+    remainder of the columns, over one panel and two, every column has the bits of the aligned block's,
+    by the block entry in place and not, the per-column and the allocation-free one, and nothing is
+    written past the block."""
+    import torch
+    import sparse_matrix_algorithms_b200 as S
+    from sparse_matrix_algorithms_b200 import _lib as L
+
+    A = {"csr": lambda: M.anderson3d(37, 16.5, 5), "anderson": lambda: M.anderson3d(37, 16.5, 5),
+         "ring": lambda: M._canonical((M.lap1d(n) - sp.coo_matrix(([1.0, 1.0], ([0, n - 1], [n - 1, 0])), shape=(n, n))).tocsr()),
+         "ragged": lambda: _ragged(n, 4)}[kind]()
+    op = S.AndersonOperator(37, 16.5, 5) if kind == "anderson" else S.SparseOperator(A)
+    smin, smax = _bounds(A)
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    lib, P = L.load(), L.PRECISIONS[precision]
+    wide = -(-max(widths) // 8) * 8
+    full = _device(M.splitmix_normal(n, n, wide)).to(dt)
+    for K in (1, 2, 3):
+        c = np.ascontiguousarray(O.build_coeffs(K, smin, smax, 0.1, -0.4, 0.3, "step", True))
+        ref = torch.empty_like(full)
+        torch.cuda.synchronize()
+        L.check(lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, full.data_ptr(), wide,
+                                             ref.data_ptr(), wide, wide, P))
+        for b in widths:
+            table = np.ascontiguousarray(np.repeat(c[:, None], b, axis=1))
+            for entry in ("block", "in place", "percol", "noalloc"):
+                if entry == "noalloc" and (precision == "fp32" or n * b > 2 ** 21):
+                    continue
+                Q = full[:, :b].contiguous()
+                store = torch.full((n * b + 9,), 7.0, dtype=dt, device="cuda")
+                Y = Q if entry == "in place" else store[1:1 + n * b].view(n, b)
+                torch.cuda.synchronize()
+                if entry == "percol":
+                    rc = lib.sma_apply_poly_block_percol_dev(op.handle, table.ctypes.data, K, smin, smax, Q.data_ptr(),
+                                                             Y.data_ptr(), b, P)
+                elif entry == "noalloc":
+                    rc = lib.sma_apply_poly_block_noalloc(op.handle, c.ctypes.data, K, smin, smax, Q.data_ptr(), b,
+                                                          Y.data_ptr(), b, b)
+                else:
+                    rc = lib.sma_apply_poly_block_dev(op.handle, c.ctypes.data, K, smin, smax, Q.data_ptr(), b,
+                                                      Y.data_ptr(), b, b, P)
+                L.check(rc)
+                assert torch.equal(Y, ref[:, :b]), (K, b, entry)
+                assert bool((store[0] == 7.0) & (store[1 + n * b:] == 7.0).all())
+    ref0 = O.apply_poly_block(A, full[:, :3].double().cpu().numpy(), c, smin, smax)
+    assert np.abs(ref[:, :3].double().cpu().numpy() - ref0).max() <= (1e-12 if precision == "fp64" else 2e-4) * 5

@@ -128,3 +128,24 @@ def test_slicing_errors(lib_built):
         S.slice_spectrum(op, [(0.1, -0.1)], [100], [16])
     with pytest.raises(S.ArgumentError):
         S.slice_spectrum(S.AndersonOperator(6, 16.5, 0), [(-0.1, 0.1)], [100], [16])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_slicing_of_odd_widths(lib_built, precision):
+    """113 columns of three windows side by side, no two in one access: segments that begin and end
+    within a thread's columns, each window's bits those of its own solve."""
+    import sparse_matrix_algorithms_b200 as S
+
+    A = M.anderson3d(12, 16.5, 0)
+    n = A.shape[0]
+    lam_all = np.linalg.eigvalsh(A.toarray())
+    op = S.SparseOperator(A)
+    smin, smax = op.gershgorin_bounds()
+    mid = int(np.searchsorted(lam_all, 0.0))
+    wins = _windows(lam_all, mid - 20, [10, 12, 9])
+    deg, m0 = [150, 131, 170], [37, 41, 35]
+    lam, X, res, win = S.slice_spectrum(op, wins, deg, m0, maxiter=4, seed=5, precision=precision)
+    for w in range(3):
+        l1, X1, r1 = _single(S, op, n, wins[w], deg[w], m0[w], w, 5, precision, 4)
+        np.testing.assert_array_equal(lam[win == w], l1)
+        np.testing.assert_array_equal(X[:, win == w], X1)
