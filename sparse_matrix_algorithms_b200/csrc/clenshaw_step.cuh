@@ -15,9 +15,10 @@
 // registers go to occupancy, not to operands in flight: at most U = 4 neighbour rows are held
 // at a time, the epilogue's rows are prefetched into L2 at the start and loaded only after the
 // gathers, and 40 registers keep 12 CTAs on an SM.  Measured on the 3D Anderson lattice
-// (n = 262144, 7 entries a row), step after step on one B200:
-//   FP32 b = 64   66 -> 43 us (6.6 TB/s of algorithmic bytes),  b = 768   640 -> 522 us,
-//   FP64 b = 64  121 -> 85 us (6.6 TB/s).
+// (n = 262144, 7 entries a row), step after step on one B200, in a burst of some steps and in whole
+// filters, which run under the power cap (SM clock 1.45-1.6 GHz):
+//   FP32 b = 64   66 -> 43 us (6.6 TB/s of algorithmic bytes) and 50,  b = 768   640 -> 522 and 580,
+//   FP64 b = 64  121 -> 85 us (6.6 TB/s) and 100.
 // Against the kernel before it: 16-byte halves at a 32-byte stride doubled the L1 wavefronts
 // (73 % of the LSU data pipe), and 63 registers left 45 % of the warps (DRAM 4.0 TB/s).
 //

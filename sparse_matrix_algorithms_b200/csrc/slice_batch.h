@@ -1,5 +1,5 @@
 // The batched (segmented) block Clenshaw filter shared by batched spectrum slicing
-// (slicing.cu) and batched POLFED (polfed_batch.cu).
+// (slicing.cu) and batched POLFED (polfed.cu).
 //
 // The windows' blocks are concatenated side by side into one row-major n x W block,
 // windows sorted by filter degree (highest first).  The Clenshaw recurrence runs from the
