@@ -461,7 +461,7 @@ int sma_apply_poly_block_percol_dev(sma_op *op, const double *coeffs, int64_t K,
     auto run = [&](auto zero) {
       using T = decltype(zero);
       // a width that wide accesses divide, Q copied, as in apply_poly_block; without the memory, b
-      const int64_t w = op->kind == OP_CSR_HALF || op->band ? b : recurrence_width(b, sizeof(T));
+      const int64_t w = op->kind == OP_CSR_HALF || op->band ? b : staged_width(op, b, sizeof(T));
       DevBuf<T> coef, B1, B2, TMP, AX, Qw;
       auto allocate = [&](int64_t width) {
         coef.alloc((K + 1) * width, st);

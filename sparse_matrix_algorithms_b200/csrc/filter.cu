@@ -84,6 +84,13 @@ int64_t recurrence_width(int64_t b, int elem_bytes) {
   return best;
 }
 
+// The same where a copy of Q is its price: not where a thread takes one column anyway (vector_width in
+// clenshaw_step.cuh: fewer than half a CTA an SM with two; n = 3000, b = 3, K = 4 27.2 us with the
+// copy, 26.1 without).
+int64_t staged_width(const sma_op *op, int64_t b, int elem_bytes) {
+  return op->n * b < 128LL * op->ctx->num_sms ? b : recurrence_width(b, elem_bytes);
+}
+
 double clenshaw_step_bytes(const sma_op *op, int64_t b, int elem_bytes) {
   // nnz*(value + column index) + row pointers + Q, B1, B2 reads and one write
   double mat = 0.0;
@@ -246,7 +253,7 @@ static FilterCount apply_poly_block_impl(const sma_op *op, cudaStream_t st,
     return banded_filter<T>(op, st, &coeffs, nullptr, K, smin, smax, Q, ldq, Y, ldy, b, buf);
   }
   if (fused && !persistent && K >= kPadMinDegree) {
-    w = recurrence_width(b, sizeof(T));
+    w = staged_width(op, b, sizeof(T));
     int64_t vec = 32;  // the access that w allows
     while ((w * (int64_t)sizeof(T)) % vec) vec /= 2;
     stage = w != b || (ldq * (int64_t)sizeof(T)) % vec || (uintptr_t)Q % vec;

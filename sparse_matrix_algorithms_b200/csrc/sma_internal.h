@@ -411,6 +411,7 @@ void op_apply(const sma_op *op, cudaStream_t st, const double *X, int64_t ldx, d
 // Width of a recurrence's own blocks for b columns of elem_bytes (filter.cu): b, or b padded to a
 // width that wider vectors divide.
 int64_t recurrence_width(int64_t b, int elem_bytes);
+int64_t staged_width(const sma_op *op, int64_t b, int elem_bytes);
 
 // Algorithmic bytes of one fused Clenshaw step over b columns
 double clenshaw_step_bytes(const sma_op *op, int64_t b, int elem_bytes);
